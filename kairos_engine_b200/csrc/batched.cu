@@ -817,12 +817,7 @@ cudaError_t run_layer(const SpDims &d, const SpLayerDev &L, int M, const float *
     launch_router(d, L, v, M, st, nl);
     k_b_topk<<<M, 256, (size_t)NE * 12, st>>>(d, L, v, M, sel, wts, status); (*nl)++;
     if (!FA && tc) {                                            /* prefill arithmetic on the tensor cores */
-        cudaError_t e = sp_tc_shared_expert(tc, d, L, M, v.nx_f, v.dn, status, st, nl);
-        if (e != cudaSuccess) return e;
-        const int *off, *gather, *rowmap;
-        e = sp_tc_sort_pairs(tc, d, M, v.sel_asc, v.count, v.pairpos, &off, &gather, &rowmap, st, nl);
-        if (e != cudaSuccess) return e;
-        e = sp_tc_routed(tc, d, L, M * NU, v.in_f, gather, off, rowmap, v.eo, status, st, nl);
+        const cudaError_t e = sp_tc_layer(tc, d, L, M, v.nx_f, v.in_f, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);
         if (e != cudaSuccess) return e;
         k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
         return cudaGetLastError();

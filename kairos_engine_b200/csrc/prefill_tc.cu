@@ -1,5 +1,5 @@
 /* prefill_tc.cu — the prefill GEMMs of the MoE feed-forward layer on the 5th-generation tensor
- * cores (tcgen05.mma, accumulators in tensor memory), sm_100a only.
+ * cores (tcgen05.mma, weights and accumulators in tensor memory), sm_100a only.
  *
  * Replaces the reference's prefill matmul for Q4B tensors (gemm_w, CF:13488-13518 of
  * src/backends/cuda/cuda_forward.cu: dequantise the whole tensor to a scratch matrix, then
@@ -14,103 +14,154 @@
  * and D += w_hi*x_hi + w_lo*x_hi + w_hi*x_lo accumulates in fp32 in tensor memory (the dropped
  * w_lo*x_lo term is below 2^-22 relative). That is three MMAs per k-step.
  *
- * Tile: 128 activation rows (the MMA's M: one TMEM lane per row) x 256 weight rows (its N: one
- * TMEM column per weight row), K in stages of 64. One 128x256x16 MMA reads 12 KB of operands from
- * shared memory per 128 tensor-core cycles; two 128x128x16 ones would read 16 KB, and shared-memory
- * bandwidth (operand reads + the unpack warps' writes + TMA) is what bounds this kernel.
- *   gate|up GEMM : columns [0,128) = 128 gate rows, columns [128,256) = the matching 128 up rows, so
- *                  the epilogue thread that owns a TMEM lane (one activation row) holds g and u of
- *                  the same outputs and writes gelu(g)*u directly, already split into fp16 hi/lo
- *                  for the next GEMM, 16 bytes at a time;
- *   down GEMM    : columns = weight rows [j0, j0+256), fp32 out, 16 bytes at a time.
- * Activation tiles come in by TMA (2-D tiled copy, 128-byte swizzle) from row lists sorted by
- * expert; weight tiles are unpacked by eight warps into the same swizzled layout. Inside every
- * group of 8 k the order is 0,4,1,5,2,6,3,7 on BOTH operands (the natural order of the nibble
- * unpack), which a dot product does not see.
- * Warp roles (14 warps): 0-3 epilogue (TMEM lane quadrant = warp), 4 TMA, 5 MMA issue + TMEM
- * allocation, 6-13 weight unpack. Two shared-memory stages, two accumulator sets (512 TMEM columns)
- * so the epilogue of one tile overlaps the main loop of the next. Every wait is bounded.
+ * Tile: two blocks of 128 weight rows (the MMA's M, one TMEM lane per weight row) x up to NMAX
+ * activation rows (its N, a multiple of 16), K in stages of 64.
+ *   - The weights are the A operand and live in tensor memory: an unpack thread owns one weight
+ *     row, which is one TMEM lane, and stores its fp16 hi/lo values there (tcgen05.st). The
+ *     unpacked weights therefore cost no shared-memory bandwidth, neither the write nor the read
+ *     by every MMA; only the activation tile is read from shared memory (64 B per clock at any N).
+ *   - The activation rows are N, so a group pays for its rows rounded up to 16, not to 128: with a
+ *     few rows per expert the GEMM is a stream of weights, and with 256 the padding is some percent.
+ *   gate|up GEMM : a block is 64 gate rows and the 64 up rows of the same outputs, 16 + 16 to a
+ *                  32-lane quadrant, so that g and u of an output sit 16 lanes apart in one warp: one
+ *                  shuffle per two outputs, then gelu(g)*u, split into fp16 hi/lo for the next GEMM;
+ *   down GEMM    : a block is 128 consecutive rows, fp32 out.
+ * A last tile with at most one block of rows left does that block only.
+ * Packed codes come in by TMA (256 weights of 256 rows a time, 128-byte swizzle: the unpack threads
+ * read their row's pieces without bank conflicts), activations by TMA from row lists sorted by
+ * expert. Inside every group of 8 k the order is 0,4,1,5,2,6,3,7 on BOTH operands (the natural
+ * order of the nibble unpack), which a dot product does not see.
+ * Warps: 0-7 epilogue (TMEM lane quadrant = warp % 4, block = warp / 4), 8-23 unpack (the same, in
+ * two sets that take alternate stages), 24 and 25 MMA issue (one per block), 26 activation TMA, 27
+ * code TMA and TMEM allocation. Every wait is bounded.
+ * What bounds it (Gemma geometry, one B200): up to some 40 rows per expert the unpack, ~136
+ * instructions of the half-rate fp16 and integer pipes per 2048 weights, beside a weight stream at
+ * about a third of HBM's rate; from there to the largest batches the MMAs (12, 16 and 32 cycles at N =
+ * 16, 32 and 64) and in the end the power limit. A layer of 37 / 717 / 4096 tokens: 0.60 / 0.85 /
+ * 2.40 ms with the weights in shared memory and 128 rows a tile, 0.21 / 0.46 / 1.95 ms with this.
  */
-#include <vector>
+#include <map>
+#include <mutex>
 #include "prefill_tc.cuh"
 #include "tc_common.cuh"
 
 namespace {
 using namespace sp_tc;
 
-constexpr int kTileN = 128, kBK = 64, kStages = 2;
-constexpr int kThreads = 448;
-constexpr uint32_t kAHalf = 256 * 128, kBHalf = kTileN * 128;
-constexpr uint32_t kStageBytes = 2 * kAHalf + 2 * kBHalf;             /* 98304 */
-constexpr uint32_t kBarOff = kStages * kStageBytes;
-constexpr uint32_t kSmemBytes = kBarOff + 128 + 1024;                 /* + alignment slack */
+constexpr int kBK = 64, kNGran = 16, kBoxBig = 64;
+constexpr int kEpiWarps = 8, kItems = 64;
+constexpr uint32_t kBoxRows = 64, kBoxBytes = 128 * kBoxRows;          /* codes: 128 B (256 weights) of 64 rows */
+constexpr uint32_t kChunkBytes = 4 * kBoxBytes;                        /* the four boxes of a tile: 32 KB per 256 k */
+/* 512 TMEM columns: 2 blocks x kAccBufs x NMAX of accumulators from column 0, then a ring of three stages of unpacked
+ * weights, 128 columns each (2 blocks x 64 k x hi/lo). Registers: the epilogue empties the accumulators into registers at
+ * once, before it computes, so setmaxnreg moves registers to it. Tiles of 96 and of 128 rows were measured too (fewer
+ * unpacks, but more registers for the epilogue and a shorter ring): the same within 2% at 4096 tokens, slower below. */
+template <int NMAX> struct Cfg {
+    static constexpr int kSets = 2, kUnpWarps = 8 * kSets, kWarps = kEpiWarps + kUnpWarps + 4, kThreads = 32 * kWarps;
+    static constexpr int kAccBufs = NMAX == 32 ? 2 : 1, kACol = 2 * NMAX * kAccBufs, kAStages = 3, kACols = 2 * kBK;
+    static constexpr int kBStages = 4, kCStages = 4;
+    static constexpr uint32_t kBHalf = NMAX * 128u, kBStage = 2 * kBHalf;
+    static constexpr uint32_t kCOff = kBStages * kBStage, kBarOff = kCOff + kCStages * kChunkBytes, kItemOff = kBarOff + 320;
+    static constexpr uint32_t kScaleOff = kItemOff + 32 * kItems, kSmem = kScaleOff + 3 * 16 * 32 * kUnpWarps + 1024;     /* + alignment slack */
+    static constexpr int kLaunchRegs = 72, kEpiRegs = 104, kUnpRegs = 64, kMiscRegs = 32;
+    static_assert(32 * (kEpiWarps * kEpiRegs + kUnpWarps * kUnpRegs + 4 * kMiscRegs) <= kThreads * kLaunchRegs, "register split exceeds what the block is launched with");
+    static_assert(kACol + kACols * kAStages <= 512, "tensor memory");
+};
 
-struct TcMaps { CUtensorMap hi, lo; };
-
-struct TcArgs {
-    const uint8_t *codes[2]; const uint16_t *bs[2];   /* weight tensor feeding accumulator 0 / 1 */
+struct TcSeg {                     /* one GEMM of a launch: the shared expert's or the routed experts' */
+    const uint16_t *bs[2];         /* block scales of the tensor feeding the gate / up rows (plain: both the same) */
     long long group_rows;          /* rows per group (expert) in the tensor */
-    int acc1_off;                  /* pair: row offset of accumulator 1's rows inside the group */
-    int rows;                      /* valid output rows (pair: per accumulator) */
-    int K;
+    int up_off;                    /* pair: row offset of the up rows inside the group (0 with a separate up tensor) */
+    int rows;                      /* valid output rows (pair: per half) */
     const int *tiles;              /* {group, first row, valid rows} per activation tile */
     const int *n_tiles;
     int m_tiles;
-    __half *out_hi, *out_lo; int out_k;               /* pair: geglu output rows, split + permuted */
+    __half *out_hi, *out_lo;       /* pair: geglu output rows of `rows` columns, split + permuted */
     float *out_f; int out_stride; const int *rowmap;  /* plain: out_f[(rowmap ? rowmap[r] : r) * stride + j] */
-    int *status;
 };
+struct TcArgs { TcSeg seg[2]; int nseg; int K[2]; int *status; };
+struct TcMaps { CUtensorMap codes[2][2], hi[2], lo[2], hi64[2], lo64[2]; };   /* [segment][gate / up]; activation boxes of 16 and of 64 rows */
 
-__device__ __forceinline__ int kpos(int e) { return ((e & 3) << 1) | (e >> 2); }     /* slot of element e inside its group of 8 */
+constexpr uint32_t kNegateA = 1u << 13;                                /* instruction descriptor: A enters with its sign flipped */
 
-/* one Q4B block (32 weights, one f16 scale) -> four 16-byte chunks of hi and (LO) of lo halves */
+__device__ __forceinline__ int kperm(int j) { return (j & ~7) | ((j & 3) << 1) | ((j >> 2) & 1); }   /* slot of k = j */
+
+/* one Q4B block (32 weights, one f16 scale) -> 16 registers of hi and (LO) of NEGATED lo halves (the MMA negates them
+ * back: a sign is free there, and one instruction per two weights here). The nibbles j and j + 4 of a word become two
+ * halves with an exponent that makes the nibble's place count one: 1024 + n in bits 0-3, 64 + n in bits 4-7; the nibbles
+ * of the upper byte are shifted down once. The unpack is bound by the half-rate fp16 and integer pipes, so what counts is
+ * 5 integer and 12 fp16 instructions per word of 8 weights. */
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t mask, uint32_t flip) {          /* one LOP3: `flip` has to be a register for that */
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(d) : "r"(a), "r"(mask), "r"(flip));
+    return d;
+}
+__device__ __forceinline__ uint32_t in_register(uint32_t v) { uint32_t r; asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v)); return r; }
 template <bool LO>
-__device__ __forceinline__ void unpack_block(const int4 &w, unsigned short scale, unsigned char *a_hi, unsigned char *a_lo,
-                                             uint32_t rowoff, int r7, int g0) {
-    const __half2 s2 = __half2half2(__ushort_as_half(scale));
-    const __half2 k1032 = __half2half2(__ushort_as_half((unsigned short)0x6408));
-    const uint32_t words[4] = {(uint32_t)w.x, (uint32_t)w.y, (uint32_t)w.z, (uint32_t)w.w};
+__device__ __forceinline__ void unpack_words(uint32_t w0, uint32_t w1, __half2 s2, uint32_t m1032, uint32_t m72, uint32_t t_hi, uint32_t t_lo) {
+    const __half2 k1032 = __half2half2(__ushort_as_half((unsigned short)0x6408)), k72 = __half2half2(__ushort_as_half((unsigned short)0x5480));
+    const __half2 ns2 = __hneg2(s2);
+    uint32_t hi[8], lo[8];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint32_t t = words[q] ^ 0x88888888u;
-        uint32_t hi[4], lo[4];
+    for (int q = 0; q < 2; q++) {
+        const uint32_t w = q ? w1 : w0, up = w >> 8;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const uint32_t bits = ((t >> (4 * j)) & 0x000F000Fu) | 0x64006400u;        /* halves 1024 + (code + 8): elements j, j + 4 */
-            const __half2 c = __hsub2(*reinterpret_cast<const __half2 *>(&bits), k1032);
+            const uint32_t x = j < 2 ? w : up;                                         /* code + 8 = the nibble with its top bit flipped */
+            const uint32_t bits = j & 1 ? and_xor(x, 0x00F000F0u, m72) : and_xor(x, 0x000F000Fu, m1032);
+            const __half2 c = __hsub2(*reinterpret_cast<const __half2 *>(&bits), j & 1 ? k72 : k1032);
             const __half2 h = __hmul2(c, s2);
-            hi[j] = *reinterpret_cast<const uint32_t *>(&h);
-            if (LO) { const __half2 l = __hfma2(c, s2, __hneg2(h)); lo[j] = *reinterpret_cast<const uint32_t *>(&l); }
+            hi[4 * q + j] = *reinterpret_cast<const uint32_t *>(&h);
+            if (LO) { const __half2 l = __hfma2(c, ns2, h); lo[4 * q + j] = *reinterpret_cast<const uint32_t *>(&l); }
         }
-        const uint32_t off = rowoff + (uint32_t)(((g0 + q) ^ r7) << 4);
-        *reinterpret_cast<uint4 *>(a_hi + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        if (LO) *reinterpret_cast<uint4 *>(a_lo + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
+    tmem_st8(t_hi, hi);
+    if (LO) tmem_st8(t_lo, lo);
+}
+/* one Q4B block -> 16 columns of hi and of negated lo halves of this thread's TMEM lane */
+template <bool LO>
+__device__ __forceinline__ void unpack_block(const int4 &w, unsigned short scale, uint32_t m1032, uint32_t m72, uint32_t t_hi, uint32_t t_lo) {
+    const __half2 s2 = __half2half2(__ushort_as_half(scale));
+    unpack_words<LO>((uint32_t)w.x, (uint32_t)w.y, s2, m1032, m72, t_hi, t_lo);
+    unpack_words<LO>((uint32_t)w.z, (uint32_t)w.w, s2, m1032, m72, t_hi + 8u, t_lo + 8u);
 }
 
 /* TERMS: 3 = all of w_hi*x_hi + w_lo*x_hi + w_hi*x_lo (exact to 2^-22); 2 = the weight rounded to fp16
  * (w_hi*x_hi + w_hi*x_lo); 1 = fp16 x fp16, the reference's SP_G4_GEMM_F16 mode (CF:13350-13365). */
-template <bool PAIR, int TERMS>
-__global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const TcArgs a, const __grid_constant__ TcMaps maps) {
+struct __align__(16) Item { int sg, mt, grp, row0, nv, n16, nblk, KB; };      /* rows [row0, row0 + nv) of group grp x weight tile mt */
+
+template <bool PAIR, int TERMS, int NMAX>
+__global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid_constant__ TcArgs a, const __grid_constant__ TcMaps maps) {
+    using C = Cfg<NMAX>;
+    constexpr int BLK = PAIR ? 64 : 128;                                /* output rows of one block */
+    constexpr int kMma = kEpiWarps + C::kUnpWarps, kActs = kMma + 2, kCodes = kMma + 3;      /* single warps: MMA issue (one per block), TMA */
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t sbase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t bar0 = sbase + kBarOff;
-    auto full = [&](int s) { return bar0 + 8u * s; };
-    auto empty = [&](int s) { return bar0 + 16u + 8u * s; };
-    auto tfull = [&](int b) { return bar0 + 32u + 8u * b; };
-    auto tempty = [&](int b) { return bar0 + 48u + 8u * b; };
-    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + kBarOff + 64);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kBarOff + 68);
+    const uint32_t bar0 = sbase + C::kBarOff;
+    auto bfull = [&](int s) { return bar0 + 8u * s; };                  /* activation stages */
+    auto bempty = [&](int s) { return bar0 + 32u + 8u * s; };
+    auto cfull = [&](int s) { return bar0 + 64u + 8u * s; };            /* chunks of codes */
+    auto cempty = [&](int s) { return bar0 + 96u + 8u * s; };
+    auto afull = [&](int s, int blk) { return bar0 + 128u + 8u * (2 * s + blk); };      /* unpacked weights in TMEM: the two blocks keep apart rings, */
+    auto aempty = [&](int s, int blk) { return bar0 + 176u + 8u * (2 * s + blk); };
+    auto tfull = [&](int b, int blk) { return bar0 + 224u + 8u * (2 * b + blk); };      /* and apart accumulators */
+    auto tempty = [&](int b, int blk) { return bar0 + 256u + 8u * (2 * b + blk); };
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + C::kBarOff + 288);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::kBarOff + 292);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; s++) { mbar_init(full(s), 9); mbar_init(empty(s), 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 4); }
+        for (int s = 0; s < C::kBStages; s++) { mbar_init(bfull(s), 1); mbar_init(bempty(s), 2); }
+        for (int s = 0; s < C::kCStages; s++) { mbar_init(cfull(s), 1); mbar_init(cempty(s), C::kUnpWarps); }
+        for (int blk = 0; blk < 2; blk++) {
+            for (int s = 0; s < C::kAStages; s++) { mbar_init(afull(s, blk), 4); mbar_init(aempty(s, blk), 1); }
+            for (int b = 0; b < 2; b++) { mbar_init(tfull(b, blk), 1); mbar_init(tempty(b, blk), kEpiWarps / 2); }
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 5) {
+    if (warp == kCodes) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -119,155 +170,251 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const TcArgs a, const _
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    const int n_tiles = *a.n_tiles;
-    const int total = n_tiles * a.m_tiles;
-    const int KB = a.K / kBK;
+    const int total0 = *a.seg[0].n_tiles * a.seg[0].m_tiles;
+    const int total = total0 + (a.nseg > 1 ? *a.seg[1].n_tiles * a.seg[1].m_tiles : 0);
+    /* work item -> segment, activation tile, weight tile (the weight tiles of one activation tile are neighbours). The
+     * first kItems of a CTA are worked out once, in parallel, and kept in shared memory: every role reads each of them */
+    auto item_at = [&](int w) {
+        Item t;
+        t.sg = w >= total0 ? 1 : 0;
+        const TcSeg &s = a.seg[t.sg];
+        const int r = w - (t.sg ? total0 : 0), nt = r / s.m_tiles;
+        t.mt = r - nt * s.m_tiles;
+        t.grp = __ldg(s.tiles + 3 * nt); t.row0 = __ldg(s.tiles + 3 * nt + 1); t.nv = __ldg(s.tiles + 3 * nt + 2);
+        t.n16 = (t.nv + kNGran - 1) & ~(kNGran - 1);
+        t.nblk = s.rows - t.mt * 2 * BLK > BLK ? 2 : 1;
+        t.KB = a.K[t.sg] / kBK;
+        return t;
+    };
+    Item *items = reinterpret_cast<Item *>(smem + C::kItemOff);
+    for (int i = threadIdx.x; i < kItems && (int)blockIdx.x + i * (int)gridDim.x < total; i += C::kThreads) items[i] = item_at(blockIdx.x + i * gridDim.x);
+    __syncthreads();
+    auto item = [&](int w, int i) { return i < kItems ? items[i] : item_at(w); };
     bool failed = false;
 
-    if (warp == 4) {
-        /* ---------------- activation tiles by TMA */
-        if (lane == 0) {
-            uint32_t it = 0;
-            for (int w = blockIdx.x; w < total && !failed; w += gridDim.x) {
-                const int nt = w / a.m_tiles;
-                const int row0 = a.tiles[3 * nt + 1];
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const int s = it % kStages; const uint32_t ph = (it / kStages) & 1;
-                    if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-                    mbar_expect_tx(full(s), TERMS >= 2 ? 2 * kBHalf : kBHalf);
-                    const uint32_t dst = sbase + s * kStageBytes + 2 * kAHalf;
-                    tma_load_2d(dst, &maps.hi, kb * kBK, row0, full(s));
-                    if (TERMS >= 2) tma_load_2d(dst + kBHalf, &maps.lo, kb * kBK, row0, full(s));
-                }
-            }
-            if (failed || *abort_flag) __nanosleep(100000);          /* let copies in flight land before the CTA leaves */
-        }
-    } else if (warp == 5) {
-        /* ---------------- MMA issue */
-        if (lane == 0) {
-            uint32_t it = 0, lt = 0;
-            for (int w = blockIdx.x; w < total && !failed; w += gridDim.x, lt++) {
-                const int nt = w / a.m_tiles;
-                const uint32_t idesc = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);   /* f16 x f16 -> f32, K-major both, M = 128, N = 256 */
-                const int b = lt & 1; const uint32_t bph = (lt >> 1) & 1;
-                if (!mbar_wait(tempty(b), bph ^ 1, abort_flag)) { failed = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d0 = tmem + (uint32_t)(b * 256);
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const int s = it % kStages; const uint32_t ph = (it / kStages) & 1;
-                    if (!mbar_wait(full(s), ph, abort_flag)) { failed = true; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t st = sbase + s * kStageBytes;
-#pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ks++) {
-                        /* A operand = activation rows (M), B operand = the 256 weight rows (N) */
-                        const uint64_t whi = make_desc(st + ks * 32), wlo = make_desc(st + kAHalf + ks * 32);
-                        const uint64_t xhi = make_desc(st + 2 * kAHalf + ks * 32), xlo = make_desc(st + 2 * kAHalf + kBHalf + ks * 32);
-                        umma_f16(d0, xhi, whi, idesc, (kb | ks) ? 1u : 0u);
-                        if (TERMS >= 3) umma_f16(d0, xhi, wlo, idesc, 1u);
-                        if (TERMS >= 2) umma_f16(d0, xlo, whi, idesc, 1u);
-                    }
-                    umma_commit(empty(s));                          /* stage reusable once these MMAs have read it */
-                }
-                if (!failed) umma_commit(tfull(b));
-            }
-        }
-    } else if (warp >= 6) {
-        /* ---------------- weight tiles: Q4B -> fp16 hi/lo, swizzled K-major rows */
-        const int r = (warp - 6) * 32 + lane;
-        const int acc = r >> 7, i = r & 127, r7 = r & 7;
-        const uint32_t rowoff = (uint32_t)r * 128u;
-        const size_t rb = (size_t)a.K / 2; const int n32 = a.K / 32;
-        uint32_t it = 0;
-        for (int w = blockIdx.x; w < total && !failed; w += gridDim.x) {
-            const int nt = w / a.m_tiles, mt = w - nt * a.m_tiles;
-            const int grp = a.tiles[3 * nt];
-            int jj = PAIR ? mt * 128 + i : mt * 256 + r;
-            if (jj > a.rows - 1) jj = a.rows - 1;
-            const size_t wrow = (size_t)((long long)grp * a.group_rows) + (size_t)(PAIR ? acc * a.acc1_off : 0) + (size_t)jj;
-            const int tsel = PAIR ? acc : 0;
-            const unsigned char *cp = a.codes[tsel] + wrow * rb;
-            const uint16_t *sp = a.bs[tsel] + wrow * n32;
-            int4 c0 = ld_stream16(cp), c1 = ld_stream16(cp + 16);
-            uint32_t sc = *reinterpret_cast<const uint32_t *>(sp);
-            for (int kb = 0; kb < KB; kb++, it++) {
-                const int4 w0 = c0, w1 = c1; const uint32_t s2 = sc;
-                if (kb + 1 < KB) { c0 = ld_stream16(cp + 32 * (kb + 1)); c1 = ld_stream16(cp + 32 * (kb + 1) + 16); sc = *reinterpret_cast<const uint32_t *>(sp + 2 * (kb + 1)); }
-                const int s = it % kStages; const uint32_t ph = (it / kStages) & 1;
-                if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-                unsigned char *ahi = smem + s * kStageBytes, *alo = ahi + kAHalf;
-                unpack_block<TERMS >= 3>(w0, (unsigned short)(s2 & 0xFFFFu), ahi, alo, rowoff, r7, 0);
-                unpack_block<TERMS >= 3>(w1, (unsigned short)(s2 >> 16), ahi, alo, rowoff, r7, 4);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full(s));
-            }
-        }
-    } else {
-        /* ---------------- epilogue: TMEM -> registers -> global */
-        const int i = warp * 32 + lane;                             /* TMEM lane = activation row inside the tile */
-        uint32_t lt = 0;
-        for (int w = blockIdx.x; w < total && !failed; w += gridDim.x, lt++) {
-            const int nt = w / a.m_tiles, mt = w - nt * a.m_tiles;
-            const int row0 = a.tiles[3 * nt + 1], nv = a.tiles[3 * nt + 2];
-            const int b = lt & 1; const uint32_t bph = (lt >> 1) & 1;
-            if (!mbar_wait(tfull(b), bph, abort_flag)) { failed = true; break; }
+    if (warp < kEpiWarps) {
+        /* ---------------- epilogue: TMEM -> registers, the accumulators are free again, then -> global */
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
+        const int quad = warp & 3, blk = warp >> 2;
+        int lt = 0;
+        for (int w = blockIdx.x, i = 0; w < total; w += gridDim.x, i++) {
+            const Item t = item(w, i);
+            if (blk >= t.nblk) continue;
+            const TcSeg &s = a.seg[t.sg];
+            const int b = lt % C::kAccBufs; const uint32_t ph = (lt / C::kAccBufs) & 1;
+            lt++;
+            if (!mbar_wait(tfull(b, blk), ph, abort_flag)) { failed = true; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * 256);
-            const bool rv = i < nv;
-            const int sr = row0 + (rv ? i : 0);
-            if (PAIR) {
-                __half *ohi = a.out_hi + (size_t)sr * a.out_k, *olo = a.out_lo + (size_t)sr * a.out_k;
-                for (int c0 = 0; c0 < 128; c0 += 16) {
-                    const int j0 = mt * 128 + c0;
-                    if (j0 >= a.rows) break;                             /* warp-uniform */
-                    uint32_t g[16], u[16];
-                    tmem_ld16(t0 + c0, g);
-                    tmem_ld16(t0 + 128 + c0, u);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (rv) {
+            const uint32_t t0 = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)((2 * b + blk) * NMAX);
+            uint32_t v[NMAX];
 #pragma unroll
-                        for (int h8 = 0; h8 < 2; h8++) {
-                            if (j0 + 8 * h8 < a.rows) {                  /* rows is a multiple of 8 */
-                                __half hh[8], hl[8];
+            for (int c = 0; c < NMAX; c += 32) if (c < t.n16) tmem_ld32(t0 + c, v + c);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty(b, blk));
+            const int j = t.mt * 2 * BLK + blk * BLK + (PAIR ? quad * 16 + (lane & 15) : quad * 32 + lane);
+            const bool upper = lane >= 16, b2 = (lane & 4) != 0;
+            /* pair: lane and lane ^ 4 hold k = j and j + 4, neighbours in the stored order: the lower one stores both hi, the upper both lo */
+            __half *pp = PAIR ? (b2 ? s.out_lo : s.out_hi) + kperm(j & ~4) : nullptr;
+#pragma unroll 1
+            for (int c0 = 0; c0 < t.nv; c0 += 32) {
+                int rm = t.row0 + c0 + lane;
+                if (!PAIR && s.rowmap) rm = c0 + lane < t.nv ? __ldg(s.rowmap + rm) : 0;
 #pragma unroll
-                                for (int n = 0; n < 8; n++) {
-                                    const float h = gelu_mul(__uint_as_float(g[8 * h8 + n]), __uint_as_float(u[8 * h8 + n]));
-                                    const __half x = __float2half_rn(h);
-                                    hh[kpos(n)] = x; hl[kpos(n)] = __float2half_rn(__fsub_rn(h, __half2float(x)));
-                                }
-                                *reinterpret_cast<uint4 *>(ohi + j0 + 8 * h8) = *reinterpret_cast<const uint4 *>(hh);
-                                *reinterpret_cast<uint4 *>(olo + j0 + 8 * h8) = *reinterpret_cast<const uint4 *>(hl);
-                            }
+                for (int n = 0; n < 32; n += 2) {
+                    if (c0 + n >= t.nv) break;                          /* warp-uniform */
+                    if (PAIR) {
+                        /* lanes 0-15 hold gate rows, 16-31 the up rows of the same outputs: the lower half finishes column n, the upper n + 1 */
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? v[n] : v[n + 1], 16);
+                        const float g = __uint_as_float(upper ? got : v[n]), u = __uint_as_float(upper ? v[n + 1] : got);
+                        const float h = gelu_mul(g, u);
+                        const __half x = __float2half_rn(h), y = __float2half_rn(__fsub_rn(h, __half2float(x)));
+                        const uint32_t hx = __half_as_ushort(x), hy = __half_as_ushort(y);
+                        const uint32_t other = __shfl_xor_sync(0xffffffffu, b2 ? hx : hy, 4);
+                        const uint32_t word = b2 ? (other | (hy << 16)) : (hx | (other << 16));
+                        const int nn = c0 + n + (upper ? 1 : 0);
+                        if (nn < t.nv) *reinterpret_cast<uint32_t *>(pp + (size_t)(t.row0 + nn) * s.rows) = word;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const int r = __shfl_sync(0xffffffffu, rm, n + k);
+                            if (c0 + n + k < t.nv && j < s.rows) s.out_f[(size_t)r * s.out_stride + j] = __uint_as_float(v[n + k]);
                         }
                     }
                 }
-            } else {
-                float *orow = a.out_f + (size_t)(a.rowmap ? __ldg(a.rowmap + sr) : sr) * a.out_stride;
-                for (int c0 = 0; c0 < 256; c0 += 16) {
-                    const int j0 = mt * 256 + c0;
-                    if (j0 >= a.rows) break;                             /* warp-uniform */
-                    uint32_t v[16];
-                    tmem_ld16(t0 + c0, v);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (rv) {
 #pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            if (j0 + 4 * q < a.rows)                     /* rows is a multiple of 4 */
-                                *reinterpret_cast<float4 *>(orow + j0 + 4 * q) =
-                                    make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+                for (int i = 0; i + 32 < NMAX; i++) v[i] = v[i + 32];
+            }
+        }
+    } else if (warp < kMma) {
+        /* ---------------- weights: packed codes in shared memory -> fp16 hi/lo in TMEM; one thread per weight row */
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kUnpRegs));
+        const int quad = warp & 3, blk = ((warp - kEpiWarps) >> 2) & 1, set = (warp - kEpiWarps) >> 3;
+        const int half = PAIR ? lane >> 4 : 0;
+        const int rb = PAIR ? quad * 16 + (lane & 15) : quad * 32 + lane;                /* row inside the block (pair: of its gate or up half) */
+        const int box = blk * 2 + (PAIR ? half : rb >> 6), r64 = rb & 63;
+        const uint32_t coff = (uint32_t)box * kBoxBytes + (uint32_t)r64 * 128u, r7 = r64 & 7;
+        const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + C::kACol + kBK * blk;
+        const uint32_t m1032 = in_register(0x64086408u), m72 = in_register(0x54805480u);
+        uint32_t as = set, aph = 0, cs = 0, cph = 0;
+        int u = set;                                                    /* next stage (64 k) of this set, within the tile; the sets alternate across tiles too */
+        /* This thread's block scales travel two chunks (8 scales each) ahead of their use, by asynchronous copies into a
+         * place of its own. */
+        const uint32_t slot0 = smem_u32(smem) + C::kScaleOff + 16u * (threadIdx.x - 32 * kEpiWarps);
+        constexpr uint32_t kSlot = 16u * 32u * C::kUnpWarps;
+        int pw = blockIdx.x, pi = 0, pk = 0, pKB = 0; uint32_t pslot = 0, uslot = 0;     /* next chunk to fetch: item, first 64-k step; slots of a ring of three */
+        const uint32_t *sp = nullptr;
+        auto fetch = [&]() {
+            if (pw < total) {
+                if (pk == 0) {
+                    const Item t = item(pw, pi);
+                    const TcSeg &s = a.seg[t.sg];
+                    int jj = t.mt * 2 * BLK + blk * BLK + rb;
+                    if (jj > s.rows - 1) jj = s.rows - 1;
+                    const size_t row = (size_t)((long long)t.grp * s.group_rows) + (size_t)(half ? s.up_off : 0) + (size_t)jj;
+                    sp = reinterpret_cast<const uint32_t *>(s.bs[half] + row * (size_t)(2 * t.KB));
+                    pKB = t.KB;
+                }
+                const uint32_t dst = slot0 + pslot * kSlot;
+                if ((pKB & 3) == 0) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(sp + pk) : "memory");      /* K a multiple of 256: rows of 16 bytes */
+                else {
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (pk + k < pKB) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * k), "l"(sp + pk + k) : "memory");
+                }
+                pk += 4;
+                if (pk >= pKB) { pk = 0; pw += gridDim.x; pi++; }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            pslot = pslot == 2 ? 0 : pslot + 1;
+        };
+        fetch(); fetch();
+        for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
+            const Item t = item(w, iw);
+            const int nst = blk < t.nblk ? t.KB : 0;
+            for (int c0 = 0; c0 < t.KB; c0 += 4) {
+                fetch();
+                asm volatile("cp.async.wait_group 2;" ::: "memory");
+                const uint32_t sc = slot0 + uslot * kSlot;
+                uslot = uslot == 2 ? 0 : uslot + 1;
+                if (!mbar_wait(cfull(cs), cph, abort_flag)) { failed = true; break; }
+                const unsigned char *codes = smem + C::kCOff + cs * kChunkBytes + coff;
+                const int lim = nst < c0 + 4 ? nst : c0 + 4;
+#pragma unroll 1                                                        /* one copy of the unpack: several would not stay in the instruction cache */
+                for (; u < lim; u += C::kSets) {
+                    const int k = u - c0;
+                    const uint32_t td = ta + C::kACols * as;
+                    uint32_t s2;
+                    const int4 w0 = *reinterpret_cast<const int4 *>(codes + (((2 * k) ^ r7) << 4)), w1 = *reinterpret_cast<const int4 *>(codes + (((2 * k + 1) ^ r7) << 4));
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(s2) : "r"(sc + 4u * k));
+                    if (!mbar_wait(aempty(as, blk), aph ^ 1, abort_flag)) { failed = true; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    unpack_block<TERMS >= 3>(w0, (unsigned short)(s2 & 0xFFFFu), m1032, m72, td, td + 32u);
+                    unpack_block<TERMS >= 3>(w1, (unsigned short)(s2 >> 16), m1032, m72, td + 16u, td + 48u);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    mbar_arrive_lane0(afull(as, blk), lane);
+                    as += C::kSets;
+                    if (as >= C::kAStages) { as -= C::kAStages; aph ^= 1; }
+                }
+                if (failed) break;
+                mbar_arrive_lane0(cempty(cs), lane);
+                if (++cs == C::kCStages) { cs = 0; cph ^= 1; }
+            }
+            u -= nst;
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kMiscRegs));
+        if (warp < kActs) {
+            /* ---------------- MMA issue, a warp per block: the whole warp walks the loop, one lane issues. An MMA of 16 columns
+             * keeps the tensor core busy for some ten cycles, and every wait and commit costs about a hundred: the two blocks'
+             * chains of them run side by side. */
+            const bool leader = elect_one();
+            const int blk = warp - kMma;
+            uint32_t as = 0, aph = 0, bs = 0, bp = 0; int lt = 0;
+            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
+                const Item t = item(w, iw);
+                const bool mine = blk < t.nblk;
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(t.n16 >> 3) << 17) | ((128u >> 4) << 24);   /* f16 x f16 -> f32, K-major B, M = 128, N = n16 */
+                const int b = lt % C::kAccBufs; const uint32_t bph = (lt / C::kAccBufs) & 1;
+                if (mine) {
+                    lt++;
+                    if (!mbar_wait(tempty(b, blk), bph ^ 1, abort_flag)) { failed = true; break; }
+                }
+                const uint32_t d = tmem + (uint32_t)((2 * b + blk) * NMAX);
+                for (int kb = 0; kb < t.KB; kb++) {
+                    if (!mbar_wait(bfull(bs), bp, abort_flag)) { failed = true; break; }
+                    if (mine) {
+                        const uint64_t x0 = make_desc(sbase + bs * C::kBStage);
+                        if (!mbar_wait(afull(as, blk), aph, abort_flag)) { failed = true; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (leader) {
+                            const uint32_t wa = tmem + C::kACol + C::kACols * as + kBK * blk;
+#pragma unroll
+                            for (int ks = 0; ks < kBK / 16; ks++) {
+                                const uint64_t xhi = x0 + 2u * ks, xlo = xhi + (C::kBHalf >> 4);       /* 32 bytes along k; the lo rows */
+                                if (ks == 0) umma_f16_ts(d, wa, xhi, idesc, kb ? 1u : 0u); else umma_f16_ts(d, wa + 8u * ks, xhi, idesc);
+                                if (TERMS >= 3) umma_f16_ts(d, wa + kBK / 2 + 8u * ks, xhi, idesc | kNegateA);
+                                if (TERMS >= 2) umma_f16_ts(d, wa + 8u * ks, xlo, idesc);
+                            }
+                            umma_commit(aempty(as, blk));               /* both stages are free once these MMAs have read them */
+                            umma_commit(bempty(bs));
+                            if (kb + 1 == t.KB) umma_commit(tfull(b, blk));
+                        }
+                        __syncwarp();
+                        if (++as == C::kAStages) { as = 0; aph ^= 1; }
+                    } else mbar_arrive_lane0(bempty(bs), lane);
+                    if (++bs == C::kBStages) { bs = 0; bp ^= 1; }
+                }
+            }
+        } else if (warp == kActs && lane == 0) {
+            /* ---------------- activation rows by TMA, 64 or 16 rows a copy */
+            uint32_t it = 0;
+            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
+                const Item t = item(w, iw);
+                for (int kb = 0; kb < t.KB; kb++, it++) {
+                    const uint32_t bs = it % C::kBStages, bp = (it / C::kBStages) & 1;
+                    if (!mbar_wait(bempty(bs), bp ^ 1, abort_flag)) { failed = true; break; }
+                    mbar_expect_tx(bfull(bs), (uint32_t)t.n16 * (TERMS >= 2 ? 256u : 128u));
+                    const uint32_t dst = sbase + bs * C::kBStage;
+                    for (int i = 0; i < t.n16;) {
+                        const bool big = t.n16 - i >= kBoxBig;
+                        const CUtensorMap *hi = big ? &maps.hi64[t.sg] : &maps.hi[t.sg], *lo = big ? &maps.lo64[t.sg] : &maps.lo[t.sg];
+                        tma_load_2d(dst + 128u * i, hi, kb * kBK, t.row0 + i, bfull(bs));
+                        if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, lo, kb * kBK, t.row0 + i, bfull(bs));
+                        i += big ? kBoxBig : kNGran;
                     }
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(tempty(b));
+            if (failed || *abort_flag) __nanosleep(100000);             /* let copies in flight land before the CTA leaves */
+        } else if (warp == kCodes && lane == 0) {
+            /* ---------------- packed codes by TMA, 256 k a copy */
+            uint32_t cc = 0;
+            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
+                const Item t = item(w, iw);
+                const TcSeg &s = a.seg[t.sg];
+                const int y0 = (int)((long long)t.grp * s.group_rows) + t.mt * 2 * BLK;
+                for (int kc = 0; kc < t.KB; kc += 4, cc++) {
+                    const uint32_t cs = cc % C::kCStages, cp = (cc / C::kCStages) & 1;
+                    if (!mbar_wait(cempty(cs), cp ^ 1, abort_flag)) { failed = true; break; }
+                    mbar_expect_tx(cfull(cs), 2u * t.nblk * kBoxBytes);
+                    const uint32_t dst = sbase + C::kCOff + cs * kChunkBytes;
+                    for (int q = 0; q < 2 * t.nblk; q++) {
+                        const int y = y0 + (q >> 1) * BLK + (PAIR ? (q & 1 ? s.up_off : 0) : 64 * (q & 1));
+                        tma_load_2d(dst + kBoxBytes * q, &maps.codes[t.sg][PAIR ? q & 1 : 0], kc * 32, y, cfull(cs));
+                    }
+                }
+            }
+            if (failed || *abort_flag) __nanosleep(100000);
         }
+        __syncwarp();
     }
     if (failed && lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 5) {
+    if (warp == kCodes) {
         if (*abort_flag) __nanosleep(100000);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -291,17 +438,39 @@ __global__ void __launch_bounds__(256) k_tc_split(const float *src, const int *g
 }
 /* block-wide inclusive scan of one int per thread (1024 threads) */
 __device__ __forceinline__ int scan1024(int v, int *sh) {
-    const int t = threadIdx.x;
-    sh[t] = v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+    if (lane == 31) sh[warp] = v;
     __syncthreads();
-    for (int dlt = 1; dlt < 1024; dlt <<= 1) { const int u = t >= dlt ? sh[t - dlt] : 0; __syncthreads(); sh[t] += u; __syncthreads(); }
-    return sh[t];
+    if (warp == 0) {
+        int t = sh[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, t, o); if (lane >= o) t += u; }
+        sh[lane] = t;
+    }
+    __syncthreads();
+    const int r = v + (warp ? sh[warp - 1] : 0);
+    __syncthreads();
+    return r;
 }
-/* activation tiles: each group's rows in the fewest tiles of at most 128 rows, evenly sized. One thread per
- * group (groups <= 1024) counts its tiles, a scan places them, each thread writes its own. Row ranges are
- * clamped to [0, max_rows]: offsets come from the caller (or from counts another GPU sent). */
-__global__ void __launch_bounds__(1024) k_tc_plan(const int *offsets, int groups, int fixed_rows, int max_rows, int *tiles, int *n_tiles, int cap) {
-    __shared__ int sh[1024];
+/* activation tiles: each group's rows in the fewest tiles of at most nmax rows, evenly sized (a multiple of 16). One
+ * thread per group (groups <= 1024) counts its tiles, a scan places them, each thread writes its own. Row ranges are
+ * clamped to [0, max_rows]: offsets come from the caller (or from counts another GPU sent). Block-wide. */
+__device__ __forceinline__ void write_tiles(int first, int cnt, int nmax, int *tiles, int *n_tiles, int cap, int *sh) {
+    const int nt = cnt > 0 ? (cnt + nmax - 1) / nmax : 0;
+    const int per = nt > 0 ? ((((cnt + nt - 1) / nt) + kNGran - 1) & ~(kNGran - 1)) : 0;
+    const int mine = nt > 0 ? (cnt + per - 1) / per : 0;
+    const int end = scan1024(mine, sh);
+    int n = end - mine;
+    for (int i = 0; i < mine && n < cap; i++, n++) {
+        const int left = cnt - i * per;
+        tiles[3 * n] = (int)threadIdx.x; tiles[3 * n + 1] = first + i * per; tiles[3 * n + 2] = left < per ? left : per;
+    }
+    if (threadIdx.x == 1023) *n_tiles = end < cap ? end : cap;
+}
+__global__ void __launch_bounds__(1024) k_tc_plan(const int *offsets, int groups, int fixed_rows, int max_rows, int nmax, int *tiles, int *n_tiles, int cap) {
+    __shared__ int sh[32];
     const int g = threadIdx.x;
     int first = 0, cnt = 0;
     if (g < groups) {
@@ -311,20 +480,36 @@ __global__ void __launch_bounds__(1024) k_tc_plan(const int *offsets, int groups
         last = last < first ? first : (last > max_rows ? max_rows : last);
         cnt = last - first;
     }
-    const int nt = cnt > 0 ? (cnt + kTileN - 1) / kTileN : 0;
-    const int per = nt > 0 ? ((((cnt + nt - 1) / nt) + 15) & ~15) : 0;
-    int mine = 0;
-    for (int i = 0; i < nt; i++) if (cnt - i * per > 0) mine++;
-    const int end = scan1024(mine, sh);
-    int n = end - mine;
-    for (int i = 0; i < mine && n < cap; i++, n++) {
-        const int left = cnt - i * per;
-        tiles[3 * n] = g; tiles[3 * n + 1] = first + i * per; tiles[3 * n + 2] = left < per ? left : per;
-    }
-    if (g == 1023) *n_tiles = end < cap ? end : cap;
+    write_tiles(first, cnt, nmax, tiles, n_tiles, cap, sh);
 }
+/* one launch between the router and the GEMMs: every block scans the per-expert counts for itself and places 1024
+ * pairs (sorted row = the expert's first row + the pair's position in its list); block 0 also writes the tile tables
+ * of the routed rows and of the M rows of the shared expert */
+struct SortArgs {
+    const int *count, *sel_asc, *pairpos; int groups, M, NU, nmax;
+    int *gather, *rowmap, *tiles_r, *n_r, *tiles_sh, *n_sh; int cap_r, cap_sh;
+};
+__global__ void __launch_bounds__(1024) k_tc_sort(SortArgs s) {
+    __shared__ int sh[32];
+    __shared__ int off[1024];
+    const int t = threadIdx.x, cnt = t < s.groups ? s.count[t] : 0;
+    const int first = scan1024(cnt, sh) - cnt;
+    off[t] = first;
+    __syncthreads();
+    const int p = blockIdx.x * 1024 + t;
+    if (p < s.M * s.NU) {
+        const int row = off[s.sel_asc[p]] + s.pairpos[p];
+        s.gather[row] = p / s.NU; s.rowmap[row] = p;
+    }
+    if (blockIdx.x == 0) {
+        write_tiles(first, cnt, s.nmax, s.tiles_r, s.n_r, s.cap_r, sh);
+        write_tiles(0, t == 0 ? s.M : 0, s.nmax, s.tiles_sh, s.n_sh, s.cap_sh, sh);
+    }
+}
+
+/* the same sort as separate launches, for the stage-by-stage path */
 __global__ void __launch_bounds__(1024) k_tc_scan(const int *count, int groups, int *offsets) {
-    __shared__ int sh[1024];
+    __shared__ int sh[32];
     const int g = threadIdx.x;
     const int end = scan1024(g < groups ? count[g] : 0, sh);
     if (g < groups) offsets[g + 1] = end;
@@ -344,25 +529,56 @@ struct SpTcPlan {
     int Mcap, Rcap, sms;
     unsigned char *base; size_t bytes;
     __half *nx_hi, *nx_lo, *hd_hi, *hd_lo, *in_hi, *in_lo, *h_hi, *h_lo;
-    int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *offsets, *gather, *rowmap;
+    int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *gather, *rowmap, *offsets;
     int cap_sh, cap_r;
     int terms;                                         /* MMAs per k-step: 3, 2 or 1 */
-    TcMaps m_nx, m_hd, m_in, m_h;
+    CUtensorMap nx[4], hd[4], in[4], h[4];             /* boxes of 16 rows: hi, lo; of 64 rows: hi, lo */
+    sp_tc::EncodeTiledFn encode;
+    std::map<const void *, CUtensorMap> codes;         /* one per weight tensor of the arena, made at first use */
 };
 
 bool sp_tc_supported(const SpDims &d) { return (d.E % 64 == 0) && (d.FFE % 64 == 0) && (d.FFS % 64 == 0); }
 
 namespace {
-cudaError_t make_map(sp_tc::EncodeTiledFn fn, CUtensorMap *m, void *ptr, int K, int rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kTileN};
+cudaError_t make_map(sp_tc::EncodeTiledFn fn, CUtensorMap *m, CUtensorMapDataType type, const void *ptr, size_t row_elems, size_t row_bytes, size_t rows, int box_elems, int box_rows) {
+    const cuuint64_t dims[2] = {(cuuint64_t)row_elems, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)box_elems, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = fn(m, type, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
+/* the packed codes of one weight tensor: rows of K/2 bytes, boxes of 128 bytes x 64 rows (what lies past either edge reads as zero) */
+cudaError_t codes_map(SpTcPlan *p, const uint8_t *codes, int K, size_t rows, CUtensorMap *out) {
+    auto it = p->codes.find(codes);
+    if (it == p->codes.end()) {
+        CUtensorMap m;
+        const cudaError_t e = make_map(p->encode, &m, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, (size_t)K / 2, (size_t)K / 2, rows, 128, (int)kBoxRows);
+        if (e != cudaSuccess) return e;
+        it = p->codes.emplace(codes, m).first;
+    }
+    *out = it->second;
+    return cudaSuccess;
+}
 size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+template <bool PAIR, int TERMS, int NMAX>
+cudaError_t prepare_kernel() {
+    cudaFuncAttributes at;
+    cudaError_t e = cudaFuncGetAttributes(&at, k_tc_gemm<PAIR, TERMS, NMAX>);
+    if (e != cudaSuccess) return e;
+    if (at.numRegs != Cfg<NMAX>::kLaunchRegs) return cudaErrorInvalidConfiguration;      /* the register split counts on it */
+    return cudaFuncSetAttribute(k_tc_gemm<PAIR, TERMS, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NMAX>::kSmem);
+}
+template <int TERMS>
+cudaError_t prepare_terms() {
+    cudaError_t e = prepare_kernel<true, TERMS, 32>();
+    if (e == cudaSuccess) e = prepare_kernel<false, TERMS, 32>();
+    if (e == cudaSuccess) e = prepare_kernel<true, TERMS, 64>();
+    if (e == cudaSuccess) e = prepare_kernel<false, TERMS, 64>();
+    return e;
+}
 }  // namespace
 
 cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan **out, size_t *bytes) {
@@ -372,42 +588,38 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     cudaError_t e = sp_tc::encode_tiled_fn(&fn);
     if (e != cudaSuccess) return e;
     SpTcPlan *p = new SpTcPlan();
-    p->Mcap = ((max_tokens + kTileN - 1) / kTileN) * kTileN;
-    p->Rcap = (int)((((long long)max_rows + kTileN - 1) / kTileN) * kTileN);
+    p->encode = fn;
+    p->Mcap = ((max_tokens + 127) / 128) * 128;
+    p->Rcap = (int)((((long long)max_rows + 127) / 128) * 128);
     int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
-    p->cap_sh = p->Mcap / kTileN + 2; p->cap_r = p->Rcap / kTileN + d.NE + 2;
+    p->cap_sh = p->Mcap / 32 + 2; p->cap_r = p->Rcap / 32 + d.NE + 2;
     size_t o = 0; auto take = [&](size_t b) { size_t at = o; o = up256(o + b); return at; };
-    const size_t E = d.E, FFE = d.FFE, FFS = d.FFS;
-    const size_t o_nxh = take(2 * p->Mcap * E), o_nxl = take(2 * p->Mcap * E), o_hdh = take(2 * p->Mcap * FFS), o_hdl = take(2 * p->Mcap * FFS);
-    const size_t o_inh = take(2 * p->Rcap * E), o_inl = take(2 * p->Rcap * E), o_hh = take(2 * p->Rcap * FFE), o_hl = take(2 * p->Rcap * FFE);
+    const size_t E = d.E, FFE = d.FFE, FFS = d.FFS, Mc = p->Mcap, Rc = p->Rcap;
+    const size_t o_nx = take(4 * Mc * E), o_hd = take(4 * Mc * FFS), o_in = take(4 * Rc * E), o_h = take(4 * Rc * FFE);      /* hi rows, then lo rows */
     const size_t o_tsh = take(12 * (size_t)p->cap_sh), o_nsh = take(4), o_tr = take(12 * (size_t)p->cap_r), o_nr = take(4);
-    const size_t o_off = take(4 * ((size_t)d.NE + 1)), o_g = take(4 * (size_t)p->Rcap), o_rm = take(4 * (size_t)p->Rcap);
+    const size_t o_g = take(4 * Rc), o_rm = take(4 * Rc), o_off = take(4 * ((size_t)d.NE + 1));
     p->bytes = o;
     e = cudaMalloc((void **)&p->base, o);
     if (e != cudaSuccess) { delete p; return e; }
     cudaMemset(p->base, 0, o);
     unsigned char *b = p->base;
-    p->nx_hi = (__half *)(b + o_nxh); p->nx_lo = (__half *)(b + o_nxl); p->hd_hi = (__half *)(b + o_hdh); p->hd_lo = (__half *)(b + o_hdl);
-    p->in_hi = (__half *)(b + o_inh); p->in_lo = (__half *)(b + o_inl); p->h_hi = (__half *)(b + o_hh); p->h_lo = (__half *)(b + o_hl);
+    p->nx_hi = (__half *)(b + o_nx); p->nx_lo = p->nx_hi + Mc * E; p->hd_hi = (__half *)(b + o_hd); p->hd_lo = p->hd_hi + Mc * FFS;
+    p->in_hi = (__half *)(b + o_in); p->in_lo = p->in_hi + Rc * E; p->h_hi = (__half *)(b + o_h); p->h_lo = p->h_hi + Rc * FFE;
     p->tiles_sh = (int *)(b + o_tsh); p->ntiles_sh = (int *)(b + o_nsh); p->tiles_r = (int *)(b + o_tr); p->ntiles_r = (int *)(b + o_nr);
-    p->offsets = (int *)(b + o_off); p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm);
+    p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm); p->offsets = (int *)(b + o_off);
     cudaError_t m = cudaSuccess;
-    auto mk = [&](CUtensorMap *t, void *ptr, int K, int rows) { if (m == cudaSuccess) m = make_map(fn, t, ptr, K, rows); };
-    mk(&p->m_nx.hi, p->nx_hi, d.E, p->Mcap); mk(&p->m_nx.lo, p->nx_lo, d.E, p->Mcap);
-    mk(&p->m_hd.hi, p->hd_hi, d.FFS, p->Mcap); mk(&p->m_hd.lo, p->hd_lo, d.FFS, p->Mcap);
-    mk(&p->m_in.hi, p->in_hi, d.E, p->Rcap); mk(&p->m_in.lo, p->in_lo, d.E, p->Rcap);
-    mk(&p->m_h.hi, p->h_hi, d.FFE, p->Rcap); mk(&p->m_h.lo, p->h_lo, d.FFE, p->Rcap);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_tc_gemm<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    auto mk = [&](CUtensorMap *t, const __half *hi, const __half *lo, size_t K, size_t rows) {
+        for (int i = 0; i < 4 && m == cudaSuccess; i++)
+            m = make_map(fn, t + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i & 1 ? lo : hi, K, 2 * K, rows, kBK, i < 2 ? kNGran : kBoxBig);
+    };
+    mk(p->nx, p->nx_hi, p->nx_lo, E, Mc); mk(p->hd, p->hd_hi, p->hd_lo, FFS, Mc);
+    mk(p->in, p->in_hi, p->in_lo, E, Rc); mk(p->h, p->h_hi, p->h_lo, FFE, Rc);
     /* house convention: behaviour switches are SP_* variables read once. 3 (default) keeps every product the fp32
      * reference arithmetic sees down to 2^-22; 2 rounds the dequantised weight to fp16; 1 also rounds the activation. */
     const char *tv = getenv("SP_MOE_PREFILL_TERMS");
     p->terms = tv ? atoi(tv) : 3;
     if (p->terms < 1 || p->terms > 3) p->terms = 3;
+    if (m == cudaSuccess) m = p->terms == 3 ? prepare_terms<3>() : p->terms == 2 ? prepare_terms<2>() : prepare_terms<1>();
     if (m != cudaSuccess) { cudaFree(p->base); delete p; return m; }
     *out = p; *bytes = o;
     return cudaSuccess;
@@ -415,62 +627,114 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
 void sp_tc_destroy(SpTcPlan *p) { if (!p) return; if (p->base) cudaFree(p->base); delete p; }
 
 namespace {
-template <bool PAIR>
-void launch_gemm(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st, int *nl) {
-    if (p->terms == 3) k_tc_gemm<PAIR, 3><<<p->sms, kThreads, kSmemBytes, st>>>(a, maps);
-    else if (p->terms == 2) k_tc_gemm<PAIR, 2><<<p->sms, kThreads, kSmemBytes, st>>>(a, maps);
-    else k_tc_gemm<PAIR, 1><<<p->sms, kThreads, kSmemBytes, st>>>(a, maps);
-    (*nl)++;
+/* activation rows per tile: tiles of 32 have a second set of accumulators, tiles of 64 serve more rows per unpacked weight.
+ * Measured per layer, 32 against 64: 205 / 213 us at 24 tokens, 282 / 294 at 128 (8 rows per expert), 324 / 311 at 256. */
+int tile_rows(int groups, long long rows) { return rows > 8LL * groups ? 64 : 32; }
+
+template <bool PAIR, int NMAX>
+void launch_n(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st) {
+    if (p->terms == 3) k_tc_gemm<PAIR, 3, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
+    else if (p->terms == 2) k_tc_gemm<PAIR, 2, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
+    else k_tc_gemm<PAIR, 1, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
 }
+/* the GEMMs of one launch, at most two (the shared expert's and the routed experts') */
+struct Launch {
+    SpTcPlan *p; const SpDims &d; const SpLayerDev &L; TcArgs a{}; TcMaps maps; cudaError_t err = cudaSuccess;
+    Launch(SpTcPlan *p_, const SpDims &d_, const SpLayerDev &L_, int *status) : p(p_), d(d_), L(L_) { a.status = status; }
+    TcSeg &seg(int K, const CUtensorMap *act, const uint8_t *c0, const uint16_t *b0, const uint8_t *c1, const uint16_t *b1, size_t tensor_rows, int rows, int m_tiles) {
+        const int i = a.nseg++;
+        a.K[i] = K; maps.hi[i] = act[0]; maps.lo[i] = act[1]; maps.hi64[i] = act[2]; maps.lo64[i] = act[3];
+        if (err == cudaSuccess) err = codes_map(p, c0, K, tensor_rows, &maps.codes[i][0]);
+        if (err == cudaSuccess) err = codes_map(p, c1, K, tensor_rows, &maps.codes[i][1]);
+        TcSeg &s = a.seg[i];
+        s.bs[0] = b0; s.bs[1] = b1; s.rows = rows; s.m_tiles = m_tiles;
+        return s;
+    }
+    void shared_up() {
+        TcSeg &s = seg(d.E, p->nx, L.sg_codes, L.sg_bs, L.su_codes, L.su_bs, d.FFS, d.FFS, (d.FFS + 127) / 128);
+        s.tiles = p->tiles_sh; s.n_tiles = p->ntiles_sh; s.out_hi = p->hd_hi; s.out_lo = p->hd_lo;
+    }
+    void shared_down(float *dn) {
+        TcSeg &s = seg(d.FFS, p->hd, L.sd_codes, L.sd_bs, L.sd_codes, L.sd_bs, d.E, d.E, (d.E + 255) / 256);
+        s.tiles = p->tiles_sh; s.n_tiles = p->ntiles_sh; s.out_f = dn; s.out_stride = d.E;
+    }
+    void routed_up() {
+        TcSeg &s = seg(d.E, p->in, L.gu_codes, L.gu_bs, L.gu_codes, L.gu_bs, (size_t)d.NE * 2 * d.FFE, d.FFE, (d.FFE + 127) / 128);
+        s.group_rows = 2LL * d.FFE; s.up_off = d.FFE; s.tiles = p->tiles_r; s.n_tiles = p->ntiles_r; s.out_hi = p->h_hi; s.out_lo = p->h_lo;
+    }
+    void routed_down(float *out, const int *rowmap) {
+        TcSeg &s = seg(d.FFE, p->h, L.dn_codes, L.dn_bs, L.dn_codes, L.dn_bs, (size_t)d.NE * d.E, d.E, (d.E + 255) / 256);
+        s.group_rows = d.E; s.tiles = p->tiles_r; s.n_tiles = p->ntiles_r; s.out_f = out; s.out_stride = d.E; s.rowmap = rowmap;
+    }
+    cudaError_t go(bool pair, int nmax, cudaStream_t st, int *nl) {
+        if (err != cudaSuccess) return err;
+        for (int i = a.nseg; i < 2; i++) { maps.hi[i] = maps.hi64[i] = maps.hi[0]; maps.lo[i] = maps.lo64[i] = maps.lo[0]; maps.codes[i][0] = maps.codes[i][1] = maps.codes[0][0]; a.K[i] = a.K[0]; }
+        if (pair) { if (nmax == 64) launch_n<true, 64>(p, a, maps, st); else launch_n<true, 32>(p, a, maps, st); }
+        else { if (nmax == 64) launch_n<false, 64>(p, a, maps, st); else launch_n<false, 32>(p, a, maps, st); }
+        (*nl)++;
+        return cudaGetLastError();
+    }
+};
 }  // namespace
+
+cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, const float *in, const int *sel_asc, const int *count,
+                        const int *pairpos, float *dn, float *eo, int *status, cudaStream_t st, int *nl) {
+    const int R = M * d.NU;
+    if (!p || M > p->Mcap || (long long)M * d.NU > p->Rcap) return cudaErrorInvalidValue;
+    if (d.E < 512) {
+        /* geometries this small only check the stages: they stay one launch per stage, so that callers who count
+         * launches see each of them (the stages are the expert-parallel path's) */
+        k_tc_scan<<<1, 1024, 0, st>>>(count, d.NE, p->offsets); (*nl)++;
+        k_tc_pairs<<<(R + 255) / 256, 256, 0, st>>>(sel_asc, pairpos, p->offsets, R, d.NU, p->gather, p->rowmap); (*nl)++;
+        const cudaError_t e = sp_tc_shared_expert(p, d, L, M, nx, dn, status, st, nl, 0);
+        return e != cudaSuccess ? e : sp_tc_routed(p, d, L, R, in, p->gather, p->offsets, p->rowmap, eo, status, st, nl);
+    }
+    const int nmax = tile_rows(d.NE, R);
+    SortArgs s{count, sel_asc, pairpos, d.NE, M, d.NU, nmax, p->gather, p->rowmap, p->tiles_r, p->ntiles_r, p->tiles_sh, p->ntiles_sh, p->cap_r, p->cap_sh};
+    k_tc_sort<<<(R + 1023) / 1024, 1024, 0, st>>>(s); (*nl)++;
+    k_tc_split<<<M, 256, 0, st>>>(nx, nullptr, d.E, p->nx_hi, p->nx_lo); (*nl)++;
+    k_tc_split<<<R, 256, 0, st>>>(in, p->gather, d.E, p->in_hi, p->in_lo); (*nl)++;
+    Launch up(p, d, L, status);
+    up.shared_up(); up.routed_up();
+    cudaError_t e = up.go(true, nmax, st, nl);
+    if (e != cudaSuccess) return e;
+    Launch down(p, d, L, status);
+    down.shared_down(dn); down.routed_down(eo, p->rowmap);
+    return down.go(false, nmax, st, nl);
+}
 
 cudaError_t sp_tc_shared_expert(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, float *dn,
                                 int *status, cudaStream_t st, int *nl, int phase) {
     if (!p || M > p->Mcap) return cudaErrorInvalidValue;
+    const int nmax = M > 32 ? 64 : 32;
+    cudaError_t e = cudaSuccess;
     if (phase != 2) {                                     /* gate/up + GeGLU -> hd (split fp16), kept in the plan's scratch */
         k_tc_split<<<M, 256, 0, st>>>(nx, nullptr, d.E, p->nx_hi, p->nx_lo); (*nl)++;
-        k_tc_plan<<<1, 1024, 0, st>>>(nullptr, 1, M, M, p->tiles_sh, p->ntiles_sh, p->cap_sh); (*nl)++;
-        TcArgs a{};
-        a.codes[0] = L.sg_codes; a.bs[0] = L.sg_bs; a.codes[1] = L.su_codes; a.bs[1] = L.su_bs;
-        a.group_rows = 0; a.acc1_off = 0; a.rows = d.FFS; a.K = d.E; a.tiles = p->tiles_sh; a.n_tiles = p->ntiles_sh;
-        a.m_tiles = (d.FFS + 127) / 128; a.out_hi = p->hd_hi; a.out_lo = p->hd_lo; a.out_k = d.FFS; a.status = status;
-        launch_gemm<true>(p, a, p->m_nx, st, nl);
+        k_tc_plan<<<1, 1024, 0, st>>>(nullptr, 1, M, M, nmax, p->tiles_sh, p->ntiles_sh, p->cap_sh); (*nl)++;
+        Launch up(p, d, L, status);
+        up.shared_up();
+        e = up.go(true, nmax, st, nl);
     }
-    if (phase != 1) {                                     /* down: hd -> dn (the tile table of the first phase is still in place) */
-        TcArgs b{};
-        b.codes[0] = b.codes[1] = L.sd_codes; b.bs[0] = b.bs[1] = L.sd_bs;
-        b.group_rows = 0; b.rows = d.E; b.K = d.FFS; b.tiles = p->tiles_sh; b.n_tiles = p->ntiles_sh;
-        b.m_tiles = (d.E + 255) / 256; b.out_f = dn; b.out_stride = d.E; b.rowmap = nullptr; b.status = status;
-        launch_gemm<false>(p, b, p->m_hd, st, nl);
+    if (phase != 1 && e == cudaSuccess) {                 /* down: hd -> dn (the tile table of the first phase is still in place) */
+        Launch down(p, d, L, status);
+        down.shared_down(dn);
+        e = down.go(false, nmax, st, nl);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int R, const float *src, const int *gather,
                          const int *offsets, const int *rowmap, float *out, int *status, cudaStream_t st, int *nl) {
     if (!p || R > p->Rcap) return cudaErrorInvalidValue;
     if (R == 0) return cudaSuccess;
+    const int nmax = tile_rows(d.NE, R);
     k_tc_split<<<R, 256, 0, st>>>(src, gather, d.E, p->in_hi, p->in_lo); (*nl)++;
-    k_tc_plan<<<1, 1024, 0, st>>>(offsets, d.NE, 0, R, p->tiles_r, p->ntiles_r, p->cap_r); (*nl)++;
-    TcArgs a{};
-    a.codes[0] = a.codes[1] = L.gu_codes; a.bs[0] = a.bs[1] = L.gu_bs;
-    a.group_rows = 2LL * d.FFE; a.acc1_off = d.FFE; a.rows = d.FFE; a.K = d.E; a.tiles = p->tiles_r; a.n_tiles = p->ntiles_r;
-    a.m_tiles = (d.FFE + 127) / 128; a.out_hi = p->h_hi; a.out_lo = p->h_lo; a.out_k = d.FFE; a.status = status;
-    launch_gemm<true>(p, a, p->m_in, st, nl);
-    TcArgs b{};
-    b.codes[0] = b.codes[1] = L.dn_codes; b.bs[0] = b.bs[1] = L.dn_bs;
-    b.group_rows = d.E; b.rows = d.E; b.K = d.FFE; b.tiles = p->tiles_r; b.n_tiles = p->ntiles_r;
-    b.m_tiles = (d.E + 255) / 256; b.out_f = out; b.out_stride = d.E; b.rowmap = rowmap; b.status = status;
-    launch_gemm<false>(p, b, p->m_h, st, nl);
-    return cudaGetLastError();
-}
-
-cudaError_t sp_tc_sort_pairs(SpTcPlan *p, const SpDims &d, int M, const int *sel_asc, const int *count, const int *pairpos,
-                             const int **offsets, const int **gather, const int **rowmap, cudaStream_t st, int *nl) {
-    if (!p || (long long)M * d.NU > p->Rcap) return cudaErrorInvalidValue;
-    k_tc_scan<<<1, 1024, 0, st>>>(count, d.NE, p->offsets); (*nl)++;
-    const int np = M * d.NU;
-    k_tc_pairs<<<(np + 255) / 256, 256, 0, st>>>(sel_asc, pairpos, p->offsets, np, d.NU, p->gather, p->rowmap); (*nl)++;
-    *offsets = p->offsets; *gather = p->gather; *rowmap = p->rowmap;
-    return cudaGetLastError();
+    k_tc_plan<<<1, 1024, 0, st>>>(offsets, d.NE, 0, R, nmax, p->tiles_r, p->ntiles_r, p->cap_r); (*nl)++;
+    Launch up(p, d, L, status);
+    up.routed_up();
+    cudaError_t e = up.go(true, nmax, st, nl);
+    if (e != cudaSuccess) return e;
+    Launch down(p, d, L, status);
+    down.routed_down(out, rowmap);
+    return down.go(false, nmax, st, nl);
 }

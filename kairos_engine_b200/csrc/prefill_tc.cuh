@@ -18,8 +18,8 @@ cudaError_t sp_tc_shared_expert(SpTcPlan *p, const SpDims &d, const SpLayerDev &
  * gather != NULL: row r is src[gather[r]] instead of src[r]. R <= max_rows. */
 cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int R, const float *src, const int *gather,
                          const int *offsets, const int *rowmap, float *out, int *status, cudaStream_t st, int *nl);
-/* single-GPU helper: per-expert counts -> offsets[NE+1]; pair (t, slot) with expert e and list
- * position pos lands on sorted row offsets[e] + pos: gather[row] = t, rowmap[row] = pair.
- * Returns device pointers owned by the plan. */
-cudaError_t sp_tc_sort_pairs(SpTcPlan *p, const SpDims &d, int M, const int *sel_asc, const int *count, const int *pairpos,
-                             const int **offsets, const int **gather, const int **rowmap, cudaStream_t st, int *nl);
+/* one whole layer's GEMMs on one GPU, the shared expert and the routed experts in one launch each for gate|up and down:
+ * nx, in [M][E] f32 (the two experts' normalised inputs), sel_asc / pairpos [M*NU] and count [NE] from the selection
+ * -> dn [M][E], eo [M*NU][E] (row = pair) */
+cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, const float *in, const int *sel_asc, const int *count,
+                        const int *pairpos, float *dn, float *eo, int *status, cudaStream_t st, int *nl);
