@@ -16,6 +16,7 @@
  */
 #include "batched.cuh"
 #include "prefill_tc.cuh"
+#include "rows_mma.cuh"
 #include <cstdlib>
 #include "../../include/sp_engine/moe_backend.h"
 
@@ -25,9 +26,8 @@ struct BView {                 /* carved scratch */
     float *rin, *nx_f, *in_f, *logits, *cw, *hd, *dn, *h, *eo, *xa, *xb;
     signed char *nx_q, *in_q, *hd_q, *h_q;
     float *nx_s, *in_s, *hd_s, *h_s;
-    int *nx_c, *in_c, *hd_c, *h_c;
     int *sel_asc, *count, *list, *pairpos, *ep_off;
-    signed char *ep_q; float *ep_s; int *ep_c;      /* expert-parallel stage: quantised received rows, [max_rows] */
+    signed char *ep_q; float *ep_s;      /* expert-parallel stage: quantised received rows, [max_rows] */
 };
 
 size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -43,23 +43,21 @@ size_t blayout(const SpDims &d, int Mx, int Rx, F place) {
     take(4 * M * E); take(4 * M * E);                                                               /* xa xb */
     take(M * E); take(M * E); take(M * FFS); take(R * FFE);                                          /* q */
     take(4 * M * (E / 16)); take(4 * M * (E / 16)); take(4 * M * (FFS / 16)); take(4 * R * (FFE / 16));        /* s */
-    take(4 * M * (E / 16)); take(4 * M * (E / 16)); take(4 * M * (FFS / 16)); take(4 * R * (FFE / 16));        /* c */
     take(4 * M * NU); take(4 * NE * kSlices); take(4 * NE * M);                                     /* sel_asc count list */
-    take(R * E); take(4 * R * (E / 16)); take(4 * R * (E / 16));                                    /* ep_q ep_s ep_c */
+    take(R * E); take(4 * R * (E / 16));                                                            /* ep_q ep_s */
     take(4 * M * NU); take(4 * (NE + 1) * kSlices);                                                 /* pairpos ep_off */
     return o;
 }
 BView bview(const SpDims &d, const SpBatchedScratch *s) {
-    unsigned char *p[31];
+    unsigned char *p[26];
     blayout(d, s->max_tokens, s->max_rows, [&](int id, size_t off) { p[id] = (unsigned char *)s->base + off; });
     BView v;
     v.rin = (float *)p[0]; v.nx_f = (float *)p[1]; v.in_f = (float *)p[2]; v.logits = (float *)p[3]; v.cw = (float *)p[4];
     v.hd = (float *)p[5]; v.dn = (float *)p[6]; v.h = (float *)p[7]; v.eo = (float *)p[8]; v.xa = (float *)p[9]; v.xb = (float *)p[10];
     v.nx_q = (signed char *)p[11]; v.in_q = (signed char *)p[12]; v.hd_q = (signed char *)p[13]; v.h_q = (signed char *)p[14];
     v.nx_s = (float *)p[15]; v.in_s = (float *)p[16]; v.hd_s = (float *)p[17]; v.h_s = (float *)p[18];
-    v.nx_c = (int *)p[19]; v.in_c = (int *)p[20]; v.hd_c = (int *)p[21]; v.h_c = (int *)p[22];
-    v.sel_asc = (int *)p[23]; v.count = (int *)p[24]; v.list = (int *)p[25];
-    v.ep_q = (signed char *)p[26]; v.ep_s = (float *)p[27]; v.ep_c = (int *)p[28]; v.pairpos = (int *)p[29]; v.ep_off = (int *)p[30];
+    v.sel_asc = (int *)p[19]; v.count = (int *)p[20]; v.list = (int *)p[21];
+    v.ep_q = (signed char *)p[22]; v.ep_s = (float *)p[23]; v.pairpos = (int *)p[24]; v.ep_off = (int *)p[25];
     return v;
 }
 /* The same scratch seen by token slice `slice` of a layer, whose first token is `t0`: everything the route stage
@@ -73,7 +71,6 @@ BView bview_slice(const SpDims &d, const SpBatchedScratch *s, int t0, int slice)
     v.rin += t * E; v.nx_f += t * E; v.in_f += t * E; v.logits += t * NE; v.cw += t * NU; v.hd += t * FFS; v.dn += t * E; v.eo += t * NU * E;
     v.nx_q += t * E; v.in_q += t * E; v.hd_q += t * FFS;
     v.nx_s += t * (E / 16); v.in_s += t * (E / 16); v.hd_s += t * (FFS / 16);
-    v.nx_c += t * (E / 16); v.in_c += t * (E / 16); v.hd_c += t * (FFS / 16);
     v.sel_asc += t * NU; v.pairpos += t * NU; v.list += t * NE;
     v.count += (size_t)slice * NE; v.ep_off += (size_t)slice * (NE + 1);
     return v;
@@ -110,13 +107,13 @@ __device__ __forceinline__ float warp_tree(float v) {
 }
 /* quantise one row with all 256 threads (k_quant_act_int8_batched, CF:1725-1746) */
 template <class F>
-__device__ __forceinline__ void quant_row(int n, signed char *q, float *sx, int *corr, F get) {
+__device__ __forceinline__ void quant_row(int n, signed char *q, float *sx, F get) {
     for (int base = 0; base < n; base += 256) {
         const int i = base + (int)threadIdx.x;
         const bool valid = i < n;
         const float v = valid ? get(i) : 0.0f;
         const int b = i >> 4;
-        quant_elem16(v, valid, q + 16 * b, sx + b, corr + b);
+        quant_elem16(v, valid, q + 16 * b, sx + b);
     }
 }
 
@@ -169,8 +166,8 @@ __global__ void __launch_bounds__(256) k_b_prep(SpDims d, SpLayerDev L, const fl
                 const float nv = __fmul_rn(xs, n1[k]), iv = __fmul_rn(xs, n2[k]);
                 if (FA) {
                     const int b = i >> 4;
-                    quant_elem16(nv, ok, v.nx_q + row + 16 * b, v.nx_s + b16 + b, v.nx_c + b16 + b);
-                    quant_elem16(iv, ok, v.in_q + row + 16 * b, v.in_s + b16 + b, v.in_c + b16 + b);
+                    quant_elem16(nv, ok, v.nx_q + row + 16 * b, v.nx_s + b16 + b);
+                    quant_elem16(iv, ok, v.in_q + row + 16 * b, v.in_s + b16 + b);
                 } else if (ok) { v.nx_f[row + i] = nv; v.in_f[row + i] = iv; }
                 if (ok) {
                     if (rows_f) rows_f[row + i] = iv;
@@ -183,8 +180,8 @@ __global__ void __launch_bounds__(256) k_b_prep(SpDims d, SpLayerDev L, const fl
     const float scale = rms_scale_from(sumsq256(xt, E, sh), E, d.eps);
     if (FA) {
         const size_t b16 = (size_t)t * (E / 16);
-        quant_row(E, v.nx_q + (size_t)t * E, v.nx_s + b16, v.nx_c + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.ffn_norm + i)); });
-        quant_row(E, v.in_q + (size_t)t * E, v.in_s + b16, v.in_c + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i)); });
+        quant_row(E, v.nx_q + (size_t)t * E, v.nx_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.ffn_norm + i)); });
+        quant_row(E, v.in_q + (size_t)t * E, v.in_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i)); });
         if (rows_f)                                             /* the routed experts' input as fp32 rows (expert-parallel dispatch) */
             for (int i = tid; i < E; i += 256) rows_f[(size_t)t * E + i] = __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i));
     } else {
@@ -362,7 +359,7 @@ __global__ void __launch_bounds__(256) k_b_topk(SpDims d, SpLayerDev L, BView v,
 }
 
 /* ---------------------------------------------------------------- K5: per-row activation quant (CF:1725-1746) */
-__global__ void __launch_bounds__(256) k_b_quant_rows(const float *x, int n, signed char *q, float *sx, int *corr) {
+__global__ void __launch_bounds__(256) k_b_quant_rows(const float *x, int n, signed char *q, float *sx) {
     const size_t r = blockIdx.x;
     const float *xr = x + r * n;
     if (n <= 256 * kPrepK) {                                    /* all of the row's loads first, then the dependent steps */
@@ -373,15 +370,15 @@ __global__ void __launch_bounds__(256) k_b_quant_rows(const float *x, int n, sig
         for (int k = 0; k < kPrepK; k++)
             if (256 * k < n) {
                 const int i = (int)threadIdx.x + 256 * k, b = i >> 4;
-                quant_elem16(v[k], i < n, q + r * n + 16 * b, sx + r * (n / 16) + b, corr + r * (n / 16) + b);
+                quant_elem16(v[k], i < n, q + r * n + 16 * b, sx + r * (n / 16) + b);
             }
         return;
     }
-    quant_row(n, q + r * n, sx + r * (n / 16), corr + r * (n / 16), [&](int i) { return xr[i]; });
+    quant_row(n, q + r * n, sx + r * (n / 16), [&](int i) { return xr[i]; });
 }
 
-/* ---------------------------------------------------------------- K4/K6: Q4B rows x a list of activations
- * One warp per output row (or gate/up row pair); its codes and block scales are loaded ONCE into
+/* ---------------------------------------------------------------- K4/K6, floating-point flavour without the tensor cores
+ * (the integer flavour's rows are rows_mma.cu's). One warp per output row (or gate/up row pair); its codes and block scales are loaded ONCE into
  * registers and reused for every activation in the group's list, so each weight byte is read from
  * HBM once per layer however many tokens share the expert. grid.y = group (expert, or 0 for the
  * shared expert whose list is every token). */
@@ -396,9 +393,6 @@ struct GroupArgs {
     const uint8_t *ucodes; const uint16_t *ubs;    /* PAIR with a separate up tensor (shared expert), else NULL */
     int act_div;                                   /* activation row = item / act_div (NU for routed gate|up, 1 otherwise) */
     const int *act_index;                          /* with offset: sorted position -> activation row, when it is not the item's own row (NULL = item / act_div) */
-    /* flavour A */
-    const signed char *q; const float *sx; const int *corr;
-    /* flavour B */
     const float *xf;
     float *out; int out_stride;                    /* out[item * out_stride + row] */
 };
@@ -411,23 +405,6 @@ __device__ __forceinline__ void load_row(const uint8_t *codes, const uint16_t *b
         if (c < n32) { w[i] = ld_stream16(codes + 16 * (size_t)c); sc[i] = h2f(ld_stream_u16(bs + c)); }
         else { w[i] = make_int4(0, 0, 0, 0); sc[i] = 0.0f; }
     }
-}
-template <int NIT>
-__device__ __forceinline__ float dot_a(const int4 (&w)[NIT], const float (&sc)[NIT], int n32, int lane,
-                                       const int4 *q, const float *sx, const int *corr) {
-    float facc = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NIT; i++) {
-        const int c = lane + 32 * i;
-        if (c < n32) {
-            const int2 cr = *reinterpret_cast<const int2 *>(corr + 2 * c);
-            const float2 s2 = *reinterpret_cast<const float2 *>(sx + 2 * c);
-            int a0, a1;
-            q4b_chunk_dot(w[i], q[2 * c], q[2 * c + 1], cr.x, cr.y, a0, a1);
-            facc = __fmaf_rn(sc[i], __fmaf_rn((float)a0, s2.x, __fmul_rn((float)a1, s2.y)), facc);
-        }
-    }
-    return warp_tree(facc);
 }
 /* flavour B: w = code * scale exactly (CF:1459-1463), fp32 dot */
 template <int NIT>
@@ -459,7 +436,7 @@ __device__ __forceinline__ float dot_b(const int4 (&w)[NIT], const float (&sc)[N
     return warp_tree(acc);
 }
 
-template <bool FA, bool PAIR, int NIT>
+template <bool PAIR, int NIT>
 __global__ void __launch_bounds__(256) k_b_rows(GroupArgs g) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = blockIdx.y;
@@ -484,293 +461,51 @@ __global__ void __launch_bounds__(256) k_b_rows(GroupArgs g) {
         else load_row<NIT>(g.codes + (row + g.up_off) * rb, g.bs + (row + g.up_off) * n32, n32, lane, reinterpret_cast<int4(&)[NIT]>(w1), reinterpret_cast<float(&)[NIT]>(s1));
     }
     const int *list = g.list ? g.list + (size_t)grp * g.list_stride : nullptr;
-    const int b16 = g.in >> 4;
     for (int i = 0; i < cnt; i++) {
         const int item = list ? list[i] : (g.index ? g.index[first + i] : first + i);
         const size_t arow = (size_t)(g.act_index ? g.act_index[first + i] : item / g.act_div);
-        float o;
-        if (FA) {
-            const int4 *q = reinterpret_cast<const int4 *>(g.q + arow * g.in);
-            const float *sx = g.sx + arow * b16; const int *corr = g.corr + arow * b16;
-            o = dot_a<NIT>(w0, s0, n32, lane, q, sx, corr);
-            if (PAIR) o = gelu_mul(o, dot_a<NIT>(reinterpret_cast<int4(&)[NIT]>(w1), reinterpret_cast<float(&)[NIT]>(s1), n32, lane, q, sx, corr));
-        } else {
-            const float *x = g.xf + arow * g.in;
-            o = dot_b<NIT>(w0, s0, n32, lane, x);
-            if (PAIR) o = gelu_mul(o, dot_b<NIT>(reinterpret_cast<int4(&)[NIT]>(w1), reinterpret_cast<float(&)[NIT]>(s1), n32, lane, x));
-        }
+        const float *x = g.xf + arow * g.in;
+        float o = dot_b<NIT>(w0, s0, n32, lane, x);
+        if (PAIR) o = gelu_mul(o, dot_b<NIT>(reinterpret_cast<int4(&)[NIT]>(w1), reinterpret_cast<float(&)[NIT]>(s1), n32, lane, x));
         if (lane == 0) g.out[(size_t)item * g.out_stride + r] = o;
     }
 }
 
-/* ---------------------------------------------------------------- K4/K6 on the tensor cores (integer flavour)
- * The same sums as dot_a, bit for bit, with the 16-weight block dots taken by mma.sync m16n8k32
- * (s8 x s8 -> s32) instead of dp4a chains. A warp owns 16 weight rows. Four chunks (4 x 32 weights)
- * go through four MMAs that accumulate into one C tile: the activation operand of MMA i is non-zero
- * only in the column (chunk, half) its k-slots belong to, so column 2q+h of C ends up holding the
- * integer dot of half h of chunk 4j+q, and lane (g, q) of the warp reads the two block sums of
- * "its" chunk for rows g and g+8 straight out of its C registers. Lane (g, q) therefore plays the
- * part that lane (4j+q) % 32 plays in dot_a: it keeps one fp32 accumulator per slot and adds its
- * chunks in ascending order; the 32 slots of a row are then added in the pairing of warp_tree.
- *   A operand: code nibbles moved to the top of a byte (value 16*code as s8, no +8 bias, no
- *              correction term); low nibbles feed k-slots 4q..4q+3, high nibbles 16+4q..16+4q+3.
- *   B operand: the activations' int8 values; the quantiser already stores every 8 of them as
- *              4 even-index then 4 odd-index bytes, which is the order the nibble split needs.
- *   C starts at 0x4B400000 (1.5 * 2^23): the s32 result read as a float is 12582912 + 16*S, and one
- *              fma by 1/16 gives float(S) exactly, without an integer-to-float conversion.
- * KS = warps per 16-row unit: 1 (in <= 768: a warp covers the whole row) or 4 (in <= 3072: warp wq
- * covers slots 8wq..8wq+7 and the slot sums meet in shared memory). */
-constexpr int kMmaTB = 4, kMmaG = 6, kMmaPartStride = 33;
-constexpr int kMmaMagic = 0x4B400000;
-
-__device__ __forceinline__ void mma_s8(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ float magic_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }
-/* the 32 slot sums of one row, added in warp_tree's pairing */
-__device__ __forceinline__ float slot_tree(const float *p) {
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = p[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < o; i++) v[i] += v[i + o];
-    return v[0];
-}
-
-/* shared-memory row stride of the staged codes: the two rows a quarter-warp reads (64 B each) must fall in different banks */
-__host__ __device__ constexpr int mma_a_stride(int in) { return in / 2 + ((64 - (in / 2) % 128 + 128) % 128); }
-template <int KS>
-constexpr size_t mma_smem_bytes(int in) {
-    return (size_t)kMmaTB * (in + 16) + (size_t)kMmaTB * (in / 16) * 4 + 16
-         + (KS == 4 ? (size_t)2 * kMmaTB * 16 * kMmaPartStride * 4 : (size_t)8 * kMmaTB * 16 * 4)
-         + (size_t)(8 / KS) * 16 * mma_a_stride(in);
-}
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((unsigned)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
-}
-/* D = A*B + {c, c, c, c}: the first MMA of a chain reads its start value from one register */
-__device__ __forceinline__ void mma_s8_first(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
-}
-
-template <bool PAIR, int KS>
-__global__ void __launch_bounds__(256, 2) k_b_rows_mma(GroupArgs g) {
-    constexpr int TB = kMmaTB, UNITS = 8 / KS, TPC = PAIR ? UNITS / 2 : UNITS, NACC = KS == 4 ? 2 : 8;
-    extern __shared__ __align__(16) unsigned char sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
-    const int grp = blockIdx.y;
-    int first = 0, cnt;
-    if (g.offset) {
-        int last = g.offset[grp + 1];
-        first = g.offset[grp];
-        first = first < 0 ? 0 : (first > g.M ? g.M : first);
-        last = last > g.M ? g.M : last;
-        cnt = last - first;
-    } else cnt = g.count ? g.count[grp] : g.M;
-    if ((int)blockIdx.z * TB >= cnt) return;
-    const int in = g.in, n32 = in >> 5, b16 = in >> 4, ngroups = (n32 + 3) >> 2, astride = mma_a_stride(in), pstride = in + 16;
-    unsigned char *P = sm;                                      /* [TB][in + 16]: a token's activations as the quantiser stored them, then 16 zero bytes */
-    float *sxs = reinterpret_cast<float *>(P + (size_t)TB * pstride);   /* [TB][in/16] activation block scales */
-    int *items = reinterpret_cast<int *>(sxs + (size_t)TB * b16);      /* [TB] (+ padding to 16 bytes) */
-    float *part = reinterpret_cast<float *>(items + 4);         /* KS=4: [2][TB][16][33] slot sums; KS=1: [8][TB][16] row sums */
-    unsigned char *A = reinterpret_cast<unsigned char *>(part + (KS == 4 ? 2 * TB * 16 * kMmaPartStride : 8 * TB * 16));   /* [UNITS][16][astride] codes */
-    const size_t rb = (size_t)in / 2;
-
-    /* the block's weight rows go to shared memory once, in one burst: warp w copies rows w, w+8, ... */
-    {
-        const int ppr = (int)(rb >> 4);
-        for (int ur = warp; ur < UNITS * 16; ur += 8) {
-            const int u = ur >> 4, r = ur & 15;
-            const int tile_u = blockIdx.x * TPC + (PAIR ? u >> 1 : u);
-            if (tile_u * 16 < g.rows) {
-                const bool up_u = PAIR && (u & 1);
-                const size_t row = (size_t)grp * g.rows_per_group + tile_u * 16 + r + (up_u && !g.ucodes ? g.up_off : 0);
-                const uint8_t *src = (up_u && g.ucodes ? g.ucodes : g.codes) + row * rb;
-                unsigned char *dst = A + (size_t)ur * astride;
-                for (int k = lane; k < ppr; k += 32) cp_async16(dst + 16 * k, src + 16 * (size_t)k);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    const int unit = warp / KS, wq = warp % KS;
-    const int tile = blockIdx.x * TPC + (PAIR ? unit >> 1 : unit);
-    const bool up = PAIR && (unit & 1);
-    const bool tile_ok = tile * 16 < g.rows;
-    const int r0 = tile_ok ? tile * 16 : 0;                     /* a warp past the last tile keeps valid pointers and computes nothing */
-    const unsigned char *A0 = A + ((size_t)unit * 16 + gq) * astride, *A1 = A0 + 8 * (size_t)astride;
-    float sc[kMmaG][2];                                         /* this lane's block scales: rows gq and gq+8, one chunk per group */
-    {
-        const size_t row = (size_t)grp * g.rows_per_group + r0 + gq + (up && !g.ucodes ? g.up_off : 0);
-        const uint16_t *bs0 = (up && g.ucodes ? g.ubs : g.bs) + row * n32, *bs1 = bs0 + 8 * (size_t)n32;
-#pragma unroll
-        for (int jj = 0; jj < kMmaG; jj++) {
-            const int j = KS == 4 ? 8 * (jj >> 1) + 2 * wq + (jj & 1) : jj;
-            const int c = 4 * j + q, cc = c < n32 ? c : n32 - 1;
-            sc[jj][0] = h2f(ld_stream_u16(bs0 + cc)); sc[jj][1] = h2f(ld_stream_u16(bs1 + cc));
-        }
-    }
-    const int *list = g.list ? g.list + (size_t)grp * g.list_stride : nullptr;
-    const bool bvalid = (gq >> 1) == q;                         /* this lane's k-slots belong to column pair (2q, 2q+1) */
-    const int bh = gq & 1;
-    if (tid < 4 * TB) reinterpret_cast<int *>(P + (size_t)(tid >> 2) * pstride + in)[tid & 3] = 0;
-    const bool vec_sx = (b16 & 3) == 0;                         /* 16-byte copies of the scales need 16-byte rows */
-
-    for (int b0 = blockIdx.z * TB; b0 < cnt; b0 += gridDim.z * TB) {   /* token batches are dealt round-robin over grid.z */
-        const int nb = cnt - b0 < TB ? cnt - b0 : TB;
-        __syncthreads();                                        /* the previous batch's readers are done */
-        /* warps 2t and 2t+1 fetch token t: its int8 row and its block scales */
-        {
-            const int t = warp >> 1, hw = warp & 1;
-            if (t < nb) {
-                const int item = list ? list[b0 + t] : (g.index ? g.index[first + b0 + t] : first + b0 + t);
-                if (hw == 0 && lane == 0) items[t] = item;
-                const size_t arow = (size_t)(g.act_index ? g.act_index[first + b0 + t] : item / g.act_div);
-                const signed char *qs = g.q + arow * in;
-                unsigned char *pd = P + (size_t)t * pstride;
-                for (int k = lane + 32 * hw; k < b16; k += 64) cp_async16(pd + 16 * k, qs + 16 * (size_t)k);
-                const float *ss = g.sx + arow * b16;
-                if (vec_sx) { for (int k = lane + 32 * hw; k < (b16 >> 2); k += 64) cp_async16(sxs + t * b16 + 4 * k, ss + 4 * k); }
-                else { for (int k = lane + 32 * hw; k < b16; k += 64) sxs[t * b16 + k] = ss[k]; }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-
-        if (tile_ok) {
-            float acc[TB][NACC][2];
-#pragma unroll
-            for (int t = 0; t < TB; t++)
-#pragma unroll
-                for (int a = 0; a < NACC; a++) acc[t][a][0] = acc[t][a][1] = 0.0f;
-#pragma unroll
-            for (int jj = 0; jj < kMmaG; jj++) {
-                const int j = KS == 4 ? 8 * (jj >> 1) + 2 * wq + (jj & 1) : jj;
-                if (j < ngroups) {
-                    const int ai = KS == 4 ? (jj & 1) : jj;
-                    const int c = 4 * j + q;
-                    const bool cv = c < n32;
-                    const int cc = cv ? c : n32 - 1;                    /* a lane past the row's end reads the last chunk and drops it */
-                    uint4 w0 = *reinterpret_cast<const uint4 *>(A0 + 16 * cc), w1 = *reinterpret_cast<const uint4 *>(A1 + 16 * cc);
-                    if (!cv) { w0 = make_uint4(0, 0, 0, 0); w1 = w0; }
-                    const float s0 = sc[jj][0], s1 = sc[jj][1];
-                    const unsigned x0[4] = {w0.x, w0.y, w0.z, w0.w};
-                    const unsigned x1[4] = {w1.x, w1.y, w1.z, w1.w};
-                    unsigned a[4][4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        a[i][0] = (x0[i] << 4) & 0xF0F0F0F0u; a[i][1] = (x1[i] << 4) & 0xF0F0F0F0u;
-                        a[i][2] = x0[i] & 0xF0F0F0F0u;        a[i][3] = x1[i] & 0xF0F0F0F0u;
-                    }
-                    /* a lane whose k-slots are not in column (chunk, half) reads the token's 16 zero bytes */
-                    const int off0 = bvalid && cv && bh == 0 ? c * 32 : in, off1 = bvalid && cv && bh == 1 ? c * 32 + 16 : in;
-#pragma unroll
-                    for (int t = 0; t < TB; t++) {
-                        if (t < nb) {
-                            const unsigned char *pt = P + (size_t)t * pstride;
-                            const uint4 l0 = *reinterpret_cast<const uint4 *>(pt + off0);
-                            const uint4 l1 = *reinterpret_cast<const uint4 *>(pt + off1);
-                            int ca[4], cb[4];
-                            mma_s8_first(ca, a[0][0], a[0][1], a[0][2], a[0][3], l0.x, l0.y, kMmaMagic);
-                            mma_s8_first(cb, a[2][0], a[2][1], a[2][2], a[2][3], l1.x, l1.y, kMmaMagic);
-                            mma_s8(ca, a[1][0], a[1][1], a[1][2], a[1][3], l0.z, l0.w);
-                            mma_s8(cb, a[3][0], a[3][1], a[3][2], a[3][3], l1.z, l1.w);
-                            if (cv) {
-                                const float2 s2 = *reinterpret_cast<const float2 *>(sxs + t * b16 + 2 * c);
-                                acc[t][ai][0] = __fmaf_rn(s0, __fmaf_rn(magic_to_float(ca[0]), s2.x, __fmul_rn(magic_to_float(cb[1]), s2.y)), acc[t][ai][0]);
-                                acc[t][ai][1] = __fmaf_rn(s1, __fmaf_rn(magic_to_float(ca[2]), s2.x, __fmul_rn(magic_to_float(cb[3]), s2.y)), acc[t][ai][1]);
-                            }
-                        }
-                    }
-                }
-            }
-            if (KS == 4) {
-#pragma unroll
-                for (int t = 0; t < TB; t++)
-                    if (t < nb)
-#pragma unroll
-                        for (int a2 = 0; a2 < NACC; a2++)
-#pragma unroll
-                            for (int r = 0; r < 2; r++)
-                                part[((size_t)(unit * TB + t) * 16 + gq + 8 * r) * kMmaPartStride + 8 * wq + 4 * a2 + q] = acc[t][a2][r];
-            } else {
-#pragma unroll
-                for (int t = 0; t < TB; t++)
-                    if (t < nb)
-#pragma unroll
-                        for (int r = 0; r < 2; r++) {
-                            float v[8];
-#pragma unroll
-                            for (int a2 = 0; a2 < 8; a2++) v[a2] = acc[t][a2][r];
-#pragma unroll
-                            for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-                                for (int i = 0; i < o; i++) v[i] += v[i + o];      /* slots s+16, s+8, s+4 sit in this lane */
-                            float s = v[0];
-                            s += __shfl_down_sync(0xffffffffu, s, 2);
-                            s += __shfl_down_sync(0xffffffffu, s, 1);
-                            if (q == 0) part[(size_t)(unit * TB + t) * 16 + gq + 8 * r] = s;
-                        }
-            }
-        }
-        __syncthreads();
-        /* one thread per (unit, token, row); with PAIR the gate thread (even lane) takes the up value from its neighbour */
-        {
-            const int per = nb * 16 * (PAIR ? 2 : 1);           /* threads per tile */
-            for (int w0 = 0; w0 < TPC * per; w0 += 256) {
-                const int w = w0 + tid;
-                const bool act = w < TPC * per;
-                const int tl = act ? w / per : 0, rem = act ? w - tl * per : 0;
-                const int half = PAIR ? rem & 1 : 0, tr = PAIR ? rem >> 1 : rem, t = tr >> 4, row = tr & 15;
-                const int u = PAIR ? 2 * tl + half : tl;
-                float o = 0.0f;
-                if (act) o = KS == 4 ? slot_tree(part + ((size_t)(u * TB + t) * 16 + row) * kMmaPartStride) : part[(size_t)(u * TB + t) * 16 + row];
-                if (PAIR) { const float other = __shfl_down_sync(0xffffffffu, o, 1); if (half == 0) o = gelu_mul(o, other); }
-                const int r = (blockIdx.x * TPC + tl) * 16 + row;
-                if (act && half == 0 && r < g.rows) g.out[(size_t)items[t] * g.out_stride + r] = o;
-            }
-        }
-    }
-}
-/* the staged rows need more than the default 48 KB of shared memory: a per-device setting */
-cudaError_t mma_rows_prepare() {
-    const int lim = 200 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(k_b_rows_mma<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_b_rows_mma<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_b_rows_mma<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_b_rows_mma<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    return e;
-}
-
-template <bool FA, bool PAIR>
+template <bool PAIR>
 void launch_rows(const GroupArgs &g, int groups, cudaStream_t st, int *nl) {
-    if (FA && (g.rows & 15) == 0 && (g.in & 31) == 0 && g.in <= 3072) {
-        const int tiles = g.rows / 16;
-        /* one group holding every token (the shared expert) spreads its token batches over grid.z; routed
-         * groups hold M*NU/groups tokens on average, so two CTAs per tile cover the long lists */
-        const int batches = (g.M + kMmaTB - 1) / kMmaTB;
-        const unsigned z = (unsigned)(groups == 1 ? (batches < 32 ? batches : 32) : (batches > 2 ? 2 : 1));
-        if (g.in <= 768) {
-            const int tpc = PAIR ? 4 : 8;
-            k_b_rows_mma<PAIR, 1><<<dim3((unsigned)((tiles + tpc - 1) / tpc), (unsigned)groups, z), 256, mma_smem_bytes<1>(g.in), st>>>(g);
-        } else {
-            const int tpc = PAIR ? 1 : 2;
-            k_b_rows_mma<PAIR, 4><<<dim3((unsigned)((tiles + tpc - 1) / tpc), (unsigned)groups, z), 256, mma_smem_bytes<4>(g.in), st>>>(g);
-        }
-        (*nl)++;
-        return;
-    }
     const dim3 grid((unsigned)((g.rows + 7) / 8), (unsigned)groups);
     const int nit = ((g.in >> 5) + 31) >> 5;
-    if (nit <= 1) k_b_rows<FA, PAIR, 1><<<grid, 256, 0, st>>>(g);
-    else if (nit == 2) k_b_rows<FA, PAIR, 2><<<grid, 256, 0, st>>>(g);
-    else if (nit == 3) k_b_rows<FA, PAIR, 3><<<grid, 256, 0, st>>>(g);
-    else k_b_rows<FA, PAIR, 4><<<grid, 256, 0, st>>>(g);
+    if (nit <= 1) k_b_rows<PAIR, 1><<<grid, 256, 0, st>>>(g);
+    else if (nit == 2) k_b_rows<PAIR, 2><<<grid, 256, 0, st>>>(g);
+    else if (nit == 3) k_b_rows<PAIR, 3><<<grid, 256, 0, st>>>(g);
+    else k_b_rows<PAIR, 4><<<grid, 256, 0, st>>>(g);
     (*nl)++;
+}
+
+/* ---------------------------------------------------------------- K4/K6, integer flavour: the four row sets as segments of rows_mma.cu */
+SpRowsSeg seg_shared_up(const SpDims &d, const SpLayerDev &L, int M, const BView &v) {
+    SpRowsSeg s{};
+    s.codes = L.sg_codes; s.bs = L.sg_bs; s.ucodes = L.su_codes; s.ubs = L.su_bs; s.in = d.E; s.rows = d.FFS; s.groups = 1; s.M = M; s.act_div = 1;
+    s.q = v.nx_q; s.sx = v.nx_s; s.out_q = v.hd_q; s.out_s = v.hd_s;
+    return s;
+}
+SpRowsSeg seg_shared_down(const SpDims &d, const SpLayerDev &L, int M, const BView &v) {
+    SpRowsSeg s{};
+    s.codes = L.sd_codes; s.bs = L.sd_bs; s.in = d.FFS; s.rows = d.E; s.groups = 1; s.M = M; s.act_div = 1;
+    s.q = v.hd_q; s.sx = v.hd_s; s.out_f = v.dn; s.out_stride = d.E;
+    return s;
+}
+SpRowsSeg seg_routed_up(const SpDims &d, const SpLayerDev &L, int M, const signed char *q, const float *sx, const BView &v) {
+    SpRowsSeg s{};
+    s.codes = s.ucodes = L.gu_codes; s.bs = s.ubs = L.gu_bs; s.rows_per_group = 2LL * d.FFE; s.up_off = d.FFE; s.in = d.E; s.rows = d.FFE; s.groups = d.NE;
+    s.M = M; s.act_div = 1; s.q = q; s.sx = sx; s.out_q = v.h_q; s.out_s = v.h_s;
+    return s;
+}
+SpRowsSeg seg_routed_down(const SpDims &d, const SpLayerDev &L, int M, const BView &v, float *out) {
+    SpRowsSeg s{};
+    s.codes = L.dn_codes; s.bs = L.dn_bs; s.rows_per_group = d.E; s.in = d.FFE; s.rows = d.E; s.groups = d.NE; s.M = M; s.act_div = 1;
+    s.q = v.h_q; s.sx = v.h_s; s.out_f = out; s.out_stride = d.E;
+    return s;
 }
 
 /* ---------------------------------------------------------------- K7: ordered combine + recombine (CF:6071-6077, 9014-9019) */
@@ -822,28 +557,37 @@ cudaError_t run_layer(const SpDims &d, const SpLayerDev &L, int M, const float *
         k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
         return cudaGetLastError();
     }
+    if (FA) {
+        /* gate|up of the shared and the routed experts, quantised as it leaves (CF:8348-8356, 8733-8737, 8958-8959), then down (CF:8358, 8739-8742, 8961) */
+        SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v.in_s, v)};
+        up[1].count = v.count; up[1].list = v.list; up[1].list_stride = M; up[1].act_div = NU;
+        cudaError_t e = sp_rows_launch(up, 2, true, status, st, nl);
+        if (e != cudaSuccess) return e;
+        SpRowsSeg down[2] = {seg_shared_down(d, L, M, v), seg_routed_down(d, L, M, v, v.eo)};
+        down[1].count = v.count; down[1].list = v.list; down[1].list_stride = M;
+        e = sp_rows_launch(down, 2, false, status, st, nl);
+        if (e != cudaSuccess) return e;
+        k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
+        return cudaGetLastError();
+    }
     GroupArgs g{};
     g.M = M;
     /* shared expert gate/up -> hd (CF:8348-8356) */
     g.codes = L.sg_codes; g.bs = L.sg_bs; g.ucodes = L.su_codes; g.ubs = L.su_bs; g.rows_per_group = 0; g.count = nullptr; g.list = nullptr;
-    g.in = E; g.rows = FFS; g.up_off = 0; g.act_div = 1; g.q = v.nx_q; g.sx = v.nx_s; g.corr = v.nx_c; g.xf = v.nx_f; g.out = v.hd; g.out_stride = FFS;
-    launch_rows<FA, true>(g, 1, st, nl);
+    g.in = E; g.rows = FFS; g.up_off = 0; g.act_div = 1; g.xf = v.nx_f; g.out = v.hd; g.out_stride = FFS;
+    launch_rows<true>(g, 1, st, nl);
     /* routed gate|up -> h (CF:8733-8737, 8958-8959) */
     g.codes = L.gu_codes; g.bs = L.gu_bs; g.ucodes = nullptr; g.ubs = nullptr; g.rows_per_group = 2LL * FFE; g.count = v.count; g.list = v.list; g.list_stride = M;
-    g.in = E; g.rows = FFE; g.up_off = FFE; g.act_div = NU; g.q = v.in_q; g.sx = v.in_s; g.corr = v.in_c; g.xf = v.in_f; g.out = v.h; g.out_stride = FFE;
-    launch_rows<FA, true>(g, NE, st, nl);
-    if (FA) {
-        k_b_quant_rows<<<M, 256, 0, st>>>(v.hd, FFS, v.hd_q, v.hd_s, v.hd_c); (*nl)++;
-        k_b_quant_rows<<<M * NU, 256, 0, st>>>(v.h, FFE, v.h_q, v.h_s, v.h_c); (*nl)++;
-    }
+    g.in = E; g.rows = FFE; g.up_off = FFE; g.act_div = NU; g.xf = v.in_f; g.out = v.h; g.out_stride = FFE;
+    launch_rows<true>(g, NE, st, nl);
     /* shared down -> dn (CF:8358) */
     g.codes = L.sd_codes; g.bs = L.sd_bs; g.rows_per_group = 0; g.count = nullptr; g.list = nullptr;
-    g.in = FFS; g.rows = E; g.act_div = 1; g.q = v.hd_q; g.sx = v.hd_s; g.corr = v.hd_c; g.xf = v.hd; g.out = v.dn; g.out_stride = E;
-    launch_rows<FA, false>(g, 1, st, nl);
+    g.in = FFS; g.rows = E; g.act_div = 1; g.xf = v.hd; g.out = v.dn; g.out_stride = E;
+    launch_rows<false>(g, 1, st, nl);
     /* routed down -> eo (CF:8739-8742, 8961) */
     g.codes = L.dn_codes; g.bs = L.dn_bs; g.rows_per_group = E; g.count = v.count; g.list = v.list; g.list_stride = M;
-    g.in = FFE; g.rows = E; g.act_div = 1; g.q = v.h_q; g.sx = v.h_s; g.corr = v.h_c; g.xf = v.h; g.out = v.eo; g.out_stride = E;
-    launch_rows<FA, false>(g, NE, st, nl);
+    g.in = FFE; g.rows = E; g.act_div = 1; g.xf = v.h; g.out = v.eo; g.out_stride = E;
+    launch_rows<false>(g, NE, st, nl);
     k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
     return cudaGetLastError();
 }
@@ -996,18 +740,23 @@ template <bool FA>
 cudaError_t ep_shared(const SpDims &d, const SpLayerDev &L, int M, BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl, int phase) {
     const int E = d.E, FFS = d.FFS;
     if (!FA && tc) return sp_tc_shared_expert(tc, d, L, M, v.nx_f, v.dn, status, st, nl, phase);
+    if (FA) {
+        const SpRowsSeg up = seg_shared_up(d, L, M, v), down = seg_shared_down(d, L, M, v);
+        cudaError_t e = phase != 2 ? sp_rows_launch(&up, 1, true, status, st, nl) : cudaSuccess;
+        if (e == cudaSuccess && phase != 1) e = sp_rows_launch(&down, 1, false, status, st, nl);
+        return e;
+    }
     GroupArgs g{};
     g.M = M; g.act_div = 1;
     if (phase != 2) {
         g.codes = L.sg_codes; g.bs = L.sg_bs; g.ucodes = L.su_codes; g.ubs = L.su_bs;
-        g.in = E; g.rows = FFS; g.q = v.nx_q; g.sx = v.nx_s; g.corr = v.nx_c; g.xf = v.nx_f; g.out = v.hd; g.out_stride = FFS;
-        launch_rows<FA, true>(g, 1, st, nl);
-        if (FA) { k_b_quant_rows<<<M, 256, 0, st>>>(v.hd, FFS, v.hd_q, v.hd_s, v.hd_c); (*nl)++; }
+        g.in = E; g.rows = FFS; g.xf = v.nx_f; g.out = v.hd; g.out_stride = FFS;
+        launch_rows<true>(g, 1, st, nl);
     }
     if (phase != 1) {
         g.codes = L.sd_codes; g.bs = L.sd_bs; g.ucodes = nullptr; g.ubs = nullptr;
-        g.in = FFS; g.rows = E; g.q = v.hd_q; g.sx = v.hd_s; g.corr = v.hd_c; g.xf = v.hd; g.out = v.dn; g.out_stride = E;
-        launch_rows<FA, false>(g, 1, st, nl);
+        g.in = FFS; g.rows = E; g.xf = v.hd; g.out = v.dn; g.out_stride = E;
+        launch_rows<false>(g, 1, st, nl);
     }
     return cudaGetLastError();
 }
@@ -1042,16 +791,21 @@ cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float 
     const int E = d.E, NE = d.NE, FFE = d.FFE;
     if (R == 0) return cudaSuccess;
     if (!FA && tc) return sp_tc_routed(tc, d, L, R, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
-    if (FA) { k_b_quant_rows<<<in_index ? n_in : R, 256, 0, st>>>(rows_in, E, v.ep_q, v.ep_s, v.ep_c); (*nl)++; }
+    if (FA) {
+        k_b_quant_rows<<<in_index ? n_in : R, 256, 0, st>>>(rows_in, E, v.ep_q, v.ep_s); (*nl)++;
+        SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v.ep_s, v), down = seg_routed_down(d, L, R, v, rows_out);
+        up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */
+        const cudaError_t e = sp_rows_launch(&up, 1, true, status, st, nl);
+        return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, status, st, nl);
+    }
     GroupArgs g{};
     g.M = R; g.offset = offsets; g.index = row_index; g.act_index = in_index;
     g.codes = L.gu_codes; g.bs = L.gu_bs; g.rows_per_group = 2LL * FFE;
-    g.in = E; g.rows = FFE; g.up_off = FFE; g.act_div = 1; g.q = v.ep_q; g.sx = v.ep_s; g.corr = v.ep_c; g.xf = rows_in; g.out = v.h; g.out_stride = FFE;
-    launch_rows<FA, true>(g, NE, st, nl);
-    if (FA) { k_b_quant_rows<<<R, 256, 0, st>>>(v.h, FFE, v.h_q, v.h_s, v.h_c); (*nl)++; }
+    g.in = E; g.rows = FFE; g.up_off = FFE; g.act_div = 1; g.xf = rows_in; g.out = v.h; g.out_stride = FFE;
+    launch_rows<true>(g, NE, st, nl);
     g.codes = L.dn_codes; g.bs = L.dn_bs; g.rows_per_group = E; g.act_index = nullptr;          /* h has one row per pair */
-    g.in = FFE; g.rows = E; g.q = v.h_q; g.sx = v.h_s; g.corr = v.h_c; g.xf = v.h; g.out = rows_out; g.out_stride = E;
-    launch_rows<FA, false>(g, NE, st, nl);
+    g.in = FFE; g.rows = E; g.xf = v.h; g.out = rows_out; g.out_stride = E;
+    launch_rows<false>(g, NE, st, nl);
     return cudaGetLastError();
 }
 
@@ -1123,7 +877,7 @@ cudaError_t sp_batched_alloc(const SpDims &d, int max_tokens, int max_rows, SpBa
     s->max_rows = max_rows > max_tokens * d.NU ? max_rows : max_tokens * d.NU;
     s->bytes = blayout(d, max_tokens, s->max_rows, [](int, size_t) {});
     s->tc = nullptr;
-    cudaError_t e = mma_rows_prepare();
+    cudaError_t e = sp_rows_prepare();
     if (e != cudaSuccess) return e;
     e = cudaMalloc(&s->base, s->bytes);
     if (e != cudaSuccess) { s->base = nullptr; return e; }

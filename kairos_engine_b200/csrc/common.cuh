@@ -192,8 +192,9 @@ __device__ __forceinline__ void quant_block16_store(const float (&v)[16], int4 *
 
 /* Same quantiser, one element per thread: the 16 lanes of a half-warp hold one block. Every
  * lane of the warp must call (shuffles use the full mask); `valid` gates only the stores.
- * dst/sx/corr point at the block's own slots. */
-__device__ __forceinline__ void quant_elem16(float v, bool valid, signed char *dst_block, float *sx_b, int *corr_b) {
+ * dst/sx point at the block's own slots. (No offset correction: the row kernels that read these
+ * blocks multiply signed codes.) */
+__device__ __forceinline__ void quant_elem16(float v, bool valid, signed char *dst_block, float *sx_b) {
     const int k = threadIdx.x & 15;
     float m = fabsf(v);
 #pragma unroll
@@ -202,13 +203,10 @@ __device__ __forceinline__ void quant_elem16(float v, bool valid, signed char *d
     const float inv = __fdiv_rn(1.0f, scale);
     int q = __float2int_rn(__fmul_rn(v, inv));
     q = q > 127 ? 127 : q; q = q < -127 ? -127 : q;
-    int s = q;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (valid) {
         const int r = k & 7;
         dst_block[(k & 8) + ((r & 1) << 2) + (r >> 1)] = (signed char)q;
-        if (k == 0) { *sx_b = scale; *corr_b = 8 * s; }
+        if (k == 0) *sx_b = scale;
     }
 }
 

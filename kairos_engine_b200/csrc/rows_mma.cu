@@ -1,0 +1,410 @@
+/* rows_mma.cu — Q4B rows x the int8 activations of a list of tokens, in the decode arithmetic, for M > 1.
+ *
+ * The sums are those of k_gemv_q4b_dp4a_v2 (CF:1688-1713 of src/backends/cuda/cuda_forward.cu), bit for bit: for every
+ * (row, token) the 32-weight chunk c adds fma(scale, fma(a0, s0, a1 * s1), acc) to slot c % 32, chunks in ascending order
+ * (a0, a1: exact integer dots of the chunk's two 16-blocks), and the 32 slots are added in the pairing of the shuffle-down
+ * tree. What is free is who does it when:
+ *   - One mma.sync m16n8k32 (s8 x s8) takes 16 weight rows x one chunk x four tokens: column 2t + h of B is token t
+ *     restricted to half h, so lane (g, q) of the warp finds both block sums of rows g and g + 8 for token q in its C
+ *     registers, for every chunk. It adds its slots by itself, in the order that completes subtrees (no shuffles, at most
+ *     four partial sums waiting). Half of the MMA multiplies zeros; the MMA pipe has room for that (2.6 cycles per
+ *     instruction and scheduler), and the epilogue's 10 fp32 instructions serve four tokens at a time.
+ *   - A operand: code nibbles moved to the top of a byte (16 * code as s8); C starts at 0x4B400000, so that one fma turns
+ *     the s32 result into the float a conversion would give.
+ *   - Gate|up: a 16-row MMA tile is 8 gate rows and the 8 up rows of the same outputs. A unit is 16 outputs = one
+ *     quantisation block: it leaves the kernel as int8 codes and a scale, ready for the down rows.
+ *
+ * Work is cut into units of ~50 KB of weights x up to 16 tokens. One CTA per SM; a producer warp asks the copy engine for
+ * the units' rows (cp.async.bulk, a ring of stages), two teams of eight warps consume them alternately, and fetch the
+ * activations of their next four tokens while they multiply the current four. So the weight stream does not stop between
+ * units, and experts nobody chose cost nothing. Row copies are padded in shared memory where a row's length would put
+ * eight rows on the same banks.
+ */
+#include "rows_mma.cuh"
+#include <cstring>
+
+namespace {
+
+constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kUnitTok = 16, kMaxStages = 4, kMaxTeams = 2;
+constexpr int kUnits = 128;                        /* unit descriptors of a CTA kept in shared memory */
+constexpr int kMagic = 0x4B400000;
+constexpr unsigned kSpin = 1u << 15, kWaitNs = 20000;
+
+struct RowsArgs {
+    SpRowsSeg seg[2]; int nseg;
+    int stages, teams;
+    unsigned stage_bytes, act_bytes;               /* one stage; one buffer of four tokens */
+    int *status;
+};
+
+__host__ __device__ inline int wide_tiles(int in) { return in <= 1024 ? 8 : 2; }      /* plain rows: 16-row tiles of a unit */
+__host__ __device__ inline int row_stride(int in, bool pair) {                         /* bytes between rows in shared memory */
+    const int rb = in / 2;
+    return pair ? (rb % 32 == 0 ? rb + 16 : rb) : (rb % 64 == 0 ? rb + 16 : rb);       /* plain: two-way conflicts are left (a row is copied with its neighbours) */
+}
+__host__ __device__ inline int act_stride(int in) { return in + ((32 - in % 128 + 128) % 128); }        /* = 32 mod 128: four tokens on four bank groups */
+__host__ __device__ inline int sx_stride(int in) { return in / 16 + ((8 - (in / 16) % 32 + 32) % 32); }   /* floats, = 8 mod 32 */
+__host__ __device__ inline unsigned up128(unsigned v) { return (v + 127u) & ~127u; }
+__host__ __device__ inline unsigned seg_stage_bytes(const SpRowsSeg &s, bool pair) {
+    const unsigned nr = pair ? 32 : 16 * wide_tiles(s.in);
+    return up128(nr * (unsigned)row_stride(s.in, pair)) + up128(nr * (unsigned)(s.in / 16));
+}
+__host__ __device__ inline unsigned seg_act_bytes(const SpRowsSeg &s) { return up128(kTok * (unsigned)act_stride(s.in)) + up128(kTok * 4u * (unsigned)sx_stride(s.in)); }
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned mbar_try(uint32_t bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity, volatile int *abort_flag) {
+    if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
+    for (unsigned i = 0; i < kSpin; i++) {
+        unsigned ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitNs) : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp8(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads) : "memory"); }
+
+/* C = A x B + {magic, ...} (a pure function of its operands: the compiler may move it) */
+__device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
+}
+__device__ __forceinline__ float magic_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }     /* bits of magic + 16 S -> float(S) */
+
+/* ---------------------------------------------------------------- units of work */
+struct Unit { int seg, grp, tile, t0, nt, pad[3]; };        /* weight tile `tile` of group grp x its tokens [t0, t0 + nt) */
+struct Plan {                                               /* in shared memory: first unit of every group, per segment */
+    const int *start[2]; int total[2];
+};
+__device__ __forceinline__ int group_first(const SpRowsSeg &s, int g) {
+    if (!s.offset) return 0;
+    const int f = __ldg(s.offset + g);                      /* caller-supplied ranges: kept inside the M rows that exist */
+    return f < 0 ? 0 : (f > s.M ? s.M : f);
+}
+__device__ __forceinline__ int group_count(const SpRowsSeg &s, int g) {
+    if (s.offset) { int l = __ldg(s.offset + g + 1); l = l > s.M ? s.M : l; const int c = l - group_first(s, g); return c < 0 ? 0 : c; }
+    if (!s.count) return s.M;
+    const int c = __ldg(s.count + g);
+    return c > s.M ? s.M : c;
+}
+template <bool PAIR> __device__ __forceinline__ int seg_tiles(const SpRowsSeg &s) {
+    const int per = PAIR ? 16 : 16 * wide_tiles(s.in);
+    return (s.rows + per - 1) / per;
+}
+template <bool PAIR>
+__device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
+    Unit r{};
+    r.seg = u >= p.total[0] ? 1 : 0;
+    const SpRowsSeg &s = a.seg[r.seg];
+    u -= r.seg ? p.total[0] : 0;
+    const int *st = p.start[r.seg];
+    int lo = 0, hi = s.groups - 1;                          /* the last group that starts at or before u: never an empty one */
+    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (st[mid] <= u) lo = mid; else hi = mid - 1; }
+    r.grp = lo;
+    const int cnt = group_count(s, lo), nr = (cnt + kUnitTok - 1) / kUnitTok, k = u - st[lo];
+    r.tile = k / nr;
+    r.t0 = (k - r.tile * nr) * kUnitTok;
+    r.nt = cnt - r.t0 < kUnitTok ? cnt - r.t0 : kUnitTok;
+    return r;
+}
+
+/* ---------------------------------------------------------------- the dots of one warp: 16 rows x four tokens */
+struct Frag {
+    const unsigned char *w0, *w1;      /* rows g and g + 8 of the tile, at this lane's word */
+    const unsigned char *s0, *s1;      /* their block scales */
+    const unsigned char *b;            /* token g >> 1, this lane's 8 bytes of a chunk */
+    const float *sx;                   /* token q's block scales */
+    bool bvalid;                       /* the lane's k-slots lie in its column's half */
+    int n32;
+};
+/* slots r, r + 4, ..., r + 28 (chunks s + 32 i of each), added as the tree adds them: s and s + 16, then + 8, then + 4 */
+template <int NI>
+__device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
+    auto slot = [&](int j) {
+        float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            const int c = r + 4 * j + 32 * i;
+            if (i + 1 < NI || c < f.n32) {                  /* warp-uniform */
+                const unsigned x0 = *reinterpret_cast<const unsigned *>(f.w0 + 16 * c), x1 = *reinterpret_cast<const unsigned *>(f.w1 + 16 * c);
+                uint2 b = make_uint2(0u, 0u);
+                if (f.bvalid) b = *reinterpret_cast<const uint2 *>(f.b + 32 * c);
+                const float2 s2 = *reinterpret_cast<const float2 *>(f.sx + 2 * c);
+                const float ws0 = h2f(*reinterpret_cast<const unsigned short *>(f.s0 + 2 * c)), ws1 = h2f(*reinterpret_cast<const unsigned short *>(f.s1 + 2 * c));
+                int d[4];
+                mma_s8(d, (x0 << 4) & 0xF0F0F0F0u, (x1 << 4) & 0xF0F0F0F0u, x0 & 0xF0F0F0F0u, x1 & 0xF0F0F0F0u, b.x, b.y, kMagic);
+                acc.x = __fmaf_rn(ws0, __fmaf_rn(magic_to_float(d[0]), s2.x, __fmul_rn(magic_to_float(d[1]), s2.y)), acc.x);
+                acc.y = __fmaf_rn(ws1, __fmaf_rn(magic_to_float(d[2]), s2.x, __fmul_rn(magic_to_float(d[3]), s2.y)), acc.y);
+            }
+        }
+        return acc;
+    };
+    auto add = [](float2 p, float2 q) { return make_float2(p.x + q.x, p.y + q.y); };
+    float2 a = add(slot(0), slot(4)); a = add(a, add(slot(2), slot(6)));
+    float2 b = add(slot(1), slot(5)); b = add(b, add(slot(3), slot(7)));
+    return add(a, b);
+}
+__device__ __forceinline__ float2 class_sum_n(const Frag &f, int r) {
+    if (f.n32 <= 32) return class_sum<1>(f, r);
+    if (f.n32 <= 64) return class_sum<2>(f, r);
+    if (f.n32 <= 96) return class_sum<3>(f, r);
+    return class_sum<4>(f, r);
+}
+
+/* ---------------------------------------------------------------- the kernel */
+template <bool PAIR>
+__global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const __grid_constant__ RowsArgs a) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ unsigned long long bars[2 * kMaxStages];
+    __shared__ int abort_s, items_s[kMaxTeams][2][kTok];
+    __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
+    __shared__ Unit units_s[kUnits];
+    __shared__ int start_s[1 + 1024], total_s[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    volatile int *abort_flag = &abort_s;
+    auto full = [&](int s) { return smem_u32(&bars[s]); };
+    auto empty = [&](int s) { return smem_u32(&bars[kMaxStages + s]); };
+    if (tid == 0) {
+        for (int s = 0; s < a.stages; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(s)) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty(s)), "n"(kTeamWarps) : "memory");
+        }
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    /* first unit of every group: segment 0 has its one entry (or the groups of an only segment), segment 1 the experts */
+    if (warp == 0) {
+        int at = 0;
+        for (int k = 0; k < 2; k++) {
+            int run = 0;
+            if (k < a.nseg) {
+                const SpRowsSeg &s = a.seg[k];
+                const int tiles = seg_tiles<PAIR>(s);
+                for (int g0 = 0; g0 < s.groups; g0 += 32) {
+                    const int g = g0 + lane;
+                    const int n = g < s.groups ? tiles * ((group_count(s, g) + kUnitTok - 1) / kUnitTok) : 0;
+                    int v = n;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t; }
+                    if (g < s.groups) start_s[at + g] = run + v - n;
+                    run += __shfl_sync(0xffffffffu, v, 31);
+                }
+                at += s.groups;
+            }
+            if (lane == 0) total_s[k] = run;
+        }
+    }
+    __syncthreads();
+    Plan plan;
+    plan.start[0] = start_s; plan.start[1] = start_s + a.seg[0].groups; plan.total[0] = total_s[0]; plan.total[1] = total_s[1];
+    const int total = plan.total[0] + plan.total[1], G = gridDim.x;
+    for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = locate<PAIR>(a, plan, blockIdx.x + i * G);
+    __syncthreads();
+    const int mine = total > (int)blockIdx.x ? (total - blockIdx.x + G - 1) / G : 0;
+    auto unit = [&](int i) { return i < kUnits ? units_s[i] : locate<PAIR>(a, plan, blockIdx.x + i * G); };
+    const uint32_t sbase = smem_u32(sm);
+    bool failed = false;
+
+    if (warp == a.teams * kTeamWarps) {
+        /* ---------------- producer: the rows of every unit, one lane per row copy */
+        for (int i = 0, s = 0, ph = 0; i < mine; i++) {
+            const Unit u = unit(i);
+            const SpRowsSeg &sg = a.seg[u.seg];
+            if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
+            const unsigned rb = (unsigned)sg.in / 2, sb = (unsigned)sg.in / 16, stride = (unsigned)row_stride(sg.in, PAIR);
+            const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, bar = full(s);
+            const size_t row0 = (size_t)((long long)u.grp * sg.rows_per_group);
+            if (PAIR) {
+                const int j0 = u.tile * 16, up = lane >> 4, col = lane & 15;
+                const uint32_t sdst = dst + up128(32 * stride);
+                if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(32 * (rb + sb)) : "memory");
+                __syncwarp();
+                const size_t row = row0 + j0 + (up ? sg.up_off : 0);
+                bulk_g2s(dst + ((col >> 3) * 16 + up * 8 + (col & 7)) * stride, (up ? sg.ucodes : sg.codes) + (row + col) * rb, rb, bar);
+                if (col == 0) bulk_g2s(sdst + up * 16 * sb, reinterpret_cast<const unsigned char *>(up ? sg.ubs : sg.bs) + row * sb, 16 * sb, bar);
+            } else {
+                const int per = 16 * wide_tiles(sg.in), r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
+                const uint32_t sdst = dst + up128(per * stride);
+                if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(nr * (rb + sb)) : "memory");
+                __syncwarp();
+                const unsigned char *src = sg.codes + (row0 + r0) * rb;
+                if (stride == rb) { if (lane == 0) bulk_g2s(dst, src, nr * rb, bar); }
+                else for (int r = lane; r < nr; r += 32) bulk_g2s(dst + r * stride, src + (size_t)r * rb, rb, bar);
+                if (lane == 0) bulk_g2s(sdst, reinterpret_cast<const unsigned char *>(sg.bs) + (row0 + r0) * sb, nr * sb, bar);
+            }
+            if (++s == a.stages) { s = 0; ph ^= 1; }
+        }
+    } else {
+        /* ---------------- a team: units team, team + teams, ... of this CTA, four tokens at a time */
+        const int team = warp / kTeamWarps, tw = warp % kTeamWarps, gq = lane >> 2, q = lane & 3;
+        const uint32_t abase = sbase + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
+        const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
+        /* a position in the team's sequence of (unit, four tokens) */
+        struct Pos { int i, b; Unit u; };
+        auto first_pos = [&]() { Pos p; p.i = team; p.b = 0; if (p.i < mine) p.u = unit(p.i); return p; };
+        auto next_pos = [&](Pos p) {
+            if (p.i >= mine) return p;
+            if ((p.b + 1) * kTok < p.u.nt) { p.b++; return p; }
+            p.i += a.teams; p.b = 0;
+            if (p.i < mine) p.u = unit(p.i);
+            return p;
+        };
+        /* the item and activation row of this warp's token (two warps fetch a token) at a position */
+        const int tk = tw >> 1;
+        auto look_up = [&](const Pos &p, int &item, int &arow) {
+            item = -1; arow = 0;
+            if (p.i >= mine || p.b * kTok + tk >= p.u.nt) return;
+            const SpRowsSeg &s = a.seg[p.u.seg];
+            const int at = p.u.t0 + p.b * kTok + tk;
+            if (s.offset) {
+                const int pos = group_first(s, p.u.grp) + at;
+                item = s.index ? __ldg(s.index + pos) : pos;
+                arow = s.act_index ? __ldg(s.act_index + pos) : item / s.act_div;
+            } else {
+                item = s.list ? __ldg(s.list + (size_t)p.u.grp * s.list_stride + at) : at;
+                arow = item / s.act_div;
+            }
+        };
+        auto fetch = [&](const Pos &p, int buf, int item, int arow) {       /* that token's codes and scales into buffer `buf` */
+            if (item >= 0) {
+                const SpRowsSeg &s = a.seg[p.u.seg];
+                const int nq = s.in / 16, ast = act_stride(s.in), sst = sx_stride(s.in), hw = tw & 1;
+                const uint32_t qd = abase + buf * a.act_bytes + tk * ast, sd = abase + buf * a.act_bytes + up128(kTok * ast) + 4u * tk * sst;
+                const signed char *qs = s.q + (size_t)arow * s.in;
+                const float *ss = s.sx + (size_t)arow * nq;
+                for (int k = lane + 32 * hw; k < nq; k += 64) cp16(qd + 16 * k, qs + 16 * k);
+                if ((nq & 3) == 0) { for (int k = lane + 32 * hw; k < (nq >> 2); k += 64) cp16(sd + 16 * k, ss + 4 * k); }
+                else { for (int k = lane + 32 * hw; k < (nq >> 1); k += 64) cp8(sd + 8 * k, ss + 2 * k); }
+            }
+            if ((tw & 1) == 0 && lane == 0) items_s[team][buf][tk] = item;
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        Pos cur = first_pos();
+        int item, arow, s = team % a.stages, ph = (team / a.stages) & 1;
+        look_up(cur, item, arow);
+        fetch(cur, 0, item, arow);
+        Pos nxt = next_pos(cur);
+        look_up(nxt, item, arow);
+        for (int n = 0; cur.i < mine; n++) {
+            const int buf = n & 1;
+            const SpRowsSeg &sg = a.seg[cur.u.seg];
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            team_sync(team);                                /* the four tokens are there, and nobody reads the other buffer any more */
+            fetch(nxt, buf ^ 1, item, arow);
+            Pos nn = next_pos(nxt);
+            look_up(nn, item, arow);                        /* in flight while this position is computed */
+            if (cur.b == 0 && !mbar_wait(full(s), ph, abort_flag)) failed = true;
+            const unsigned stride = (unsigned)row_stride(sg.in, PAIR), sb = (unsigned)sg.in / 16;
+            const int mt_n = PAIR ? 2 : wide_tiles(sg.in);
+            const int mt = mt_n == 8 ? tw : tw >> 2;
+            const unsigned char *codes = sm + (unsigned)s * a.stage_bytes, *scales = codes + up128(16 * mt_n * stride);
+            const unsigned char *act = aptr + buf * a.act_bytes;
+            Frag f;
+            f.w0 = codes + (mt * 16 + gq) * stride + 4 * q; f.w1 = f.w0 + 8 * stride;
+            if (PAIR) { f.s0 = scales + (mt * 8 + gq) * sb; f.s1 = f.s0 + 16 * sb; }        /* gate rows, then the up rows */
+            else { f.s0 = scales + (mt * 16 + gq) * sb; f.s1 = f.s0 + 8 * sb; }
+            f.bvalid = (q >> 1) == (gq & 1);
+            f.b = act + (gq >> 1) * act_stride(sg.in) + 8 * q;
+            f.sx = reinterpret_cast<const float *>(act + up128(kTok * act_stride(sg.in))) + q * sx_stride(sg.in);
+            f.n32 = sg.in >> 5;
+            const bool last = (cur.b + 1) * kTok >= cur.u.nt;
+            const int r0 = cur.u.tile * 16 * mt_n;
+            if (!PAIR && mt_n == 8) {
+                if (r0 + mt * 16 < sg.rows) {
+                    float2 v = make_float2(0.0f, 0.0f), o = v;
+#pragma unroll 1
+                    for (int k = 0; k < 4; k++) {           /* classes 0, 2, 1, 3: (0 + 2) + (1 + 3) */
+                        const float2 c = class_sum<1>(f, k == 1 ? 2 : k == 2 ? 1 : k);
+                        if (k == 0 || k == 2) o = c;
+                        else { o.x += c.x; o.y += c.y; if (k == 1) v = o; else { v.x += o.x; v.y += o.y; } }
+                    }
+                    const int it = items_s[team][buf][q];
+                    if (it >= 0) {
+                        float *out = sg.out_f + (size_t)it * sg.out_stride + r0 + mt * 16 + gq;
+                        out[0] = v.x; out[8] = v.y;
+                    }
+                }
+                if (last) { __syncwarp(); if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(empty(s)) : "memory"); }
+            } else {
+                float *part = part_s[team][buf];
+                if (PAIR || r0 + mt * 16 < sg.rows) {
+                    const float2 v = class_sum_n(f, tw & 3);
+                    float *p = part + (((tw & 3) * 2 + mt) * 16 + gq) * kTok + q;
+                    p[0] = v.x; p[8 * kTok] = v.y;
+                }
+                if (last) { __syncwarp(); if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(empty(s)) : "memory"); }
+                team_sync(team);
+                auto total_of = [&](int m, int row, int t) {                /* the last two levels of the tree */
+                    const float *p = part + (m * 16 + row) * kTok + t;
+                    return (p[0] + p[2 * 2 * 16 * kTok]) + (p[2 * 16 * kTok] + p[3 * 2 * 16 * kTok]);
+                };
+                if (PAIR) {
+                    const int w0 = 2 * (n & 3);             /* two warps finish, other ones each time */
+                    if (tw == w0 || tw == w0 + 1) {
+                        const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
+                        const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
+                        const int it = items_s[team][buf][t];
+                        const size_t o = (size_t)(it < 0 ? 0 : it) * sg.rows + r0 / 2;
+                        quant_elem16(h, it >= 0, sg.out_q + o, sg.out_s + o / 16);
+                    }
+                } else {
+                    const int w0 = 4 * (n & 1), t = tw - w0;
+                    if (t >= 0 && t < 4) {
+                        const int it = items_s[team][buf][t];
+                        if (it >= 0 && r0 + lane < sg.rows) sg.out_f[(size_t)it * sg.out_stride + r0 + lane] = total_of(lane >> 4, lane & 15, t);
+                    }
+                }
+            }
+            if (last) { s += a.teams; while (s >= a.stages) { s -= a.stages; ph ^= 1; } }
+            cur = nxt; nxt = nn;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    if (failed && lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
+}
+
+constexpr size_t kSmemLimit = 227 * 1024 - 17 * 1024;      /* dynamic part: the static arrays of the kernel take 16.3 KB */
+
+}  // namespace
+
+cudaError_t sp_rows_prepare() {
+    cudaError_t e = cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) : e;
+}
+
+cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *status, cudaStream_t st, int *nl) {
+    RowsArgs a{};
+    a.nseg = nseg; a.status = status;
+    for (int i = 0; i < nseg; i++) {
+        a.seg[i] = seg[i];
+        const unsigned sb = seg_stage_bytes(seg[i], pair), ab = seg_act_bytes(seg[i]);
+        a.stage_bytes = sb > a.stage_bytes ? sb : a.stage_bytes; a.act_bytes = ab > a.act_bytes ? ab : a.act_bytes;
+    }
+    /* two teams with three stages where they fit (one being filled while two are used), else one team with two */
+    a.teams = (size_t)3 * a.stage_bytes + 4 * (size_t)a.act_bytes <= kSmemLimit ? 2 : 1;
+    const size_t acts = (size_t)a.teams * 2 * a.act_bytes;
+    a.stages = (int)((kSmemLimit - acts) / a.stage_bytes);
+    if (a.stages > kMaxStages) a.stages = kMaxStages;
+    if (a.stages < 1) return cudaErrorInvalidValue;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32);
+    const size_t smem = acts + (size_t)a.stages * a.stage_bytes;
+    if (pair) k_rows<true><<<(unsigned)sms, threads, smem, st>>>(a); else k_rows<false><<<(unsigned)sms, threads, smem, st>>>(a);
+    (*nl)++;
+    return cudaGetLastError();
+}
