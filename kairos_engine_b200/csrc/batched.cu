@@ -42,9 +42,9 @@ size_t blayout(const SpDims &d, int Mx, int Rx, F place) {
     take(4 * M * FFS); take(4 * M * E); take(4 * R * FFE); take(4 * M * NU * E);                     /* hd dn h eo */
     take(4 * M * E); take(4 * M * E);                                                               /* xa xb */
     take(M * E); take(M * E); take(M * FFS); take(R * FFE);                                          /* q */
-    take(4 * M * (E / 16)); take(4 * M * (E / 16)); take(4 * M * (FFS / 16)); take(4 * R * (FFE / 16));        /* s */
+    take(4 * M * sp_sx_row(d.E)); take(4 * M * sp_sx_row(d.E)); take(4 * M * sp_sx_row(d.FFS)); take(4 * R * sp_sx_row(d.FFE));        /* s */
     take(4 * M * NU); take(4 * NE * kSlices); take(4 * NE * M);                                     /* sel_asc count list */
-    take(R * E); take(4 * R * (E / 16));                                                            /* ep_q ep_s */
+    take(R * E); take(4 * R * sp_sx_row(d.E));                                                        /* ep_q ep_s */
     take(4 * M * NU); take(4 * (NE + 1) * kSlices);                                                 /* pairpos ep_off */
     return o;
 }
@@ -70,7 +70,7 @@ BView bview_slice(const SpDims &d, const SpBatchedScratch *s, int t0, int slice)
     const size_t E = d.E, NE = d.NE, NU = d.NU, FFS = d.FFS, t = (size_t)t0;
     v.rin += t * E; v.nx_f += t * E; v.in_f += t * E; v.logits += t * NE; v.cw += t * NU; v.hd += t * FFS; v.dn += t * E; v.eo += t * NU * E;
     v.nx_q += t * E; v.in_q += t * E; v.hd_q += t * FFS;
-    v.nx_s += t * (E / 16); v.in_s += t * (E / 16); v.hd_s += t * (FFS / 16);
+    v.nx_s += t * sp_sx_row(d.E); v.in_s += t * sp_sx_row(d.E); v.hd_s += t * sp_sx_row(d.FFS);
     v.sel_asc += t * NU; v.pairpos += t * NU; v.list += t * NE;
     v.count += (size_t)slice * NE; v.ep_off += (size_t)slice * (NE + 1);
     return v;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(256) k_b_prep(SpDims d, SpLayerDev L, const fl
 #pragma unroll
         for (int k = 0; k < kPrepK; k++) if (256 * k < E) { const double a = xv[k]; if (tid + 256 * k < E) ss += a * a; }
         const float scale = rms_scale_from(block_sum256(ss, sh), E, d.eps);
-        const size_t b16 = (size_t)t * (E / 16), row = (size_t)t * E;
+        const size_t b16 = (size_t)t * sp_sx_row(E), row = (size_t)t * E;
 #pragma unroll
         for (int k = 0; k < kPrepK; k++) {
             if (256 * k < E) {                                  /* block-uniform: every lane of a warp reaches the shuffles */
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) k_b_prep(SpDims d, SpLayerDev L, const fl
     }
     const float scale = rms_scale_from(sumsq256(xt, E, sh), E, d.eps);
     if (FA) {
-        const size_t b16 = (size_t)t * (E / 16);
+        const size_t b16 = (size_t)t * sp_sx_row(E);
         quant_row(E, v.nx_q + (size_t)t * E, v.nx_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.ffn_norm + i)); });
         quant_row(E, v.in_q + (size_t)t * E, v.in_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i)); });
         if (rows_f)                                             /* the routed experts' input as fp32 rows (expert-parallel dispatch) */
@@ -370,11 +370,11 @@ __global__ void __launch_bounds__(256) k_b_quant_rows(const float *x, int n, sig
         for (int k = 0; k < kPrepK; k++)
             if (256 * k < n) {
                 const int i = (int)threadIdx.x + 256 * k, b = i >> 4;
-                quant_elem16(v[k], i < n, q + r * n + 16 * b, sx + r * (n / 16) + b);
+                quant_elem16(v[k], i < n, q + r * n + 16 * b, sx + r * sp_sx_row(n) + b);
             }
         return;
     }
-    quant_row(n, q + r * n, sx + r * (n / 16), [&](int i) { return xr[i]; });
+    quant_row(n, q + r * n, sx + r * sp_sx_row(n), [&](int i) { return xr[i]; });
 }
 
 /* ---------------------------------------------------------------- K4/K6, floating-point flavour without the tensor cores

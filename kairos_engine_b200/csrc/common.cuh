@@ -210,6 +210,9 @@ __device__ __forceinline__ void quant_elem16(float v, bool valid, signed char *d
     }
 }
 
+/* floats between the block-scale rows of quantised activations: [row][n / 16], rows padded to whole 16-byte pieces */
+__host__ __device__ __forceinline__ int sp_sx_row(int n) { return (n / 16 + 3) & ~3; }
+
 /* ---------------------------------------------------------------- block-wide f64 sum of squares (CF:497-514)
  * The reference sums in double with 256 strided threads and a halving tree. This keeps the
  * double accumulation and a fixed order (thread-strided partials, warp shuffles, then warps in

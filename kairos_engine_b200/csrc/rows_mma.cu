@@ -14,10 +14,10 @@
  *   - Gate|up: a 16-row MMA tile is 8 gate rows and the 8 up rows of the same outputs. A unit is 16 outputs = one
  *     quantisation block: it leaves the kernel as int8 codes and a scale, ready for the down rows.
  *
- * Work is cut into units of ~50 KB of weights x up to 16 tokens. One CTA per SM; a producer warp asks the copy engine for
- * the units' rows (cp.async.bulk, a ring of stages), two teams of eight warps consume them alternately, and fetch the
- * activations of their next four tokens while they multiply the current four. So the weight stream does not stop between
- * units, and experts nobody chose cost nothing. Row copies are padded in shared memory where a row's length would put
+ * Work is cut into units of ~50 KB of weights x up to 16 tokens. One CTA per SM; one warp asks the copy engine for the
+ * units' rows (cp.async.bulk, a ring of stages), two teams of eight warps consume them alternately, and a warp per team
+ * has the activations of its next four tokens copied while it multiplies the current four. So the weight stream does not
+ * stop between units, and experts nobody chose cost nothing. Row copies are padded in shared memory where a row's length would put
  * eight rows on the same banks.
  */
 #include "rows_mma.cuh"
@@ -30,26 +30,32 @@ constexpr int kUnits = 128;                        /* unit descriptors of a CTA 
 constexpr int kMagic = 0x4B400000;
 constexpr unsigned kSpin = 1u << 15, kWaitNs = 20000;
 
+struct SegGeo {                                    /* what the copies and the dots need of a segment's shape */
+    int tiles, mt_n, n32;                          /* weight tiles per group, 16-row MMA tiles of one, chunks of a row */
+    unsigned rb, sb, stride, scale_off;            /* bytes of a row's codes / scales; row stride and where the scales start in a stage */
+    unsigned ast, sst, sx_off;                     /* bytes between tokens, floats between their scale rows, where those start in a buffer */
+};
 struct RowsArgs {
-    SpRowsSeg seg[2]; int nseg;
+    SpRowsSeg seg[2]; SegGeo geo[2]; int nseg;
     int stages, teams;
     unsigned stage_bytes, act_bytes;               /* one stage; one buffer of four tokens */
     int *status;
 };
 
-__host__ __device__ inline int wide_tiles(int in) { return in <= 1024 ? 8 : 2; }      /* plain rows: 16-row tiles of a unit */
-__host__ __device__ inline int row_stride(int in, bool pair) {                         /* bytes between rows in shared memory */
-    const int rb = in / 2;
-    return pair ? (rb % 32 == 0 ? rb + 16 : rb) : (rb % 64 == 0 ? rb + 16 : rb);       /* plain: two-way conflicts are left (a row is copied with its neighbours) */
+/* shapes in shared memory */
+unsigned up128(unsigned v) { return (v + 127u) & ~127u; }
+SegGeo seg_geo(const SpRowsSeg &s, bool pair) {
+    SegGeo g;
+    g.mt_n = pair ? 2 : (s.in <= 1024 ? 8 : 2);
+    const int per = pair ? 16 : 16 * g.mt_n;                /* output rows of a unit */
+    g.tiles = (s.rows + per - 1) / per; g.n32 = s.in / 32; g.rb = s.in / 2; g.sb = s.in / 16;
+    g.stride = pair ? (g.rb % 32 == 0 ? g.rb + 16 : g.rb) : (g.rb % 64 == 0 ? g.rb + 16 : g.rb);   /* plain: two-way conflicts are left, such rows are copied in one piece */
+    g.scale_off = up128(16 * g.mt_n * g.stride);
+    g.ast = s.in + (32 - s.in % 128 + 128) % 128;           /* = 32 mod 128: four tokens on four bank groups */
+    g.sst = s.in / 16 + (8 - (s.in / 16) % 32 + 32) % 32;   /* = 8 mod 32 */
+    g.sx_off = up128(kTok * g.ast);
+    return g;
 }
-__host__ __device__ inline int act_stride(int in) { return in + ((32 - in % 128 + 128) % 128); }        /* = 32 mod 128: four tokens on four bank groups */
-__host__ __device__ inline int sx_stride(int in) { return in / 16 + ((8 - (in / 16) % 32 + 32) % 32); }   /* floats, = 8 mod 32 */
-__host__ __device__ inline unsigned up128(unsigned v) { return (v + 127u) & ~127u; }
-__host__ __device__ inline unsigned seg_stage_bytes(const SpRowsSeg &s, bool pair) {
-    const unsigned nr = pair ? 32 : 16 * wide_tiles(s.in);
-    return up128(nr * (unsigned)row_stride(s.in, pair)) + up128(nr * (unsigned)(s.in / 16));
-}
-__host__ __device__ inline unsigned seg_act_bytes(const SpRowsSeg &s) { return up128(kTok * (unsigned)act_stride(s.in)) + up128(kTok * 4u * (unsigned)sx_stride(s.in)); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned mbar_try(uint32_t bar, unsigned parity) {
@@ -72,8 +78,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity, volatil
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void cp8(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void expect_tx(uint32_t bar, unsigned bytes) {
+    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void arrive_lane0(uint32_t bar, int lane) {     /* predicated, not branched around */
+    asm volatile("{ .reg .pred p; .reg .b64 st; setp.eq.s32 p, %1, 0; @p mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar), "r"(lane) : "memory");
+}
 __device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads) : "memory"); }
 
 /* C = A x B + {magic, ...} (a pure function of its operands: the compiler may move it) */
@@ -99,11 +109,6 @@ __device__ __forceinline__ int group_count(const SpRowsSeg &s, int g) {
     const int c = __ldg(s.count + g);
     return c > s.M ? s.M : c;
 }
-template <bool PAIR> __device__ __forceinline__ int seg_tiles(const SpRowsSeg &s) {
-    const int per = PAIR ? 16 : 16 * wide_tiles(s.in);
-    return (s.rows + per - 1) / per;
-}
-template <bool PAIR>
 __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     Unit r{};
     r.seg = u >= p.total[0] ? 1 : 0;
@@ -129,11 +134,13 @@ struct Frag {
     bool bvalid;                       /* the lane's k-slots lie in its column's half */
     int n32;
 };
-/* slots r, r + 4, ..., r + 28 (chunks s + 32 i of each), added as the tree adds them: s and s + 16, then + 8, then + 4 */
-template <int NI>
+/* slots r, r + 4, ..., r + 28 (chunks s + 32 i of each), added as the tree adds them: s and s + 16, then + 8, then + 4.
+ * Rows of one chunk per slot may have fewer than 32: slots from 4 * NJ on are known to be empty (NJ even). */
+template <int NI, int NJ = 8>
 __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
     auto slot = [&](int j) {
         float2 acc = make_float2(0.0f, 0.0f);
+        if (j >= NJ) return acc;
 #pragma unroll
         for (int i = 0; i < NI; i++) {
             const int c = r + 4 * j + 32 * i;
@@ -163,38 +170,49 @@ __device__ __forceinline__ float2 class_sum_n(const Frag &f, int r) {
     return class_sum<4>(f, r);
 }
 
-/* ---------------------------------------------------------------- the kernel */
+/* ---------------------------------------------------------------- the kernel
+ * Warps: teams x 8 that multiply, one that copies weights, one per team that copies activations. */
+struct Batch { int seg, tile, flags, item[kTok], pad; };     /* four tokens of a unit; flags: 1 = the unit's first, 2 = its last, 4 = the team is done */
+
 template <bool PAIR>
-__global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const __grid_constant__ RowsArgs a) {
+__global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const __grid_constant__ RowsArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ unsigned long long bars[2 * kMaxStages];
-    __shared__ int abort_s, items_s[kMaxTeams][2][kTok];
+    __shared__ unsigned long long bars[2 * kMaxStages + 4 * kMaxTeams];
+    __shared__ int abort_s;
+    __shared__ Batch batch_s[kMaxTeams][2];
     __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
     __shared__ Unit units_s[kUnits];
     __shared__ int start_s[1 + 1024], total_s[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     volatile int *abort_flag = &abort_s;
-    auto full = [&](int s) { return smem_u32(&bars[s]); };
-    auto empty = [&](int s) { return smem_u32(&bars[kMaxStages + s]); };
+    const uint32_t bar0 = smem_u32(bars);
+    auto full = [&](int s) { return bar0 + 8u * s; };                   /* weight stages */
+    auto empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
+    auto afull = [&](int team, int b) { return bar0 + 8u * (2 * kMaxStages + 4 * team + b); };      /* a team's two buffers of activations */
+    auto aempty = [&](int team, int b) { return bar0 + 8u * (2 * kMaxStages + 4 * team + 2 + b); };
     if (tid == 0) {
         for (int s = 0; s < a.stages; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(s)) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty(s)), "n"(kTeamWarps) : "memory");
         }
+        for (int t = 0; t < a.teams; t++)
+            for (int b = 0; b < 2; b++) {
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(afull(t, b)) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(aempty(t, b)), "n"(kTeamWarps) : "memory");
+            }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    /* first unit of every group: segment 0 has its one entry (or the groups of an only segment), segment 1 the experts */
+    /* first unit of every group, per segment (segment 0 is the only one or has one group) */
     if (warp == 0) {
         int at = 0;
         for (int k = 0; k < 2; k++) {
             int run = 0;
             if (k < a.nseg) {
                 const SpRowsSeg &s = a.seg[k];
-                const int tiles = seg_tiles<PAIR>(s);
                 for (int g0 = 0; g0 < s.groups; g0 += 32) {
                     const int g = g0 + lane;
-                    const int n = g < s.groups ? tiles * ((group_count(s, g) + kUnitTok - 1) / kUnitTok) : 0;
+                    const int n = g < s.groups ? a.geo[k].tiles * ((group_count(s, g) + kUnitTok - 1) / kUnitTok) : 0;
                     int v = n;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t; }
@@ -210,34 +228,33 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const 
     Plan plan;
     plan.start[0] = start_s; plan.start[1] = start_s + a.seg[0].groups; plan.total[0] = total_s[0]; plan.total[1] = total_s[1];
     const int total = plan.total[0] + plan.total[1], G = gridDim.x;
-    for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = locate<PAIR>(a, plan, blockIdx.x + i * G);
+    for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = locate(a, plan, blockIdx.x + i * G);
     __syncthreads();
     const int mine = total > (int)blockIdx.x ? (total - blockIdx.x + G - 1) / G : 0;
-    auto unit = [&](int i) { return i < kUnits ? units_s[i] : locate<PAIR>(a, plan, blockIdx.x + i * G); };
+    auto unit = [&](int i) { return i < kUnits ? units_s[i] : locate(a, plan, blockIdx.x + i * G); };
     const uint32_t sbase = smem_u32(sm);
     bool failed = false;
 
     if (warp == a.teams * kTeamWarps) {
-        /* ---------------- producer: the rows of every unit, one lane per row copy */
+        /* ---------------- weights: the rows of every unit, one lane per row copy */
         for (int i = 0, s = 0, ph = 0; i < mine; i++) {
             const Unit u = unit(i);
             const SpRowsSeg &sg = a.seg[u.seg];
+            const SegGeo &ge = a.geo[u.seg];
             if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-            const unsigned rb = (unsigned)sg.in / 2, sb = (unsigned)sg.in / 16, stride = (unsigned)row_stride(sg.in, PAIR);
-            const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, bar = full(s);
+            const unsigned rb = ge.rb, sb = ge.sb, stride = ge.stride;
+            const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(s);
             const size_t row0 = (size_t)((long long)u.grp * sg.rows_per_group);
             if (PAIR) {
                 const int j0 = u.tile * 16, up = lane >> 4, col = lane & 15;
-                const uint32_t sdst = dst + up128(32 * stride);
-                if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(32 * (rb + sb)) : "memory");
+                if (lane == 0) expect_tx(bar, 32 * (rb + sb));
                 __syncwarp();
                 const size_t row = row0 + j0 + (up ? sg.up_off : 0);
                 bulk_g2s(dst + ((col >> 3) * 16 + up * 8 + (col & 7)) * stride, (up ? sg.ucodes : sg.codes) + (row + col) * rb, rb, bar);
                 if (col == 0) bulk_g2s(sdst + up * 16 * sb, reinterpret_cast<const unsigned char *>(up ? sg.ubs : sg.bs) + row * sb, 16 * sb, bar);
             } else {
-                const int per = 16 * wide_tiles(sg.in), r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
-                const uint32_t sdst = dst + up128(per * stride);
-                if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(nr * (rb + sb)) : "memory");
+                const int per = 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
+                if (lane == 0) expect_tx(bar, nr * (rb + sb));
                 __syncwarp();
                 const unsigned char *src = sg.codes + (row0 + r0) * rb;
                 if (stride == rb) { if (lane == 0) bulk_g2s(dst, src, nr * rb, bar); }
@@ -246,97 +263,88 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const 
             }
             if (++s == a.stages) { s = 0; ph ^= 1; }
         }
+    } else if (warp > a.teams * kTeamWarps) {
+        /* ---------------- activations of one team: four tokens ahead of it, one lane per token */
+        const int team = warp - a.teams * kTeamWarps - 1;
+        const uint32_t abase = sbase + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
+        int n = 0;
+        for (int i = team; i < mine && !failed; i += a.teams) {
+            const Unit u = unit(i);
+            const SpRowsSeg &s = a.seg[u.seg];
+            const SegGeo &ge = a.geo[u.seg];
+            const int first = group_first(s, u.grp) + u.t0;
+            for (int b = 0; b < u.nt; b += kTok, n++) {
+                int item = -1, arow = 0;
+                if (lane < kTok && b + lane < u.nt) {
+                    const int at = first + b + lane;
+                    if (s.offset) { item = s.index ? __ldg(s.index + at) : at; arow = s.act_index ? __ldg(s.act_index + at) : item; }
+                    else { item = s.list ? __ldg(s.list + (size_t)u.grp * s.list_stride + at) : at; arow = item; }
+                    if (!s.act_index && s.act_div > 1) arow /= s.act_div;
+                }
+                const int buf = n & 1, have = u.nt - b < kTok ? u.nt - b : kTok;
+                if (!mbar_wait(aempty(team, buf), ((n >> 1) & 1) ^ 1, abort_flag)) { failed = true; break; }
+                Batch *d = &batch_s[team][buf];
+                if (lane < kTok) d->item[lane] = item;
+                if (lane == 0) { d->seg = u.seg; d->tile = u.tile; d->flags = (b == 0 ? 1 : 0) | (b + kTok >= u.nt ? 2 : 0); }
+                __syncwarp();
+                if (lane == 0) expect_tx(afull(team, buf), (unsigned)have * ((unsigned)s.in + 4u * (unsigned)sp_sx_row(s.in)));        /* its arrival also publishes the descriptor */
+                __syncwarp();
+                if (item >= 0) {
+                    const uint32_t qd = abase + buf * a.act_bytes + lane * ge.ast, sd = abase + buf * a.act_bytes + ge.sx_off + 4u * lane * ge.sst;
+                    bulk_g2s(qd, s.q + (size_t)arow * s.in, (unsigned)s.in, afull(team, buf));
+                    bulk_g2s(sd, s.sx + (size_t)arow * sp_sx_row(s.in), 4u * (unsigned)sp_sx_row(s.in), afull(team, buf));
+                }
+            }
+        }
+        if (!failed) {                                      /* one more descriptor: nothing left */
+            const int buf = n & 1;
+            if (!mbar_wait(aempty(team, buf), ((n >> 1) & 1) ^ 1, abort_flag)) failed = true;
+            else if (lane == 0) {
+                batch_s[team][buf].flags = 4;
+                asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(afull(team, buf)) : "memory");
+            }
+        }
     } else {
         /* ---------------- a team: units team, team + teams, ... of this CTA, four tokens at a time */
         const int team = warp / kTeamWarps, tw = warp % kTeamWarps, gq = lane >> 2, q = lane & 3;
-        const uint32_t abase = sbase + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
-        /* a position in the team's sequence of (unit, four tokens) */
-        struct Pos { int i, b; Unit u; };
-        auto first_pos = [&]() { Pos p; p.i = team; p.b = 0; if (p.i < mine) p.u = unit(p.i); return p; };
-        auto next_pos = [&](Pos p) {
-            if (p.i >= mine) return p;
-            if ((p.b + 1) * kTok < p.u.nt) { p.b++; return p; }
-            p.i += a.teams; p.b = 0;
-            if (p.i < mine) p.u = unit(p.i);
-            return p;
-        };
-        /* the item and activation row of this warp's token (two warps fetch a token) at a position */
-        const int tk = tw >> 1;
-        auto look_up = [&](const Pos &p, int &item, int &arow) {
-            item = -1; arow = 0;
-            if (p.i >= mine || p.b * kTok + tk >= p.u.nt) return;
-            const SpRowsSeg &s = a.seg[p.u.seg];
-            const int at = p.u.t0 + p.b * kTok + tk;
-            if (s.offset) {
-                const int pos = group_first(s, p.u.grp) + at;
-                item = s.index ? __ldg(s.index + pos) : pos;
-                arow = s.act_index ? __ldg(s.act_index + pos) : item / s.act_div;
-            } else {
-                item = s.list ? __ldg(s.list + (size_t)p.u.grp * s.list_stride + at) : at;
-                arow = item / s.act_div;
-            }
-        };
-        auto fetch = [&](const Pos &p, int buf, int item, int arow) {       /* that token's codes and scales into buffer `buf` */
-            if (item >= 0) {
-                const SpRowsSeg &s = a.seg[p.u.seg];
-                const int nq = s.in / 16, ast = act_stride(s.in), sst = sx_stride(s.in), hw = tw & 1;
-                const uint32_t qd = abase + buf * a.act_bytes + tk * ast, sd = abase + buf * a.act_bytes + up128(kTok * ast) + 4u * tk * sst;
-                const signed char *qs = s.q + (size_t)arow * s.in;
-                const float *ss = s.sx + (size_t)arow * nq;
-                for (int k = lane + 32 * hw; k < nq; k += 64) cp16(qd + 16 * k, qs + 16 * k);
-                if ((nq & 3) == 0) { for (int k = lane + 32 * hw; k < (nq >> 2); k += 64) cp16(sd + 16 * k, ss + 4 * k); }
-                else { for (int k = lane + 32 * hw; k < (nq >> 1); k += 64) cp8(sd + 8 * k, ss + 2 * k); }
-            }
-            if ((tw & 1) == 0 && lane == 0) items_s[team][buf][tk] = item;
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        Pos cur = first_pos();
-        int item, arow, s = team % a.stages, ph = (team / a.stages) & 1;
-        look_up(cur, item, arow);
-        fetch(cur, 0, item, arow);
-        Pos nxt = next_pos(cur);
-        look_up(nxt, item, arow);
-        for (int n = 0; cur.i < mine; n++) {
+        int s = team % a.stages, ph = (team / a.stages) & 1;
+        Frag f;
+        f.bvalid = (q >> 1) == (gq & 1);
+        for (int n = 0;; n++) {
             const int buf = n & 1;
-            const SpRowsSeg &sg = a.seg[cur.u.seg];
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            team_sync(team);                                /* the four tokens are there, and nobody reads the other buffer any more */
-            fetch(nxt, buf ^ 1, item, arow);
-            Pos nn = next_pos(nxt);
-            look_up(nn, item, arow);                        /* in flight while this position is computed */
-            if (cur.b == 0 && !mbar_wait(full(s), ph, abort_flag)) failed = true;
-            const unsigned stride = (unsigned)row_stride(sg.in, PAIR), sb = (unsigned)sg.in / 16;
-            const int mt_n = PAIR ? 2 : wide_tiles(sg.in);
-            const int mt = mt_n == 8 ? tw : tw >> 2;
-            const unsigned char *codes = sm + (unsigned)s * a.stage_bytes, *scales = codes + up128(16 * mt_n * stride);
-            const unsigned char *act = aptr + buf * a.act_bytes;
-            Frag f;
-            f.w0 = codes + (mt * 16 + gq) * stride + 4 * q; f.w1 = f.w0 + 8 * stride;
-            if (PAIR) { f.s0 = scales + (mt * 8 + gq) * sb; f.s1 = f.s0 + 16 * sb; }        /* gate rows, then the up rows */
-            else { f.s0 = scales + (mt * 16 + gq) * sb; f.s1 = f.s0 + 8 * sb; }
-            f.bvalid = (q >> 1) == (gq & 1);
-            f.b = act + (gq >> 1) * act_stride(sg.in) + 8 * q;
-            f.sx = reinterpret_cast<const float *>(act + up128(kTok * act_stride(sg.in))) + q * sx_stride(sg.in);
-            f.n32 = sg.in >> 5;
-            const bool last = (cur.b + 1) * kTok >= cur.u.nt;
-            const int r0 = cur.u.tile * 16 * mt_n;
+            if (!mbar_wait(afull(team, buf), (n >> 1) & 1, abort_flag)) { failed = true; break; }
+            const Batch &bt = batch_s[team][buf];
+            const int flags = bt.flags;
+            if (flags & 4) break;
+            const int sgi = bt.seg, tile = bt.tile;
+            const SpRowsSeg &sg = a.seg[sgi];
+            const SegGeo &ge = a.geo[sgi];
+            if ((flags & 1) && !mbar_wait(full(s), ph, abort_flag)) { failed = true; break; }
+            const int mt_n = PAIR ? 2 : ge.mt_n, mt = mt_n == 8 ? tw : tw >> 2, r0 = tile * 16 * mt_n;
+            const unsigned char *codes = sm + (unsigned)s * a.stage_bytes, *scales = codes + ge.scale_off, *act = aptr + buf * a.act_bytes;
+            f.w0 = codes + (mt * 16 + gq) * ge.stride + 4 * q; f.w1 = f.w0 + 8 * ge.stride;
+            if (PAIR) { f.s0 = scales + (mt * 8 + gq) * ge.sb; f.s1 = f.s0 + 16 * ge.sb; }         /* gate rows, then the up rows */
+            else { f.s0 = scales + (mt * 16 + gq) * ge.sb; f.s1 = f.s0 + 8 * ge.sb; }
+            f.b = act + (gq >> 1) * ge.ast + 8 * q;
+            f.sx = reinterpret_cast<const float *>(act + ge.sx_off) + q * ge.sst;
+            f.n32 = ge.n32;
             if (!PAIR && mt_n == 8) {
                 if (r0 + mt * 16 < sg.rows) {
                     float2 v = make_float2(0.0f, 0.0f), o = v;
 #pragma unroll 1
                     for (int k = 0; k < 4; k++) {           /* classes 0, 2, 1, 3: (0 + 2) + (1 + 3) */
-                        const float2 c = class_sum<1>(f, k == 1 ? 2 : k == 2 ? 1 : k);
+                        const int r = k == 1 ? 2 : k == 2 ? 1 : k;
+                        const float2 c = f.n32 <= 8 ? class_sum<1, 2>(f, r) : f.n32 <= 16 ? class_sum<1, 4>(f, r) : f.n32 <= 24 ? class_sum<1, 6>(f, r) : class_sum<1, 8>(f, r);
                         if (k == 0 || k == 2) o = c;
                         else { o.x += c.x; o.y += c.y; if (k == 1) v = o; else { v.x += o.x; v.y += o.y; } }
                     }
-                    const int it = items_s[team][buf][q];
+                    const int it = bt.item[q];
                     if (it >= 0) {
                         float *out = sg.out_f + (size_t)it * sg.out_stride + r0 + mt * 16 + gq;
                         out[0] = v.x; out[8] = v.y;
                     }
                 }
-                if (last) { __syncwarp(); if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(empty(s)) : "memory"); }
             } else {
                 float *part = part_s[team][buf];
                 if (PAIR || r0 + mt * 16 < sg.rows) {
@@ -344,7 +352,6 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const 
                     float *p = part + (((tw & 3) * 2 + mt) * 16 + gq) * kTok + q;
                     p[0] = v.x; p[8 * kTok] = v.y;
                 }
-                if (last) { __syncwarp(); if (lane == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(empty(s)) : "memory"); }
                 team_sync(team);
                 auto total_of = [&](int m, int row, int t) {                /* the last two levels of the tree */
                     const float *p = part + (m * 16 + row) * kTok + t;
@@ -355,24 +362,30 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 32, 1) k_rows(const 
                     if (tw == w0 || tw == w0 + 1) {
                         const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
                         const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
-                        const int it = items_s[team][buf][t];
-                        const size_t o = (size_t)(it < 0 ? 0 : it) * sg.rows + r0 / 2;
-                        quant_elem16(h, it >= 0, sg.out_q + o, sg.out_s + o / 16);
+                        const int it = bt.item[t] < 0 ? 0 : bt.item[t];
+                        quant_elem16(h, bt.item[t] >= 0, sg.out_q + (size_t)it * sg.rows + tile * 16, sg.out_s + (size_t)it * sp_sx_row(sg.rows) + tile);
                     }
                 } else {
-                    const int w0 = 4 * (n & 1), t = tw - w0;
+                    const int t = tw - 4 * (n & 1);
                     if (t >= 0 && t < 4) {
-                        const int it = items_s[team][buf][t];
+                        const int it = bt.item[t];
                         if (it >= 0 && r0 + lane < sg.rows) sg.out_f[(size_t)it * sg.out_stride + r0 + lane] = total_of(lane >> 4, lane & 15, t);
                     }
                 }
             }
-            if (last) { s += a.teams; while (s >= a.stages) { s -= a.stages; ph ^= 1; } }
-            cur = nxt; nxt = nn;
+            __syncwarp();
+            arrive_lane0(aempty(team, buf), lane);
+            if (flags & 2) {
+                arrive_lane0(empty(s), lane);
+                s += a.teams;
+                while (s >= a.stages) { s -= a.stages; ph ^= 1; }
+            }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    if (failed && lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
+    if (failed) {
+        if (lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
+        __nanosleep(100000);                                /* let copies in flight land before the CTA leaves */
+    }
 }
 
 constexpr size_t kSmemLimit = 227 * 1024 - 17 * 1024;      /* dynamic part: the static arrays of the kernel take 16.3 KB */
@@ -389,7 +402,8 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *statu
     a.nseg = nseg; a.status = status;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
-        const unsigned sb = seg_stage_bytes(seg[i], pair), ab = seg_act_bytes(seg[i]);
+        const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
+        const unsigned sb = g.scale_off + up128(16 * g.mt_n * g.sb), ab = g.sx_off + up128(kTok * 4 * g.sst);
         a.stage_bytes = sb > a.stage_bytes ? sb : a.stage_bytes; a.act_bytes = ab > a.act_bytes ? ab : a.act_bytes;
     }
     /* two teams with three stages where they fit (one being filled while two are used), else one team with two */
@@ -402,7 +416,7 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *statu
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32);
+    const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32 + 32 * a.teams);
     const size_t smem = acts + (size_t)a.stages * a.stage_bytes;
     if (pair) k_rows<true><<<(unsigned)sms, threads, smem, st>>>(a); else k_rows<false><<<(unsigned)sms, threads, smem, st>>>(a);
     (*nl)++;

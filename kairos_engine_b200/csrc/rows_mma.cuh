@@ -15,8 +15,8 @@ struct SpRowsSeg {
     const int *count, *list; int list_stride;
     const int *offset, *index, *act_index;         /* act_index: position -> activation row when it is not item / act_div */
     int M, act_div;
-    const signed char *q; const float *sx;         /* int8 activations [row][in] (de-interleaved by 8), block scales [row][in / 16] */
-    /* pair: geglu(gate . x, up . x), quantised again in blocks of 16: out_q[item][rows], out_s[item][rows / 16];
+    const signed char *q; const float *sx;         /* int8 activations [row][in] (de-interleaved by 8), block scales [row][sp_sx_row(in)] */
+    /* pair: geglu(gate . x, up . x), quantised again in blocks of 16: out_q[item][rows], out_s[item][sp_sx_row(rows)];
      * otherwise out_f[item * out_stride + row] */
     signed char *out_q; float *out_s; float *out_f; int out_stride;
 };
