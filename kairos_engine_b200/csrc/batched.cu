@@ -17,6 +17,7 @@
 #include "batched.cuh"
 #include "prefill_tc.cuh"
 #include "rows_mma.cuh"
+#include "launch.cuh"
 #include <cstdlib>
 #include "../../include/sp_engine/moe_backend.h"
 
@@ -77,25 +78,6 @@ BView bview_slice(const SpDims &d, const SpBatchedScratch *s, int t0, int slice)
 }
 
 /* ---------------------------------------------------------------- device helpers */
-/* sum of squares in the reference's order (k_rmsnorm, CF:503-511); blockDim.x == 256 */
-__device__ double sumsq256(const float *v, int n, double *sh) {
-    const int t = threadIdx.x;
-    double s = 0.0;
-    for (int i = t; i < n; i += 256) { const double a = v[i]; s += a * a; }
-    sh[t] = s;
-    __syncthreads();
-    for (int o = 128; o >= 32; o >>= 1) { if (t < o) sh[t] += sh[t + o]; __syncthreads(); }
-    if (t < 32) {
-        double a = sh[t];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (t == 0) sh[0] = a;
-    }
-    __syncthreads();
-    const double r = sh[0];
-    __syncthreads();
-    return r;
-}
 __device__ __forceinline__ float rms_scale_from(double ss, int n, float eps) {
     const float ms = (float)(ss / (double)n);
     return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ms, eps)));
@@ -105,96 +87,196 @@ __device__ __forceinline__ float warp_tree(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
-/* quantise one row with all 256 threads (k_quant_act_int8_batched, CF:1725-1746) */
-template <class F>
-__device__ __forceinline__ void quant_row(int n, signed char *q, float *sx, F get) {
-    for (int base = 0; base < n; base += 256) {
-        const int i = base + (int)threadIdx.x;
-        const bool valid = i < n;
-        const float v = valid ? get(i) : 0.0f;
-        const int b = i >> 4;
-        quant_elem16(v, valid, q + 16 * b, sx + b);
+/* ---------------------------------------------------------------- K1/K7: everything a layer does per token
+ * FIN: ordered combine and recombine of the layer that ends (CF:6071-6077, 9014-9019), which gives the residual y.
+ * PREP: norms of y (or of x, without FIN) for the layer that begins (CF:8347, 8402-8404, 8425): the router's input and the
+ * two experts' inputs as int8 blocks, fp32 rows, or fp16 hi/lo rows in the tensor-core GEMMs' k order.
+ * One block per token, a thread takes two groups of four consecutive elements; what a thread needs is fetched before the
+ * first dependent step, and what is left is three or four block-wide double sums in a row. Bound by their instructions (each
+ * sum costs a warp some fifty, so few warps with more elements each), then by the pair rows it reads: see the figures at
+ * launch_token. */
+enum { kOutNone = 0, kOutInt8 = 1, kOutF32 = 2, kOutSplit = 3 };
+struct TokArgs {
+    const float *x;
+    const float *dn, *eo, *cw; const int *pair_index; const float *post_ffw1, *post_ffw2, *post_ffw; float *y;       /* FIN */
+    const float *ffn_norm, *pre_ffw2, *router_scale; float *rin; int *count;                                         /* PREP */
+    signed char *nx_q, *in_q; float *nx_s, *in_s; float *nx_f, *in_f, *rows_f; __half *nx_hi, *nx_lo, *in_hi, *in_lo;
+};
+/* block-wide sums: shuffle tree per warp, then every warp adds the (at most 16) warps' sums by a second tree. `red` has 16
+ * slots per sum, used once. */
+template <int N>
+__device__ __forceinline__ void block_sum(double (&a)[N], double *red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; k++) a[k] += __shfl_down_sync(0xffffffffu, a[k], o);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < N; k++) red[16 * k + warp] = a[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; k++) a[k] = (lane & 15) < nw ? red[16 * k + (lane & 15)] : 0.0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; k++) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+}
+__device__ __forceinline__ double sumsq4(const float4 &f) { return ((double)f.x * f.x + (double)f.y * f.y) + ((double)f.z * f.z + (double)f.w * f.w); }
+__device__ __forceinline__ float4 scale4(const float4 &f, float s, const float4 &w) {
+    return make_float4(__fmul_rn(__fmul_rn(f.x, s), w.x), __fmul_rn(__fmul_rn(f.y, s), w.y), __fmul_rn(__fmul_rn(f.z, s), w.z), __fmul_rn(__fmul_rn(f.w, s), w.w));
+}
+/* four elements of a 16-block, four threads per block: quant_elem16's arithmetic and layout */
+__device__ __forceinline__ void quant_quad(const float4 &f, bool ok, int i, signed char *q, float *sx) {
+    float m = fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w)));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1)); m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    const float scale = m > 0.0f ? __fmul_rn(m, 1.0f / 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, scale);
+    auto one = [&](float v) { int t = __float2int_rn(__fmul_rn(v, inv)); t = t > 127 ? 127 : t; return t < -127 ? -127 : t; };
+    const int a = one(f.x), b = one(f.y), c = one(f.z), d = one(f.w);
+    if (ok) {
+        signed char *g = q + 8 * (i >> 1) + 2 * (i & 1);        /* the even elements of a group of 8, then the odd ones */
+        *reinterpret_cast<unsigned short *>(g) = (unsigned short)((a & 0xFF) | ((c & 0xFF) << 8));
+        *reinterpret_cast<unsigned short *>(g + 4) = (unsigned short)((b & 0xFF) | ((d & 0xFF) << 8));
+        if ((i & 3) == 0) sx[i >> 2] = scale;
     }
 }
-
-/* ---------------------------------------------------------------- K1: per-token norms of x (CF:8347, 8402-8404, 8425) */
-/* block sum of 256 per-thread doubles in sumsq256's order */
-__device__ double block_sum256(double s, double *sh) {
-    const int t = threadIdx.x;
-    sh[t] = s;
-    __syncthreads();
-    for (int o = 128; o >= 32; o >>= 1) { if (t < o) sh[t] += sh[t + o]; __syncthreads(); }
-    if (t < 32) {
-        double a = sh[t];
+/* four elements of a group of 8, two threads per group: fp16 hi and lo in the order 0,4,1,5,2,6,3,7; the lower thread
+ * stores the group's hi, the upper its lo */
+__device__ __forceinline__ void split_quad(const float4 &f, bool ok, int i, __half *hi, __half *lo) {
+    const float v[4] = {f.x, f.y, f.z, f.w};
+    unsigned h[4], l[4];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (t == 0) sh[0] = a;
+    for (int k = 0; k < 4; k++) {
+        const __half x = __float2half_rn(v[k]), y = __float2half_rn(__fsub_rn(v[k], __half2float(x)));
+        h[k] = __half_as_ushort(x); l[k] = __half_as_ushort(y);
     }
-    __syncthreads();
-    const double r = sh[0];
-    __syncthreads();
-    return r;
+    const bool up = i & 1;
+    unsigned w[4];
+    const unsigned s0 = up ? (h[0] | (h[1] << 16)) : (l[0] | (l[1] << 16)), s1 = up ? (h[2] | (h[3] << 16)) : (l[2] | (l[3] << 16));
+    const unsigned r0 = __shfl_xor_sync(0xffffffffu, s0, 1), r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+    const unsigned other[4] = {r0 & 0xFFFFu, r0 >> 16, r1 & 0xFFFFu, r1 >> 16};
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = up ? (other[k] | (l[k] << 16)) : (h[k] | (other[k] << 16));
+    if (ok) *reinterpret_cast<uint4 *>((up ? lo : hi) + 8 * (i >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
 }
-/* One block per token. Everything a thread needs (its 256-strided elements of x and of the three norm
- * vectors) is fetched before the first dependent step, so a block pays the memory latency once and not
- * once per 256 elements; rows wider than 256 * kPrepK take the plain loops. */
-constexpr int kPrepK = 12;
-template <bool FA>
-__global__ void __launch_bounds__(256) k_b_prep(SpDims d, SpLayerDev L, const float *x, BView v, float *rows_f) {
-    __shared__ double sh[256];
-    const int t = blockIdx.x, E = d.E, tid = threadIdx.x;
-    const float *xt = x + (size_t)t * E;
-    if (t == 0) for (int i = tid; i < d.NE; i += 256) v.count[i] = 0;
-    if (E <= 256 * kPrepK) {
-        float xv[kPrepK], n1[kPrepK], n2[kPrepK], rs[kPrepK];
+/* FEW: at most one block per SM, so its latency counts: the norm weights are fetched while the previous kernel drains, all
+ * pair rows at once. Otherwise three blocks (two of E above 3072) share an SM and the registers. */
+template <bool FIN, int OUT, bool WIDE, bool FEW>
+__global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_token(SpDims d, TokArgs a) {
+    constexpr int KB = FEW ? SP_MAX_NU : 4;
+    __shared__ double red[3][32];
+    const int t = blockIdx.x, E = d.E, NU = d.NU, T = blockDim.x;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int ix[2]; bool ok[2];
 #pragma unroll
-        for (int k = 0; k < kPrepK; k++) {
-            const int i = tid + 256 * k; const bool ok = i < E;
-            xv[k] = ok ? xt[i] : 0.0f; n1[k] = ok ? __ldg(L.ffn_norm + i) : 0.0f;
-            n2[k] = ok ? __ldg(L.pre_ffw2 + i) : 0.0f; rs[k] = ok ? __ldg(L.router_scale + i) : 0.0f;
-        }
-        double ss = 0.0;
+    for (int h = 0; h < 2; h++) { ix[h] = threadIdx.x + h * T; ok[h] = 4 * ix[h] < E; }
+    auto load = [&](const float *p, int h) { return ok[h] ? __ldg(reinterpret_cast<const float4 *>(p) + ix[h]) : zero; };       /* weights: not an earlier kernel's work */
+    const float *const wptr[6] = {a.post_ffw1, a.post_ffw2, a.post_ffw, a.ffn_norm, a.pre_ffw2, a.router_scale};
+    float4 pre[6][2];
+    if (FEW) {
 #pragma unroll
-        for (int k = 0; k < kPrepK; k++) if (256 * k < E) { const double a = xv[k]; if (tid + 256 * k < E) ss += a * a; }
-        const float scale = rms_scale_from(block_sum256(ss, sh), E, d.eps);
-        const size_t b16 = (size_t)t * sp_sx_row(E), row = (size_t)t * E;
+        for (int k = FIN ? 0 : 3; k < (OUT ? 6 : 3); k++)
 #pragma unroll
-        for (int k = 0; k < kPrepK; k++) {
-            if (256 * k < E) {                                  /* block-uniform: every lane of a warp reaches the shuffles */
-                const int i = tid + 256 * k; const bool ok = i < E;
-                const float xs = __fmul_rn(xv[k], scale);
-                const float nv = __fmul_rn(xs, n1[k]), iv = __fmul_rn(xs, n2[k]);
-                if (FA) {
-                    const int b = i >> 4;
-                    quant_elem16(nv, ok, v.nx_q + row + 16 * b, v.nx_s + b16 + b);
-                    quant_elem16(iv, ok, v.in_q + row + 16 * b, v.in_s + b16 + b);
-                } else if (ok) { v.nx_f[row + i] = nv; v.in_f[row + i] = iv; }
-                if (ok) {
-                    if (rows_f) rows_f[row + i] = iv;
-                    v.rin[row + i] = __fmul_rn(__fmul_rn(xs, d.inv_sqrt_e), rs[k]);
+            for (int h = 0; h < 2; h++) pre[k][h] = load(wptr[k], h);
+    }
+    auto vec = [&](int k, int h) { return FEW ? pre[k][h] : load(wptr[k], h); };
+    sp_pdl_wait();
+    sp_pdl_next();
+    if (OUT && t == 0) for (int k = threadIdx.x; k < d.NE; k += T) a.count[k] = 0;
+    const size_t row = (size_t)t * E;
+    auto row4 = [&](const float *p, int h) { return ok[h] ? __ldcs(reinterpret_cast<const float4 *>(p) + ix[h]) : zero; };
+    float4 x[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) x[h] = row4(a.x + row, h);
+    if (FIN) {
+        float4 dn[2], c[2] = {zero, zero};
+#pragma unroll
+        for (int h = 0; h < 2; h++) dn[h] = row4(a.dn + row, h);
+#pragma unroll
+        for (int k0 = 0; k0 < SP_MAX_NU; k0 += KB) {            /* KB pair rows in flight */
+            float4 o[KB][2]; float cw[KB];
+#pragma unroll
+            for (int k = 0; k < KB; k++) {
+                cw[k] = 0.0f; o[k][0] = o[k][1] = zero;
+                if (k0 + k < NU) {
+                    const size_t p = (size_t)t * NU + k0 + k;
+                    cw[k] = a.cw[p];
+                    const float *r = a.eo + (size_t)(a.pair_index ? a.pair_index[p] : (int)p) * E;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) o[k][h] = row4(r, h);
                 }
             }
+#pragma unroll
+            for (int k = 0; k < KB; k++)
+                if (k0 + k < NU)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        c[h].x = __fadd_rn(c[h].x, __fmul_rn(cw[k], o[k][h].x)); c[h].y = __fadd_rn(c[h].y, __fmul_rn(cw[k], o[k][h].y));
+                        c[h].z = __fadd_rn(c[h].z, __fmul_rn(cw[k], o[k][h].z)); c[h].w = __fadd_rn(c[h].w, __fmul_rn(cw[k], o[k][h].w));
+                    }
         }
-        return;
-    }
-    const float scale = rms_scale_from(sumsq256(xt, E, sh), E, d.eps);
-    if (FA) {
-        const size_t b16 = (size_t)t * sp_sx_row(E);
-        quant_row(E, v.nx_q + (size_t)t * E, v.nx_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.ffn_norm + i)); });
-        quant_row(E, v.in_q + (size_t)t * E, v.in_s + b16, [&](int i) { return __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i)); });
-        if (rows_f)                                             /* the routed experts' input as fp32 rows (expert-parallel dispatch) */
-            for (int i = tid; i < E; i += 256) rows_f[(size_t)t * E + i] = __fmul_rn(__fmul_rn(xt[i], scale), __ldg(L.pre_ffw2 + i));
-    } else {
-        for (int i = tid; i < E; i += 256) {
-            const float xs = __fmul_rn(xt[i], scale);
-            v.nx_f[(size_t)t * E + i] = __fmul_rn(xs, __ldg(L.ffn_norm + i));
-            const float iv = __fmul_rn(xs, __ldg(L.pre_ffw2 + i));
-            v.in_f[(size_t)t * E + i] = iv;
-            if (rows_f) rows_f[(size_t)t * E + i] = iv;
+        double s2[2] = {sumsq4(dn[0]) + sumsq4(dn[1]), sumsq4(c[0]) + sumsq4(c[1])};
+        block_sum<2>(s2, red[0]);
+        const float sc1 = rms_scale_from(s2[0], E, d.eps), sc2 = rms_scale_from(s2[1], E, d.eps);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float4 m = scale4(dn[h], sc1, vec(0, h)), u = scale4(c[h], sc2, vec(1, h));
+            dn[h] = make_float4(__fadd_rn(m.x, u.x), __fadd_rn(m.y, u.y), __fadd_rn(m.z, u.z), __fadd_rn(m.w, u.w));
+        }
+        double s1[1] = {sumsq4(dn[0]) + sumsq4(dn[1])};
+        block_sum<1>(s1, red[1]);
+        const float sc3 = rms_scale_from(s1[0], E, d.eps);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float4 r = scale4(dn[h], sc3, vec(2, h));
+            x[h] = make_float4(__fadd_rn(x[h].x, r.x), __fadd_rn(x[h].y, r.y), __fadd_rn(x[h].z, r.z), __fadd_rn(x[h].w, r.w));
+            if (ok[h]) reinterpret_cast<float4 *>(a.y + row)[ix[h]] = x[h];
         }
     }
-    for (int i = tid; i < E; i += 256)
-        v.rin[(size_t)t * E + i] = __fmul_rn(__fmul_rn(__fmul_rn(xt[i], scale), d.inv_sqrt_e), __ldg(L.router_scale + i));
+    if (OUT) {
+        double s1[1] = {sumsq4(x[0]) + sumsq4(x[1])};
+        block_sum<1>(s1, red[2]);
+        const float sc = rms_scale_from(s1[0], E, d.eps);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int i = ix[h];
+            const float4 n = scale4(x[h], sc, vec(3, h)), in = scale4(x[h], sc, vec(4, h));
+            if (ok[h]) {
+                const float4 xs = make_float4(__fmul_rn(x[h].x, sc), __fmul_rn(x[h].y, sc), __fmul_rn(x[h].z, sc), __fmul_rn(x[h].w, sc));
+                reinterpret_cast<float4 *>(a.rin + row)[i] = scale4(xs, d.inv_sqrt_e, vec(5, h));
+            }
+            if (OUT == kOutInt8) {
+                const size_t b = (size_t)t * sp_sx_row(E);
+                quant_quad(n, ok[h], i, a.nx_q + row, a.nx_s + b);
+                quant_quad(in, ok[h], i, a.in_q + row, a.in_s + b);
+            } else if (OUT == kOutSplit) {
+                split_quad(n, ok[h], i, a.nx_hi + row, a.nx_lo + row);
+                split_quad(in, ok[h], i, a.in_hi + row, a.in_lo + row);
+            } else if (ok[h]) {
+                reinterpret_cast<float4 *>(a.nx_f + row)[i] = n;
+                reinterpret_cast<float4 *>(a.in_f + row)[i] = in;
+            }
+            if (a.rows_f && ok[h]) reinterpret_cast<float4 *>(a.rows_f + row)[i] = in;
+        }
+    }
+}
+/* End of a layer + beginning of the next: as two kernels of 256 threads that walked the row in shared memory 229 us for 4096
+ * tokens, as this one 111 us (625 MB of it pair rows and rows in and out). */
+constexpr int kFewTokens = 148;
+template <bool FIN, int OUT>
+cudaError_t launch_token(const SpDims &d, int M, const TokArgs &a, cudaStream_t st, int *nl) {
+    const unsigned threads = (unsigned)((d.E / 8 + 31) & ~31);
+    const bool wide = d.E > 3072, few = M <= kFewTokens;
+    return sp_launch(wide ? (few ? k_b_token<FIN, OUT, true, true> : k_b_token<FIN, OUT, true, false>) : (few ? k_b_token<FIN, OUT, false, true> : k_b_token<FIN, OUT, false, false>),
+                     dim3((unsigned)M), threads, 0, st, nl, d, a);
+}
+void set_prep(TokArgs &a, const SpLayerDev &L, const BView &v, SpTcPlan *split) {
+    a.ffn_norm = L.ffn_norm; a.pre_ffw2 = L.pre_ffw2; a.router_scale = L.router_scale; a.rin = v.rin; a.count = v.count;
+    a.nx_q = v.nx_q; a.in_q = v.in_q; a.nx_s = v.nx_s; a.in_s = v.in_s; a.nx_f = v.nx_f; a.in_f = v.in_f;
+    if (split) sp_tc_inputs(split, &a.nx_hi, &a.nx_lo, &a.in_hi, &a.in_lo);
+}
+void set_finish(TokArgs &a, const SpLayerDev &L, const BView &v, const float *eo, const int *pair_index, float *y) {
+    a.dn = v.dn; a.eo = eo; a.cw = v.cw; a.pair_index = pair_index; a.post_ffw1 = L.post_ffw1; a.post_ffw2 = L.post_ffw2; a.post_ffw = L.post_ffw; a.y = y;
 }
 
 /* ---------------------------------------------------------------- K2: router logits, fp32, fixed order
@@ -214,6 +296,8 @@ __global__ void __launch_bounds__(256, 2) k_b_router(SpDims d, SpLayerDev L, BVi
     const int E = d.E, G = E >> 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int we = warp & 3, wt = warp >> 2;
     const int e0 = blockIdx.x * kRouterTE, t0 = blockIdx.y * kRouterTT;
+    sp_pdl_wait();
+    sp_pdl_next();
     float acc[8][8];
 #pragma unroll
     for (int i = 0; i < 8; i++)
@@ -276,7 +360,9 @@ __global__ void __launch_bounds__(256) k_b_router_small(SpDims d, SpLayerDev L, 
     extern __shared__ __align__(16) float4 rw[];               /* [E/4] */
     const int E = d.E, G = E >> 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x;
     const float4 *wrow = reinterpret_cast<const float4 *>(L.router_w + (size_t)e * E);
-    for (int g = threadIdx.x; g < G; g += 256) rw[g] = __ldg(wrow + g);
+    for (int g = threadIdx.x; g < G; g += 256) rw[g] = __ldg(wrow + g);      /* a weight: fetched before the wait */
+    sp_pdl_wait();
+    sp_pdl_next();
     __syncthreads();
     const int t = blockIdx.y * 8 + warp;
     if (t >= M) return;
@@ -295,14 +381,74 @@ __global__ void __launch_bounds__(256) k_b_router_small(SpDims d, SpLayerDev L, 
 #define SP_ROUTER_SMALL_M 64
 #endif
 constexpr int kRouterSmallM = SP_ROUTER_SMALL_M;   /* up to this many tokens the per-(expert, eight tokens) blocks beat the tiled kernel */
-void launch_router(const SpDims &d, const SpLayerDev &L, BView &v, int M, cudaStream_t st, int *nl) {
-    if (M <= kRouterSmallM && (size_t)d.E * 4 <= 48 * 1024) k_b_router_small<<<dim3((unsigned)d.NE, (unsigned)((M + 7) / 8)), 256, (size_t)d.E * 4, st>>>(d, L, v, M);
-    else k_b_router<<<dim3((d.NE + kRouterTE - 1) / kRouterTE, (M + kRouterTT - 1) / kRouterTT), 256, kRouterSmem, st>>>(d, L, v, M);
-    (*nl)++;
+cudaError_t launch_router(const SpDims &d, const SpLayerDev &L, BView &v, int M, cudaStream_t st, int *nl) {
+    if (M <= kRouterSmallM && (size_t)d.E * 4 <= 48 * 1024)
+        return sp_launch(k_b_router_small, dim3((unsigned)d.NE, (unsigned)((M + 7) / 8)), 256, (size_t)d.E * 4, st, nl, d, L, v, M);
+    return sp_launch(k_b_router, dim3((d.NE + kRouterTE - 1) / kRouterTE, (M + kRouterTT - 1) / kRouterTT), 256, kRouterSmem, st, nl, d, L, v, M);
 }
 
 /* ---------------------------------------------------------------- K3: moe_topk_host (CF:6220-6240) + bucketing by expert (CF:8594-8624) */
-__global__ void __launch_bounds__(256) k_b_topk(SpDims d, SpLayerDev L, BView v, int M, int32_t *sel_out, float *wts_out, int *status) {
+struct TopkOut { int32_t *sel; float *wts; int *status; };
+/* the selection of one token, expert e in place k of the descending order with probability p: clamped weights, ascending
+ * slots, bucketing */
+__device__ __forceinline__ void topk_store(const SpDims &d, const SpLayerDev &L, const BView &v, int M, int tok, int k, int e, float p, float wsum, int slot, const TopkOut &o) {
+    if (wsum < 6.103515625e-5f) wsum = 6.103515625e-5f;
+    const float w = __fdiv_rn(p, wsum);
+    const int pair = tok * d.NU + slot;
+    v.sel_asc[pair] = e;
+    v.cw[pair] = __fmul_rn(w, __ldg(L.dexps_scale + e));                 /* CF:8709 */
+    const int pos = atomicAdd(&v.count[e], 1);
+    v.pairpos[pair] = pos;
+    if (pos < M) v.list[(size_t)e * M + pos] = pair; else atomicExch(o.status, SP_KERR_OVERFLOW);
+    if (o.sel) o.sel[(size_t)tok * d.NU + k] = e;
+    if (o.wts) o.wts[(size_t)tok * d.NU + k] = w;
+}
+/* NE <= 128: one warp per token, four candidates a lane; NU rounds of (largest probability, then the lowest id among its
+ * holders), the order moe_topk_host's strict > insertion produces. key = bits(p) + 1 for a usable probability (p >= 0, so
+ * its bits order like its value), 0 for a NaN or an absent candidate. */
+__global__ void __launch_bounds__(128) k_b_topk_warp(SpDims d, SpLayerDev L, BView v, int M, TopkOut o) {
+    const int lane = threadIdx.x & 31, tok = blockIdx.x * 4 + (threadIdx.x >> 5), NE = d.NE, NU = d.NU;
+    sp_pdl_wait();
+    sp_pdl_next();
+    if (tok >= M) return;
+    const float *lg = v.logits + (size_t)tok * NE;
+    float l[4], mx = -INFINITY; bool bad = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) { l[k] = lane + 32 * k < NE ? lg[lane + 32 * k] : -INFINITY; bad |= l[k] != l[k]; mx = fmaxf(mx, l[k]); }
+#pragma unroll
+    for (int q = 16; q > 0; q >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, q));
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(o.status, SP_KERR_NAN_ROUTER);
+    double ex[4], sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) { ex[k] = lane + 32 * k < NE ? exp((double)l[k] - (double)mx) : 0.0; sum += ex[k]; }
+#pragma unroll
+    for (int q = 16; q > 0; q >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, q);
+    unsigned key[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) { const float p = (float)(ex[k] / sum); key[k] = (lane + 32 * k < NE && p == p) ? __float_as_uint(p) + 1u : 0u; }
+    int e = lane < NE ? lane : 0; float p = 0.0f;               /* lane r keeps the r-th of the descending order */
+#pragma unroll 1
+    for (int r = 0; r < NU; r++) {
+        unsigned lm = key[0] > key[1] ? key[0] : key[1]; const unsigned l2 = key[2] > key[3] ? key[2] : key[3]; lm = lm > l2 ? lm : l2;
+        const unsigned m = __reduce_max_sync(0xffffffffu, lm);
+        if (m == 0u) break;
+        unsigned cand = 0x7fffffffu;
+#pragma unroll
+        for (int k = 3; k >= 0; k--) if (key[k] == m) cand = (unsigned)(lane + 32 * k);
+        const unsigned w = __reduce_min_sync(0xffffffffu, cand);
+#pragma unroll
+        for (int k = 0; k < 4; k++) if ((unsigned)(lane + 32 * k) == w) key[k] = 0u;
+        if (lane == r) { e = (int)w; p = __uint_as_float(m - 1u); }
+    }
+    float wsum = 0.0f; int slot = 0;
+    for (int k = 0; k < NU; k++) {
+        wsum = __fadd_rn(wsum, __shfl_sync(0xffffffffu, p, k));
+        slot += __shfl_sync(0xffffffffu, e, k) < e;
+    }
+    if (lane < NU) topk_store(d, L, v, M, tok, lane, e, p, wsum, slot, o);
+}
+/* any NE: one block per token, the rank of a candidate counted against all others */
+__global__ void __launch_bounds__(256) k_b_topk(SpDims d, SpLayerDev L, BView v, int M, TopkOut o) {
     extern __shared__ __align__(16) unsigned char tsm[];
     const int NE = d.NE, NU = d.NU, t = threadIdx.x, tok = blockIdx.x;
     double *ex = reinterpret_cast<double *>(tsm);               /* [NE] */
@@ -311,13 +457,15 @@ __global__ void __launch_bounds__(256) k_b_topk(SpDims d, SpLayerDev L, BView v,
     __shared__ float wmax[8];
     __shared__ int sel_desc[SP_MAX_NU];
     __shared__ float p_desc[SP_MAX_NU];
+    sp_pdl_wait();
+    sp_pdl_next();
     const float *lg = v.logits + (size_t)tok * NE;
     float mx = -INFINITY; int bad = 0;
     for (int i = t; i < NE; i += 256) { const float l = lg[i]; if (l != l) bad = 1; mx = fmaxf(mx, l); }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); bad |= __shfl_xor_sync(0xffffffffu, bad, o); }
     if ((t & 31) == 0) wmax[t >> 5] = mx;
-    if (bad && (t & 31) == 0) atomicExch(status, SP_KERR_NAN_ROUTER);
+    if (bad && (t & 31) == 0) atomicExch(o.status, SP_KERR_NAN_ROUTER);
     __syncthreads();
     mx = wmax[0];
 #pragma unroll
@@ -342,39 +490,27 @@ __global__ void __launch_bounds__(256) k_b_topk(SpDims d, SpLayerDev L, BView v,
     if (t < NU) {
         float wsum = 0.0f;
         for (int k = 0; k < NU; k++) wsum = __fadd_rn(wsum, p_desc[k]);
-        if (wsum < 6.103515625e-5f) wsum = 6.103515625e-5f;
         const int e = sel_desc[t];
-        const float w = __fdiv_rn(p_desc[t], wsum);
         int slot = 0;
         for (int j = 0; j < NU; j++) slot += (sel_desc[j] < e);
-        const int pair = tok * NU + slot;
-        v.sel_asc[pair] = e;
-        v.cw[pair] = __fmul_rn(w, __ldg(L.dexps_scale + e));             /* CF:8709 */
-        const int pos = atomicAdd(&v.count[e], 1);
-        v.pairpos[pair] = pos;
-        if (pos < M) v.list[(size_t)e * M + pos] = pair; else atomicExch(status, SP_KERR_OVERFLOW);
-        if (sel_out) sel_out[(size_t)tok * NU + t] = e;
-        if (wts_out) wts_out[(size_t)tok * NU + t] = w;
+        topk_store(d, L, v, M, tok, t, e, p_desc[t], wsum, slot, o);
     }
 }
+cudaError_t launch_topk(const SpDims &d, const SpLayerDev &L, BView &v, int M, int32_t *sel, float *wts, int *status, cudaStream_t st, int *nl) {
+    const TopkOut o{sel, wts, status};
+    if (d.NE <= 128) return sp_launch(k_b_topk_warp, dim3((unsigned)((M + 3) / 4)), 128, 0, st, nl, d, L, v, M, o);
+    return sp_launch(k_b_topk, dim3((unsigned)M), 256, (size_t)d.NE * 12, st, nl, d, L, v, M, o);
+}
 
-/* ---------------------------------------------------------------- K5: per-row activation quant (CF:1725-1746) */
-__global__ void __launch_bounds__(256) k_b_quant_rows(const float *x, int n, signed char *q, float *sx) {
+/* ---------------------------------------------------------------- per-row activation quant (CF:1725-1746): received rows of an expert-parallel run */
+__global__ void __launch_bounds__(1024) k_b_quant_rows(const float *x, int n, signed char *q, float *sx) {
     const size_t r = blockIdx.x;
-    const float *xr = x + r * n;
-    if (n <= 256 * kPrepK) {                                    /* all of the row's loads first, then the dependent steps */
-        float v[kPrepK];
-#pragma unroll
-        for (int k = 0; k < kPrepK; k++) { const int i = (int)threadIdx.x + 256 * k; v[k] = i < n ? xr[i] : 0.0f; }
-#pragma unroll
-        for (int k = 0; k < kPrepK; k++)
-            if (256 * k < n) {
-                const int i = (int)threadIdx.x + 256 * k, b = i >> 4;
-                quant_elem16(v[k], i < n, q + r * n + 16 * b, sx + r * sp_sx_row(n) + b);
-            }
-        return;
-    }
-    quant_row(n, q + r * n, sx + r * sp_sx_row(n), [&](int i) { return xr[i]; });
+    const int i = threadIdx.x;
+    const bool ok = 4 * i < n;
+    sp_pdl_wait();
+    sp_pdl_next();
+    const float4 f = ok ? reinterpret_cast<const float4 *>(x + r * n)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    quant_quad(f, ok, i, q + r * n, sx + r * sp_sx_row(n));
 }
 
 /* ---------------------------------------------------------------- K4/K6, floating-point flavour without the tensor cores
@@ -508,67 +644,20 @@ SpRowsSeg seg_routed_down(const SpDims &d, const SpLayerDev &L, int M, const BVi
     return s;
 }
 
-/* ---------------------------------------------------------------- K7: ordered combine + recombine (CF:6071-6077, 9014-9019) */
-__global__ void __launch_bounds__(256) k_b_finish(SpDims d, SpLayerDev L, const float *x, BView v, const float *eo, const int *pair_index, float *y) {
-    extern __shared__ __align__(16) float fsm[];              /* [2][E] */
-    __shared__ double sh[256];
-    const int t = blockIdx.x, E = d.E, NU = d.NU, tid = threadIdx.x;
-    float cw[SP_MAX_NU]; size_t er[SP_MAX_NU];
-#pragma unroll
-    for (int k = 0; k < SP_MAX_NU; k++) {
-        cw[k] = k < NU ? v.cw[(size_t)t * NU + k] : 0.0f;
-        er[k] = k < NU ? (size_t)(pair_index ? pair_index[(size_t)t * NU + k] : t * NU + k) * E : 0;
-    }
-    float *va = fsm, *vb = fsm + E;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < E; i += 256) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < SP_MAX_NU; k++) if (k < NU) acc = __fadd_rn(acc, __fmul_rn(cw[k], eo[er[k] + i]));
-        vb[i] = acc;
-        va[i] = v.dn[(size_t)t * E + i];
-    }
-    __syncthreads();
-    const float sc1 = rms_scale_from(sumsq256(va, E, sh), E, d.eps);
-    const float sc2 = rms_scale_from(sumsq256(vb, E, sh), E, d.eps);
-    for (int i = threadIdx.x; i < E; i += 256) {
-        const float mlp = __fmul_rn(__fmul_rn(va[i], sc1), __ldg(L.post_ffw1 + i));
-        const float t1 = __fmul_rn(__fmul_rn(vb[i], sc2), __ldg(L.post_ffw2 + i));
-        va[i] = __fadd_rn(mlp, t1);
-    }
-    __syncthreads();
-    const float sc3 = rms_scale_from(sumsq256(va, E, sh), E, d.eps);
-    for (int i = threadIdx.x; i < E; i += 256)
-        y[(size_t)t * E + i] = __fadd_rn(x[(size_t)t * E + i], __fmul_rn(__fmul_rn(va[i], sc3), __ldg(L.post_ffw + i)));
-}
-
-static size_t finish_smem(int E) { return (size_t)2 * E * 4; }
-
+/* the experts of one layer: the inputs the prep half left -> dn and eo */
 template <bool FA>
-cudaError_t run_layer(const SpDims &d, const SpLayerDev &L, int M, const float *x, float *y, int32_t *sel, float *wts,
-                      BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
+cudaError_t run_experts(const SpDims &d, const SpLayerDev &L, int M, BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
     const int E = d.E, NE = d.NE, NU = d.NU, FFE = d.FFE, FFS = d.FFS;
-    k_b_prep<FA><<<M, 256, 0, st>>>(d, L, x, v, nullptr); (*nl)++;
-    launch_router(d, L, v, M, st, nl);
-    k_b_topk<<<M, 256, (size_t)NE * 12, st>>>(d, L, v, M, sel, wts, status); (*nl)++;
-    if (!FA && tc) {                                            /* prefill arithmetic on the tensor cores */
-        const cudaError_t e = sp_tc_layer(tc, d, L, M, v.nx_f, v.in_f, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);
-        if (e != cudaSuccess) return e;
-        k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
-        return cudaGetLastError();
-    }
+    if (!FA && tc) return sp_tc_layer(tc, d, L, M, v.nx_f, v.in_f, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);      /* prefill arithmetic on the tensor cores */
     if (FA) {
         /* gate|up of the shared and the routed experts, quantised as it leaves (CF:8348-8356, 8733-8737, 8958-8959), then down (CF:8358, 8739-8742, 8961) */
         SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v.in_s, v)};
         up[1].count = v.count; up[1].list = v.list; up[1].list_stride = M; up[1].act_div = NU;
-        cudaError_t e = sp_rows_launch(up, 2, true, status, st, nl);
+        const cudaError_t e = sp_rows_launch(up, 2, true, status, st, nl);
         if (e != cudaSuccess) return e;
         SpRowsSeg down[2] = {seg_shared_down(d, L, M, v), seg_routed_down(d, L, M, v, v.eo)};
         down[1].count = v.count; down[1].list = v.list; down[1].list_stride = M;
-        e = sp_rows_launch(down, 2, false, status, st, nl);
-        if (e != cudaSuccess) return e;
-        k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
-        return cudaGetLastError();
+        return sp_rows_launch(down, 2, false, status, st, nl);
     }
     GroupArgs g{};
     g.M = M;
@@ -588,8 +677,37 @@ cudaError_t run_layer(const SpDims &d, const SpLayerDev &L, int M, const float *
     g.codes = L.dn_codes; g.bs = L.dn_bs; g.rows_per_group = E; g.count = v.count; g.list = v.list; g.list_stride = M;
     g.in = FFE; g.rows = E; g.act_div = 1; g.xf = v.h; g.out = v.eo; g.out_stride = E;
     launch_rows<false>(g, NE, st, nl);
-    k_b_finish<<<M, 256, finish_smem(E), st>>>(d, L, x, v, v.eo, nullptr, y); (*nl)++;
     return cudaGetLastError();
+}
+template <bool FA>
+cudaError_t run_layers(const SpDims &d, const SpLayerDev *layers, int n, int M, const float *x, float *y, int32_t *sel, float *wts,
+                       BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
+    /* where the experts' kernels take int8 or split rows, the end of a layer and the beginning of the next are one launch */
+    const bool split = !FA && tc && sp_tc_takes_split(d), fused = FA || split;
+    const float *cur = x;
+    cudaError_t e = cudaSuccess;
+    for (int li = 0; li < n && e == cudaSuccess; li++) {
+        const SpLayerDev &L = layers[li];
+        float *dst = li == n - 1 ? y : (li & 1) ? v.xb : v.xa;
+        TokArgs a{};
+        a.x = cur;
+        if (li == 0 || !fused) {
+            set_prep(a, L, v, split ? tc : nullptr);
+            e = FA ? launch_token<false, kOutInt8>(d, M, a, st, nl) : split ? launch_token<false, kOutSplit>(d, M, a, st, nl)
+                   : launch_token<false, kOutF32>(d, M, a, st, nl);
+        }
+        if (e == cudaSuccess) e = launch_router(d, L, v, M, st, nl);
+        if (e == cudaSuccess) e = launch_topk(d, L, v, M, sel ? sel + (size_t)li * M * d.NU : nullptr, wts ? wts + (size_t)li * M * d.NU : nullptr, status, st, nl);
+        if (e == cudaSuccess) e = run_experts<FA>(d, L, M, v, tc, status, st, nl);
+        if (e != cudaSuccess) break;
+        set_finish(a, L, v, v.eo, nullptr, dst);
+        if (fused && li + 1 < n) {
+            set_prep(a, layers[li + 1], v, split ? tc : nullptr);
+            e = FA ? launch_token<true, kOutInt8>(d, M, a, st, nl) : launch_token<true, kOutSplit>(d, M, a, st, nl);
+        } else e = launch_token<true, kOutNone>(d, M, a, st, nl);
+        cur = dst;
+    }
+    return e;
 }
 
 /* per-expert counts -> exclusive offsets (NE is at most 1024: one block) */
@@ -766,10 +884,15 @@ cudaError_t ep_route(const SpDims &d, const SpLayerDev &L, int M, const float *x
                      int32_t *pair_index, int32_t *sel, float *wts, int defer_shared, int n_ranks, int capacity, BView &v, SpTcPlan *tc, int *status,
                      cudaStream_t st, int *nl) {
     const int E = d.E, NE = d.NE, NU = d.NU;
-    k_b_prep<FA><<<M, 256, 0, st>>>(d, L, x, v, FA ? v.in_f : nullptr); (*nl)++;
-    cudaError_t e = cudaSuccess;
-    launch_router(d, L, v, M, st, nl);
-    k_b_topk<<<M, 256, (size_t)NE * 12, st>>>(d, L, v, M, sel, wts, status); (*nl)++;
+    TokArgs a{};
+    a.x = x;
+    set_prep(a, L, v, nullptr);
+    if (FA) a.rows_f = v.in_f;                                  /* the routed experts' input as fp32 rows too, for the dispatch */
+    cudaError_t e = FA ? launch_token<false, kOutInt8>(d, M, a, st, nl)
+                       : launch_token<false, kOutF32>(d, M, a, st, nl);
+    if (e == cudaSuccess) e = launch_router(d, L, v, M, st, nl);
+    if (e == cudaSuccess) e = launch_topk(d, L, v, M, sel, wts, status, st, nl);
+    if (e != cudaSuccess) return e;
     /* the send buffer: rows sorted by expert (so also by owner), ready for the all-to-all */
     k_b_scan<<<1, 1024, 0, st>>>(v.count, NE, v.ep_off); (*nl)++;
     k_b_dispatch_rows<<<M * NU, 256, 0, st>>>(v.in_f, v.sel_asc, v.pairpos, v.ep_off, NU, E, capacity > 0 ? NE / n_ranks : NE, capacity, rows, pair_index, status); (*nl)++;
@@ -792,10 +915,11 @@ cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float 
     if (R == 0) return cudaSuccess;
     if (!FA && tc) return sp_tc_routed(tc, d, L, R, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
     if (FA) {
-        k_b_quant_rows<<<in_index ? n_in : R, 256, 0, st>>>(rows_in, E, v.ep_q, v.ep_s); (*nl)++;
+        cudaError_t e = sp_launch(k_b_quant_rows, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q, v.ep_s);
+        if (e != cudaSuccess) return e;
         SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v.ep_s, v), down = seg_routed_down(d, L, R, v, rows_out);
         up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */
-        const cudaError_t e = sp_rows_launch(&up, 1, true, status, st, nl);
+        e = sp_rows_launch(&up, 1, true, status, st, nl);
         return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, status, st, nl);
     }
     GroupArgs g{};
@@ -868,8 +992,10 @@ cudaError_t sp_batched_ep_finish(const SpDims &d, const SpLayerDev &L, int M, co
     *nlaunch = 0;
     if (!s->base || t0 < 0 || t0 + M > s->max_tokens || slice < 0 || slice >= kSlices) return cudaErrorInvalidValue;
     BView v = bview_slice(d, s, t0, slice);
-    k_b_finish<<<M, 256, finish_smem(d.E), st>>>(d, L, x, v, pair_rows, pair_index, y); (*nlaunch)++;
-    return cudaGetLastError();
+    TokArgs a{};
+    a.x = x;
+    set_finish(a, L, v, pair_rows, pair_index, y);
+    return launch_token<true, kOutNone>(d, M, a, st, nlaunch);
 }
 
 cudaError_t sp_batched_alloc(const SpDims &d, int max_tokens, int max_rows, SpBatchedScratch *s, size_t *bytes) {
@@ -905,16 +1031,6 @@ cudaError_t sp_batched_forward(const SpDims &d, const SpLayerDev *layers_host, i
     *nlaunch = 0;
     if (!s->base || M > s->max_tokens) return cudaErrorInvalidValue;
     BView v = bview(d, s);
-    const float *cur = x;
-    for (int li = 0; li < nl_; li++) {
-        float *dst = (li == nl_ - 1) ? y : ((li & 1) ? v.xb : v.xa);
-        int32_t *sl = sel ? sel + (size_t)li * M * d.NU : nullptr;
-        float *wl = wts ? wts + (size_t)li * M * d.NU : nullptr;
-        const cudaError_t e = (flavour == SP_MOE_FLAVOUR_DECODE)
-            ? run_layer<true>(d, layers_host[lf + li], M, cur, dst, sl, wl, v, s->tc, status, st, nlaunch)
-            : run_layer<false>(d, layers_host[lf + li], M, cur, dst, sl, wl, v, s->tc, status, st, nlaunch);
-        if (e != cudaSuccess) return e;
-        cur = dst;
-    }
-    return cudaSuccess;
+    return flavour == SP_MOE_FLAVOUR_DECODE ? run_layers<true>(d, layers_host + lf, nl_, M, x, y, sel, wts, v, s->tc, status, st, nlaunch)
+                                            : run_layers<false>(d, layers_host + lf, nl_, M, x, y, sel, wts, v, s->tc, status, st, nlaunch);
 }

@@ -44,6 +44,7 @@
 #include <mutex>
 #include "prefill_tc.cuh"
 #include "tc_common.cuh"
+#include "launch.cuh"
 
 namespace {
 using namespace sp_tc;
@@ -169,6 +170,8 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    sp_pdl_wait();
+    sp_pdl_next();
 
     const int total0 = *a.seg[0].n_tiles * a.seg[0].m_tiles;
     const int total = total0 + (a.nseg > 1 ? *a.seg[1].n_tiles * a.seg[1].m_tiles : 0);
@@ -369,22 +372,25 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                     if (++bs == C::kBStages) { bs = 0; bp ^= 1; }
                 }
             }
-        } else if (warp == kActs && lane == 0) {
-            /* ---------------- activation rows by TMA, 64 or 16 rows a copy */
-            uint32_t it = 0;
-            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
-                const Item t = item(w, iw);
-                for (int kb = 0; kb < t.KB; kb++, it++) {
-                    const uint32_t bs = it % C::kBStages, bp = (it / C::kBStages) & 1;
-                    if (!mbar_wait(bempty(bs), bp ^ 1, abort_flag)) { failed = true; break; }
-                    mbar_expect_tx(bfull(bs), (uint32_t)t.n16 * (TERMS >= 2 ? 256u : 128u));
-                    const uint32_t dst = sbase + bs * C::kBStage;
-                    for (int i = 0; i < t.n16;) {
-                        const bool big = t.n16 - i >= kBoxBig;
-                        const CUtensorMap *hi = big ? &maps.hi64[t.sg] : &maps.hi[t.sg], *lo = big ? &maps.lo64[t.sg] : &maps.lo[t.sg];
-                        tma_load_2d(dst + 128u * i, hi, kb * kBK, t.row0 + i, bfull(bs));
-                        if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, lo, kb * kBK, t.row0 + i, bfull(bs));
-                        i += big ? kBoxBig : kNGran;
+        } else if (warp == kActs) {
+            /* ---------------- activation rows by TMA, 64 or 16 rows a copy. (Four gathered rows a copy, tile::gather4 from one
+             * row per token, would save the sorted copy of the rows, but such copies are too slow: 1640 against 870 us for the
+             * gate|up launch of 4096 tokens.) */
+            if (lane == 0) {
+                uint32_t bs = 0, bp = 0;
+                for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
+                    const Item t = item(w, iw);
+                    for (int kb = 0; kb < t.KB; kb++) {
+                        if (!mbar_wait(bempty(bs), bp ^ 1, abort_flag)) { failed = true; break; }
+                        const uint32_t dst = sbase + bs * C::kBStage, bar = bfull(bs);
+                        mbar_expect_tx(bar, (uint32_t)t.n16 * (TERMS >= 2 ? 256u : 128u));
+                        for (int i = 0; i < t.n16;) {
+                            const bool big = t.n16 - i >= kBoxBig;
+                            tma_load_2d(dst + 128u * i, big ? &maps.hi64[t.sg] : &maps.hi[t.sg], kb * kBK, t.row0 + i, bar);
+                            if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, big ? &maps.lo64[t.sg] : &maps.lo[t.sg], kb * kBK, t.row0 + i, bar);
+                            i += big ? kBoxBig : kNGran;
+                        }
+                        if (++bs == C::kBStages) { bs = 0; bp ^= 1; }
                     }
                 }
             }
@@ -435,6 +441,17 @@ __global__ void __launch_bounds__(256) k_tc_split(const float *src, const int *g
         *reinterpret_cast<uint4 *>(hi + r * K + 8 * c) = *reinterpret_cast<const uint4 *>(h);
         *reinterpret_cast<uint4 *>(lo + r * K + 8 * c) = *reinterpret_cast<const uint4 *>(l);
     }
+}
+/* fp16 hi/lo rows of the tokens -> the rows of the pairs, sorted by expert; one block per sorted row, one thread per 16 bytes
+ * of hi and of lo */
+__global__ void __launch_bounds__(512) k_tc_permute(const __half *src_hi, const __half *src_lo, const int *gather, int K, __half *hi, __half *lo) {
+    sp_pdl_wait();
+    sp_pdl_next();
+    const size_t r = (size_t)blockIdx.x * (K / 8), s = (size_t)gather[blockIdx.x] * (K / 8);
+    const int c = threadIdx.x;
+    if (c >= K / 8) return;
+    const uint4 h = reinterpret_cast<const uint4 *>(src_hi)[s + c], l = reinterpret_cast<const uint4 *>(src_lo)[s + c];
+    reinterpret_cast<uint4 *>(hi)[r + c] = h; reinterpret_cast<uint4 *>(lo)[r + c] = l;
 }
 /* block-wide inclusive scan of one int per thread (1024 threads) */
 __device__ __forceinline__ int scan1024(int v, int *sh) {
@@ -492,6 +509,8 @@ struct SortArgs {
 __global__ void __launch_bounds__(1024) k_tc_sort(SortArgs s) {
     __shared__ int sh[32];
     __shared__ int off[1024];
+    sp_pdl_wait();
+    sp_pdl_next();
     const int t = threadIdx.x, cnt = t < s.groups ? s.count[t] : 0;
     const int first = scan1024(cnt, sh) - cnt;
     off[t] = first;
@@ -528,7 +547,7 @@ __global__ void __launch_bounds__(256) k_tc_pairs(const int *sel_asc, const int 
 struct SpTcPlan {
     int Mcap, Rcap, sms;
     unsigned char *base; size_t bytes;
-    __half *nx_hi, *nx_lo, *hd_hi, *hd_lo, *in_hi, *in_lo, *h_hi, *h_lo;
+    __half *nx_hi, *nx_lo, *hd_hi, *hd_lo, *in_hi, *in_lo, *h_hi, *h_lo, *tk_hi, *tk_lo;           /* tk: the routed experts' input, one row per token; in: one per pair */
     int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *gather, *rowmap, *offsets;
     int cap_sh, cap_r;
     int terms;                                         /* MMAs per k-step: 3, 2 or 1 */
@@ -537,6 +556,10 @@ struct SpTcPlan {
     std::map<const void *, CUtensorMap> codes;         /* one per weight tensor of the arena, made at first use */
 };
 
+/* Geometries with E below 512 only check the stages: they stay one launch per stage (the expert-parallel path's stages), so
+ * that callers who count launches see each of them. */
+bool sp_tc_takes_split(const SpDims &d) { return d.E >= 512; }
+void sp_tc_inputs(SpTcPlan *p, __half **nx_hi, __half **nx_lo, __half **in_hi, __half **in_lo) { *nx_hi = p->nx_hi; *nx_lo = p->nx_lo; *in_hi = p->tk_hi; *in_lo = p->tk_lo; }
 bool sp_tc_supported(const SpDims &d) { return (d.E % 64 == 0) && (d.FFE % 64 == 0) && (d.FFS % 64 == 0); }
 
 namespace {
@@ -595,7 +618,7 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     p->cap_sh = p->Mcap / 32 + 2; p->cap_r = p->Rcap / 32 + d.NE + 2;
     size_t o = 0; auto take = [&](size_t b) { size_t at = o; o = up256(o + b); return at; };
     const size_t E = d.E, FFE = d.FFE, FFS = d.FFS, Mc = p->Mcap, Rc = p->Rcap;
-    const size_t o_nx = take(4 * Mc * E), o_hd = take(4 * Mc * FFS), o_in = take(4 * Rc * E), o_h = take(4 * Rc * FFE);      /* hi rows, then lo rows */
+    const size_t o_nx = take(4 * Mc * E), o_hd = take(4 * Mc * FFS), o_in = take(4 * Rc * E), o_h = take(4 * Rc * FFE), o_tk = take(4 * Mc * E);      /* hi rows, then lo rows */
     const size_t o_tsh = take(12 * (size_t)p->cap_sh), o_nsh = take(4), o_tr = take(12 * (size_t)p->cap_r), o_nr = take(4);
     const size_t o_g = take(4 * Rc), o_rm = take(4 * Rc), o_off = take(4 * ((size_t)d.NE + 1));
     p->bytes = o;
@@ -605,6 +628,7 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     unsigned char *b = p->base;
     p->nx_hi = (__half *)(b + o_nx); p->nx_lo = p->nx_hi + Mc * E; p->hd_hi = (__half *)(b + o_hd); p->hd_lo = p->hd_hi + Mc * FFS;
     p->in_hi = (__half *)(b + o_in); p->in_lo = p->in_hi + Rc * E; p->h_hi = (__half *)(b + o_h); p->h_lo = p->h_hi + Rc * FFE;
+    p->tk_hi = (__half *)(b + o_tk); p->tk_lo = p->tk_hi + Mc * E;
     p->tiles_sh = (int *)(b + o_tsh); p->ntiles_sh = (int *)(b + o_nsh); p->tiles_r = (int *)(b + o_tr); p->ntiles_r = (int *)(b + o_nr);
     p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm); p->offsets = (int *)(b + o_off);
     cudaError_t m = cudaSuccess;
@@ -632,10 +656,9 @@ namespace {
 int tile_rows(int groups, long long rows) { return rows > 8LL * groups ? 64 : 32; }
 
 template <bool PAIR, int NMAX>
-void launch_n(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st) {
-    if (p->terms == 3) k_tc_gemm<PAIR, 3, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
-    else if (p->terms == 2) k_tc_gemm<PAIR, 2, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
-    else k_tc_gemm<PAIR, 1, NMAX><<<p->sms, Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st>>>(a, maps);
+cudaError_t launch_n(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st, int *nl) {
+    return sp_launch(p->terms == 3 ? k_tc_gemm<PAIR, 3, NMAX> : p->terms == 2 ? k_tc_gemm<PAIR, 2, NMAX> : k_tc_gemm<PAIR, 1, NMAX>,
+                     dim3((unsigned)p->sms), Cfg<NMAX>::kThreads, Cfg<NMAX>::kSmem, st, nl, a, maps);
 }
 /* the GEMMs of one launch, at most two (the shared expert's and the routed experts') */
 struct Launch {
@@ -669,10 +692,8 @@ struct Launch {
     cudaError_t go(bool pair, int nmax, cudaStream_t st, int *nl) {
         if (err != cudaSuccess) return err;
         for (int i = a.nseg; i < 2; i++) { maps.hi[i] = maps.hi64[i] = maps.hi[0]; maps.lo[i] = maps.lo64[i] = maps.lo[0]; maps.codes[i][0] = maps.codes[i][1] = maps.codes[0][0]; a.K[i] = a.K[0]; }
-        if (pair) { if (nmax == 64) launch_n<true, 64>(p, a, maps, st); else launch_n<true, 32>(p, a, maps, st); }
-        else { if (nmax == 64) launch_n<false, 64>(p, a, maps, st); else launch_n<false, 32>(p, a, maps, st); }
-        (*nl)++;
-        return cudaGetLastError();
+        if (pair) return nmax == 64 ? launch_n<true, 64>(p, a, maps, st, nl) : launch_n<true, 32>(p, a, maps, st, nl);
+        return nmax == 64 ? launch_n<false, 64>(p, a, maps, st, nl) : launch_n<false, 32>(p, a, maps, st, nl);
     }
 };
 }  // namespace
@@ -681,9 +702,7 @@ cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M
                         const int *pairpos, float *dn, float *eo, int *status, cudaStream_t st, int *nl) {
     const int R = M * d.NU;
     if (!p || M > p->Mcap || (long long)M * d.NU > p->Rcap) return cudaErrorInvalidValue;
-    if (d.E < 512) {
-        /* geometries this small only check the stages: they stay one launch per stage, so that callers who count
-         * launches see each of them (the stages are the expert-parallel path's) */
+    if (!sp_tc_takes_split(d)) {
         k_tc_scan<<<1, 1024, 0, st>>>(count, d.NE, p->offsets); (*nl)++;
         k_tc_pairs<<<(R + 255) / 256, 256, 0, st>>>(sel_asc, pairpos, p->offsets, R, d.NU, p->gather, p->rowmap); (*nl)++;
         const cudaError_t e = sp_tc_shared_expert(p, d, L, M, nx, dn, status, st, nl, 0);
@@ -691,12 +710,13 @@ cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M
     }
     const int nmax = tile_rows(d.NE, R);
     SortArgs s{count, sel_asc, pairpos, d.NE, M, d.NU, nmax, p->gather, p->rowmap, p->tiles_r, p->ntiles_r, p->tiles_sh, p->ntiles_sh, p->cap_r, p->cap_sh};
-    k_tc_sort<<<(R + 1023) / 1024, 1024, 0, st>>>(s); (*nl)++;
-    k_tc_split<<<M, 256, 0, st>>>(nx, nullptr, d.E, p->nx_hi, p->nx_lo); (*nl)++;
-    k_tc_split<<<R, 256, 0, st>>>(in, p->gather, d.E, p->in_hi, p->in_lo); (*nl)++;
+    cudaError_t e = sp_launch(k_tc_sort, dim3((unsigned)((R + 1023) / 1024)), 1024, 0, st, nl, s);
+    if (e != cudaSuccess) return e;
+    e = sp_launch(k_tc_permute, dim3((unsigned)R), (unsigned)((d.E / 8 + 31) & ~31), 0, st, nl, p->tk_hi, p->tk_lo, p->gather, d.E, p->in_hi, p->in_lo);
+    if (e != cudaSuccess) return e;
     Launch up(p, d, L, status);
     up.shared_up(); up.routed_up();
-    cudaError_t e = up.go(true, nmax, st, nl);
+    e = up.go(true, nmax, st, nl);
     if (e != cudaSuccess) return e;
     Launch down(p, d, L, status);
     down.shared_down(dn); down.routed_down(eo, p->rowmap);

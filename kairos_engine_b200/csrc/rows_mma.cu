@@ -21,6 +21,7 @@
  * eight rows on the same banks.
  */
 #include "rows_mma.cuh"
+#include "launch.cuh"
 #include <cstring>
 
 namespace {
@@ -203,6 +204,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    sp_pdl_wait();
+    sp_pdl_next();
     /* first unit of every group, per segment (segment 0 is the only one or has one group) */
     if (warp == 0) {
         int at = 0;
@@ -418,7 +421,5 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *statu
     if (e != cudaSuccess) return e;
     const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32 + 32 * a.teams);
     const size_t smem = acts + (size_t)a.stages * a.stage_bytes;
-    if (pair) k_rows<true><<<(unsigned)sms, threads, smem, st>>>(a); else k_rows<false><<<(unsigned)sms, threads, smem, st>>>(a);
-    (*nl)++;
-    return cudaGetLastError();
+    return sp_launch(pair ? k_rows<true> : k_rows<false>, dim3((unsigned)sms), threads, smem, st, nl, a);
 }
