@@ -254,6 +254,7 @@ static int check_forward(sp_moe *h, int lf, int nl, int flavour, int M, const vo
     return SP_MOE_OK;
 }
 
+constexpr int kDirectLayers = 4;
 extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
                                   const float *x_dev, float *y_dev, int32_t *sel_dev, float *wts_dev, void *stream) {
     int rc = check_forward(h, lf, nl, flavour, M, x_dev, y_dev, "sp_moe_forward_dev");
@@ -263,6 +264,16 @@ extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
     h->last_stream = st;
     if (M <= h->seq_tokens && flavour == SP_MOE_FLAVOUR_DECODE) {
         /* One token (or, by the switch, a few of them one after the other) replays the single-token graph. */
+        if (M == 1 && nl <= kDirectLayers) {
+            /* a short run (an engine with attention between the layers calls once per layer): launched as it is, on the
+             * caller's stream and pointers. A graph would add two copies and its own start to three kernels per layer. */
+            int nlaunch = 0;
+            const cudaError_t e = h->decode_impl == 0
+                ? sp_staged_decode_enqueue(h->d, h->layers_host.data(), lf, nl, x_dev, y_dev, sel_dev, wts_dev, h->gs, h->sms, h->staged_flags, h->stamps, st, true, &nlaunch)
+                : sp_graph_decode_enqueue(h->d, h->layers_host.data(), lf, nl, x_dev, y_dev, sel_dev, wts_dev, h->gs, h->sms, st, true, &nlaunch);
+            h->launches += (uint64_t)nlaunch;
+            return e == cudaSuccess ? SP_MOE_OK : fail_cuda(e, "decode launch");
+        }
         const bool routing = sel_dev || wts_dev;
         sp_moe::DecodeGraph *dg = nullptr;
         for (auto &g : h->graphs) if (g.lf == lf && g.nl == nl && g.routing == routing) dg = &g;

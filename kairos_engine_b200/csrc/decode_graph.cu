@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(kT, 1) k_dg_finish(GArgs a, float *y) {
     for (int k = 0; k < KE; k++) { const int i = t + kT * k; const bool in = i < E;
         w1[k] = in ? __ldg(a.s.prev_post_ffw1 + i) : 0.0f; w2[k] = in ? __ldg(a.s.prev_post_ffw2 + i) : 0.0f; w3[k] = in ? __ldg(a.s.prev_post_ffw + i) : 0.0f; }
     pdl_wait();
+    pdl_launch();
 #pragma unroll
     for (int k = 0; k < KE; k++) { const int i = t + kT * k; const bool in = i < E; dn[k] = in ? __ldcg(a.s.dn + i) : 0.0f; ac[k] = in ? __ldcg(a.s.acc + i) : 0.0f; x[k] = in ? __ldcg(a.x_prev + i) : 0.0f; }
     double p1 = 0.0, p2 = 0.0;
@@ -581,7 +582,7 @@ cudaError_t sp_graph_decode_enqueue(const SpDims &d, const SpLayerDev *layers_ho
         if (li > 0) { a.s.prev_post_ffw1 = layers_host[lf + li - 1].post_ffw1; a.s.prev_post_ffw2 = layers_host[lf + li - 1].post_ffw2; a.s.prev_post_ffw = layers_host[lf + li - 1].post_ffw; }
         a.sel_out = sel ? sel + (size_t)li * NU : nullptr; a.wts_out = wts ? wts + (size_t)li * NU : nullptr;
         a.has_next = li + 1 < nl; if (a.has_next) a.Ln = layers_host[lf + li + 1];
-        e = (E <= 6 * kT) ? launch_pdl(k_dg_router_shared<6>, grid, sm1, st, pdl && li > 0, a) : launch_pdl(k_dg_router_shared<8>, grid, sm1, st, pdl && li > 0, a); (*nlaunch)++;
+        e = (E <= 6 * kT) ? launch_pdl(k_dg_router_shared<6>, grid, sm1, st, pdl, a) : launch_pdl(k_dg_router_shared<8>, grid, sm1, st, pdl, a); (*nlaunch)++;
         if (e == cudaSuccess) { e = launch_pdl(k_dg_experts_up, grid, sm2, st, pdl, a); (*nlaunch)++; }
         if (e == cudaSuccess) { e = launch_pdl(k_dg_experts_down, grid, sm3, st, pdl, a); (*nlaunch)++; }
     }
