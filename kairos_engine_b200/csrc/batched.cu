@@ -25,10 +25,9 @@ namespace {
 
 struct BView {                 /* carved scratch */
     float *rin, *nx_f, *in_f, *logits, *cw, *hd, *dn, *h, *eo, *xa, *xb;
-    signed char *nx_q, *in_q, *hd_q, *h_q;
-    float *nx_s, *in_s, *hd_s, *h_s;
+    unsigned char *nx_q, *in_q, *hd_q, *h_q;      /* quantised rows, sp_act_pitch apart */
     int *sel_asc, *count, *list, *pairpos, *ep_off;
-    signed char *ep_q; float *ep_s;      /* expert-parallel stage: quantised received rows, [max_rows] */
+    unsigned char *ep_q;      /* expert-parallel stage: quantised received rows, [max_rows] */
 };
 
 size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -42,23 +41,21 @@ size_t blayout(const SpDims &d, int Mx, int Rx, F place) {
     take(4 * M * E); take(4 * M * E); take(4 * M * E); take(4 * M * NE); take(4 * M * NU);            /* rin nx_f in_f logits cw */
     take(4 * M * FFS); take(4 * M * E); take(4 * R * FFE); take(4 * M * NU * E);                     /* hd dn h eo */
     take(4 * M * E); take(4 * M * E);                                                               /* xa xb */
-    take(M * E); take(M * E); take(M * FFS); take(R * FFE);                                          /* q */
-    take(4 * M * sp_sx_row(d.E)); take(4 * M * sp_sx_row(d.E)); take(4 * M * sp_sx_row(d.FFS)); take(4 * R * sp_sx_row(d.FFE));        /* s */
+    take(M * sp_act_pitch(d.E)); take(M * sp_act_pitch(d.E)); take(M * sp_act_pitch(d.FFS)); take(R * sp_act_pitch(d.FFE));        /* q */
     take(4 * M * NU); take(4 * NE * kSlices); take(4 * NE * M);                                     /* sel_asc count list */
-    take(R * E); take(4 * R * sp_sx_row(d.E));                                                        /* ep_q ep_s */
+    take(R * sp_act_pitch(d.E));                                                                     /* ep_q */
     take(4 * M * NU); take(4 * (NE + 1) * kSlices);                                                 /* pairpos ep_off */
     return o;
 }
 BView bview(const SpDims &d, const SpBatchedScratch *s) {
-    unsigned char *p[26];
+    unsigned char *p[21];
     blayout(d, s->max_tokens, s->max_rows, [&](int id, size_t off) { p[id] = (unsigned char *)s->base + off; });
     BView v;
     v.rin = (float *)p[0]; v.nx_f = (float *)p[1]; v.in_f = (float *)p[2]; v.logits = (float *)p[3]; v.cw = (float *)p[4];
     v.hd = (float *)p[5]; v.dn = (float *)p[6]; v.h = (float *)p[7]; v.eo = (float *)p[8]; v.xa = (float *)p[9]; v.xb = (float *)p[10];
-    v.nx_q = (signed char *)p[11]; v.in_q = (signed char *)p[12]; v.hd_q = (signed char *)p[13]; v.h_q = (signed char *)p[14];
-    v.nx_s = (float *)p[15]; v.in_s = (float *)p[16]; v.hd_s = (float *)p[17]; v.h_s = (float *)p[18];
-    v.sel_asc = (int *)p[19]; v.count = (int *)p[20]; v.list = (int *)p[21];
-    v.ep_q = (signed char *)p[22]; v.ep_s = (float *)p[23]; v.pairpos = (int *)p[24]; v.ep_off = (int *)p[25];
+    v.nx_q = p[11]; v.in_q = p[12]; v.hd_q = p[13]; v.h_q = p[14];
+    v.sel_asc = (int *)p[15]; v.count = (int *)p[16]; v.list = (int *)p[17];
+    v.ep_q = p[18]; v.pairpos = (int *)p[19]; v.ep_off = (int *)p[20];
     return v;
 }
 /* The same scratch seen by token slice `slice` of a layer, whose first token is `t0`: everything the route stage
@@ -70,8 +67,7 @@ BView bview_slice(const SpDims &d, const SpBatchedScratch *s, int t0, int slice)
     BView v = bview(d, s);
     const size_t E = d.E, NE = d.NE, NU = d.NU, FFS = d.FFS, t = (size_t)t0;
     v.rin += t * E; v.nx_f += t * E; v.in_f += t * E; v.logits += t * NE; v.cw += t * NU; v.hd += t * FFS; v.dn += t * E; v.eo += t * NU * E;
-    v.nx_q += t * E; v.in_q += t * E; v.hd_q += t * FFS;
-    v.nx_s += t * sp_sx_row(d.E); v.in_s += t * sp_sx_row(d.E); v.hd_s += t * sp_sx_row(d.FFS);
+    v.nx_q += t * sp_act_pitch(d.E); v.in_q += t * sp_act_pitch(d.E); v.hd_q += t * sp_act_pitch(d.FFS);
     v.sel_asc += t * NU; v.pairpos += t * NU; v.list += t * NE;
     v.count += (size_t)slice * NE; v.ep_off += (size_t)slice * (NE + 1);
     return v;
@@ -100,7 +96,7 @@ struct TokArgs {
     const float *x;
     const float *dn, *eo, *cw; const int *pair_index; const float *post_ffw1, *post_ffw2, *post_ffw; float *y;       /* FIN */
     const float *ffn_norm, *pre_ffw2, *router_scale; float *rin; int *count;                                         /* PREP */
-    signed char *nx_q, *in_q; float *nx_s, *in_s; float *nx_f, *in_f, *rows_f; __half *nx_hi, *nx_lo, *in_hi, *in_lo;
+    unsigned char *nx_q, *in_q; float *nx_f, *in_f, *rows_f; __half *nx_hi, *nx_lo, *in_hi, *in_lo;
 };
 /* block-wide sums: shuffle tree per warp, then every warp adds the (at most 16) warps' sums by a second tree. `red` has 16
  * slots per sum, used once. */
@@ -127,17 +123,17 @@ __device__ __forceinline__ float4 scale4(const float4 &f, float s, const float4 
     return make_float4(__fmul_rn(__fmul_rn(f.x, s), w.x), __fmul_rn(__fmul_rn(f.y, s), w.y), __fmul_rn(__fmul_rn(f.z, s), w.z), __fmul_rn(__fmul_rn(f.w, s), w.w));
 }
 /* four elements of a 16-block, four threads per block: quant_elem16's arithmetic and layout */
-__device__ __forceinline__ void quant_quad(const float4 &f, bool ok, int i, signed char *q, float *sx) {
+__device__ __forceinline__ void quant_quad(const float4 &f, bool ok, int i, unsigned char *act, int n) {
     float m = fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w)));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1)); m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
     const float scale = m > 0.0f ? __fmul_rn(m, 1.0f / 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, scale);
     auto one = [&](float v) { int t = __float2int_rn(__fmul_rn(v, inv)); t = t > 127 ? 127 : t; return t < -127 ? -127 : t; };
     const int a = one(f.x), b = one(f.y), c = one(f.z), d = one(f.w);
     if (ok) {
-        signed char *g = q + 8 * (i >> 1) + 2 * (i & 1);        /* the even elements of a group of 8, then the odd ones */
+        unsigned char *g = act + 8 * (i >> 1) + 2 * (i & 1);        /* the even elements of a group of 8, then the odd ones */
         *reinterpret_cast<unsigned short *>(g) = (unsigned short)((a & 0xFF) | ((c & 0xFF) << 8));
         *reinterpret_cast<unsigned short *>(g + 4) = (unsigned short)((b & 0xFF) | ((d & 0xFF) << 8));
-        if ((i & 3) == 0) sx[i >> 2] = scale;
+        if ((i & 3) == 0) reinterpret_cast<float *>(act + n)[i >> 2] = scale;
     }
 }
 /* four elements of a group of 8, two threads per group: fp16 hi and lo in the order 0,4,1,5,2,6,3,7; the lower thread
@@ -246,9 +242,8 @@ __global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_
                 reinterpret_cast<float4 *>(a.rin + row)[i] = scale4(xs, d.inv_sqrt_e, vec(5, h));
             }
             if (OUT == kOutInt8) {
-                const size_t b = (size_t)t * sp_sx_row(E);
-                quant_quad(n, ok[h], i, a.nx_q + row, a.nx_s + b);
-                quant_quad(in, ok[h], i, a.in_q + row, a.in_s + b);
+                quant_quad(n, ok[h], i, a.nx_q + (size_t)t * sp_act_pitch(E), E);
+                quant_quad(in, ok[h], i, a.in_q + (size_t)t * sp_act_pitch(E), E);
             } else if (OUT == kOutSplit) {
                 split_quad(n, ok[h], i, a.nx_hi + row, a.nx_lo + row);
                 split_quad(in, ok[h], i, a.in_hi + row, a.in_lo + row);
@@ -272,7 +267,7 @@ cudaError_t launch_token(const SpDims &d, int M, const TokArgs &a, cudaStream_t 
 }
 void set_prep(TokArgs &a, const SpLayerDev &L, const BView &v, SpTcPlan *split) {
     a.ffn_norm = L.ffn_norm; a.pre_ffw2 = L.pre_ffw2; a.router_scale = L.router_scale; a.rin = v.rin; a.count = v.count;
-    a.nx_q = v.nx_q; a.in_q = v.in_q; a.nx_s = v.nx_s; a.in_s = v.in_s; a.nx_f = v.nx_f; a.in_f = v.in_f;
+    a.nx_q = v.nx_q; a.in_q = v.in_q; a.nx_f = v.nx_f; a.in_f = v.in_f;
     if (split) sp_tc_inputs(split, &a.nx_hi, &a.nx_lo, &a.in_hi, &a.in_lo);
 }
 void set_finish(TokArgs &a, const SpLayerDev &L, const BView &v, const float *eo, const int *pair_index, float *y) {
@@ -503,14 +498,14 @@ cudaError_t launch_topk(const SpDims &d, const SpLayerDev &L, BView &v, int M, i
 }
 
 /* ---------------------------------------------------------------- per-row activation quant (CF:1725-1746): received rows of an expert-parallel run */
-__global__ void __launch_bounds__(1024) k_b_quant_rows(const float *x, int n, signed char *q, float *sx) {
+__global__ void __launch_bounds__(1024) k_b_quant_rows(const float *x, int n, unsigned char *act) {
     const size_t r = blockIdx.x;
     const int i = threadIdx.x;
     const bool ok = 4 * i < n;
     sp_pdl_wait();
     sp_pdl_next();
     const float4 f = ok ? reinterpret_cast<const float4 *>(x + r * n)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    quant_quad(f, ok, i, q + r * n, sx + r * sp_sx_row(n));
+    quant_quad(f, ok, i, act + r * sp_act_pitch(n), n);
 }
 
 /* ---------------------------------------------------------------- K4/K6, floating-point flavour without the tensor cores
@@ -622,25 +617,25 @@ void launch_rows(const GroupArgs &g, int groups, cudaStream_t st, int *nl) {
 SpRowsSeg seg_shared_up(const SpDims &d, const SpLayerDev &L, int M, const BView &v) {
     SpRowsSeg s{};
     s.codes = L.sg_codes; s.bs = L.sg_bs; s.ucodes = L.su_codes; s.ubs = L.su_bs; s.in = d.E; s.rows = d.FFS; s.groups = 1; s.M = M; s.act_div = 1;
-    s.q = v.nx_q; s.sx = v.nx_s; s.out_q = v.hd_q; s.out_s = v.hd_s;
+    s.act = v.nx_q; s.out_act = v.hd_q;
     return s;
 }
 SpRowsSeg seg_shared_down(const SpDims &d, const SpLayerDev &L, int M, const BView &v) {
     SpRowsSeg s{};
     s.codes = L.sd_codes; s.bs = L.sd_bs; s.in = d.FFS; s.rows = d.E; s.groups = 1; s.M = M; s.act_div = 1;
-    s.q = v.hd_q; s.sx = v.hd_s; s.out_f = v.dn; s.out_stride = d.E;
+    s.act = v.hd_q; s.out_f = v.dn; s.out_stride = d.E;
     return s;
 }
-SpRowsSeg seg_routed_up(const SpDims &d, const SpLayerDev &L, int M, const signed char *q, const float *sx, const BView &v) {
+SpRowsSeg seg_routed_up(const SpDims &d, const SpLayerDev &L, int M, const unsigned char *act, const BView &v) {
     SpRowsSeg s{};
     s.codes = s.ucodes = L.gu_codes; s.bs = s.ubs = L.gu_bs; s.rows_per_group = 2LL * d.FFE; s.up_off = d.FFE; s.in = d.E; s.rows = d.FFE; s.groups = d.NE;
-    s.M = M; s.act_div = 1; s.q = q; s.sx = sx; s.out_q = v.h_q; s.out_s = v.h_s;
+    s.M = M; s.act_div = 1; s.act = act; s.out_act = v.h_q;
     return s;
 }
 SpRowsSeg seg_routed_down(const SpDims &d, const SpLayerDev &L, int M, const BView &v, float *out) {
     SpRowsSeg s{};
     s.codes = L.dn_codes; s.bs = L.dn_bs; s.rows_per_group = d.E; s.in = d.FFE; s.rows = d.E; s.groups = d.NE; s.M = M; s.act_div = 1;
-    s.q = v.h_q; s.sx = v.h_s; s.out_f = out; s.out_stride = d.E;
+    s.act = v.h_q; s.out_f = out; s.out_stride = d.E;
     return s;
 }
 
@@ -651,7 +646,7 @@ cudaError_t run_experts(const SpDims &d, const SpLayerDev &L, int M, BView &v, S
     if (!FA && tc) return sp_tc_layer(tc, d, L, M, v.nx_f, v.in_f, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);      /* prefill arithmetic on the tensor cores */
     if (FA) {
         /* gate|up of the shared and the routed experts, quantised as it leaves (CF:8348-8356, 8733-8737, 8958-8959), then down (CF:8358, 8739-8742, 8961) */
-        SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v.in_s, v)};
+        SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v)};
         up[1].count = v.count; up[1].list = v.list; up[1].list_stride = M; up[1].act_div = NU;
         const cudaError_t e = sp_rows_launch(up, 2, true, status, st, nl);
         if (e != cudaSuccess) return e;
@@ -915,9 +910,9 @@ cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float 
     if (R == 0) return cudaSuccess;
     if (!FA && tc) return sp_tc_routed(tc, d, L, R, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
     if (FA) {
-        cudaError_t e = sp_launch(k_b_quant_rows, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q, v.ep_s);
+        cudaError_t e = sp_launch(k_b_quant_rows, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q);
         if (e != cudaSuccess) return e;
-        SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v.ep_s, v), down = seg_routed_down(d, L, R, v, rows_out);
+        SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v), down = seg_routed_down(d, L, R, v, rows_out);
         up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */
         e = sp_rows_launch(&up, 1, true, status, st, nl);
         return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, status, st, nl);

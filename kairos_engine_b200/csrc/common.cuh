@@ -210,8 +210,8 @@ __device__ __forceinline__ void quant_elem16(float v, bool valid, signed char *d
     }
 }
 
-/* floats between the block-scale rows of quantised activations: [row][n / 16], rows padded to whole 16-byte pieces */
-__host__ __device__ __forceinline__ int sp_sx_row(int n) { return (n / 16 + 3) & ~3; }
+/* bytes between rows of quantised activations of n elements: n int8, then n / 16 fp32 block scales, in whole 16-byte pieces */
+__host__ __device__ __forceinline__ int sp_act_pitch(int n) { return n + 4 * ((n / 16 + 3) & ~3); }
 
 /* ---------------------------------------------------------------- block-wide f64 sum of squares (CF:497-514)
  * The reference sums in double with 256 strided threads and a halving tree. This keeps the

@@ -15,13 +15,15 @@
  *     quantisation block: it leaves the kernel as int8 codes and a scale, ready for the down rows.
  *
  * Work is cut into units of ~50 KB of weights x up to 16 tokens. One CTA per SM; one warp asks the copy engine for the
- * units' rows (cp.async.bulk, a ring of stages), two teams of eight warps consume them alternately, and a warp per team
- * has the activations of its next four tokens copied while it multiplies the current four. So the weight stream does not
- * stop between units, and experts nobody chose cost nothing. Row copies are padded in shared memory where a row's length would put
- * eight rows on the same banks.
+ * units' rows (a ring of stages), two teams of eight warps consume them alternately, and a warp per team has the activations
+ * of its next four tokens copied while it multiplies the current four. So the weight stream does not stop between units,
+ * and experts nobody chose cost nothing. A unit's codes are one or two tensor copies (a box of all 128-byte slices of 16 to
+ * 128 rows, swizzled, so that the eight rows an MMA operand takes lie on different banks): a copy costs its warp ~85 cycles
+ * whatever its size, and a copy per row (for padded rows) took longer than the multiplication.
  */
 #include "rows_mma.cuh"
 #include "launch.cuh"
+#include "tc_common.cuh"
 #include <cstring>
 
 namespace {
@@ -33,28 +35,28 @@ constexpr unsigned kSpin = 1u << 15, kWaitNs = 20000;
 
 struct SegGeo {                                    /* what the copies and the dots need of a segment's shape */
     int tiles, mt_n, n32;                          /* weight tiles per group, 16-row MMA tiles of one, chunks of a row */
-    unsigned rb, sb, stride, scale_off;            /* bytes of a row's codes / scales; row stride and where the scales start in a stage */
-    unsigned ast, sst, sx_off;                     /* bytes between tokens, floats between their scale rows, where those start in a buffer */
+    unsigned sb, box_bytes, scale_off;             /* bytes of a row's scales, of one box of codes; where the scales start in a stage */
+    unsigned ast;                                  /* bytes between tokens in a buffer */
 };
 struct RowsArgs {
     SpRowsSeg seg[2]; SegGeo geo[2]; int nseg;
     int stages, teams;
     unsigned stage_bytes, act_bytes;               /* one stage; one buffer of four tokens */
     int *status;
+    CUtensorMap codes[2][2];                       /* [segment][gate or only / up] */
 };
 
 /* shapes in shared memory */
-unsigned up128(unsigned v) { return (v + 127u) & ~127u; }
+unsigned up1024(unsigned v) { return (v + 1023u) & ~1023u; }
+int box_rows(const SegGeo &g, bool pair) { return pair ? 16 : 16 * g.mt_n; }
 SegGeo seg_geo(const SpRowsSeg &s, bool pair) {
     SegGeo g;
     g.mt_n = pair ? 2 : (s.in <= 1024 ? 8 : 2);
-    const int per = pair ? 16 : 16 * g.mt_n;                /* output rows of a unit */
-    g.tiles = (s.rows + per - 1) / per; g.n32 = s.in / 32; g.rb = s.in / 2; g.sb = s.in / 16;
-    g.stride = pair ? (g.rb % 32 == 0 ? g.rb + 16 : g.rb) : (g.rb % 64 == 0 ? g.rb + 16 : g.rb);   /* plain: two-way conflicts are left, such rows are copied in one piece */
-    g.scale_off = up128(16 * g.mt_n * g.stride);
-    g.ast = s.in + (32 - s.in % 128 + 128) % 128;           /* = 32 mod 128: four tokens on four bank groups */
-    g.sst = s.in / 16 + (8 - (s.in / 16) % 32 + 32) % 32;   /* = 8 mod 32 */
-    g.sx_off = up128(kTok * g.ast);
+    const int per = box_rows(g, pair);                      /* output rows of a unit */
+    g.tiles = (s.rows + per - 1) / per; g.n32 = s.in / 32; g.sb = s.in / 16;
+    g.box_bytes = 128u * per * ((s.in / 2 + 127) / 128);
+    g.scale_off = (pair ? 2 : 1) * g.box_bytes;
+    g.ast = (unsigned)sp_act_pitch(s.in); g.ast += (32 - g.ast % 128 + 128) % 128;         /* = 32 mod 128: four tokens on four bank groups */
     return g;
 }
 
@@ -79,6 +81,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity, volatil
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+/* a box of codes: all 128-byte slices of some consecutive rows, slice-major, 128-byte swizzle */
+__device__ __forceinline__ void box_g2s(uint32_t dst, const CUtensorMap *map, int row, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%4, %2, %4}], [%3];" ::"r"(dst), "l"(map), "r"(row), "r"(bar), "r"(0) : "memory");
+}
 __device__ __forceinline__ void expect_tx(uint32_t bar, unsigned bytes) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -98,6 +104,7 @@ __device__ __forceinline__ float magic_to_float(int c) { return __fmaf_rn(__int_
 struct Unit { int seg, grp, tile, t0, nt, pad[3]; };        /* weight tile `tile` of group grp x its tokens [t0, t0 + nt) */
 struct Plan {                                               /* in shared memory: first unit of every group, per segment */
     const int *start[2]; int total[2];
+    const int *count;                                       /* items of segment 1's groups while the table is in place, else NULL */
 };
 __device__ __forceinline__ int group_first(const SpRowsSeg &s, int g) {
     if (!s.offset) return 0;
@@ -119,7 +126,7 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     int lo = 0, hi = s.groups - 1;                          /* the last group that starts at or before u: never an empty one */
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (st[mid] <= u) lo = mid; else hi = mid - 1; }
     r.grp = lo;
-    const int cnt = group_count(s, lo), nr = (cnt + kUnitTok - 1) / kUnitTok, k = u - st[lo];
+    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), nr = (cnt + kUnitTok - 1) / kUnitTok, k = u - st[lo];
     r.tile = k / nr;
     r.t0 = (k - r.tile * nr) * kUnitTok;
     r.nt = cnt - r.t0 < kUnitTok ? cnt - r.t0 : kUnitTok;
@@ -133,26 +140,31 @@ struct Frag {
     const unsigned char *b;            /* token g >> 1, this lane's 8 bytes of a chunk */
     const float *sx;                   /* token q's block scales */
     bool bvalid;                       /* the lane's k-slots lie in its column's half */
-    int n32;
+    int n32, gq;
 };
 /* slots r, r + 4, ..., r + 28 (chunks s + 32 i of each), added as the tree adds them: s and s + 16, then + 8, then + 4.
- * Rows of one chunk per slot may have fewer than 32: slots from 4 * NJ on are known to be empty (NJ even). */
-template <int NI, int NJ = 8>
+ * Rows of one chunk per slot may have fewer than 32: slots from 4 * NJ on are known to be empty (NJ even). Chunk c of a row
+ * is piece c % 8 of slice c / 8 (SL bytes apart), swizzled by the row. */
+template <int SL, int NI, int NJ = 8>
 __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
+    const unsigned p = (unsigned)((r ^ f.gq) << 4);
+    const unsigned char *const w0e = f.w0 + p, *const w0o = f.w0 + (p ^ 64u), *const w1e = f.w1 + p, *const w1o = f.w1 + (p ^ 64u);
+    const unsigned char *const b0 = f.b + 32 * r, *const s0 = f.s0 + 2 * r, *const s1 = f.s1 + 2 * r;
+    const float *const x0 = f.sx + 2 * r;
     auto slot = [&](int j) {
         float2 acc = make_float2(0.0f, 0.0f);
         if (j >= NJ) return acc;
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-            const int c = r + 4 * j + 32 * i;
-            if (i + 1 < NI || c < f.n32) {                  /* warp-uniform */
-                const unsigned x0 = *reinterpret_cast<const unsigned *>(f.w0 + 16 * c), x1 = *reinterpret_cast<const unsigned *>(f.w1 + 16 * c);
+            const int c = 4 * j + 32 * i, at = ((j >> 1) + 4 * i) * SL;      /* c: beyond r */
+            if (i + 1 < NI || r + c < f.n32) {              /* warp-uniform */
+                const unsigned u0 = *reinterpret_cast<const unsigned *>((j & 1 ? w0o : w0e) + at), u1 = *reinterpret_cast<const unsigned *>((j & 1 ? w1o : w1e) + at);
                 uint2 b = make_uint2(0u, 0u);
-                if (f.bvalid) b = *reinterpret_cast<const uint2 *>(f.b + 32 * c);
-                const float2 s2 = *reinterpret_cast<const float2 *>(f.sx + 2 * c);
-                const float ws0 = h2f(*reinterpret_cast<const unsigned short *>(f.s0 + 2 * c)), ws1 = h2f(*reinterpret_cast<const unsigned short *>(f.s1 + 2 * c));
+                if (f.bvalid) b = *reinterpret_cast<const uint2 *>(b0 + 32 * c);
+                const float2 s2 = *reinterpret_cast<const float2 *>(x0 + 2 * c);
+                const float ws0 = h2f(*reinterpret_cast<const unsigned short *>(s0 + 2 * c)), ws1 = h2f(*reinterpret_cast<const unsigned short *>(s1 + 2 * c));
                 int d[4];
-                mma_s8(d, (x0 << 4) & 0xF0F0F0F0u, (x1 << 4) & 0xF0F0F0F0u, x0 & 0xF0F0F0F0u, x1 & 0xF0F0F0F0u, b.x, b.y, kMagic);
+                mma_s8(d, (u0 << 4) & 0xF0F0F0F0u, (u1 << 4) & 0xF0F0F0F0u, u0 & 0xF0F0F0F0u, u1 & 0xF0F0F0F0u, b.x, b.y, kMagic);
                 acc.x = __fmaf_rn(ws0, __fmaf_rn(magic_to_float(d[0]), s2.x, __fmul_rn(magic_to_float(d[1]), s2.y)), acc.x);
                 acc.y = __fmaf_rn(ws1, __fmaf_rn(magic_to_float(d[2]), s2.x, __fmul_rn(magic_to_float(d[3]), s2.y)), acc.y);
             }
@@ -164,11 +176,12 @@ __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
     float2 b = add(slot(1), slot(5)); b = add(b, add(slot(3), slot(7)));
     return add(a, b);
 }
+template <int SL>
 __device__ __forceinline__ float2 class_sum_n(const Frag &f, int r) {
-    if (f.n32 <= 32) return class_sum<1>(f, r);
-    if (f.n32 <= 64) return class_sum<2>(f, r);
-    if (f.n32 <= 96) return class_sum<3>(f, r);
-    return class_sum<4>(f, r);
+    if (f.n32 <= 32) return class_sum<SL, 1>(f, r);
+    if (f.n32 <= 64) return class_sum<SL, 2>(f, r);
+    if (f.n32 <= 96) return class_sum<SL, 3>(f, r);
+    return class_sum<SL, 4>(f, r);
 }
 
 /* ---------------------------------------------------------------- the kernel
@@ -177,7 +190,8 @@ struct Batch { int seg, tile, flags, item[kTok], pad; };     /* four tokens of a
 
 template <bool PAIR>
 __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const __grid_constant__ RowsArgs a) {
-    extern __shared__ __align__(128) unsigned char sm[];
+    extern __shared__ unsigned char sm_raw[];
+    unsigned char *const sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
     __shared__ unsigned long long bars[2 * kMaxStages + 4 * kMaxTeams];
     __shared__ int abort_s;
     __shared__ Batch batch_s[kMaxTeams][2];
@@ -207,6 +221,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     sp_pdl_wait();
     sp_pdl_next();
     /* first unit of every group, per segment (segment 0 is the only one or has one group) */
+    int *const count_s = reinterpret_cast<int *>(part_s);     /* until the teams start */
     if (warp == 0) {
         int at = 0;
         for (int k = 0; k < 2; k++) {
@@ -215,7 +230,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const SpRowsSeg &s = a.seg[k];
                 for (int g0 = 0; g0 < s.groups; g0 += 32) {
                     const int g = g0 + lane;
-                    const int n = g < s.groups ? a.geo[k].tiles * ((group_count(s, g) + kUnitTok - 1) / kUnitTok) : 0;
+                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * ((cnt + kUnitTok - 1) / kUnitTok);
+                    if (k == 1 && g < s.groups) count_s[g] = cnt;
                     int v = n;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t; }
@@ -229,9 +245,10 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     }
     __syncthreads();
     Plan plan;
-    plan.start[0] = start_s; plan.start[1] = start_s + a.seg[0].groups; plan.total[0] = total_s[0]; plan.total[1] = total_s[1];
+    plan.start[0] = start_s; plan.start[1] = start_s + a.seg[0].groups; plan.total[0] = total_s[0]; plan.total[1] = total_s[1]; plan.count = count_s;
     const int total = plan.total[0] + plan.total[1], G = gridDim.x;
     for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = locate(a, plan, blockIdx.x + i * G);
+    plan.count = nullptr;
     __syncthreads();
     const int mine = total > (int)blockIdx.x ? (total - blockIdx.x + G - 1) / G : 0;
     auto unit = [&](int i) { return i < kUnits ? units_s[i] : locate(a, plan, blockIdx.x + i * G); };
@@ -239,33 +256,27 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     bool failed = false;
 
     if (warp == a.teams * kTeamWarps) {
-        /* ---------------- weights: the rows of every unit, one lane per row copy */
-        for (int i = 0, s = 0, ph = 0; i < mine; i++) {
-            const Unit u = unit(i);
-            const SpRowsSeg &sg = a.seg[u.seg];
-            const SegGeo &ge = a.geo[u.seg];
-            if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-            const unsigned rb = ge.rb, sb = ge.sb, stride = ge.stride;
-            const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(s);
-            const size_t row0 = (size_t)((long long)u.grp * sg.rows_per_group);
-            if (PAIR) {
-                const int j0 = u.tile * 16, up = lane >> 4, col = lane & 15;
-                if (lane == 0) expect_tx(bar, 32 * (rb + sb));
-                __syncwarp();
-                const size_t row = row0 + j0 + (up ? sg.up_off : 0);
-                bulk_g2s(dst + ((col >> 3) * 16 + up * 8 + (col & 7)) * stride, (up ? sg.ucodes : sg.codes) + (row + col) * rb, rb, bar);
-                if (col == 0) bulk_g2s(sdst + up * 16 * sb, reinterpret_cast<const unsigned char *>(up ? sg.ubs : sg.bs) + row * sb, 16 * sb, bar);
-            } else {
-                const int per = 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
-                if (lane == 0) expect_tx(bar, nr * (rb + sb));
-                __syncwarp();
-                const unsigned char *src = sg.codes + (row0 + r0) * rb;
-                if (stride == rb) { if (lane == 0) bulk_g2s(dst, src, nr * rb, bar); }
-                else for (int r = lane; r < nr; r += 32) bulk_g2s(dst + r * stride, src + (size_t)r * rb, rb, bar);
-                if (lane == 0) bulk_g2s(sdst, reinterpret_cast<const unsigned char *>(sg.bs) + (row0 + r0) * sb, nr * sb, bar);
+        /* ---------------- weights */
+        if (lane == 0)
+            for (int i = 0, s = 0, ph = 0; i < mine; i++) {
+                const Unit u = unit(i);
+                const SpRowsSeg &sg = a.seg[u.seg];
+                const SegGeo &ge = a.geo[u.seg];
+                if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
+                const int per = PAIR ? 16 : 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
+                const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(s);
+                const int row = (int)((long long)u.grp * sg.rows_per_group) + r0;
+                const unsigned sbytes = (unsigned)nr * ge.sb;
+                expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
+                box_g2s(dst, &a.codes[u.seg][0], row, bar);
+                bulk_g2s(sdst, reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb, sbytes, bar);
+                if (PAIR) {
+                    box_g2s(dst + ge.box_bytes, &a.codes[u.seg][1], row + sg.up_off, bar);
+                    bulk_g2s(sdst + 16 * ge.sb, reinterpret_cast<const unsigned char *>(sg.ubs) + (size_t)(row + sg.up_off) * ge.sb, sbytes, bar);
+                }
+                if (++s == a.stages) { s = 0; ph ^= 1; }
             }
-            if (++s == a.stages) { s = 0; ph ^= 1; }
-        }
+        __syncwarp();
     } else if (warp > a.teams * kTeamWarps) {
         /* ---------------- activations of one team: four tokens ahead of it, one lane per token */
         const int team = warp - a.teams * kTeamWarps - 1;
@@ -290,13 +301,10 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 if (lane < kTok) d->item[lane] = item;
                 if (lane == 0) { d->seg = u.seg; d->tile = u.tile; d->flags = (b == 0 ? 1 : 0) | (b + kTok >= u.nt ? 2 : 0); }
                 __syncwarp();
-                if (lane == 0) expect_tx(afull(team, buf), (unsigned)have * ((unsigned)s.in + 4u * (unsigned)sp_sx_row(s.in)));        /* its arrival also publishes the descriptor */
+                if (lane == 0) expect_tx(afull(team, buf), (unsigned)have * (unsigned)sp_act_pitch(s.in));        /* its arrival also publishes the descriptor */
                 __syncwarp();
-                if (item >= 0) {
-                    const uint32_t qd = abase + buf * a.act_bytes + lane * ge.ast, sd = abase + buf * a.act_bytes + ge.sx_off + 4u * lane * ge.sst;
-                    bulk_g2s(qd, s.q + (size_t)arow * s.in, (unsigned)s.in, afull(team, buf));
-                    bulk_g2s(sd, s.sx + (size_t)arow * sp_sx_row(s.in), 4u * (unsigned)sp_sx_row(s.in), afull(team, buf));
-                }
+                if (item >= 0)
+                    bulk_g2s(abase + buf * a.act_bytes + lane * ge.ast, s.act + (size_t)arow * sp_act_pitch(s.in), (unsigned)sp_act_pitch(s.in), afull(team, buf));
             }
         }
         if (!failed) {                                      /* one more descriptor: nothing left */
@@ -313,7 +321,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
         int s = team % a.stages, ph = (team / a.stages) & 1;
         Frag f;
-        f.bvalid = (q >> 1) == (gq & 1);
+        f.bvalid = (q >> 1) == (gq & 1); f.gq = gq;
         for (int n = 0;; n++) {
             const int buf = n & 1;
             if (!mbar_wait(afull(team, buf), (n >> 1) & 1, abort_flag)) { failed = true; break; }
@@ -326,11 +334,10 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             if ((flags & 1) && !mbar_wait(full(s), ph, abort_flag)) { failed = true; break; }
             const int mt_n = PAIR ? 2 : ge.mt_n, mt = mt_n == 8 ? tw : tw >> 2, r0 = tile * 16 * mt_n;
             const unsigned char *codes = sm + (unsigned)s * a.stage_bytes, *scales = codes + ge.scale_off, *act = aptr + buf * a.act_bytes;
-            f.w0 = codes + (mt * 16 + gq) * ge.stride + 4 * q; f.w1 = f.w0 + 8 * ge.stride;
-            if (PAIR) { f.s0 = scales + (mt * 8 + gq) * ge.sb; f.s1 = f.s0 + 16 * ge.sb; }         /* gate rows, then the up rows */
-            else { f.s0 = scales + (mt * 16 + gq) * ge.sb; f.s1 = f.s0 + 8 * ge.sb; }
+            if (PAIR) { f.w0 = codes + (mt * 8 + gq) * 128 + 4 * q; f.w1 = f.w0 + ge.box_bytes; f.s0 = scales + (mt * 8 + gq) * ge.sb; f.s1 = f.s0 + 16 * ge.sb; }      /* gate rows, then the up rows */
+            else { f.w0 = codes + (mt * 16 + gq) * 128 + 4 * q; f.w1 = f.w0 + 8 * 128; f.s0 = scales + (mt * 16 + gq) * ge.sb; f.s1 = f.s0 + 8 * ge.sb; }
             f.b = act + (gq >> 1) * ge.ast + 8 * q;
-            f.sx = reinterpret_cast<const float *>(act + ge.sx_off) + q * ge.sst;
+            f.sx = reinterpret_cast<const float *>(act + q * ge.ast + sg.in);
             f.n32 = ge.n32;
             if (!PAIR && mt_n == 8) {
                 if (r0 + mt * 16 < sg.rows) {
@@ -338,7 +345,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
 #pragma unroll 1
                     for (int k = 0; k < 4; k++) {           /* classes 0, 2, 1, 3: (0 + 2) + (1 + 3) */
                         const int r = k == 1 ? 2 : k == 2 ? 1 : k;
-                        const float2 c = f.n32 <= 8 ? class_sum<1, 2>(f, r) : f.n32 <= 16 ? class_sum<1, 4>(f, r) : f.n32 <= 24 ? class_sum<1, 6>(f, r) : class_sum<1, 8>(f, r);
+                        const float2 c = f.n32 <= 8 ? class_sum<128 * 128, 1, 2>(f, r) : f.n32 <= 16 ? class_sum<128 * 128, 1, 4>(f, r) : f.n32 <= 24 ? class_sum<128 * 128, 1, 6>(f, r) : class_sum<128 * 128, 1, 8>(f, r);
                         if (k == 0 || k == 2) o = c;
                         else { o.x += c.x; o.y += c.y; if (k == 1) v = o; else { v.x += o.x; v.y += o.y; } }
                     }
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             } else {
                 float *part = part_s[team][buf];
                 if (PAIR || r0 + mt * 16 < sg.rows) {
-                    const float2 v = class_sum_n(f, tw & 3);
+                    const float2 v = class_sum_n<PAIR ? 16 * 128 : 32 * 128>(f, tw & 3);
                     float *p = part + (((tw & 3) * 2 + mt) * 16 + gq) * kTok + q;
                     p[0] = v.x; p[8 * kTok] = v.y;
                 }
@@ -366,7 +373,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                         const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
                         const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
                         const int it = bt.item[t] < 0 ? 0 : bt.item[t];
-                        quant_elem16(h, bt.item[t] >= 0, sg.out_q + (size_t)it * sg.rows + tile * 16, sg.out_s + (size_t)it * sp_sx_row(sg.rows) + tile);
+                        unsigned char *o = sg.out_act + (size_t)it * sp_act_pitch(sg.rows);
+                        quant_elem16(h, bt.item[t] >= 0, reinterpret_cast<signed char *>(o) + tile * 16, reinterpret_cast<float *>(o + sg.rows) + tile);
                     }
                 } else {
                     const int t = tw - 4 * (n & 1);
@@ -391,6 +399,20 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     }
 }
 
+/* the codes of a tensor as [128-byte slice][row][128 bytes]: the last slice of a row may reach into the next row (or into the
+ * scales that follow the tensor in the arena); such chunks are not multiplied */
+cudaError_t codes_map(const uint8_t *codes, const SpRowsSeg &s, const SegGeo &g, bool pair, CUtensorMap *m) {
+    sp_tc::EncodeTiledFn fn = nullptr;
+    const cudaError_t e = sp_tc::encode_tiled_fn(&fn);
+    if (e != cudaSuccess) return e;
+    const size_t rows = s.rows_per_group ? (size_t)s.groups * (size_t)s.rows_per_group : (size_t)s.rows;
+    const cuuint64_t rb = (cuuint64_t)s.in / 2, slices = (rb + 127) / 128;
+    const cuuint64_t dims[3] = {128, (cuuint64_t)rows, slices}, strides[2] = {rb, 128};
+    const cuuint32_t box[3] = {128, (cuuint32_t)box_rows(g, pair), (cuuint32_t)slices}, estr[3] = {1, 1, 1};
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t *>(codes), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
 constexpr size_t kSmemLimit = 227 * 1024 - 17 * 1024;      /* dynamic part: the static arrays of the kernel take 16.3 KB */
 
 }  // namespace
@@ -402,24 +424,30 @@ cudaError_t sp_rows_prepare() {
 
 cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *status, cudaStream_t st, int *nl) {
     RowsArgs a{};
+    cudaError_t e = cudaSuccess;
     a.nseg = nseg; a.status = status;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
         const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
-        const unsigned sb = g.scale_off + up128(16 * g.mt_n * g.sb), ab = g.sx_off + up128(kTok * 4 * g.sst);
+        const unsigned sb = up1024(g.scale_off + 16 * g.mt_n * g.sb), ab = kTok * g.ast;
         a.stage_bytes = sb > a.stage_bytes ? sb : a.stage_bytes; a.act_bytes = ab > a.act_bytes ? ab : a.act_bytes;
     }
     /* two teams with three stages where they fit (one being filled while two are used), else one team with two */
-    a.teams = (size_t)3 * a.stage_bytes + 4 * (size_t)a.act_bytes <= kSmemLimit ? 2 : 1;
+    for (int i = 0; i < nseg; i++) {
+        e = codes_map(seg[i].codes, seg[i], a.geo[i], pair, &a.codes[i][0]);
+        if (e == cudaSuccess && pair) e = codes_map(seg[i].ucodes, seg[i], a.geo[i], pair, &a.codes[i][1]);
+        if (e != cudaSuccess) return e;
+    }
+    a.teams = (size_t)3 * a.stage_bytes + 4 * (size_t)a.act_bytes + 1024 <= kSmemLimit ? 2 : 1;
     const size_t acts = (size_t)a.teams * 2 * a.act_bytes;
-    a.stages = (int)((kSmemLimit - acts) / a.stage_bytes);
+    a.stages = (int)((kSmemLimit - 1024 - acts) / a.stage_bytes);
     if (a.stages > kMaxStages) a.stages = kMaxStages;
     if (a.stages < 1) return cudaErrorInvalidValue;
     int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32 + 32 * a.teams);
-    const size_t smem = acts + (size_t)a.stages * a.stage_bytes;
+    const size_t smem = acts + (size_t)a.stages * a.stage_bytes + 1024;
     return sp_launch(pair ? k_rows<true> : k_rows<false>, dim3((unsigned)sms), threads, smem, st, nl, a);
 }

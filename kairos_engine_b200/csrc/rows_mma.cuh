@@ -15,10 +15,10 @@ struct SpRowsSeg {
     const int *count, *list; int list_stride;
     const int *offset, *index, *act_index;         /* act_index: position -> activation row when it is not item / act_div */
     int M, act_div;
-    const signed char *q; const float *sx;         /* int8 activations [row][in] (de-interleaved by 8), block scales [row][sp_sx_row(in)] */
-    /* pair: geglu(gate . x, up . x), quantised again in blocks of 16: out_q[item][rows], out_s[item][sp_sx_row(rows)];
+    const unsigned char *act;                      /* quantised rows, sp_act_pitch(in) apart: in int8 (de-interleaved by 8), then in / 16 block scales */
+    /* pair: geglu(gate . x, up . x), quantised again in blocks of 16, in the same form: out_act + item * sp_act_pitch(rows);
      * otherwise out_f[item * out_stride + row] */
-    signed char *out_q; float *out_s; float *out_f; int out_stride;
+    unsigned char *out_act; float *out_f; int out_stride;
 };
 
 cudaError_t sp_rows_prepare();                     /* per device: the kernels' dynamic shared-memory limits */
