@@ -648,11 +648,11 @@ cudaError_t run_experts(const SpDims &d, const SpLayerDev &L, int M, BView &v, S
         /* gate|up of the shared and the routed experts, quantised as it leaves (CF:8348-8356, 8733-8737, 8958-8959), then down (CF:8358, 8739-8742, 8961) */
         SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v)};
         up[1].count = v.count; up[1].list = v.list; up[1].list_stride = M; up[1].act_div = NU;
-        const cudaError_t e = sp_rows_launch(up, 2, true, status, st, nl);
+        const cudaError_t e = sp_rows_launch(up, 2, true, (long long)M * NU, status, st, nl);
         if (e != cudaSuccess) return e;
         SpRowsSeg down[2] = {seg_shared_down(d, L, M, v), seg_routed_down(d, L, M, v, v.eo)};
         down[1].count = v.count; down[1].list = v.list; down[1].list_stride = M;
-        return sp_rows_launch(down, 2, false, status, st, nl);
+        return sp_rows_launch(down, 2, false, (long long)M * NU, status, st, nl);
     }
     GroupArgs g{};
     g.M = M;
@@ -855,8 +855,8 @@ cudaError_t ep_shared(const SpDims &d, const SpLayerDev &L, int M, BView &v, SpT
     if (!FA && tc) return sp_tc_shared_expert(tc, d, L, M, v.nx_f, v.dn, status, st, nl, phase);
     if (FA) {
         const SpRowsSeg up = seg_shared_up(d, L, M, v), down = seg_shared_down(d, L, M, v);
-        cudaError_t e = phase != 2 ? sp_rows_launch(&up, 1, true, status, st, nl) : cudaSuccess;
-        if (e == cudaSuccess && phase != 1) e = sp_rows_launch(&down, 1, false, status, st, nl);
+        cudaError_t e = phase != 2 ? sp_rows_launch(&up, 1, true, M, status, st, nl) : cudaSuccess;
+        if (e == cudaSuccess && phase != 1) e = sp_rows_launch(&down, 1, false, M, status, st, nl);
         return e;
     }
     GroupArgs g{};
@@ -914,8 +914,8 @@ cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float 
         if (e != cudaSuccess) return e;
         SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v), down = seg_routed_down(d, L, R, v, rows_out);
         up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */
-        e = sp_rows_launch(&up, 1, true, status, st, nl);
-        return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, status, st, nl);
+        e = sp_rows_launch(&up, 1, true, R, status, st, nl);
+        return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, R, status, st, nl);
     }
     GroupArgs g{};
     g.M = R; g.offset = offsets; g.index = row_index; g.act_index = in_index;

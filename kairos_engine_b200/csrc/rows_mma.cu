@@ -8,7 +8,8 @@
  *     restricted to half h, so lane (g, q) of the warp finds both block sums of rows g and g + 8 for token q in its C
  *     registers, for every chunk. It adds its slots by itself, in the order that completes subtrees (no shuffles, at most
  *     four partial sums waiting). Half of the MMA multiplies zeros; the MMA pipe has room for that (2.6 cycles per
- *     instruction and scheduler), and the epilogue's 10 fp32 instructions serve four tokens at a time.
+ *     instruction and scheduler), and the epilogue's 10 fp32 instructions serve four tokens at a time. While most experts
+ *     have one or two tokens, two neighbouring chunks x two tokens share an epilogue instead (W = 2 below).
  *   - A operand: code nibbles moved to the top of a byte (16 * code as s8); C starts at 0x4B400000, so that one fma turns
  *     the s32 result into the float a conversion would give.
  *   - Gate|up: a 16-row MMA tile is 8 gate rows and the 8 up rows of the same outputs. A unit is 16 outputs = one
@@ -19,7 +20,9 @@
  * of its next four tokens copied while it multiplies the current four. So the weight stream does not stop between units,
  * and experts nobody chose cost nothing. A unit's codes are one or two tensor copies (a box of all 128-byte slices of 16 to
  * 128 rows, swizzled, so that the eight rows an MMA operand takes lie on different banks): a copy costs its warp ~85 cycles
- * whatever its size, and a copy per row (for padded rows) took longer than the multiplication.
+ * whatever its size, and a copy per row (for padded rows) took longer than the multiplication. What bounds it now is the
+ * multiplying warps: ~30 instructions and 7 shared-memory wavefronts a chunk. One team of sixteen warps on a unit was slower
+ * (199 us a layer at 64 tokens against 176): the latencies of a batch are then paid one after the other.
  */
 #include "rows_mma.cuh"
 #include "launch.cuh"
@@ -41,7 +44,7 @@ struct SegGeo {                                    /* what the copies and the do
 struct RowsArgs {
     SpRowsSeg seg[2]; SegGeo geo[2]; int nseg;
     int stages, teams;
-    unsigned stage_bytes, act_bytes;               /* one stage; one buffer of four tokens */
+    unsigned stage_bytes, act_bytes, zero_bytes;   /* one stage; one buffer of four tokens; the zeros B's other columns read */
     int *status;
     CUtensorMap codes[2][2];                       /* [segment][gate or only / up] */
 };
@@ -93,15 +96,22 @@ __device__ __forceinline__ void arrive_lane0(uint32_t bar, int lane) {     /* pr
 }
 __device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads) : "memory"); }
 
-/* C = A x B + {magic, ...} (a pure function of its operands: the compiler may move it) */
+/* D = A x B + {magic, ...}, D += A x B (pure functions of their operands: the compiler may move them) */
 __device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
+__device__ __forceinline__ void mma_s8_add(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 __device__ __forceinline__ float magic_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }     /* bits of magic + 16 S -> float(S) */
 
 /* ---------------------------------------------------------------- units of work */
-struct Unit { int seg, grp, tile, t0, nt, pad[3]; };        /* weight tile `tile` of group grp x its tokens [t0, t0 + nt) */
+struct Unit { int seg, grp, tile, t0, nt; };                /* weight tile `tile` of group grp x its tokens [t0, t0 + nt) */
+struct UnitWord { unsigned w; int t0; };                    /* the same as it is kept: nt 5 bits, seg 1, grp 10, tile 16 */
+__device__ __forceinline__ UnitWord pack(const Unit &u) { return UnitWord{(unsigned)u.nt | (unsigned)u.seg << 5 | (unsigned)u.grp << 6 | (unsigned)u.tile << 16, u.t0}; }
+__device__ __forceinline__ Unit unpack(const UnitWord &p) { return Unit{(int)(p.w >> 5 & 1u), (int)(p.w >> 6 & 1023u), (int)(p.w >> 16), p.t0, (int)(p.w & 31u)}; }
 struct Plan {                                               /* in shared memory: first unit of every group, per segment */
     const int *start[2]; int total[2];
     const int *count;                                       /* items of segment 1's groups while the table is in place, else NULL */
@@ -134,37 +144,47 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
 }
 
 /* ---------------------------------------------------------------- the dots of one warp: 16 rows x four tokens */
+/* W = 1: one chunk x four tokens fill the eight columns of B. W = 2: two neighbouring chunks (a group) x two tokens; lane q of
+ * a row reads two words, one per MMA, and column 2 u + h takes half h of the (token, chunk) u. Either way lane q's C registers
+ * hold both block sums of one (row, token, chunk) for two rows. */
+extern __shared__ unsigned char sm_raw[];
+/* loads by offset: pointers that are chosen at run time would become generic loads, which take the long way */
+template <class T> __device__ __forceinline__ T lds(unsigned at) { return *reinterpret_cast<const T *>(sm_raw + at); }
 struct Frag {
-    const unsigned char *w0, *w1;      /* rows g and g + 8 of the tile, at this lane's word */
-    const unsigned char *s0, *s1;      /* their block scales */
-    const unsigned char *b;            /* token g >> 1, this lane's 8 bytes of a chunk */
-    const float *sx;                   /* token q's block scales */
-    bool bvalid;                       /* the lane's k-slots lie in its column's half */
-    int n32, gq;
+    unsigned w0, w1;                   /* (offsets in shared memory) this lane's two rows, at its words of a piece */
+    unsigned s0, s1;                   /* their block scales, at the lane's chunk of a group */
+    unsigned b;                        /* the lane's bytes of its column's token and half, or zeros */
+    unsigned sx;                       /* block scales of the lane's token, at its chunk of a group */
+    int n32, row, piece;               /* row % 8; the chunk of a group whose words the lane reads */
 };
-/* slots r, r + 4, ..., r + 28 (chunks s + 32 i of each), added as the tree adds them: s and s + 16, then + 8, then + 4.
- * Rows of one chunk per slot may have fewer than 32: slots from 4 * NJ on are known to be empty (NJ even). Chunk c of a row
- * is piece c % 8 of slice c / 8 (SL bytes apart), swizzled by the row. */
-template <int SL, int NI, int NJ = 8>
+/* group slots r, r + 4, ... (32 / W of them, groups s + 32 / W i of each), added as the tree adds them: s and s + 16 (chunks),
+ * then + 8, then, W = 1, + 4. Slots from chunk 4 * NJ on are known to be empty (NJ even). Chunk c of a row is piece c % 8 of
+ * slice c / 8 (SL bytes apart), swizzled by the row. */
+template <int W, int SL, int NI, int NJ = 8>
 __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
-    const unsigned p = (unsigned)((r ^ f.gq) << 4);
-    const unsigned char *const w0e = f.w0 + p, *const w0o = f.w0 + (p ^ 64u), *const w1e = f.w1 + p, *const w1o = f.w1 + (p ^ 64u);
-    const unsigned char *const b0 = f.b + 32 * r, *const s0 = f.s0 + 2 * r, *const s1 = f.s1 + 2 * r;
-    const float *const x0 = f.sx + 2 * r;
+    const unsigned p = (unsigned)((W * r + f.piece) ^ f.row) << 4;
+    const unsigned w0e = f.w0 + p, w0o = f.w0 + (p ^ 64u), w1e = f.w1 + p, w1o = f.w1 + (p ^ 64u);
+    const unsigned b0 = f.b + 32 * W * r, s0 = f.s0 + 2 * W * r, s1 = f.s1 + 2 * W * r, x0 = f.sx + 8 * W * r;
     auto slot = [&](int j) {
         float2 acc = make_float2(0.0f, 0.0f);
-        if (j >= NJ) return acc;
+        if (j * W >= NJ) return acc;
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-            const int c = 4 * j + 32 * i, at = ((j >> 1) + 4 * i) * SL;      /* c: beyond r */
-            if (i + 1 < NI || r + c < f.n32) {              /* warp-uniform */
-                const unsigned u0 = *reinterpret_cast<const unsigned *>((j & 1 ? w0o : w0e) + at), u1 = *reinterpret_cast<const unsigned *>((j & 1 ? w1o : w1e) + at);
-                uint2 b = make_uint2(0u, 0u);
-                if (f.bvalid) b = *reinterpret_cast<const uint2 *>(b0 + 32 * c);
-                const float2 s2 = *reinterpret_cast<const float2 *>(x0 + 2 * c);
-                const float ws0 = h2f(*reinterpret_cast<const unsigned short *>(s0 + 2 * c)), ws1 = h2f(*reinterpret_cast<const unsigned short *>(s1 + 2 * c));
+            const int c = 4 * W * j + 32 * i, at = ((W * j >> 1) + 4 * i) * SL;      /* c: beyond W r */
+            if (i + 1 < NI || W * r + c < f.n32) {          /* warp-uniform */
+                const float2 s2 = lds<float2>(x0 + 8 * c);
+                const float ws0 = h2f(lds<unsigned short>(s0 + 2 * c)), ws1 = h2f(lds<unsigned short>(s1 + 2 * c));
                 int d[4];
-                mma_s8(d, (u0 << 4) & 0xF0F0F0F0u, (u1 << 4) & 0xF0F0F0F0u, u0 & 0xF0F0F0F0u, u1 & 0xF0F0F0F0u, b.x, b.y, kMagic);
+                if (W == 1) {
+                    const unsigned u0 = lds<unsigned>((j & 1 ? w0o : w0e) + at), u1 = lds<unsigned>((j & 1 ? w1o : w1e) + at);
+                    const uint2 b = lds<uint2>(b0 + 32 * c);
+                    mma_s8(d, (u0 << 4) & 0xF0F0F0F0u, (u1 << 4) & 0xF0F0F0F0u, u0 & 0xF0F0F0F0u, u1 & 0xF0F0F0F0u, b.x, b.y, kMagic);
+                } else {
+                    const uint2 u0 = lds<uint2>(w0e + at), u1 = lds<uint2>(w1e + at);
+                    const uint4 b = lds<uint4>(b0 + 32 * c);
+                    mma_s8(d, (u0.x << 4) & 0xF0F0F0F0u, (u1.x << 4) & 0xF0F0F0F0u, u0.x & 0xF0F0F0F0u, u1.x & 0xF0F0F0F0u, b.x, b.y, kMagic);
+                    mma_s8_add(d, (u0.y << 4) & 0xF0F0F0F0u, (u1.y << 4) & 0xF0F0F0F0u, u0.y & 0xF0F0F0F0u, u1.y & 0xF0F0F0F0u, b.z, b.w);
+                }
                 acc.x = __fmaf_rn(ws0, __fmaf_rn(magic_to_float(d[0]), s2.x, __fmul_rn(magic_to_float(d[1]), s2.y)), acc.x);
                 acc.y = __fmaf_rn(ws1, __fmaf_rn(magic_to_float(d[2]), s2.x, __fmul_rn(magic_to_float(d[3]), s2.y)), acc.y);
             }
@@ -172,31 +192,45 @@ __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
         return acc;
     };
     auto add = [](float2 p, float2 q) { return make_float2(p.x + q.x, p.y + q.y); };
+    if (W == 2) { const float2 a = add(slot(0), slot(2)); return add(a, add(slot(1), slot(3))); }
     float2 a = add(slot(0), slot(4)); a = add(a, add(slot(2), slot(6)));
     float2 b = add(slot(1), slot(5)); b = add(b, add(slot(3), slot(7)));
     return add(a, b);
 }
-template <int SL>
+template <int W, int SL>
 __device__ __forceinline__ float2 class_sum_n(const Frag &f, int r) {
-    if (f.n32 <= 32) return class_sum<SL, 1>(f, r);
-    if (f.n32 <= 64) return class_sum<SL, 2>(f, r);
-    if (f.n32 <= 96) return class_sum<SL, 3>(f, r);
-    return class_sum<SL, 4>(f, r);
+    if (f.n32 <= 32) return class_sum<W, SL, 1>(f, r);
+    if (f.n32 <= 64) return class_sum<W, SL, 2>(f, r);
+    if (f.n32 <= 96) return class_sum<W, SL, 3>(f, r);
+    return class_sum<W, SL, 4>(f, r);
+}
+/* rows of up to 32 chunks: all four classes by one warp, (0 + 2) + (1 + 3), then the two chunks of a group (lanes q, q ^ 1) */
+template <int W, int SL>
+__device__ __forceinline__ float2 row_sum(const Frag &f) {
+    float2 v = make_float2(0.0f, 0.0f), o = v;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+        const int r = k == 1 ? 2 : k == 2 ? 1 : k;
+        const float2 c = f.n32 <= 8 ? class_sum<W, SL, 1, 2>(f, r) : f.n32 <= 16 ? class_sum<W, SL, 1, 4>(f, r) : f.n32 <= 24 ? class_sum<W, SL, 1, 6>(f, r) : class_sum<W, SL, 1, 8>(f, r);
+        if (k == 0 || k == 2) o = c;
+        else { o.x += c.x; o.y += c.y; if (k == 1) v = o; else { v.x += o.x; v.y += o.y; } }
+    }
+    if (W == 2) { v.x += __shfl_xor_sync(0xffffffffu, v.x, 1); v.y += __shfl_xor_sync(0xffffffffu, v.y, 1); }
+    return v;
 }
 
 /* ---------------------------------------------------------------- the kernel
  * Warps: teams x 8 that multiply, one that copies weights, one per team that copies activations. */
-struct Batch { int seg, tile, flags, item[kTok], pad; };     /* four tokens of a unit; flags: 1 = the unit's first, 2 = its last, 4 = the team is done */
+struct Batch { int seg, tile, flags, item[kTok], pad; };     /* up to four tokens of a unit; flags: 1 = the unit's first, 2 = its last, 4 = the team is done, 8 = more than two tokens */
 
-template <bool PAIR>
+template <bool PAIR, int W>
 __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const __grid_constant__ RowsArgs a) {
-    extern __shared__ unsigned char sm_raw[];
     unsigned char *const sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
     __shared__ unsigned long long bars[2 * kMaxStages + 4 * kMaxTeams];
     __shared__ int abort_s;
     __shared__ Batch batch_s[kMaxTeams][2];
     __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
-    __shared__ Unit units_s[kUnits];
+    __shared__ UnitWord units_s[kUnits];
     __shared__ int start_s[1 + 1024], total_s[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     volatile int *abort_flag = &abort_s;
@@ -218,6 +252,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    unsigned char *const zeros = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)a.teams * 2u * a.act_bytes;
+    for (unsigned i = tid; i < a.zero_bytes / 16; i += blockDim.x) reinterpret_cast<uint4 *>(zeros)[i] = make_uint4(0u, 0u, 0u, 0u);
     sp_pdl_wait();
     sp_pdl_next();
     /* first unit of every group, per segment (segment 0 is the only one or has one group) */
@@ -247,11 +283,11 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     Plan plan;
     plan.start[0] = start_s; plan.start[1] = start_s + a.seg[0].groups; plan.total[0] = total_s[0]; plan.total[1] = total_s[1]; plan.count = count_s;
     const int total = plan.total[0] + plan.total[1], G = gridDim.x;
-    for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = locate(a, plan, blockIdx.x + i * G);
+    for (int i = tid; i < kUnits && (int)blockIdx.x + i * G < total; i += blockDim.x) units_s[i] = pack(locate(a, plan, blockIdx.x + i * G));
     plan.count = nullptr;
     __syncthreads();
     const int mine = total > (int)blockIdx.x ? (total - blockIdx.x + G - 1) / G : 0;
-    auto unit = [&](int i) { return i < kUnits ? units_s[i] : locate(a, plan, blockIdx.x + i * G); };
+    auto unit = [&](int i) { return i < kUnits ? unpack(units_s[i]) : locate(a, plan, blockIdx.x + i * G); };
     const uint32_t sbase = smem_u32(sm);
     bool failed = false;
 
@@ -262,18 +298,19 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const Unit u = unit(i);
                 const SpRowsSeg &sg = a.seg[u.seg];
                 const SegGeo &ge = a.geo[u.seg];
-                if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
                 const int per = PAIR ? 16 : 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
                 const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(s);
                 const int row = (int)((long long)u.grp * sg.rows_per_group) + r0;
                 const unsigned sbytes = (unsigned)nr * ge.sb;
+                const unsigned char *const ssrc = reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb;
+                if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
                 expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
                 box_g2s(dst, &a.codes[u.seg][0], row, bar);
-                bulk_g2s(sdst, reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb, sbytes, bar);
                 if (PAIR) {
                     box_g2s(dst + ge.box_bytes, &a.codes[u.seg][1], row + sg.up_off, bar);
                     bulk_g2s(sdst + 16 * ge.sb, reinterpret_cast<const unsigned char *>(sg.ubs) + (size_t)(row + sg.up_off) * ge.sb, sbytes, bar);
                 }
+                bulk_g2s(sdst, ssrc, sbytes, bar);
                 if (++s == a.stages) { s = 0; ph ^= 1; }
             }
         __syncwarp();
@@ -299,7 +336,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 if (!mbar_wait(aempty(team, buf), ((n >> 1) & 1) ^ 1, abort_flag)) { failed = true; break; }
                 Batch *d = &batch_s[team][buf];
                 if (lane < kTok) d->item[lane] = item;
-                if (lane == 0) { d->seg = u.seg; d->tile = u.tile; d->flags = (b == 0 ? 1 : 0) | (b + kTok >= u.nt ? 2 : 0); }
+                if (lane == 0) { d->seg = u.seg; d->tile = u.tile; d->flags = (b == 0 ? 1 : 0) | (b + kTok >= u.nt ? 2 : 0) | (have > 2 ? 8 : 0); }
                 __syncwarp();
                 if (lane == 0) expect_tx(afull(team, buf), (unsigned)have * (unsigned)sp_act_pitch(s.in));        /* its arrival also publishes the descriptor */
                 __syncwarp();
@@ -321,7 +358,14 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
         int s = team % a.stages, ph = (team / a.stages) & 1;
         Frag f;
-        f.bvalid = (q >> 1) == (gq & 1); f.gq = gq;
+        /* lanes whose 8-byte loads share a wavefront (W = 2) take rows whose pieces differ by more than the group's two */
+        f.row = W == 1 ? gq : (gq & 1) << 2 | (gq & 2) | gq >> 2;
+        f.piece = W == 1 ? 0 : q >> 1;
+        const int cs = W == 1 ? 0 : q & 1, row = f.row;     /* cs: the chunk of a group in the lane's C registers */
+        const bool bvalid = W == 1 ? (q >> 1) == (gq & 1) : q == (gq & 3);
+        const int btok = W == 1 ? gq >> 1 : gq >> 2, ctok = W == 1 ? q : q >> 1;
+        const unsigned z = (unsigned)(zeros - sm_raw) + (W == 1 ? (gq < 4 ? 64 : 0) + 8 * q : 96);      /* on banks the other lanes of the wavefront do not use */
+        const int wo = W == 1 ? 4 * q : 8 * (q & 1), bo = (W == 1 ? 8 : 16) * q;
         for (int n = 0;; n++) {
             const int buf = n & 1;
             if (!mbar_wait(afull(team, buf), (n >> 1) & 1, abort_flag)) { failed = true; break; }
@@ -333,43 +377,71 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             const SegGeo &ge = a.geo[sgi];
             if ((flags & 1) && !mbar_wait(full(s), ph, abort_flag)) { failed = true; break; }
             const int mt_n = PAIR ? 2 : ge.mt_n, mt = mt_n == 8 ? tw : tw >> 2, r0 = tile * 16 * mt_n;
-            const unsigned char *codes = sm + (unsigned)s * a.stage_bytes, *scales = codes + ge.scale_off, *act = aptr + buf * a.act_bytes;
-            if (PAIR) { f.w0 = codes + (mt * 8 + gq) * 128 + 4 * q; f.w1 = f.w0 + ge.box_bytes; f.s0 = scales + (mt * 8 + gq) * ge.sb; f.s1 = f.s0 + 16 * ge.sb; }      /* gate rows, then the up rows */
-            else { f.w0 = codes + (mt * 16 + gq) * 128 + 4 * q; f.w1 = f.w0 + 8 * 128; f.s0 = scales + (mt * 16 + gq) * ge.sb; f.s1 = f.s0 + 8 * ge.sb; }
-            f.b = act + (gq >> 1) * ge.ast + 8 * q;
-            f.sx = reinterpret_cast<const float *>(act + q * ge.ast + sg.in);
+            const unsigned codes = (unsigned)(sm - sm_raw) + (unsigned)s * a.stage_bytes, scales = codes + ge.scale_off, act = (unsigned)(aptr - sm_raw) + buf * a.act_bytes;
+            if (PAIR) { f.w0 = codes + (mt * 8 + row) * 128 + wo; f.w1 = f.w0 + ge.box_bytes; f.s0 = scales + (mt * 8 + row) * ge.sb + 2 * cs; f.s1 = f.s0 + 16 * ge.sb; }      /* gate rows, then the up rows */
+            else { f.w0 = codes + (mt * 16 + row) * 128 + wo; f.w1 = f.w0 + 8 * 128; f.s0 = scales + (mt * 16 + row) * ge.sb + 2 * cs; f.s1 = f.s0 + 8 * ge.sb; }
             f.n32 = ge.n32;
+            const bool many = W == 2 && (flags & 8);        /* two pairs of tokens */
+            auto tokens = [&](int first) {                  /* point the fragment at the W = 1: four, 2: two tokens from `first` */
+                f.b = bvalid ? act + (first + btok) * ge.ast + bo : z;
+                f.sx = act + (first + ctok) * ge.ast + sg.in + 8 * cs;
+            };
+            auto release = [&] {                            /* the stage, once the warp has read it for the last time */
+                if (flags & 2) {
+                    __syncwarp();
+                    arrive_lane0(empty(s), lane);
+                    s += a.teams;
+                    while (s >= a.stages) { s -= a.stages; ph ^= 1; }
+                }
+            };
             if (!PAIR && mt_n == 8) {
                 if (r0 + mt * 16 < sg.rows) {
-                    float2 v = make_float2(0.0f, 0.0f), o = v;
 #pragma unroll 1
-                    for (int k = 0; k < 4; k++) {           /* classes 0, 2, 1, 3: (0 + 2) + (1 + 3) */
-                        const int r = k == 1 ? 2 : k == 2 ? 1 : k;
-                        const float2 c = f.n32 <= 8 ? class_sum<128 * 128, 1, 2>(f, r) : f.n32 <= 16 ? class_sum<128 * 128, 1, 4>(f, r) : f.n32 <= 24 ? class_sum<128 * 128, 1, 6>(f, r) : class_sum<128 * 128, 1, 8>(f, r);
-                        if (k == 0 || k == 2) o = c;
-                        else { o.x += c.x; o.y += c.y; if (k == 1) v = o; else { v.x += o.x; v.y += o.y; } }
-                    }
-                    const int it = bt.item[q];
-                    if (it >= 0) {
-                        float *out = sg.out_f + (size_t)it * sg.out_stride + r0 + mt * 16 + gq;
-                        out[0] = v.x; out[8] = v.y;
+                    for (int first = 0; first < (many ? 4 : 2); first += 4 / W) {
+                        tokens(first);
+                        const float2 v = row_sum<W, 128 * 128>(f);
+                        const int it = bt.item[first + ctok];
+                        if (it >= 0 && cs == 0) {
+                            float *out = sg.out_f + (size_t)it * sg.out_stride + r0 + mt * 16 + row;
+                            out[0] = v.x; out[8] = v.y;
+                        }
                     }
                 }
+                release();
             } else {
+                /* the eight warps: two 16-row tiles x four classes, or (W = 2, more than two tokens) two tiles x two pairs of
+                 * tokens x two pairs of classes. part: [class sums left][tile][row][token] */
                 float *part = part_s[team][buf];
+                constexpr int SL = PAIR ? 16 * 128 : 32 * 128;
+                const int T = W == 1 || many ? 4 : 2;
                 if (PAIR || r0 + mt * 16 < sg.rows) {
-                    const float2 v = class_sum_n<PAIR ? 16 * 128 : 32 * 128>(f, tw & 3);
-                    float *p = part + (((tw & 3) * 2 + mt) * 16 + gq) * kTok + q;
-                    p[0] = v.x; p[8 * kTok] = v.y;
+                    int r = many ? tw & 1 : tw & 3;
+                    tokens(many ? tw & 2 : 0);
+                    float *p = part + (((W * r + cs) * 2 + mt) * 16 + row) * T + (many ? tw & 2 : 0) + ctok;
+                    float2 v = make_float2(0.0f, 0.0f);
+                    if (W == 1) v = class_sum_n<W, SL>(f, r);
+                    else {
+#pragma unroll 1
+                        for (;; r += 2) {
+                            const float2 c = class_sum_n<W, SL>(f, r);
+                            if (r >= 2 && many) { v.x += c.x; v.y += c.y; break; }
+                            v = c;
+                            if (!many) break;
+                        }
+                    }
+                    p[0] = v.x; p[8 * T] = v.y;
                 }
+                release();
                 team_sync(team);
-                auto total_of = [&](int m, int row, int t) {                /* the last two levels of the tree */
-                    const float *p = part + (m * 16 + row) * kTok + t;
-                    return (p[0] + p[2 * 2 * 16 * kTok]) + (p[2 * 16 * kTok] + p[3 * 2 * 16 * kTok]);
+                auto total_of = [&](int m, int rw, int t) {                 /* the last levels of the tree */
+                    const float *p = part + (m * 16 + rw) * T + t;
+                    const int k = 32 * T;
+                    if (T == 4) return (p[0] + p[2 * k]) + (p[k] + p[3 * k]);
+                    return ((p[0] + p[4 * k]) + (p[2 * k] + p[6 * k])) + ((p[k] + p[5 * k]) + (p[3 * k] + p[7 * k]));
                 };
                 if (PAIR) {
                     const int w0 = 2 * (n & 3);             /* two warps finish, other ones each time */
-                    if (tw == w0 || tw == w0 + 1) {
+                    if (tw == w0 || (tw == w0 + 1 && T == 4)) {
                         const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
                         const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
                         const int it = bt.item[t] < 0 ? 0 : bt.item[t];
@@ -378,7 +450,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                     }
                 } else {
                     const int t = tw - 4 * (n & 1);
-                    if (t >= 0 && t < 4) {
+                    if (t >= 0 && t < T) {
                         const int it = bt.item[t];
                         if (it >= 0 && r0 + lane < sg.rows) sg.out_f[(size_t)it * sg.out_stride + r0 + lane] = total_of(lane >> 4, lane & 15, t);
                     }
@@ -386,11 +458,6 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             }
             __syncwarp();
             arrive_lane0(aempty(team, buf), lane);
-            if (flags & 2) {
-                arrive_lane0(empty(s), lane);
-                s += a.teams;
-                while (s >= a.stages) { s -= a.stages; ph ^= 1; }
-            }
         }
     }
     if (failed) {
@@ -413,23 +480,32 @@ cudaError_t codes_map(const uint8_t *codes, const SpRowsSeg &s, const SegGeo &g,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
-constexpr size_t kSmemLimit = 227 * 1024 - 17 * 1024;      /* dynamic part: the static arrays of the kernel take 16.3 KB */
+constexpr size_t kSmemLimit = 227 * 1024 - 14 * 1024;      /* dynamic part: the static arrays of the kernel take 13.3 KB */
 
 }  // namespace
 
 cudaError_t sp_rows_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
-    return e == cudaSuccess ? cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) : e;
+    for (const auto k : {k_rows<true, 1>, k_rows<true, 2>, k_rows<false, 1>, k_rows<false, 2>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *status, cudaStream_t st, int *nl) {
+cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long items, int *status, cudaStream_t st, int *nl) {
     RowsArgs a{};
     cudaError_t e = cudaSuccess;
     a.nseg = nseg; a.status = status;
+    /* two chunks x two tokens per MMA while most chosen experts have one or two tokens (55 instead of 58 us a layer at five
+     * tokens of eight of 128 experts, even at 16, 204 instead of 176 at 64) and the rows are whole groups */
+    bool whole = items <= seg[nseg - 1].groups;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
         const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
         const unsigned sb = up1024(g.scale_off + 16 * g.mt_n * g.sb), ab = kTok * g.ast;
+        const unsigned zb = (unsigned)seg[i].in + 128;
+        a.zero_bytes = zb > a.zero_bytes ? zb : a.zero_bytes;
+        whole = whole && g.n32 % 2 == 0;
         a.stage_bytes = sb > a.stage_bytes ? sb : a.stage_bytes; a.act_bytes = ab > a.act_bytes ? ab : a.act_bytes;
     }
     /* two teams with three stages where they fit (one being filled while two are used), else one team with two */
@@ -438,8 +514,8 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *statu
         if (e == cudaSuccess && pair) e = codes_map(seg[i].ucodes, seg[i], a.geo[i], pair, &a.codes[i][1]);
         if (e != cudaSuccess) return e;
     }
-    a.teams = (size_t)3 * a.stage_bytes + 4 * (size_t)a.act_bytes + 1024 <= kSmemLimit ? 2 : 1;
-    const size_t acts = (size_t)a.teams * 2 * a.act_bytes;
+    a.teams = (size_t)3 * a.stage_bytes + 4 * (size_t)a.act_bytes + a.zero_bytes + 1024 <= kSmemLimit ? 2 : 1;
+    const size_t acts = (size_t)a.teams * 2 * a.act_bytes + a.zero_bytes;
     a.stages = (int)((kSmemLimit - 1024 - acts) / a.stage_bytes);
     if (a.stages > kMaxStages) a.stages = kMaxStages;
     if (a.stages < 1) return cudaErrorInvalidValue;
@@ -449,5 +525,5 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *statu
     if (e != cudaSuccess) return e;
     const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32 + 32 * a.teams);
     const size_t smem = acts + (size_t)a.stages * a.stage_bytes + 1024;
-    return sp_launch(pair ? k_rows<true> : k_rows<false>, dim3((unsigned)sms), threads, smem, st, nl, a);
+    return sp_launch(pair ? whole ? k_rows<true, 2> : k_rows<true, 1> : whole ? k_rows<false, 2> : k_rows<false, 1>, dim3((unsigned)sms), threads, smem, st, nl, a);
 }

@@ -22,5 +22,6 @@ struct SpRowsSeg {
 };
 
 cudaError_t sp_rows_prepare();                     /* per device: the kernels' dynamic shared-memory limits */
-/* one launch over `nseg` (1 or 2) segments; pair: all of them gate|up with GeGLU */
-cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, int *status, cudaStream_t st, int *nl);
+/* one launch over `nseg` (1 or 2) segments; pair: all of them gate|up with GeGLU; items: how many the last segment's groups
+ * have together */
+cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long items, int *status, cudaStream_t st, int *nl);
