@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
         const TcSeg &s = a.seg[t.sg];
         const int r = w - (t.sg ? total0 : 0), nt = r / s.m_tiles;
         t.mt = r - nt * s.m_tiles;
-        t.grp = __ldg(s.tiles + 3 * nt); t.row0 = __ldg(s.tiles + 3 * nt + 1); t.nv = __ldg(s.tiles + 3 * nt + 2);
+        t.grp = __ldcg(s.tiles + 3 * nt); t.row0 = __ldcg(s.tiles + 3 * nt + 1); t.nv = __ldcg(s.tiles + 3 * nt + 2);
         t.n16 = (t.nv + kNGran - 1) & ~(kNGran - 1);
         t.nblk = s.rows - t.mt * 2 * BLK > BLK ? 2 : 1;
         t.KB = a.K[t.sg] / kBK;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
 #pragma unroll 1
             for (int c0 = 0; c0 < t.nv; c0 += 32) {
                 int rm = t.row0 + c0 + lane;
-                if (!PAIR && s.rowmap) rm = c0 + lane < t.nv ? __ldg(s.rowmap + rm) : 0;
+                if (!PAIR && s.rowmap) rm = c0 + lane < t.nv ? __ldcg(s.rowmap + rm) : 0;
 #pragma unroll
                 for (int n = 0; n < 32; n += 2) {
                     if (c0 + n >= t.nv) break;                          /* warp-uniform */

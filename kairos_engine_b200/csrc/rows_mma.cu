@@ -116,15 +116,17 @@ struct Plan {                                               /* in shared memory:
     const int *start[2]; int total[2];
     const int *count;                                       /* items of segment 1's groups while the table is in place, else NULL */
 };
+/* counts, lists and ranges are written by the kernel before this one, which may still run when this one starts: no read-only
+ * (__ldg) loads, which the compiler may move before the wait for it */
 __device__ __forceinline__ int group_first(const SpRowsSeg &s, int g) {
     if (!s.offset) return 0;
-    const int f = __ldg(s.offset + g);                      /* caller-supplied ranges: kept inside the M rows that exist */
+    const int f = __ldcg(s.offset + g);                      /* caller-supplied ranges: kept inside the M rows that exist */
     return f < 0 ? 0 : (f > s.M ? s.M : f);
 }
 __device__ __forceinline__ int group_count(const SpRowsSeg &s, int g) {
-    if (s.offset) { int l = __ldg(s.offset + g + 1); l = l > s.M ? s.M : l; const int c = l - group_first(s, g); return c < 0 ? 0 : c; }
+    if (s.offset) { int l = __ldcg(s.offset + g + 1); l = l > s.M ? s.M : l; const int c = l - group_first(s, g); return c < 0 ? 0 : c; }
     if (!s.count) return s.M;
-    const int c = __ldg(s.count + g);
+    const int c = __ldcg(s.count + g);
     return c > s.M ? s.M : c;
 }
 __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
@@ -226,7 +228,7 @@ struct Batch { int seg, tile, flags, item[kTok], pad; };     /* up to four token
 template <bool PAIR, int W>
 __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const __grid_constant__ RowsArgs a) {
     unsigned char *const sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
-    __shared__ unsigned long long bars[2 * kMaxStages + 4 * kMaxTeams];
+    __shared__ unsigned long long bars[(1 + kMaxTeams) * kMaxStages + 4 * kMaxTeams];
     __shared__ int abort_s;
     __shared__ Batch batch_s[kMaxTeams][2];
     __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
@@ -235,13 +237,16 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     volatile int *abort_flag = &abort_s;
     const uint32_t bar0 = smem_u32(bars);
-    auto full = [&](int s) { return bar0 + 8u * s; };                   /* weight stages */
-    auto empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
-    auto afull = [&](int team, int b) { return bar0 + 8u * (2 * kMaxStages + 4 * team + b); };      /* a team's two buffers of activations */
-    auto aempty = [&](int team, int b) { return bar0 + 8u * (2 * kMaxStages + 4 * team + 2 + b); };
+    /* weight stages. A stage may serve the teams in turn, and its fills land in any order: each team waits on barriers that count
+     * its own fills only (on a shared one, a team could take the phase before the other's fill for its own) */
+    auto full = [&](int team, int s) { return bar0 + 8u * (kMaxStages * (1 + team) + s); };
+    auto empty = [&](int s) { return bar0 + 8u * s; };
+    constexpr int kActBars = (1 + kMaxTeams) * kMaxStages;
+    auto afull = [&](int team, int b) { return bar0 + 8u * (kActBars + 4 * team + b); };      /* a team's two buffers of activations */
+    auto aempty = [&](int team, int b) { return bar0 + 8u * (kActBars + 4 * team + 2 + b); };
     if (tid == 0) {
         for (int s = 0; s < a.stages; s++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(s)) : "memory");
+            for (int t = 0; t < a.teams; t++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(t, s)) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty(s)), "n"(kTeamWarps) : "memory");
         }
         for (int t = 0; t < a.teams; t++)
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const SpRowsSeg &sg = a.seg[u.seg];
                 const SegGeo &ge = a.geo[u.seg];
                 const int per = PAIR ? 16 : 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
-                const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(s);
+                const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(i % a.teams, s);
                 const int row = (int)((long long)u.grp * sg.rows_per_group) + r0;
                 const unsigned sbytes = (unsigned)nr * ge.sb;
                 const unsigned char *const ssrc = reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb;
@@ -328,8 +333,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 int item = -1, arow = 0;
                 if (lane < kTok && b + lane < u.nt) {
                     const int at = first + b + lane;
-                    if (s.offset) { item = s.index ? __ldg(s.index + at) : at; arow = s.act_index ? __ldg(s.act_index + at) : item; }
-                    else { item = s.list ? __ldg(s.list + (size_t)u.grp * s.list_stride + at) : at; arow = item; }
+                    if (s.offset) { item = s.index ? __ldcg(s.index + at) : at; arow = s.act_index ? __ldcg(s.act_index + at) : item; }
+                    else { item = s.list ? __ldcg(s.list + (size_t)u.grp * s.list_stride + at) : at; arow = item; }
                     if (!s.act_index && s.act_div > 1) arow /= s.act_div;
                 }
                 const int buf = n & 1, have = u.nt - b < kTok ? u.nt - b : kTok;
@@ -356,7 +361,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         /* ---------------- a team: units team, team + teams, ... of this CTA, four tokens at a time */
         const int team = warp / kTeamWarps, tw = warp % kTeamWarps, gq = lane >> 2, q = lane & 3;
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
-        int s = team % a.stages, ph = (team / a.stages) & 1;
+        int s = team % a.stages;
+        unsigned phs = 0;                                   /* bit s: parity of this team's next use of stage s */
         Frag f;
         /* lanes whose 8-byte loads share a wavefront (W = 2) take rows whose pieces differ by more than the group's two */
         f.row = W == 1 ? gq : (gq & 1) << 2 | (gq & 2) | gq >> 2;
@@ -375,7 +381,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             const int sgi = bt.seg, tile = bt.tile;
             const SpRowsSeg &sg = a.seg[sgi];
             const SegGeo &ge = a.geo[sgi];
-            if ((flags & 1) && !mbar_wait(full(s), ph, abort_flag)) { failed = true; break; }
+            if ((flags & 1) && !mbar_wait(full(team, s), phs >> s & 1u, abort_flag)) { failed = true; break; }
             const int mt_n = PAIR ? 2 : ge.mt_n, mt = mt_n == 8 ? tw : tw >> 2, r0 = tile * 16 * mt_n;
             const unsigned codes = (unsigned)(sm - sm_raw) + (unsigned)s * a.stage_bytes, scales = codes + ge.scale_off, act = (unsigned)(aptr - sm_raw) + buf * a.act_bytes;
             if (PAIR) { f.w0 = codes + (mt * 8 + row) * 128 + wo; f.w1 = f.w0 + ge.box_bytes; f.s0 = scales + (mt * 8 + row) * ge.sb + 2 * cs; f.s1 = f.s0 + 16 * ge.sb; }      /* gate rows, then the up rows */
@@ -383,6 +389,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             f.n32 = ge.n32;
             const bool many = W == 2 && (flags & 8);        /* two pairs of tokens */
             auto tokens = [&](int first) {                  /* point the fragment at the W = 1: four, 2: two tokens from `first` */
+                __syncwarp();                               /* the MMAs take the whole warp; a wait or the last tokens' stores may have split it */
                 f.b = bvalid ? act + (first + btok) * ge.ast + bo : z;
                 f.sx = act + (first + ctok) * ge.ast + sg.in + 8 * cs;
             };
@@ -390,8 +397,9 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 if (flags & 2) {
                     __syncwarp();
                     arrive_lane0(empty(s), lane);
+                    phs ^= 1u << s;
                     s += a.teams;
-                    while (s >= a.stages) { s -= a.stages; ph ^= 1; }
+                    while (s >= a.stages) s -= a.stages;
                 }
             };
             if (!PAIR && mt_n == 8) {
