@@ -627,17 +627,17 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
         }
         STAMP(1, 7);
         if (warp == 0) {
-            float wnorm = 0.0f; int e = 0, slot = 0;
-            if (lane < NU) {
-                float ws = 0.0f;
-#pragma unroll 1
-                for (int k = 0; k < NU; k++) ws = __fadd_rn(ws, ctl->p_desc[k]);
-                if (ws < 6.103515625e-5f) ws = 6.103515625e-5f;
-                e = ctl->sel_desc[lane];
-                wnorm = __fdiv_rn(ctl->p_desc[lane], ws);
-#pragma unroll 1
-                for (int j = 0; j < NU; j++) slot += (ctl->sel_desc[j] < e);
+            /* the sum and the ascending place by shuffles, unrolled: the routed copies wait for this (23.2 -> 23.0 us a layer) */
+            static_assert(SP_MAX_NU <= 32, "one lane per selected expert");
+            const int e = lane < NU ? ctl->sel_desc[lane] : 0; const float pe = lane < NU ? ctl->p_desc[lane] : 0.0f;
+            float ws = 0.0f; int slot = 0;
+#pragma unroll
+            for (int k = 0; k < SP_MAX_NU; k++) {
+                const float pk = __shfl_sync(0xffffffffu, pe, k); const int ek = __shfl_sync(0xffffffffu, e, k);
+                if (k < NU) { ws = __fadd_rn(ws, pk); slot += ek < e; }
             }
+            if (ws < 6.103515625e-5f) ws = 6.103515625e-5f;
+            const float wnorm = __fdiv_rn(pe, ws);
             __syncwarp();
             if (lane < NU) { ctl->sel_asc[slot] = e; ctl->cw[slot] = __fmul_rn(wnorm, dsc[e]); ctl->p_desc[lane] = wnorm; }
             __syncwarp();
