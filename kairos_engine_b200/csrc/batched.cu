@@ -279,15 +279,18 @@ void set_finish(TokArgs &a, const SpLayerDev &L, const BView &v, const float *eo
  * elements in order, then the shuffle tree (the same order the decode kernel uses). One block =
  * 32 experts x 16 tokens; E is walked in chunks of 32 float4 groups staged in shared memory, and
  * each warp keeps an 8-expert x 8-token register tile (16 shared-memory loads per 256 FMAs), so every
- * (expert, token) chain keeps the order above while 64 independent chains hide the FMA latency. */
+ * (expert, token) chain keeps the order above while 64 independent chains hide the FMA latency. Bound by shared memory
+ * (as many cycles of loads as of FMAs, and the copies in) and the last wave: 129 us at 4096 tokens with two stages and 64
+ * separate trees, 90 us with four stages, one barrier a chunk and the trees together. */
 constexpr int kRouterTE = 32, kRouterTT = 16;
-constexpr size_t kRouterSmem = 2 * (size_t)(kRouterTE + kRouterTT) * 32 * sizeof(float4);     /* two stages of 24 KB */
+constexpr int kRouterStages = 4;
+constexpr size_t kRouterSmem = kRouterStages * (size_t)(kRouterTE + kRouterTT) * 32 * sizeof(float4);     /* stages of 24 KB */
 /* 16-byte asynchronous copy that writes zeros when `take` is false (the source address stays valid either way) */
 __device__ __forceinline__ void cp_async16_zfill(void *smem_dst, const void *src, bool take) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"((unsigned)__cvta_generic_to_shared(smem_dst)), "l"(src), "r"(take ? 16 : 0) : "memory");
 }
 __global__ void __launch_bounds__(256, 2) k_b_router(SpDims d, SpLayerDev L, BView v, int M) {
-    extern __shared__ __align__(16) float4 rsm[];              /* [2] x { w[32][32], x[16][32] }: the next chunk lands while this one is used */
+    extern __shared__ __align__(16) float4 rsm[];              /* [kRouterStages] x { w[32][32], x[16][32] }: the next chunks land while this one is used */
     const int E = d.E, G = E >> 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int we = warp & 3, wt = warp >> 2;
     const int e0 = blockIdx.x * kRouterTE, t0 = blockIdx.y * kRouterTT;
@@ -314,12 +317,13 @@ __global__ void __launch_bounds__(256, 2) k_b_router(SpDims d, SpLayerDev L, BVi
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nch = (G + 31) >> 5;
-    stage(0, 0);
-    for (int c = 0; c < nch; c++) {
-        if (c + 1 < nch) { stage(32 * (c + 1), (c + 1) & 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-        else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const float4 *wS = rsm + (size_t)(c & 1) * (kRouterTE + kRouterTT) * 32, *xS = wS + kRouterTE * 32;
+    for (int c = 0; c < kRouterStages - 1; c++) { if (c < nch) stage(32 * c, c); else asm volatile("cp.async.commit_group;" ::: "memory"); }
+    for (int c = 0, buf = 0, nbuf = kRouterStages - 1; c < nch; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRouterStages - 2) : "memory");
+        __syncthreads();                                        /* chunk c is there; every warp has read chunk c - 1, whose place the new one takes */
+        if (c + kRouterStages - 1 < nch) stage(32 * (c + kRouterStages - 1), nbuf); else asm volatile("cp.async.commit_group;" ::: "memory");
+        const float4 *wS = rsm + (size_t)buf * (kRouterTE + kRouterTT) * 32, *xS = wS + kRouterTE * 32;
+        buf = buf == kRouterStages - 1 ? 0 : buf + 1; nbuf = nbuf == kRouterStages - 1 ? 0 : nbuf + 1;
         float4 w[8];                                            /* zero padding beyond E leaves acc unchanged: fma(0, 0, acc) = acc */
 #pragma unroll
         for (int i = 0; i < 8; i++) w[i] = wS[(8 * we + i) * 32 + lane];
@@ -334,17 +338,26 @@ __global__ void __launch_bounds__(256, 2) k_b_router(SpDims d, SpLayerDev L, BVi
                 acc[i][j] = a;
             }
         }
-        __syncthreads();                                        /* this stage is overwritten two chunks on */
     }
+    /* all 64 sums at once: at every level of the tree a lane keeps half of the values and hands the others over (the pairs that
+     * warp_tree adds, 62 shuffles instead of 320); it ends with two neighbouring tokens of one expert */
+    float f[64];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int k = 0; k < 64; k++) f[k] = acc[k >> 3][k & 7];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float r = warp_tree(acc[i][j]);
-            const int e = e0 + 8 * we + i, t = t0 + 8 * wt + j;
-            if (lane == 0 && e < d.NE && t < M)
-                v.logits[(size_t)t * d.NE + e] = L.router_bias ? __fadd_rn(r, __ldg(L.router_bias + e)) : r;
-        }
+    for (int o = 16, n = 32; o > 0; o >>= 1, n >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int k = 0; k < 32; k++)
+            if (k < n) f[k] = (hi ? f[k + n] : f[k]) + __shfl_xor_sync(0xffffffffu, hi ? f[k] : f[k + n], o);
+    }
+    const int e = e0 + 8 * we + (lane >> 2), t = t0 + 8 * wt + 2 * (lane & 3);
+    if (e < d.NE) {
+        const float bias = L.router_bias ? __ldg(L.router_bias + e) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (t + j < M) v.logits[(size_t)(t + j) * d.NE + e] = L.router_bias ? __fadd_rn(f[j], bias) : f[j];
+    }
 }
 
 /* The same logits for a handful of tokens: one block per (expert, eight tokens), so that a small batch
@@ -999,6 +1012,7 @@ cudaError_t sp_batched_alloc(const SpDims &d, int max_tokens, int max_rows, SpBa
     s->bytes = blayout(d, max_tokens, s->max_rows, [](int, size_t) {});
     s->tc = nullptr;
     cudaError_t e = sp_rows_prepare();
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_b_router, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouterSmem);
     if (e != cudaSuccess) return e;
     e = cudaMalloc(&s->base, s->bytes);
     if (e != cudaSuccess) { s->base = nullptr; return e; }
