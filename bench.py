@@ -306,7 +306,7 @@ def small_batch_leg(eng, NL, local_rank, rank, peak_gbs):
         eng.status()
         out[f"M={M}"] = {"tokens_per_s": M / (ms / 1e3), "ms_per_step": ms, "distinct_experts_per_layer_mean": sum(U) / len(U),
                          "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak_gbs, "unit": "GB/s", "frac": gbs / peak_gbs, "algorithmic_bytes": nbytes},
-                         "route": "token by token through the single-token graph" if M <= int(os.environ.get("SP_MOE_SEQ_TOKENS", "5")) else "batched kernels (mma.sync row dots)",
+                         "route": "token by token through the single-token graph" if M <= int(os.environ.get("SP_MOE_SEQ_TOKENS", "1")) else "batched kernels (mma.sync row dots)",
                          "row0_equals_single_token_step": bool(torch.equal(y1.view(torch.int32), y[0].view(torch.int32)))}
     return out
 
