@@ -113,7 +113,7 @@ int  sp_moe_forward(sp_moe *h, int layer_first, int n_layers, int flavour, int M
                     const float *x, float *y, int32_t *sel, float *wts);
 /* Same with DEVICE pointers on a caller stream (a cudaStream_t passed as void*); enqueues only.
  * A router row with a NaN (the reference's hard error, CF:8596-8620) is reported by the next
- * sp_moe_status call. */
+ * sp_moe_status call. x_dev and y_dev may start on any float (16-byte boundaries save a copy of x beyond 64 tokens). */
 int  sp_moe_forward_dev(sp_moe *h, int layer_first, int n_layers, int flavour, int M,
                         const float *x_dev, float *y_dev, int32_t *sel_dev, float *wts_dev,
                         void *stream);
@@ -147,6 +147,8 @@ int  sp_moe_status(sp_moe *h);
  *             n_rows <= max_expert_rows of the config
  *   finish  : token t's k-th expert output (sel_asc order) is row pair_index[t*NU+k] of pair_rows
  *             (pair_index NULL = row t*NU+k) -> y = the layer's output residual
+ * x, y and pair_rows may start on any float, rows_in too in the decode arithmetic; rows, and rows_in in the prefill
+ * arithmetic, start on 16-byte boundaries (anything else is refused with SP_MOE_EBADARG).
  * A run through the three stages is bit-identical to sp_moe_forward_dev on the same tokens. */
 int sp_moe_ep_route_dev(sp_moe *h, int layer, int flavour, int M, const float *x_dev,
                         int32_t *sel_asc_dev, float *cw_dev, float *rows_dev, int32_t *counts_dev,

@@ -254,6 +254,13 @@ static int check_forward(sp_moe *h, int lf, int nl, int flavour, int M, const vo
     return SP_MOE_OK;
 }
 
+/* A layer begins with 16-byte loads of x: an x on some other float boundary is read through the handle's own copy. */
+static cudaError_t align_x(sp_moe *h, const float **x, int M, cudaStream_t st) {
+    if (!((uintptr_t)*x & 15)) return cudaSuccess;
+    const cudaError_t e = cudaMemcpyAsync(h->x_dev, *x, (size_t)M * h->cfg.E * 4, cudaMemcpyDeviceToDevice, st);
+    *x = h->x_dev;
+    return e;
+}
 constexpr int kDirectLayers = 4;
 extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
                                   const float *x_dev, float *y_dev, int32_t *sel_dev, float *wts_dev, void *stream) {
@@ -336,6 +343,7 @@ extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
         h->launches += (uint64_t)bg->launches;
         return SP_MOE_OK;
     }
+    CK(align_x(h, &x_dev, M, st), "x staging");
     int nlaunch = 0;
     cudaError_t e = sp_batched_forward(h->d, h->layers_host.data(), lf, nl, flavour, M, x_dev, y_dev, sel_dev, wts_dev, &h->bs, h->status, st, &nlaunch);
     h->launches += (uint64_t)nlaunch;
@@ -357,11 +365,13 @@ extern "C" int sp_moe_ep_route_dev(sp_moe *h, int layer, int flavour, int M, con
     int rc = check_ep(h, layer, flavour, "sp_moe_ep_route_dev");
     if (rc) return rc;
     if (!x_dev || !sel_asc_dev || !cw_dev || !rows_dev || !counts_dev || !pair_index_dev) return fail(SP_MOE_EBADARG, "sp_moe_ep_route_dev: NULL argument");
+    if ((uintptr_t)rows_dev & 15) return fail(SP_MOE_EBADARG, "sp_moe_ep_route_dev: rows must start on a 16-byte boundary");
     if (M <= 0 || M > h->cfg.max_tokens) return fail(SP_MOE_EBADARG, "sp_moe_ep_route_dev: M=%d outside (0, max_tokens=%d]", M, h->cfg.max_tokens);
     if (capacity < 0 || (capacity > 0 && (n_ranks <= 0 || h->cfg.NE % n_ranks)))
         return fail(SP_MOE_EBADARG, "sp_moe_ep_route_dev: a capacity needs n_ranks > 0 dividing NE=%d (got n_ranks=%d capacity=%d)", h->cfg.NE, n_ranks, capacity);
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     cudaStream_t st = (cudaStream_t)stream; h->last_stream = st;
+    CK(align_x(h, &x_dev, M, st), "x staging");
     int nlaunch = 0;
     cudaError_t e = sp_batched_ep_route(h->d, h->layers_host[layer], flavour, M, x_dev, sel_asc_dev, cw_dev, rows_dev, counts_dev, pair_index_dev, sel_dev, wts_dev,
                                         defer_shared, n_ranks, capacity, &h->bs, h->status, st, &nlaunch);
@@ -402,6 +412,8 @@ extern "C" int sp_moe_ep_experts_dev(sp_moe *h, int layer, int flavour, int n_ro
                                     "worst case an expert-parallel rank can receive)", n_rows, h->bs.max_rows);
     if (n_rows == 0) return SP_MOE_OK;
     if (!rows_in_dev || !offsets_dev || !rows_out_dev) return fail(SP_MOE_EBADARG, "sp_moe_ep_experts_dev: NULL argument");
+    if (flavour == SP_MOE_FLAVOUR_PREFILL && ((uintptr_t)rows_in_dev & 15))
+        return fail(SP_MOE_EBADARG, "sp_moe_ep_experts_dev: in the prefill arithmetic rows_in must start on a 16-byte boundary");
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     cudaStream_t st = (cudaStream_t)stream; h->last_stream = st;
     int nlaunch = 0;

@@ -156,8 +156,10 @@ __device__ __forceinline__ void split_quad(const float4 &f, bool ok, int i, __ha
     if (ok) *reinterpret_cast<uint4 *>((up ? lo : hi) + 8 * (i >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 /* FEW: at most one block per SM, so its latency counts: the norm weights are fetched while the previous kernel drains, all
- * pair rows at once. Otherwise three blocks (two of E above 3072) share an SM and the registers. */
-template <bool FIN, int OUT, bool WIDE, bool FEW>
+ * pair rows at once. Otherwise three blocks (two of E above 3072) share an SM and the registers.
+ * VEC: rows by 16-byte accesses. Without it (a caller's x, pair rows or y on some other float boundary) by single floats; the
+ * handle's own vectors are aligned either way. */
+template <bool FIN, int OUT, bool WIDE, bool FEW, bool VEC = true>
 __global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_token(SpDims d, TokArgs a) {
     constexpr int KB = FEW ? SP_MAX_NU : 4;
     __shared__ double red[3][32];
@@ -180,7 +182,12 @@ __global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_
     sp_pdl_next();
     if (OUT && t == 0) for (int k = threadIdx.x; k < d.NE; k += T) a.count[k] = 0;
     const size_t row = (size_t)t * E;
-    auto row4 = [&](const float *p, int h) { return ok[h] ? __ldcs(reinterpret_cast<const float4 *>(p) + ix[h]) : zero; };
+    auto row4 = [&](const float *p, int h) {
+        if (!ok[h]) return zero;
+        if (VEC) return __ldcs(reinterpret_cast<const float4 *>(p) + ix[h]);
+        const float *q = p + 4 * ix[h];
+        return make_float4(__ldcs(q), __ldcs(q + 1), __ldcs(q + 2), __ldcs(q + 3));
+    };
     float4 x[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) x[h] = row4(a.x + row, h);
@@ -226,7 +233,10 @@ __global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_
         for (int h = 0; h < 2; h++) {
             const float4 r = scale4(dn[h], sc3, vec(2, h));
             x[h] = make_float4(__fadd_rn(x[h].x, r.x), __fadd_rn(x[h].y, r.y), __fadd_rn(x[h].z, r.z), __fadd_rn(x[h].w, r.w));
-            if (ok[h]) reinterpret_cast<float4 *>(a.y + row)[ix[h]] = x[h];
+            if (ok[h]) {
+                if (VEC) reinterpret_cast<float4 *>(a.y + row)[ix[h]] = x[h];
+                else { float *q = a.y + row + 4 * ix[h]; q[0] = x[h].x; q[1] = x[h].y; q[2] = x[h].z; q[3] = x[h].w; }
+            }
         }
     }
     if (OUT) {
@@ -262,6 +272,12 @@ template <bool FIN, int OUT>
 cudaError_t launch_token(const SpDims &d, int M, const TokArgs &a, cudaStream_t st, int *nl) {
     const unsigned threads = (unsigned)((d.E / 8 + 31) & ~31);
     const bool wide = d.E > 3072, few = M <= kFewTokens;
+    if (((uintptr_t)a.x | (uintptr_t)a.eo | (uintptr_t)a.y) & 15) {
+        /* only the end of a layer meets a caller's pointers as they are (sp_moe_forward_dev, sp_moe_ep_finish_dev); an x that a
+         * layer begins with is copied to the handle's own buffer first */
+        if constexpr (FIN && OUT == kOutNone) return sp_launch(wide ? k_b_token<FIN, OUT, true, false, false> : k_b_token<FIN, OUT, false, false, false>, dim3((unsigned)M), threads, 0, st, nl, d, a);
+        else return cudaErrorInvalidValue;
+    }
     return sp_launch(wide ? (few ? k_b_token<FIN, OUT, true, true> : k_b_token<FIN, OUT, true, false>) : (few ? k_b_token<FIN, OUT, false, true> : k_b_token<FIN, OUT, false, false>),
                      dim3((unsigned)M), threads, 0, st, nl, d, a);
 }
@@ -511,13 +527,15 @@ cudaError_t launch_topk(const SpDims &d, const SpLayerDev &L, BView &v, int M, i
 }
 
 /* ---------------------------------------------------------------- per-row activation quant (CF:1725-1746): received rows of an expert-parallel run */
+template <bool VEC>                                                             /* a caller's rows on some other float boundary: single floats */
 __global__ void __launch_bounds__(1024) k_b_quant_rows(const float *x, int n, unsigned char *act) {
     const size_t r = blockIdx.x;
     const int i = threadIdx.x;
     const bool ok = 4 * i < n;
     sp_pdl_wait();
     sp_pdl_next();
-    const float4 f = ok ? reinterpret_cast<const float4 *>(x + r * n)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float *p = x + r * n + 4 * i;
+    const float4 f = !ok ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : VEC ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
     quant_quad(f, ok, i, act + r * sp_act_pitch(n), n);
 }
 
@@ -923,7 +941,7 @@ cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float 
     if (R == 0) return cudaSuccess;
     if (!FA && tc) return sp_tc_routed(tc, d, L, R, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
     if (FA) {
-        cudaError_t e = sp_launch(k_b_quant_rows, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q);
+        cudaError_t e = sp_launch((uintptr_t)rows_in & 15 ? k_b_quant_rows<false> : k_b_quant_rows<true>, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q);
         if (e != cudaSuccess) return e;
         SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v), down = seg_routed_down(d, L, R, v, rows_out);
         up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */

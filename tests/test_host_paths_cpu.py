@@ -1,0 +1,84 @@
+"""Host side of the entry points without a GPU: which kernels a call launches with which pointers, and what it does when a
+launch fails (the library's own objects over the runtime of fake_cudart.c)."""
+import ctypes as C
+import re
+
+import numpy as np
+import pytest
+
+import fake_cuda
+import orc
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    return fake_cuda.load(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture(autouse=True)
+def _reset(fake):
+    yield
+    fake.log.clear(); fake.read = {}; fake.on_launch = None
+    fake.L.fake_set_sms(148)
+
+
+def _floats(n, off):
+    """n floats that start `off` bytes past a 64-byte boundary."""
+    raw = np.zeros(4 * n + 128, np.uint8)
+    at = (-raw.ctypes.data) % 64 + off
+    return raw[at:at + 4 * n].view(np.float32)
+
+
+def _vectorised(name):
+    """Does this instance of k_b_token / k_b_quant_rows use 16-byte accesses of the rows it is given?"""
+    m = re.search(r"k_b_tokenILb[01]ELi\dELb[01]ELb[01]E(?:Lb([01])E)?|k_b_quant_rows(?:ILb([01])E)?", name)
+    return "0" not in (m.group(1), m.group(2))
+
+
+def _token_kernels_are_safe(fake):
+    seen = fake.launches("k_b_token")
+    for k in seen:
+        fin = "k_b_tokenILb1" in k.name
+        x, eo, y = k.words[0], k.words[2], k.words[8]
+        misaligned = any(p & 15 for p in ((x, eo, y) if fin else (x,)))
+        assert not (misaligned and _vectorised(k.name)), f"{k.name} is given {x:#x} {eo:#x} {y:#x}"
+    return len(seen)
+
+
+@pytest.mark.parametrize("flavour", [0, 1])
+@pytest.mark.parametrize("n_layers", [1, 3])
+@pytest.mark.parametrize("xo,yo", [(0, 0), (4, 0), (0, 8), (12, 4)])
+def test_forward_takes_any_float_boundary(fake, flavour, n_layers, xo, yo):
+    """Beyond 64 tokens the kernels run on the caller's x and y: no kernel with 16-byte accesses may meet another boundary."""
+    cfg, M = orc.SMALL, 70
+    h = fake.engine(cfg, n_layers=n_layers, max_tokens=M)
+    fake.read = {"k_b_token": (1, 9)}
+    x, y = _floats(M * cfg["E"], xo), _floats(M * cfg["E"], yo)
+    assert fake.L.sp_moe_forward_dev(h, 0, n_layers, flavour, M, x.ctypes.data, y.ctypes.data, None, None, None) == 0
+    assert _token_kernels_are_safe(fake) >= n_layers + 1
+    fake.L.sp_moe_close(h)
+
+
+@pytest.mark.parametrize("flavour", [0, 1])
+@pytest.mark.parametrize("off", [0, 4, 8])
+def test_expert_parallel_stages_take_any_float_boundary(fake, flavour, off):
+    cfg, M = orc.SMALL, 6
+    E, NE, NU = cfg["E"], cfg["NE"], cfg["NU"]
+    h = fake.engine(cfg, max_tokens=M)
+    fake.read = {"k_b_token": (1, 9), "k_b_quant_rows": (0, 1)}
+    x, y, pairs = _floats(M * E, off), _floats(M * E, off), _floats(M * NU * E, off)
+    rows, out, ints = _floats(M * NU * E, 0), _floats(M * NU * E, 0), np.zeros(M * NU + NE + 1, np.int32)
+    p = lambda a: a.ctypes.data
+    route = lambda r: fake.L.sp_moe_ep_route_dev(h, 0, flavour, M, p(x), p(ints), p(_floats(M * NU, 0)), p(r), p(ints), p(ints), None, None, 0, 0, 0, None)
+    assert route(rows) == 0
+    assert fake.L.sp_moe_ep_finish_dev(h, 0, M, p(x), p(pairs), None, p(y), None) == 0
+    assert _token_kernels_are_safe(fake) == 2
+    experts = lambda r: fake.L.sp_moe_ep_experts_dev(h, 0, flavour, M * NU, p(r), None, p(ints), p(out), None)
+    if flavour == 0 or off == 0:
+        assert experts(pairs) == 0
+        for k in fake.launches("k_b_quant_rows"):
+            assert not (k.words[0] & 15 and _vectorised(k.name))
+    else:                                                    # what only ever ran on 16-byte boundaries is refused, not launched
+        before = len(fake.launches())
+        assert experts(pairs) == -3 and route(pairs) == -3 and len(fake.launches()) == before
+    fake.L.sp_moe_close(h)

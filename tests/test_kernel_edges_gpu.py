@@ -104,3 +104,37 @@ def test_hook_edges(E, FF, NE, NU):
     diff = y.astype(np.float64) - ref
     assert np.abs(diff).max() <= MAX_ABS and np.linalg.norm(diff) / np.linalg.norm(ref) <= REL_L2
     ext.close()
+
+
+def _at(t, off):
+    """The values of t in a buffer that starts `off` floats past a 16-byte boundary."""
+    import torch
+    buf = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+    out = buf[off:off + t.numel()].view(t.shape)
+    assert out.data_ptr() % 16 == 4 * off
+    return out.copy_(t)
+
+
+@pytest.mark.parametrize("flavour", [A, B])
+@pytest.mark.parametrize("cfg,M", [(SMALL, 66), (SMALL, 200), (_cfg(3200, 8, 2, 64, 64), 65)])
+def test_vectors_on_any_float_boundary(cfg, M, flavour):
+    """x, y and pair rows where only floats are aligned: the bits of the aligned call, through the layer and through its
+    expert-parallel stages."""
+    import torch
+    eng, _ = make_stack(cfg, 2, seed=74, rand_norms=True, max_tokens=M)
+    x = torch.randn(M, cfg["E"], generator=torch.Generator().manual_seed(M)).cuda()
+    for n in (1, 2):
+        want = torch.empty_like(x)
+        eng.forward_dev(x, want, n_layers=n, flavour=flavour)
+        for xo, yo in ((1, 0), (0, 2), (3, 3)):
+            xm, y = _at(x, xo), _at(torch.zeros_like(x), yo)
+            eng.forward_dev(xm, y, n_layers=n, flavour=flavour)
+            assert torch.equal(y, want) and torch.equal(xm, x)
+            eng.forward_dev(xm, xm, n_layers=n, flavour=flavour)          # in place
+            assert torch.equal(xm, want)
+    eng.forward_dev(x, want, n_layers=1, flavour=flavour)
+    _, _, rows, counts, pair_index = eng.ep_route(0, _at(x, 1), flavour)
+    off = torch.cat([torch.zeros(1, dtype=torch.int32, device="cuda"), counts.cumsum(0).int()])
+    out = eng.ep_experts(0, _at(rows, 1) if flavour == A else rows, off, flavour)
+    assert torch.equal(eng.ep_finish(0, _at(x, 2), _at(out, 3), pair_index=pair_index), want)
+    eng.status(); eng.close()
