@@ -36,6 +36,7 @@ __device__ __forceinline__ void ext_quant(const float *p, int4 *q, float *sx, in
     quant_block16_store(v, q, sx, corr);
 }
 __global__ void __launch_bounds__(256) k_ext_quant(const float *x, int E, int4 *q, float *sx, int *corr) {
+    sp_pdl_wait();
     sp_pdl_next();
     for (int b = threadIdx.x; b < (E >> 4); b += 256) ext_quant(x + 16 * b, q + b, sx + b, corr + b);
 }
@@ -259,7 +260,7 @@ extern "C" int sp_moe_ext_moe(void *vh, const char *tag, const int *idx, const f
     for (int k = 0; k < NU; k++) if (idx[k] < 0 || idx[k] >= M->NE) { sp_set_error("sp_moe_ext_moe: expert index out of range"); return -1; }
     if (cudaSetDevice(h->device) != cudaSuccess) return -1;
     cudaStream_t st = h->st;
-    memcpy(h->s.hx, x, 4 * (size_t)E);                                  /* the stream is idle between calls */
+    memcpy(h->s.hx, x, 4 * (size_t)E);                                  /* the stream is idle between calls, also after one that failed */
     ExtArgs a{};
     a.g_codes = M->g_codes; a.u_codes = M->u_codes; a.d_codes = M->d_codes; a.g_bs = M->g_bs; a.u_bs = M->u_bs; a.d_bs = M->d_bs;
     a.E = E; a.FF = FF; a.qx = h->s.qx; a.sx = h->s.sx; a.cx = h->s.cx; a.h = h->s.h; a.acc = h->s.acc; a.y = h->s.hy;
@@ -272,7 +273,8 @@ extern "C" int sp_moe_ext_moe(void *vh, const char *tag, const int *idx, const f
         e = sp_launch(ext_up_for(E), dim3((unsigned)ext_grid(h, a.pick.n * FF)), kExtT, ext_smem(E), st, &nl, a);
         if (e == cudaSuccess) e = sp_launch(ext_down_for(FF), dim3((unsigned)ext_grid(h, E)), kExtT, ext_smem(a.pick.n * FF), st, &nl, a);
     }
-    if (e != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return -1;
+    const cudaError_t done = cudaStreamSynchronize(st);                 /* what was launched still reads hx, also when a later launch failed */
+    if (e != cudaSuccess || done != cudaSuccess) { cudaGetLastError(); sp_set_error("sp_moe_ext_moe: a kernel of the call failed"); return -1; }
     memcpy(y, h->s.hy, 4 * (size_t)E);
     return 0;
 }

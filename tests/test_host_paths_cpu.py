@@ -1,6 +1,8 @@
 """Host side of the entry points without a GPU: which kernels a call launches with which pointers, and what it does when a
 launch fails (the library's own objects over the runtime of fake_cudart.c)."""
 import ctypes as C
+import glob
+import os
 import re
 
 import numpy as np
@@ -82,3 +84,49 @@ def test_expert_parallel_stages_take_any_float_boundary(fake, flavour, off):
         before = len(fake.launches())
         assert experts(pairs) == -3 and route(pairs) == -3 and len(fake.launches()) == before
     fake.L.sp_moe_close(h)
+
+
+def _hook(fake, E=64, FF=32, NE=4):
+    h = C.c_void_p()
+    assert fake.L.sp_moe_ext_open(0, C.byref(h)) == 0
+    blob = np.zeros(NE * FF * E, np.uint8).ctypes.data
+    assert fake.L.sp_moe_ext_upload_experts(h, b"t", blob, blob, blob, blob, blob, blob, NE, FF, E) == 0
+    idx, wt, x, y = np.zeros(20, np.int32), np.zeros(20, np.float32), np.zeros(E, np.float32), np.zeros(E, np.float32)
+    return h, lambda n: fake.L.sp_moe_ext_moe(h, b"t", idx.ctypes.data, wt.ctypes.data, n, x.ctypes.data, E, FF, y.ctypes.data)
+
+
+@pytest.mark.parametrize("n,failing", [(2, 0), (2, 1), (2, 2), (20, 3)])
+def test_hook_leaves_nothing_running_when_a_launch_fails(fake, n, failing):
+    """The call reads its x from a buffer of the handle that the next call overwrites: also a call that fails waits for
+    what it had launched."""
+    h, call = _hook(fake)
+    count = [0]
+
+    def fail_one(_):
+        count[0] += 1
+        return 700 if count[0] == failing + 1 else 0
+    fake.log.clear(); fake.on_launch = fail_one
+    assert call(n) != 0
+    assert isinstance(fake.log[-1], tuple) and fake.log[-1][0] == "sync"
+    fake.on_launch = None; fake.log.clear()
+    assert call(n) == 0 and fake.log[-1][0] == "sync"
+    fake.L.sp_moe_ext_close(h)
+
+
+def test_kernels_launched_programmatically_wait():
+    """launch.cuh's rule, over the sources: a kernel launched with sp_launch, or one that lets its successor start early, waits
+    for its predecessor before it lets the successor start."""
+    checked = 0
+    for path in glob.glob(os.path.join(os.path.dirname(fake_cuda.HERE), "kairos_engine_b200", "csrc", "*.cu")):
+        src = re.sub(r"/\*.*?\*/", "", open(path).read(), flags=re.S)
+        if '"launch.cuh"' not in src:
+            continue
+        named = set(re.findall(r"k_\w+", " ".join(re.findall(r"sp_launch\(.*?;", src, flags=re.S))))
+        for part in re.split(r"__global__", src)[1:]:
+            name, body = re.search(r"\b(k_\w+)\s*\(", part).group(1), part[part.index("{"):]
+            body = body[:body.index("\n}\n")]
+            if name in named or "sp_pdl_next()" in body:
+                wait, nxt = body.find("sp_pdl_wait()"), body.find("sp_pdl_next()")
+                assert wait >= 0 and (nxt < 0 or wait < nxt), f"{name} ({os.path.basename(path)})"
+                checked += 1
+    assert checked >= 12
