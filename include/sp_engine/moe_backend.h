@@ -232,7 +232,8 @@ int sp_moe_ext_moe(void *h, const char *tag, const int *idx, const float *wt, in
  *   C[m][n] (f16 bits) = f16( float(sum_k A[m][k] * B[n][k]) * scale_a[m] * scale_b[n] ),
  * A [M][K] and B [N][K] int8 (q8) or packed signed int4, two per byte, low nibble first (q4);
  * int32 accumulate; K a multiple of 16, operand pointers 16-byte aligned. Enqueues on `stream`;
- * the q4 entry unpacks inside the kernel (no scratch) and, as before, returns after synchronising the stream. */
+ * the q4 entry unpacks inside the kernel (no scratch) and returns after synchronising the stream, with its own kernel's
+ * verdict. */
 int sp_frob_matmul_q8_dev(const int8_t *A_dev, const int8_t *B_dev, const float *scale_a_dev,
                           const float *scale_b_dev, uint16_t *C_f16_dev, int M, int K, int N, void *stream);
 int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q4_dev, const float *scale_a_dev,

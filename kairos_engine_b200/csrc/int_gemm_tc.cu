@@ -17,6 +17,7 @@
  * Warp roles: 0-7 epilogue (TMEM lane quadrant = warp % 4), 8 TMA, 9 MMA issue + TMEM allocation, 10-25 int4 unpack. Every
  * wait is bounded.
  */
+#include <condition_variable>
 #include <mutex>
 #include "tc_common.cuh"
 #include "../../include/sp_engine/moe_backend.h"
@@ -259,7 +260,15 @@ int pick_tile(int M, int K, int N, int sms) {
     }
     return best;
 }
-struct IgDevice { int *status; int sms; bool ready; };     /* status: a page-locked word a kernel writes when a bounded wait ran out */
+/* Per device, made at first use there. words: page-locked, a kernel writes the one it is given when a bounded wait ran out.
+ * Word 0 is the int8 entry's, which returns before its kernel runs; an int4 call has one of the others to itself, so that calls
+ * from several threads do not read each other's verdict. */
+constexpr int kWords = 64;
+struct IgDevice { int *words; int sms; bool ready; unsigned long long taken; };
+std::mutex g_mu;
+std::condition_variable g_word_free;
+IgDevice g_devices[kMaxDevices];
+EncodeTiledFn g_encode = nullptr;
 
 template <int MH, int NT, bool PACKED>
 cudaError_t ig_prepare() { return cudaFuncSetAttribute(k_i8_gemm<MH, NT, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IgCfg<MH, NT, PACKED>::kSmem); }
@@ -276,34 +285,38 @@ void ig_launch(const IgMaps &maps, const IgArgs &g, int sms, cudaStream_t st) {
     k_i8_gemm<MH, NT, PACKED><<<(unsigned)(tiles < sms ? tiles : sms), IgCfg<MH, NT, PACKED>::kThreads, IgCfg<MH, NT, PACKED>::kSmem, st>>>(maps, g);
 }
 
-template <bool PACKED>
-int run(const void *A, const void *B, const float *sa, const float *sb, uint16_t *C, int M, int K, int N, cudaStream_t st, int **status_out = nullptr) {
+int check_args(const void *A, const void *B, const float *sa, const float *sb, const uint16_t *C, int M, int K, int N) {
     if (!A || !B || !sa || !sb || !C) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: NULL argument");
     if (M <= 0 || N <= 0 || K <= 0 || (K & 15)) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: M, N, K must be positive and K a multiple of 16");
     if (((uintptr_t)A | (uintptr_t)B) & 15) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: operand pointers must be 16-byte aligned");
+    return SP_MOE_OK;
+}
+/* the current device, ready for use */
+int device_state(IgDevice **out) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return ig_fail(SP_MOE_ECUDA, "quantised GEMM: no CUDA device");
     if (dev < 0 || dev >= kMaxDevices) return ig_fail(SP_MOE_EUNSUPPORTED, "quantised GEMM: device ordinal out of range");
-    static std::mutex mu;                                 /* one status word and the kernels' attributes per device, at first use there */
-    static IgDevice devices[kMaxDevices] = {};
-    static EncodeTiledFn fn = nullptr;
-    int *status = nullptr, sms = 0;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!fn && encode_tiled_fn(&fn) != cudaSuccess) return ig_fail(SP_MOE_EUNSUPPORTED, "quantised GEMM: cuTensorMapEncodeTiled is not available");
-        IgDevice &d = devices[dev];
-        if (!d.ready) {
-            if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || ig_prepare_all<false>() != cudaSuccess || ig_prepare_all<true>() != cudaSuccess)
-                return ig_fail(SP_MOE_ECUDA, "quantised GEMM: kernel attributes");
-            if (!d.status && cudaMallocHost((void **)&d.status, 64) != cudaSuccess) { d.status = nullptr; cudaGetLastError(); return ig_fail(SP_MOE_ECUDA, "quantised GEMM: status word allocation failed"); }
-            *d.status = 0;
-            d.ready = true;
-        }
-        status = d.status; sms = d.sms;
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_encode && encode_tiled_fn(&g_encode) != cudaSuccess) return ig_fail(SP_MOE_EUNSUPPORTED, "quantised GEMM: cuTensorMapEncodeTiled is not available");
+    IgDevice &d = g_devices[dev];
+    if (!d.ready) {
+        if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || ig_prepare_all<false>() != cudaSuccess || ig_prepare_all<true>() != cudaSuccess)
+            return ig_fail(SP_MOE_ECUDA, "quantised GEMM: kernel attributes");
+        if (!d.words && cudaMallocHost((void **)&d.words, kWords * sizeof(int)) != cudaSuccess) { d.words = nullptr; cudaGetLastError(); return ig_fail(SP_MOE_ECUDA, "quantised GEMM: status word allocation failed"); }
+        for (int i = 0; i < kWords; i++) d.words[i] = 0;
+        d.taken = 1;                                      /* word 0 */
+        d.ready = true;
     }
+    *out = &d;
+    return SP_MOE_OK;
+}
+
+template <bool PACKED>
+int enqueue(const IgDevice &dev, int *status, const void *A, const void *B, const float *sa, const float *sb, uint16_t *C, int M, int K, int N, cudaStream_t st) {
+    const int sms = dev.sms;
     const int t = pick_tile(M, K, N, sms);
     IgMaps maps = {};
-    if (!PACKED && (make_u8_map(fn, &maps.a, A, K, M, kTiles[t].mh * 128) != cudaSuccess || make_u8_map(fn, &maps.b, B, K, N, kTiles[t].nt) != cudaSuccess))
+    if (!PACKED && (make_u8_map(g_encode, &maps.a, A, K, M, kTiles[t].mh * 128) != cudaSuccess || make_u8_map(g_encode, &maps.b, B, K, N, kTiles[t].nt) != cudaSuccess))
         return ig_fail(SP_MOE_EBADARG, "quantised GEMM: could not describe the operands to the TMA unit");
     const IgArgs g{(const uint8_t *)A, (const uint8_t *)B, sa, sb, reinterpret_cast<__half *>(C), M, K, N, status};
     switch (t) {
@@ -313,7 +326,6 @@ int run(const void *A, const void *B, const float *sa, const float *sb, uint16_t
     default: ig_launch<1, 64, PACKED>(maps, g, sms, st);
     }
     if (cudaGetLastError() != cudaSuccess) return ig_fail(SP_MOE_ECUDA, "quantised GEMM: kernel launch failed");
-    if (status_out) *status_out = status;
     return SP_MOE_OK;
 }
 
@@ -321,17 +333,36 @@ int run(const void *A, const void *B, const float *sa, const float *sb, uint16_t
 
 extern "C" int sp_frob_matmul_q8_dev(const int8_t *A_dev, const int8_t *B_dev, const float *scale_a_dev, const float *scale_b_dev,
                                      uint16_t *C_f16_dev, int M, int K, int N, void *stream) {
-    return run<false>(A_dev, B_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream);
+    int rc = check_args(A_dev, B_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N);
+    IgDevice *d = nullptr;
+    if (rc == SP_MOE_OK) rc = device_state(&d);
+    if (rc != SP_MOE_OK) return rc;
+    return enqueue<false>(*d, d->words, A_dev, B_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream);
 }
 
 extern "C" int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q4_dev, const float *scale_a_dev, const float *scale_b_dev,
                                      uint16_t *C_f16_dev, int M, int K, int N, void *stream) {
-    int *status = nullptr;
-    const int rc = run<true>(A_q4_dev, B_q4_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream, &status);
+    int rc = check_args(A_q4_dev, B_q4_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N);
+    IgDevice *d = nullptr;
+    if (rc == SP_MOE_OK) rc = device_state(&d);
     if (rc != SP_MOE_OK) return rc;
+    int w = 0;
+    {
+        std::unique_lock<std::mutex> lk(g_mu);
+        g_word_free.wait(lk, [&] { return ~d->taken != 0; });          /* every call that holds one is about to return */
+        while (d->taken >> w & 1) w++;
+        d->taken |= 1ull << w;
+    }
+    volatile int *word = d->words + w;
+    *word = 0;
+    rc = enqueue<true>(*d, d->words + w, A_q4_dev, B_q4_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream);
     /* this entry returns when the result is there, with the kernel's own verdict */
-    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q4_dev: the stream reported an error");
-    volatile int *word = status;
-    if (*word) { *word = 0; return ig_fail(SP_MOE_ECUDA, "quantised GEMM: a bounded wait inside the kernel ran out"); }
-    return SP_MOE_OK;
+    if (rc == SP_MOE_OK && cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) rc = ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q4_dev: the stream reported an error");
+    if (rc == SP_MOE_OK && *word) rc = ig_fail(SP_MOE_ECUDA, "quantised GEMM: a bounded wait inside the kernel ran out");
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        d->taken &= ~(1ull << w);
+    }
+    g_word_free.notify_one();
+    return rc;
 }

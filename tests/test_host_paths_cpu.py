@@ -130,3 +130,32 @@ def test_kernels_launched_programmatically_wait():
                 assert wait >= 0 and (nxt < 0 or wait < nxt), f"{name} ({os.path.basename(path)})"
                 checked += 1
     assert checked >= 12
+
+
+def _gemm(fake, entry, A=None, B=None, out=None, M=32, K=32, N=32):
+    a = np.zeros(4 * M * max(K, N) + 256, np.uint8)
+    base = a.ctypes.data + (-a.ctypes.data) % 64
+    p = lambda given: base if given is None else given
+    return getattr(fake.L, entry)(p(A), p(B), base, base, p(out), M, K, N, None)
+
+
+def _fail_wait(launch):
+    C.cast(launch.words[7], C.POINTER(C.c_int))[0] = 2      # what the kernel does when a bounded wait runs out
+
+
+def test_int4_calls_in_flight_together_have_their_own_verdict(fake):
+    fake.read = {"k_i8_gemm": (1, 8)}
+    inner = []
+
+    def first(launch):
+        _fail_wait(launch)
+        fake.on_launch = None
+        inner.append(_gemm(fake, "sp_frob_matmul_q4_dev"))  # another thread's call, while this one has not returned
+    fake.on_launch = first
+    assert _gemm(fake, "sp_frob_matmul_q4_dev") == -40 and inner == [0]
+    assert _gemm(fake, "sp_frob_matmul_q4_dev") == 0
+    for _ in range(200):                                    # the words are given back, by failed calls too
+        fake.on_launch = _fail_wait
+        assert _gemm(fake, "sp_frob_matmul_q4_dev") == -40
+        fake.on_launch = lambda launch: 700
+        assert _gemm(fake, "sp_frob_matmul_q4_dev") == -40
