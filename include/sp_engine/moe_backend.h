@@ -233,7 +233,8 @@ int sp_moe_ext_moe(void *h, const char *tag, const int *idx, const float *wt, in
  * A [M][K] and B [N][K] int8 (q8) or packed signed int4, two per byte, low nibble first (q4);
  * int32 accumulate; K a multiple of 16, operand pointers 16-byte aligned. Enqueues on `stream`;
  * the q4 entry unpacks inside the kernel (no scratch) and returns after synchronising the stream, with its own kernel's
- * verdict. */
+ * verdict. The q8 entry returns before its kernel runs: should a bounded wait inside it run out, the next q8 call on that
+ * device says so (SP_MOE_ECUDA) and enqueues nothing. */
 int sp_frob_matmul_q8_dev(const int8_t *A_dev, const int8_t *B_dev, const float *scale_a_dev,
                           const float *scale_b_dev, uint16_t *C_f16_dev, int M, int K, int N, void *stream);
 int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q4_dev, const float *scale_a_dev,

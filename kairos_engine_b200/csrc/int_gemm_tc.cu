@@ -337,6 +337,8 @@ extern "C" int sp_frob_matmul_q8_dev(const int8_t *A_dev, const int8_t *B_dev, c
     IgDevice *d = nullptr;
     if (rc == SP_MOE_OK) rc = device_state(&d);
     if (rc != SP_MOE_OK) return rc;
+    volatile int *word = d->words;                        /* the kernel runs after this call has returned: what went wrong there is told to the next one */
+    if (*word) { *word = 0; return ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q8_dev: in an earlier int8 call on this device a bounded wait inside the kernel ran out and its result is invalid; this call enqueued nothing"); }
     return enqueue<false>(*d, d->words, A_dev, B_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream);
 }
 

@@ -159,3 +159,14 @@ def test_int4_calls_in_flight_together_have_their_own_verdict(fake):
         assert _gemm(fake, "sp_frob_matmul_q4_dev") == -40
         fake.on_launch = lambda launch: 700
         assert _gemm(fake, "sp_frob_matmul_q4_dev") == -40
+
+
+def test_int8_verdict_reaches_the_next_int8_call_only(fake):
+    fake.read = {"k_i8_gemm": (1, 8)}
+    fake.on_launch = _fail_wait
+    assert _gemm(fake, "sp_frob_matmul_q8_dev") == 0        # returns before its kernel runs
+    fake.on_launch = None
+    assert _gemm(fake, "sp_frob_matmul_q4_dev") == 0
+    before = len(fake.launches())
+    assert _gemm(fake, "sp_frob_matmul_q8_dev") == -40 and b"earlier" in fake.L.sp_last_error() and len(fake.launches()) == before
+    assert _gemm(fake, "sp_frob_matmul_q8_dev") == 0 and len(fake.launches()) == before + 1
