@@ -288,7 +288,6 @@ void ig_launch(const IgMaps &maps, const IgArgs &g, int sms, cudaStream_t st) {
 int check_args(const void *A, const void *B, const float *sa, const float *sb, const uint16_t *C, int M, int K, int N) {
     if (!A || !B || !sa || !sb || !C) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: NULL argument");
     if (M <= 0 || N <= 0 || K <= 0 || (K & 15)) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: M, N, K must be positive and K a multiple of 16");
-    if (((uintptr_t)A | (uintptr_t)B) & 15) return ig_fail(SP_MOE_EBADARG, "quantised GEMM: operand pointers must be 16-byte aligned");
     return SP_MOE_OK;
 }
 /* the current device, ready for use */
@@ -334,6 +333,7 @@ int enqueue(const IgDevice &dev, int *status, const void *A, const void *B, cons
 extern "C" int sp_frob_matmul_q8_dev(const int8_t *A_dev, const int8_t *B_dev, const float *scale_a_dev, const float *scale_b_dev,
                                      uint16_t *C_f16_dev, int M, int K, int N, void *stream) {
     int rc = check_args(A_dev, B_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N);
+    if (rc == SP_MOE_OK && ((uintptr_t)A_dev | (uintptr_t)B_dev) & 15) rc = ig_fail(SP_MOE_EBADARG, "quantised GEMM: operand pointers must be 16-byte aligned");
     IgDevice *d = nullptr;
     if (rc == SP_MOE_OK) rc = device_state(&d);
     if (rc != SP_MOE_OK) return rc;
@@ -348,6 +348,18 @@ extern "C" int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q
     IgDevice *d = nullptr;
     if (rc == SP_MOE_OK) rc = device_state(&d);
     if (rc != SP_MOE_OK) return rc;
+    /* the kernel copies pieces of 8 or 16 bytes: operands that start on another byte are moved first */
+    cudaStream_t st = (cudaStream_t)stream;
+    uint8_t *moved = nullptr;
+    if (((uintptr_t)A_q4_dev | (uintptr_t)B_q4_dev) & 15) {
+        const size_t na = (size_t)M * (K / 2), nb = (size_t)N * (K / 2), at = (na + 255) & ~(size_t)255;
+        if (cudaMalloc((void **)&moved, at + nb) != cudaSuccess) { cudaGetLastError(); return ig_fail(SP_MOE_EBACKEND_OOM, "sp_frob_matmul_q4_dev: scratch allocation failed"); }
+        if (cudaMemcpyAsync(moved, A_q4_dev, na, cudaMemcpyDeviceToDevice, st) != cudaSuccess || cudaMemcpyAsync(moved + at, B_q4_dev, nb, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+            cudaStreamSynchronize(st); cudaFree(moved); cudaGetLastError();
+            return ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q4_dev: copying the operands failed");
+        }
+        A_q4_dev = moved; B_q4_dev = moved + at;
+    }
     int w = 0;
     {
         std::unique_lock<std::mutex> lk(g_mu);
@@ -357,14 +369,15 @@ extern "C" int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q
     }
     volatile int *word = d->words + w;
     *word = 0;
-    rc = enqueue<true>(*d, d->words + w, A_q4_dev, B_q4_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, (cudaStream_t)stream);
+    rc = enqueue<true>(*d, d->words + w, A_q4_dev, B_q4_dev, scale_a_dev, scale_b_dev, C_f16_dev, M, K, N, st);
     /* this entry returns when the result is there, with the kernel's own verdict */
-    if (rc == SP_MOE_OK && cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) rc = ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q4_dev: the stream reported an error");
+    if (cudaStreamSynchronize(st) != cudaSuccess && rc == SP_MOE_OK) rc = ig_fail(SP_MOE_ECUDA, "sp_frob_matmul_q4_dev: the stream reported an error");
     if (rc == SP_MOE_OK && *word) rc = ig_fail(SP_MOE_ECUDA, "quantised GEMM: a bounded wait inside the kernel ran out");
     {
         std::lock_guard<std::mutex> lk(g_mu);
         d->taken &= ~(1ull << w);
     }
     g_word_free.notify_one();
+    if (moved) cudaFree(moved);
     return rc;
 }

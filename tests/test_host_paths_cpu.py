@@ -170,3 +170,17 @@ def test_int8_verdict_reaches_the_next_int8_call_only(fake):
     before = len(fake.launches())
     assert _gemm(fake, "sp_frob_matmul_q8_dev") == -40 and b"earlier" in fake.L.sp_last_error() and len(fake.launches()) == before
     assert _gemm(fake, "sp_frob_matmul_q8_dev") == 0 and len(fake.launches()) == before + 1
+
+
+@pytest.mark.parametrize("off", [(1, 0), (0, 8), (7, 3)])
+def test_packed_operands_start_on_any_byte(fake, off):
+    """They are moved to where the kernel's copies can read them; int8 operands on another boundary stay refused."""
+    fake.read = {"k_i8_gemm": (1, 8)}
+    raw = np.arange(4096, dtype=np.uint8)
+    base = raw.ctypes.data + (-raw.ctypes.data) % 64
+    assert _gemm(fake, "sp_frob_matmul_q4_dev", A=base + off[0], B=base + 1024 + off[1]) == 0
+    a, b = fake.launches()[-1].words[:2]
+    assert a % 16 == 0 and b % 16 == 0
+    copies = [(src, n) for what, dst, src, n in (x for x in fake.log if isinstance(x, tuple)) if what == "memcpy"]
+    assert copies == [(base + off[0], 32 * 16), (base + 1024 + off[1], 32 * 16)]
+    assert _gemm(fake, "sp_frob_matmul_q8_dev", A=base + off[0], B=base + 1024 + off[1]) == -3

@@ -52,6 +52,21 @@ def test_packed_int4_bit_exact(M, N, K):
     assert np.array_equal(got.cpu().numpy().view(np.uint16), ref)
 
 
+def test_packed_operands_on_any_byte():
+    """Row 1 onwards of an operand whose rows are 24 bytes starts on 8 bytes, a view into raw bytes on any."""
+    import torch
+    from kairos_engine_b200.engine import int_gemm_scaled
+    r = np.random.default_rng(5)
+    M, N, K = 70, 72, 48
+    sa, sb = torch.rand(M, device="cuda"), torch.rand(N, device="cuda")
+    A, B = (torch.from_numpy(r.integers(0, 256, (n, K // 2), dtype=np.uint8)).cuda() for n in (M + 1, N))
+    raw = torch.empty(N * K // 2 + 3, dtype=torch.uint8, device="cuda")
+    Bm = raw[3:].view(N, K // 2).copy_(B)
+    assert A[1:].data_ptr() % 16 == 8 and Bm.data_ptr() % 16 == 3
+    want = int_gemm_scaled(A[1:].clone(), B, sa, sb, packed_int4=True)
+    assert torch.equal(int_gemm_scaled(A[1:], Bm, sa, sb, packed_int4=True), want)
+
+
 def test_bad_arguments_are_refused():
     import torch
     from kairos_engine_b200 import SpMoeError
