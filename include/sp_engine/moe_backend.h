@@ -231,7 +231,7 @@ int sp_moe_ext_moe(void *h, const char *tag, const int *idx, const float *wt, in
  * and the int4 kernels, ptx_mma.cuh:268-353) on DEVICE memory:
  *   C[m][n] (f16 bits) = f16( float(sum_k A[m][k] * B[n][k]) * scale_a[m] * scale_b[n] ),
  * A [M][K] and B [N][K] int8 (q8) or packed signed int4, two per byte, low nibble first (q4);
- * int32 accumulate; K a multiple of 16, operand pointers 16-byte aligned (packed operands may start on any byte, at the
+ * int32 accumulate; K a multiple of 16, C on any half, operand pointers 16-byte aligned (packed operands may start on any byte, at the
  * price of scratch and a copy). Enqueues on `stream`;
  * the q4 entry unpacks inside the kernel (no scratch) and returns after synchronising the stream, with its own kernel's
  * verdict. The q8 entry returns before its kernel runs: should a bounded wait inside it run out, the next q8 call on that

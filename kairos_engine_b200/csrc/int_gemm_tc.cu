@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(IgCfg<MH, NT, PACKED>::kThreads, 1) k_i8_gemm(
         /* epilogue (ptx_mma_tile_common.cuh:157-176): f16(float(acc) * sa[row] * sb[col]), left to right. The two warps of a
          * lane quadrant take alternate 16-column groups. */
         const int quad = warp & 3;
-        const bool vec = (N & 7) == 0;
+        const bool vec = (N & 7) == 0 && ((uintptr_t)g.C & 15) == 0;          /* every row on 16 bytes */
         int lt = 0;
         for (int w = blockIdx.x; w < total && !failed; w += gridDim.x, lt++) {
             const int n0 = (w % tn) * NT;

@@ -67,6 +67,23 @@ def test_packed_operands_on_any_byte():
     assert torch.equal(int_gemm_scaled(A[1:], Bm, sa, sb, packed_int4=True), want)
 
 
+@pytest.mark.parametrize("off", [1, 4])
+def test_result_on_any_half(off):
+    """C may start off a 16-byte boundary, where its rows are whole 16-byte pieces too."""
+    import torch
+    from kairos_engine_b200 import _lib
+    M, N, K = 130, 136, 64
+    A, B, sa, sb = (torch.from_numpy(a).cuda() for a in _case(M, N, K, 9))
+    raw = torch.zeros(M * N + 8, dtype=torch.float16, device="cuda")
+    for at in (0, off):
+        raw.zero_()
+        _lib.check(_lib.lib().sp_frob_matmul_q8_dev(A.data_ptr(), B.data_ptr(), sa.data_ptr(), sb.data_ptr(), raw[at:].data_ptr(), M, K, N,
+                                                    torch.cuda.current_stream().cuda_stream))
+        if at == 0:
+            want = raw[:M * N].clone()
+    assert torch.equal(raw[off:off + M * N], want) and not raw[:off].any() and not raw[off + M * N:].any()
+
+
 def test_bad_arguments_are_refused():
     import torch
     from kairos_engine_b200 import SpMoeError
