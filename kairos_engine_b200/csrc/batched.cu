@@ -674,7 +674,7 @@ SpRowsSeg seg_routed_down(const SpDims &d, const SpLayerDev &L, int M, const BVi
 template <bool FA>
 cudaError_t run_experts(const SpDims &d, const SpLayerDev &L, int M, BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
     const int E = d.E, NE = d.NE, NU = d.NU, FFE = d.FFE, FFS = d.FFS;
-    if (!FA && tc) return sp_tc_layer(tc, d, L, M, v.nx_f, v.in_f, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);      /* prefill arithmetic on the tensor cores */
+    if (!FA && tc) return sp_tc_layer(tc, d, L, M, v.sel_asc, v.count, v.pairpos, v.dn, v.eo, status, st, nl);      /* prefill arithmetic on the tensor cores */
     if (FA) {
         /* gate|up of the shared and the routed experts, quantised as it leaves (CF:8348-8356, 8733-8737, 8958-8959), then down (CF:8358, 8739-8742, 8961) */
         SpRowsSeg up[2] = {seg_shared_up(d, L, M, v), seg_routed_up(d, L, M, v.in_q, v)};
@@ -709,7 +709,7 @@ template <bool FA>
 cudaError_t run_layers(const SpDims &d, const SpLayerDev *layers, int n, int M, const float *x, float *y, int32_t *sel, float *wts,
                        BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
     /* where the experts' kernels take int8 or split rows, the end of a layer and the beginning of the next are one launch */
-    const bool split = !FA && tc && sp_tc_takes_split(d), fused = FA || split;
+    const bool split = !FA && tc, fused = FA || split;
     const float *cur = x;
     cudaError_t e = cudaSuccess;
     for (int li = 0; li < n && e == cudaSuccess; li++) {

@@ -526,21 +526,6 @@ __global__ void __launch_bounds__(1024) k_tc_sort(SortArgs s) {
     }
 }
 
-/* the same sort as separate launches, for the stage-by-stage path */
-__global__ void __launch_bounds__(1024) k_tc_scan(const int *count, int groups, int *offsets) {
-    __shared__ int sh[32];
-    const int g = threadIdx.x;
-    const int end = scan1024(g < groups ? count[g] : 0, sh);
-    if (g < groups) offsets[g + 1] = end;
-    if (g == 0) offsets[0] = 0;
-}
-__global__ void __launch_bounds__(256) k_tc_pairs(const int *sel_asc, const int *pairpos, const int *offsets, int n_pairs, int NU, int *gather, int *rowmap) {
-    const int p = blockIdx.x * 256 + threadIdx.x;
-    if (p >= n_pairs) return;
-    const int row = offsets[sel_asc[p]] + pairpos[p];
-    gather[row] = p / NU; rowmap[row] = p;
-}
-
 }  // namespace
 
 /* ---------------------------------------------------------------- host side */
@@ -548,7 +533,7 @@ struct SpTcPlan {
     int Mcap, Rcap, sms;
     unsigned char *base; size_t bytes;
     __half *nx_hi, *nx_lo, *hd_hi, *hd_lo, *in_hi, *in_lo, *h_hi, *h_lo, *tk_hi, *tk_lo;           /* tk: the routed experts' input, one row per token; in: one per pair */
-    int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *gather, *rowmap, *offsets;
+    int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *gather, *rowmap;
     int cap_sh, cap_r;
     int terms;                                         /* MMAs per k-step: 3, 2 or 1 */
     CUtensorMap nx[4], hd[4], in[4], h[4];             /* boxes of 16 rows: hi, lo; of 64 rows: hi, lo */
@@ -556,9 +541,6 @@ struct SpTcPlan {
     std::map<const void *, CUtensorMap> codes;         /* one per weight tensor of the arena, made at first use */
 };
 
-/* Geometries with E below 512 only check the stages: they stay one launch per stage (the expert-parallel path's stages), so
- * that callers who count launches see each of them. */
-bool sp_tc_takes_split(const SpDims &d) { return d.E >= 512; }
 void sp_tc_inputs(SpTcPlan *p, __half **nx_hi, __half **nx_lo, __half **in_hi, __half **in_lo) { *nx_hi = p->nx_hi; *nx_lo = p->nx_lo; *in_hi = p->tk_hi; *in_lo = p->tk_lo; }
 bool sp_tc_supported(const SpDims &d) { return (d.E % 64 == 0) && (d.FFE % 64 == 0) && (d.FFS % 64 == 0); }
 
@@ -620,7 +602,7 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     const size_t E = d.E, FFE = d.FFE, FFS = d.FFS, Mc = p->Mcap, Rc = p->Rcap;
     const size_t o_nx = take(4 * Mc * E), o_hd = take(4 * Mc * FFS), o_in = take(4 * Rc * E), o_h = take(4 * Rc * FFE), o_tk = take(4 * Mc * E);      /* hi rows, then lo rows */
     const size_t o_tsh = take(12 * (size_t)p->cap_sh), o_nsh = take(4), o_tr = take(12 * (size_t)p->cap_r), o_nr = take(4);
-    const size_t o_g = take(4 * Rc), o_rm = take(4 * Rc), o_off = take(4 * ((size_t)d.NE + 1));
+    const size_t o_g = take(4 * Rc), o_rm = take(4 * Rc);
     p->bytes = o;
     e = cudaMalloc((void **)&p->base, o);
     if (e != cudaSuccess) { delete p; return e; }
@@ -630,7 +612,7 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     p->in_hi = (__half *)(b + o_in); p->in_lo = p->in_hi + Rc * E; p->h_hi = (__half *)(b + o_h); p->h_lo = p->h_hi + Rc * FFE;
     p->tk_hi = (__half *)(b + o_tk); p->tk_lo = p->tk_hi + Mc * E;
     p->tiles_sh = (int *)(b + o_tsh); p->ntiles_sh = (int *)(b + o_nsh); p->tiles_r = (int *)(b + o_tr); p->ntiles_r = (int *)(b + o_nr);
-    p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm); p->offsets = (int *)(b + o_off);
+    p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm);
     cudaError_t m = cudaSuccess;
     auto mk = [&](CUtensorMap *t, const __half *hi, const __half *lo, size_t K, size_t rows) {
         for (int i = 0; i < 4 && m == cudaSuccess; i++)
@@ -698,16 +680,10 @@ struct Launch {
 };
 }  // namespace
 
-cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, const float *in, const int *sel_asc, const int *count,
-                        const int *pairpos, float *dn, float *eo, int *status, cudaStream_t st, int *nl) {
+cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const int *sel_asc, const int *count, const int *pairpos, float *dn, float *eo,
+                        int *status, cudaStream_t st, int *nl) {
     const int R = M * d.NU;
     if (!p || M > p->Mcap || (long long)M * d.NU > p->Rcap) return cudaErrorInvalidValue;
-    if (!sp_tc_takes_split(d)) {
-        k_tc_scan<<<1, 1024, 0, st>>>(count, d.NE, p->offsets); (*nl)++;
-        k_tc_pairs<<<(R + 255) / 256, 256, 0, st>>>(sel_asc, pairpos, p->offsets, R, d.NU, p->gather, p->rowmap); (*nl)++;
-        const cudaError_t e = sp_tc_shared_expert(p, d, L, M, nx, dn, status, st, nl, 0);
-        return e != cudaSuccess ? e : sp_tc_routed(p, d, L, R, in, p->gather, p->offsets, p->rowmap, eo, status, st, nl);
-    }
     const int nmax = tile_rows(d.NE, R);
     SortArgs s{count, sel_asc, pairpos, d.NE, M, d.NU, nmax, p->gather, p->rowmap, p->tiles_r, p->ntiles_r, p->tiles_sh, p->ntiles_sh, p->cap_r, p->cap_sh};
     cudaError_t e = sp_launch(k_tc_sort, dim3((unsigned)((R + 1023) / 1024)), 1024, 0, st, nl, s);

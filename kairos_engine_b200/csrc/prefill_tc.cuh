@@ -20,9 +20,7 @@ cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int 
                          const int *offsets, const int *rowmap, float *out, int *status, cudaStream_t st, int *nl);
 /* one whole layer's GEMMs on one GPU, the shared expert and the routed experts in one launch each for gate|up and down:
  * sel_asc / pairpos [M*NU] and count [NE] from the selection -> dn [M][E], eo [M*NU][E] (row = pair). The experts' normalised
- * inputs [M][E]: where sp_tc_takes_split, written beforehand into sp_tc_inputs' rows as fp16 hi/lo (k order 0,4,1,5,2,6,3,7
- * in each group of 8); else fp32 rows nx and in. */
-bool sp_tc_takes_split(const SpDims &d);
+ * inputs [M][E] are written beforehand into sp_tc_inputs' rows as fp16 hi/lo (k order 0,4,1,5,2,6,3,7 in each group of 8). */
 void sp_tc_inputs(SpTcPlan *p, __half **nx_hi, __half **nx_lo, __half **in_hi, __half **in_lo);
-cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, const float *in, const int *sel_asc, const int *count,
-                        const int *pairpos, float *dn, float *eo, int *status, cudaStream_t st, int *nl);
+cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const int *sel_asc, const int *count, const int *pairpos, float *dn, float *eo,
+                        int *status, cudaStream_t st, int *nl);

@@ -184,3 +184,14 @@ def test_packed_operands_start_on_any_byte(fake, off):
     copies = [(src, n) for what, dst, src, n in (x for x in fake.log if isinstance(x, tuple)) if what == "memcpy"]
     assert copies == [(base + off[0], 32 * 16), (base + 1024 + off[1], 32 * 16)]
     assert _gemm(fake, "sp_frob_matmul_q8_dev", A=base + off[0], B=base + 1024 + off[1]) == -3
+
+
+@pytest.mark.parametrize("E,M", [(64, 2), (128, 70), (448, 33), (512, 70), (4096, 2)])
+def test_prefill_takes_the_fused_preparation_at_every_width(fake, E, M):
+    """Seven launches a layer and one more, whatever the width: no geometry has a path that only its tests take."""
+    cfg = dict(E=E, NE=8, NU=2, FFE=64, FFS=128, eps=1e-6)
+    h = fake.engine(cfg, n_layers=2, max_tokens=M)
+    x = _floats(M * E, 0)
+    assert fake.L.sp_moe_forward_dev(h, 0, 2, 1, M, x.ctypes.data, x.ctypes.data, None, None, None) == 0
+    assert len(fake.launches()) == 15 and len(fake.launches("k_tc_sort")) == 2 and len(fake.launches("k_tc_permute")) == 2
+    fake.L.sp_moe_close(h)
