@@ -28,9 +28,9 @@ def test_batched_decode_flavour_small(cfg, n_layers, M):
 
 @pytest.mark.parametrize("cfg,n_layers,M", [(orc.TINY, 2, 2), (orc.SMALL, 2, 5), (orc.GEMMA, 1, 3)])
 def test_small_decode_batch_both_routes(cfg, n_layers, M, monkeypatch):
-    """A decode batch of a few tokens runs token by token through the single-token graph by default;
-    SP_MOE_SEQ_TOKENS=1 sends it to the batched kernels instead (tensor-core row dots, per-expert router
-    blocks). Both give the checker's result and each other's, bit for bit, routing tables included."""
+    """A decode batch of a few tokens runs on the batched kernels (tensor-core row dots, per-expert router blocks), which is
+    SP_MOE_SEQ_TOKENS=1, the default; SP_MOE_SEQ_TOKENS=8 sends it token by token through the single-token graph. Both give
+    the checker's result and each other's, bit for bit, routing tables included."""
     x = np.random.default_rng(50 + M).standard_normal((M, cfg["E"])).astype(np.float32)
     outs = []
     for seq in ("8", "1"):

@@ -35,6 +35,10 @@ def test_decode_batch_edges(cfg, M, monkeypatch):
     assert_close(y, ry, "decode batch")
     for _ in range(20):
         assert np.array_equal(eng.forward(x, flavour=A)[0].view(np.uint32), y.view(np.uint32))
+    for t in {0, 1, M - 1}:                 # the single-token kernels' bits
+        y1, sel1, wts1 = eng.forward(x[t:t + 1], flavour=A)
+        assert np.array_equal(sel1[:, 0], sel[:, t])
+        assert np.array_equal(y1[0].view(np.uint32), y[t].view(np.uint32)) and np.array_equal(wts1[:, 0].view(np.uint32), wts[:, t].view(np.uint32))
     eng.close()
 
 
@@ -52,12 +56,18 @@ def test_single_token_runs_direct_and_replayed(n):
     eng.close()
 
 
-PRE = _cfg(512, 8, 2, 160, 96)          # the smallest rows that take the fused staging; ragged 128-row weight tiles
+PRE = _cfg(512, 8, 2, 160, 96)          # FFE and FFS off multiples of 64: the CUDA-core kernels
+TC = _cfg(512, 8, 2, 192, 320)          # the tensor-core kernels with a last weight tile of one block, in both GEMMs
+TC_MIN = _cfg(64, 4, 2, 64, 64)         # one k-step of 64, less than one block of down rows
+TC_MANY = _cfg(576, 160, 8, 64, 192)    # more experts than the warp-wide selection takes, K off multiples of 256
 
 
-@pytest.mark.parametrize("cfg,M", [(PRE, 2), (PRE, 32), (PRE, 33), (PRE, 64), (PRE, 129), (PRE, 257), (_cfg(544, 160, 8, 96, 608), 50), (_cfg(4096, 4, 2, 64, 128), 40)])
+@pytest.mark.parametrize("cfg,M", [(PRE, 2), (PRE, 32), (PRE, 33), (PRE, 64), (PRE, 129), (PRE, 257), (_cfg(544, 160, 8, 96, 608), 50), (_cfg(4096, 4, 2, 64, 128), 40),
+                                   (TC, 2), (TC, 15), (TC, 32), (TC, 33), (TC, 64), (TC, 65), (TC, 129), (TC, 257), (TC_MIN, 2), (TC_MIN, 17), (TC_MIN, 33), (TC_MIN, 130),
+                                   (TC_MANY, 3), (TC_MANY, 50), (TC_MANY, 170), (TC_MANY, 400)])
 def test_prefill_tile_edges(cfg, M):
-    """Rows per expert on both sides of the eight at which the GEMMs go from 32 to 64 rows a tile."""
+    """Rows per expert on both sides of the eight at which the GEMMs go from 32 to 64 rows a tile, and of tiles of 16, 32 and
+    64 rows."""
     eng, host = make_stack(cfg, 1, seed=73, rand_norms=True, max_tokens=M)
     x = np.random.default_rng(M).standard_normal((M, cfg["E"])).astype(np.float32)
     y, sel, wts = eng.forward(x, flavour=B)
