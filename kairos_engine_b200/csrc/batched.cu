@@ -266,12 +266,17 @@ __global__ void __launch_bounds__(WIDE ? 512 : 384, FEW ? 1 : WIDE ? 2 : 3) k_b_
     }
 }
 /* End of a layer + beginning of the next: as two kernels of 256 threads that walked the row in shared memory 229 us for 4096
- * tokens, as this one 111 us (625 MB of it pair rows and rows in and out). */
-constexpr int kFewTokens = 148;
+ * tokens, as this one 111 us (625 MB of it pair rows and rows in and out). FEW while no SM has a second block: a layer of 65 /
+ * 100 tokens 184 / 237 us with it and 193 / 245 without (decode arithmetic, E 2816; prefill 224 / 226 and 229 / 231), the
+ * same within 1% from 148 to 444. */
 template <bool FIN, int OUT>
 cudaError_t launch_token(const SpDims &d, int M, const TokArgs &a, cudaStream_t st, int *nl) {
     const unsigned threads = (unsigned)((d.E / 8 + 31) & ~31);
-    const bool wide = d.E > 3072, few = M <= kFewTokens;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const bool wide = d.E > 3072, few = M <= sms;
     if (((uintptr_t)a.x | (uintptr_t)a.eo | (uintptr_t)a.y) & 15) {
         /* only the end of a layer meets a caller's pointers as they are (sp_moe_forward_dev, sp_moe_ep_finish_dev); an x that a
          * layer begins with is copied to the handle's own buffer first */

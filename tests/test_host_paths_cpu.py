@@ -195,3 +195,16 @@ def test_prefill_takes_the_fused_preparation_at_every_width(fake, E, M):
     assert fake.L.sp_moe_forward_dev(h, 0, 2, 1, M, x.ctypes.data, x.ctypes.data, None, None, None) == 0
     assert len(fake.launches()) == 15 and len(fake.launches("k_tc_sort")) == 2 and len(fake.launches("k_tc_permute")) == 2
     fake.L.sp_moe_close(h)
+
+
+@pytest.mark.parametrize("sms,M", [(148, 148), (148, 149), (100, 100), (100, 101), (160, 160)])
+def test_one_block_per_sm_form_follows_the_device(fake, sms, M):
+    """The token kernel's form for at most one block per SM: the device says how many SMs there are."""
+    cfg = orc.SMALL
+    fake.L.fake_set_sms(sms)
+    h = fake.engine(cfg, max_tokens=M)
+    x = _floats(M * cfg["E"], 0)
+    assert fake.L.sp_moe_forward_dev(h, 0, 1, 0, M, x.ctypes.data, x.ctypes.data, None, None, None) == 0
+    few = [re.search(r"k_b_tokenILb[01]ELi\dELb[01]ELb([01])E", k.name).group(1) for k in fake.launches("k_b_token")]
+    assert few == ["1" if M <= sms else "0"] * 2
+    fake.L.sp_moe_close(h)
