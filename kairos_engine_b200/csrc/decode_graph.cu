@@ -25,6 +25,7 @@
  */
 #include "common.cuh"
 #include "decode.cuh"
+#include "launch.cuh"
 
 
 namespace {
@@ -43,9 +44,6 @@ struct GArgs {
     SpLayerDev Ln;            /* the next layer (K3 asks L2 for its routing-independent rows) */
     int has_next;
 };
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 /* sum over the CTA in double: shuffle tree per warp, warp totals in order */
 __device__ __forceinline__ double cta_sum(double v, double *sh) {
@@ -172,7 +170,7 @@ __global__ void __launch_bounds__(kT, 1) k_dg_router_shared(GArgs a) {
                 l2_prefetch(L.sg_bs + c * (E / 32), E / 16, lane); l2_prefetch(L.su_bs + c * (E / 32), E / 16, lane); }
         }
     }
-    pdl_wait();
+    sp_pdl_wait();
     float x[KE];
     if (a.first) {
 #pragma unroll
@@ -232,7 +230,7 @@ __global__ void __launch_bounds__(kT, 1) k_dg_router_shared(GArgs a) {
         for (int i = t; i < E / 16; i += kT) { reinterpret_cast<int4 *>(a.s.in_q)[i] = reinterpret_cast<const int4 *>(q_in)[i]; a.s.in_s[i] = s_in[i]; a.s.in_c[i] = c_in[i]; }
     }
     __syncthreads();
-    pdl_launch();
+    sp_pdl_next();
     {   /* the next kernel's routing-independent rows (shared-expert down): ask L2 for them now */
         const int j0 = (int)((long long)b * E / G), nj = (int)((long long)(b + 1) * E / G) - j0;
         if (warp == kW - 1) { l2_prefetch(L.sd_codes + (size_t)j0 * (d.FFS / 2), nj * (d.FFS / 2), lane); l2_prefetch(L.sd_bs + (size_t)j0 * (d.FFS / 32), nj * (d.FFS / 16), lane); }
@@ -334,7 +332,7 @@ __global__ void __launch_bounds__(kT, 1) k_dg_experts_up(GArgs a) {
     const SpLayerDev &L = a.L;
     float *dsc = p + NE;                                  /* [NE] per-expert down scales */
     for (int i = t; i < NE; i += kT) dsc[i] = __ldg(L.dexps_scale + i);      /* weights: before the wait */
-    pdl_wait();
+    sp_pdl_wait();
     /* the activations this CTA needs, requested in one batch before the top-k chain */
     for (int i = t; i < E / 16; i += kT) { reinterpret_cast<int4 *>(q_in)[i] = __ldcg(reinterpret_cast<const int4 *>(a.s.in_q) + i); s_in[i] = __ldcg(a.s.in_s + i); c_in[i] = __ldcg(a.s.in_c + i); }
     {
@@ -360,7 +358,7 @@ __global__ void __launch_bounds__(kT, 1) k_dg_experts_up(GArgs a) {
         if (a.wts_out) a.wts_out[t] = p_desc[t];
     }
     __syncthreads();
-    pdl_launch();
+    sp_pdl_next();
     {   /* the routed down rows the next kernel will read in this CTA's slice: known now, ask L2 for them */
         const int j0p = (int)((long long)b * E / G), njp = (int)((long long)(b + 1) * E / G) - j0p;
         for (int sl = warp; sl < NU; sl += kW) {
@@ -429,11 +427,11 @@ __global__ void __launch_bounds__(kT, 1) k_dg_experts_down(GArgs a) {
     float *out = reinterpret_cast<float *>(c_h + nblk);                   /* [NU][rows_max] */
     int *sel_asc = reinterpret_cast<int *>(out + (size_t)NU * rows_max); float *cw = reinterpret_cast<float *>(sel_asc + SP_MAX_NU);
     const SpLayerDev &L = a.L;
-    pdl_wait();
+    sp_pdl_wait();
     quant_blocks(NU * FFE, q_h, s_h, c_h, [&](int i) { return __ldcg(a.s.h + i); });
     if (t < NU) { sel_asc[t] = __ldcg(a.s.sel_asc + t); cw[t] = __ldcg(a.s.cw + t); }
     __syncthreads();
-    pdl_launch();
+    sp_pdl_next();
     if (a.has_next) {   /* the next layer's router rows and shared gate/up pairs of this CTA's slice */
         const SpLayerDev &N = a.Ln;
         const int r0 = (int)((long long)b * d.NE / G), nr = (int)((long long)(b + 1) * d.NE / G) - r0;
@@ -508,8 +506,8 @@ __global__ void __launch_bounds__(kT, 1) k_dg_finish(GArgs a, float *y) {
 #pragma unroll
     for (int k = 0; k < KE; k++) { const int i = t + kT * k; const bool in = i < E;
         w1[k] = in ? __ldg(a.s.prev_post_ffw1 + i) : 0.0f; w2[k] = in ? __ldg(a.s.prev_post_ffw2 + i) : 0.0f; w3[k] = in ? __ldg(a.s.prev_post_ffw + i) : 0.0f; }
-    pdl_wait();
-    pdl_launch();
+    sp_pdl_wait();
+    sp_pdl_next();
 #pragma unroll
     for (int k = 0; k < KE; k++) { const int i = t + kT * k; const bool in = i < E; dn[k] = in ? __ldcg(a.s.dn + i) : 0.0f; ac[k] = in ? __ldcg(a.s.acc + i) : 0.0f; x[k] = in ? __ldcg(a.x_prev + i) : 0.0f; }
     double p1 = 0.0, p2 = 0.0;

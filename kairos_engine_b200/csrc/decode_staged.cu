@@ -24,9 +24,12 @@
  */
 #include "common.cuh"
 #include "decode.cuh"
+#include "launch.cuh"
+#include "tc_common.cuh"
 #include <cstring>
 
 namespace {
+using namespace sp_tc;
 
 #ifndef SP_DS_THREADS
 #define SP_DS_THREADS 640
@@ -34,8 +37,6 @@ namespace {
 constexpr int kT = SP_DS_THREADS;       /* threads per CTA (a multiple of 128, at least 256) */
 constexpr int kW = kT / 32;
 constexpr int kRW = 4;                  /* K2: warps that run the softmax / top-NU while the others do the shared-expert rows */
-constexpr unsigned kSpin = 1u << 15;    /* suspended polls before a wait on a copy gives up (each may sleep kWaitNs) */
-constexpr unsigned kWaitNs = 20000;     /* upper bound the hardware may keep a polling thread suspended, per poll */
 #ifndef SP_DS_AHEAD
 #define SP_DS_AHEAD 3
 #endif
@@ -64,33 +65,11 @@ struct SArgs {
 #define STAMP(k, i) do { if (a.stamps && blockIdx.x == 0 && threadIdx.x == 0) { long long t_; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_)); a.stamps[(k) * 16 + (i)] = t_; } } while (0)
 
 /* ---------------------------------------------------------------- PTX helpers */
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, unsigned bytes) {
-    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
-}
-/* one poll: plain first (14 cycles when the phase is complete, 99 with a suspend-time hint), then with the thread suspended
- * until the phase completes or kWaitNs pass, so that a waiting warp does not take issue slots from the warps that still work */
-__device__ __forceinline__ unsigned mbar_try(uint32_t bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok;
-}
-__device__ __forceinline__ unsigned mbar_try_suspend(uint32_t bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitNs) : "memory");
-    return ok;
-}
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 /* Waits for the copies counted on `bar` (each barrier is used once per launch: parity 0). Bounded:
  * when the limit runs out the error word is set, every later wait of this CTA falls through, and
@@ -98,7 +77,7 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void bar_wait(uint32_t bar, volatile int *abort_flag, int *status) {
     if (mbar_try(bar, 0)) return;
 #pragma unroll 1
-    for (unsigned i = 0; i < kSpin; i++) {
+    for (unsigned i = 0; i < kSpinLimit; i++) {
         if (mbar_try_suspend(bar, 0)) return;
         if (*abort_flag) return;
     }
@@ -356,8 +335,8 @@ __global__ void __launch_bounds__(kT, 1) k_ds_router_shared(SArgs a) {
         }
     }
     __syncthreads();                                     /* barriers initialised before any warp can wait on one */
-    pdl_launch();
-    pdl_wait();
+    sp_pdl_next();
+    sp_pdl_wait();
     STAMP(0, 1);
     float x[KE];
     if (a.first) {
@@ -559,8 +538,8 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
      * be launched only once every CTA has signalled, so CTA 0 - the one that publishes the selection - signals
      * after the write and a fence (one lane, right there: a CTA's first signal is the one that counts); the
      * others signal here. */
-    if (b != 0) pdl_launch();
-    pdl_wait();
+    if (b != 0) sp_pdl_next();
+    sp_pdl_wait();
     STAMP(1, 1);
     if (warp < kRW) {
         /* ---- moe_topk_host (CF:6220-6240): double softmax, order by (p descending, id ascending), clamp, renormalise */
@@ -659,7 +638,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
                 __threadfence();
             }
             __syncwarp();
-            if (lane == 0) pdl_launch();
+            if (lane == 0) sp_pdl_next();
         }
     } else {
         /* ---- the routed experts' input (for the pairs below), the shared expert's hidden vector, its down rows */
@@ -903,7 +882,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
         fence_barrier_init();
     }
     __syncthreads();
-    pdl_launch();
+    sp_pdl_next();
     if (warp == 0) {                                      /* the selection was published and fenced before this kernel could be launched: start this
                                                              CTA's rows of every selected expert now, before waiting for the predecessor's hidden vectors */
         const int e = lane < NU ? __ldcg(a.s.sel_asc + lane) : 0;
@@ -929,7 +908,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
         }
     }
     STAMP(2, 5);
-    pdl_wait();
+    sp_pdl_wait();
     STAMP(2, 1);
     float hv[16];
     if (t < nblk) {

@@ -41,7 +41,6 @@
  * 2.40 ms with the weights in shared memory and 128 rows a tile, 0.21 / 0.46 / 1.95 ms with this.
  */
 #include <map>
-#include <mutex>
 #include "prefill_tc.cuh"
 #include "tc_common.cuh"
 #include "launch.cuh"

@@ -30,11 +30,11 @@
 #include <cstring>
 
 namespace {
+using namespace sp_tc;
 
 constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kUnitTok = 16, kMaxStages = 4, kMaxTeams = 2;
 constexpr int kUnits = 128;                        /* unit descriptors of a CTA kept in shared memory */
 constexpr int kMagic = 0x4B400000;
-constexpr unsigned kSpin = 1u << 15, kWaitNs = 20000;
 
 struct SegGeo {                                    /* what the copies and the dots need of a segment's shape */
     int tiles, mt_n, n32;                          /* weight tiles per group, 16-row MMA tiles of one, chunks of a row */
@@ -63,36 +63,12 @@ SegGeo seg_geo(const SpRowsSeg &s, bool pair) {
     return g;
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned mbar_try(uint32_t bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity, volatile int *abort_flag) {
-    if (mbar_try(bar, parity)) return true;
-#pragma unroll 1
-    for (unsigned i = 0; i < kSpin; i++) {
-        unsigned ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitNs) : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 /* a box of codes: all 128-byte slices of some consecutive rows, slice-major, 128-byte swizzle */
 __device__ __forceinline__ void box_g2s(uint32_t dst, const CUtensorMap *map, int row, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%4, %2, %4}], [%3];" ::"r"(dst), "l"(map), "r"(row), "r"(bar), "r"(0) : "memory");
-}
-__device__ __forceinline__ void expect_tx(uint32_t bar, unsigned bytes) {
-    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void arrive_lane0(uint32_t bar, int lane) {     /* predicated, not branched around */
-    asm volatile("{ .reg .pred p; .reg .b64 st; setp.eq.s32 p, %1, 0; @p mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar), "r"(lane) : "memory");
 }
 __device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads) : "memory"); }
 
@@ -246,13 +222,12 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     auto aempty = [&](int team, int b) { return bar0 + 8u * (kActBars + 4 * team + 2 + b); };
     if (tid == 0) {
         for (int s = 0; s < a.stages; s++) {
-            for (int t = 0; t < a.teams; t++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(t, s)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty(s)), "n"(kTeamWarps) : "memory");
+            for (int t = 0; t < a.teams; t++) mbar_init(full(t, s), 1);
+            mbar_init(empty(s), kTeamWarps);
         }
         for (int t = 0; t < a.teams; t++)
             for (int b = 0; b < 2; b++) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(afull(t, b)) : "memory");
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(aempty(t, b)), "n"(kTeamWarps) : "memory");
+                mbar_init(afull(t, b), 1); mbar_init(aempty(t, b), kTeamWarps);
             }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -309,7 +284,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const unsigned sbytes = (unsigned)nr * ge.sb;
                 const unsigned char *const ssrc = reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb;
                 if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-                expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
+                mbar_expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
                 box_g2s(dst, &a.codes[u.seg][0], row, bar);
                 if (PAIR) {
                     box_g2s(dst + ge.box_bytes, &a.codes[u.seg][1], row + sg.up_off, bar);
@@ -343,7 +318,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 if (lane < kTok) d->item[lane] = item;
                 if (lane == 0) { d->seg = u.seg; d->tile = u.tile; d->flags = (b == 0 ? 1 : 0) | (b + kTok >= u.nt ? 2 : 0) | (have > 2 ? 8 : 0); }
                 __syncwarp();
-                if (lane == 0) expect_tx(afull(team, buf), (unsigned)have * (unsigned)sp_act_pitch(s.in));        /* its arrival also publishes the descriptor */
+                if (lane == 0) mbar_expect_tx(afull(team, buf), (unsigned)have * (unsigned)sp_act_pitch(s.in));        /* its arrival also publishes the descriptor */
                 __syncwarp();
                 if (item >= 0)
                     bulk_g2s(abase + buf * a.act_bytes + lane * ge.ast, s.act + (size_t)arow * sp_act_pitch(s.in), (unsigned)sp_act_pitch(s.in), afull(team, buf));
@@ -354,7 +329,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             if (!mbar_wait(aempty(team, buf), ((n >> 1) & 1) ^ 1, abort_flag)) failed = true;
             else if (lane == 0) {
                 batch_s[team][buf].flags = 4;
-                asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(afull(team, buf)) : "memory");
+                mbar_arrive(afull(team, buf));
             }
         }
     } else {
@@ -396,7 +371,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
             auto release = [&] {                            /* the stage, once the warp has read it for the last time */
                 if (flags & 2) {
                     __syncwarp();
-                    arrive_lane0(empty(s), lane);
+                    mbar_arrive_lane0(empty(s), lane);
                     phs ^= 1u << s;
                     s += a.teams;
                     while (s >= a.stages) s -= a.stages;
@@ -465,7 +440,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 }
             }
             __syncwarp();
-            arrive_lane0(aempty(team, buf), lane);
+            mbar_arrive_lane0(aempty(team, buf), lane);
         }
     }
     if (failed) {
@@ -477,8 +452,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
 /* the codes of a tensor as [128-byte slice][row][128 bytes]: the last slice of a row may reach into the next row (or into the
  * scales that follow the tensor in the arena); such chunks are not multiplied */
 cudaError_t codes_map(const uint8_t *codes, const SpRowsSeg &s, const SegGeo &g, bool pair, CUtensorMap *m) {
-    sp_tc::EncodeTiledFn fn = nullptr;
-    const cudaError_t e = sp_tc::encode_tiled_fn(&fn);
+    EncodeTiledFn fn = nullptr;
+    const cudaError_t e = encode_tiled_fn(&fn);
     if (e != cudaSuccess) return e;
     const size_t rows = s.rows_per_group ? (size_t)s.groups * (size_t)s.rows_per_group : (size_t)s.rows;
     const cuuint64_t rb = (cuuint64_t)s.in / 2, slices = (rb + 127) / 128;
