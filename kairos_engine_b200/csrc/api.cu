@@ -148,7 +148,7 @@ extern "C" int sp_moe_open(const sp_moe_config *cfg, sp_moe **out) {
         const char *fv = getenv("SP_MOE_STAGED_FLAGS");
         h->staged_flags = fv ? (unsigned)strtoul(fv, nullptr, 0) : (unsigned)SP_STAGED_DEFAULT;
         /* tuning switch: decode batches of up to this many tokens go token by token through the single-token graph. The batched
-         * kernels are ahead from two tokens on (per layer, 30 layers: 42.5 against 46.7 us at two, 62 against 116 at five). */
+         * kernels are ahead from two tokens on (per layer: 39.6 against 45.6 us at two, 54 against 115 at five). */
         const char *sq = getenv("SP_MOE_SEQ_TOKENS");
         h->seq_tokens = sq ? atoi(sq) : 1;
         if (h->seq_tokens < 1) h->seq_tokens = 1;
@@ -261,6 +261,11 @@ static cudaError_t align_x(sp_moe *h, const float **x, int M, cudaStream_t st) {
     *x = h->x_dev;
     return e;
 }
+/* Short runs of one token are launched one kernel after the other, longer ones replayed from a graph. On the device the launches
+ * are ahead up to about twelve layers (us a layer, launched / replayed: 24.0 / 33.7 at one layer a call, 23.3 / 28.0 at two,
+ * 23.0 / 24.8 at four, 22.8 / 23.4 at eight, 22.75 / 22.90 at twelve, 22.65 / 22.32 at thirty), but they cost the calling thread 7 us
+ * a layer where a replay costs it 17 us a call. At four layers the device still gains 7 us for 14 of the thread's; beyond, the
+ * gain of a call shrinks while the thread's share grows. */
 constexpr int kDirectLayers = 4;
 extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
                                   const float *x_dev, float *y_dev, int32_t *sel_dev, float *wts_dev, void *stream) {
@@ -272,8 +277,8 @@ extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
     if (M <= h->seq_tokens && flavour == SP_MOE_FLAVOUR_DECODE) {
         /* One token (or, by the switch, a few of them one after the other) replays the single-token graph. */
         if (M == 1 && nl <= kDirectLayers) {
-            /* a short run (an engine with attention between the layers calls once per layer): launched as it is, on the
-             * caller's stream and pointers. A graph would add two copies and its own start to three kernels per layer. */
+            /* an engine with attention between the layers calls once per layer: on the caller's stream and pointers. A graph
+             * would add two copies and its own start to three kernels per layer. */
             int nlaunch = 0;
             const cudaError_t e = h->decode_impl == 0
                 ? sp_staged_decode_enqueue(h->d, h->layers_host.data(), lf, nl, x_dev, y_dev, sel_dev, wts_dev, h->gs, h->sms, h->staged_flags, h->stamps, st, true, &nlaunch)

@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
         }
         STAMP(1, 7);
         if (warp == 0) {
-            /* the sum and the ascending place by shuffles, unrolled: the routed copies wait for this (23.2 -> 23.0 us a layer) */
+            /* the sum and the ascending place by shuffles, unrolled: the routed copies wait for this (22.50 -> 22.33 us a layer, 30 layers) */
             static_assert(SP_MAX_NU <= 32, "one lane per selected expert");
             const int e = lane < NU ? ctl->sel_desc[lane] : 0; const float pe = lane < NU ? ctl->p_desc[lane] : 0.0f;
             float ws = 0.0f; int slot = 0;

@@ -11,8 +11,9 @@
  * three launches and one synchronisation: x is read from page-locked memory and quantised; gate and up
  * rows of all chosen experts with silu*mul; down rows of all of them with the accumulation, written
  * to page-locked memory. What bounds a call (14 MB of weights at E 2048, FF 512, eight experts: 2 us of
- * HBM) is the latency of these steps; eight calls in a row measured 1784 us with six launches per
- * expert and pageable copies. Only Q4B tensors are served here.
+ * HBM) is the latency of these steps: 8 us to enqueue, then 18.5 us of waiting (the kernels take 4, 7 and 12 us one by one, cold),
+ * of 33 us with a ctypes caller. Eight calls in a row: 263 us, 1784 us with six launches per expert and
+ * pageable copies. Only Q4B tensors are served here.
  */
 #include "common.cuh"
 #include "launch.cuh"

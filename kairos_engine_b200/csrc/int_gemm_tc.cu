@@ -8,10 +8,13 @@
  * tensor memory, the same epilogue arithmetic and operation order, so results are bit-identical to
  * the reference's.
  * A is [M][K], B is [N][K] (the tiled kernels' layout); K a multiple of 16.
- * Tile: MH x 128 rows of A x NT rows of B, k in stages of 128. What bounds it is shared memory: an MMA of 128 x NT x 32
- * reads 4 + NT/32 KB, and the copies write each stage once, so a tile of 256 x 256 (two MMAs share a B tile; its accumulators
- * fill tensor memory, so there is one set) keeps the tensor cores 80% busy where 128 x 256 keeps them 66%. 3072 x 8192 x
- * 3072: 69.8 us with 128 x 256. Small problems take smaller tiles, to have one for every SM (pick_tile).
+ * Tile: MH x 128 rows of A x NT rows of B, k in stages of 128. What bounds it is moving operands: an MMA of 128 x NT x 32
+ * reads 4 + NT/32 KB of shared memory, and each stage comes from L2 once. A tile of 256 x 256 (two MMAs share a B tile; its
+ * accumulators fill tensor memory, so there is one set) takes 0.37 GB from L2 for 3072 x 8192 x 3072 and 4.1 GB for 8192^3
+ * where 128 x 256 takes 0.66 and 6.6. Calls in a row, 256 x 256 / 128 x 256: 55.8 / 57.7 us, 442 / 501 us (at the power limit, where
+ * the traffic saved becomes clock), 34 / 37 us at 2048 x 8192 x 2048, but about 66 / 62 us at 4096^3, where the second set of
+ * accumulators hides the emptying. The tensor pipe is active 69 to 75% of the cycles an SM is active with 256 x 256, 72
+ * to 80% with 128 x 256. Small problems take smaller tiles, to have one for every SM (pick_tile).
  * Packed int4 operands are unpacked on the way: sixteen warps read the packed rows and write the int8 tiles (the even
  * elements of every 8, then the odd ones, in both operands: an integer dot product does not see the order).
  * Warp roles: 0-7 epilogue (TMEM lane quadrant = warp % 4), 8 TMA, 9 MMA issue + TMEM allocation, 10-25 int4 unpack. Every

@@ -36,9 +36,10 @@
  * code TMA and TMEM allocation. Every wait is bounded.
  * What bounds it (Gemma geometry, one B200): up to some 40 rows per expert the unpack, ~136
  * instructions of the half-rate fp16 and integer pipes per 2048 weights, beside a weight stream at
- * about a third of HBM's rate; from there to the largest batches the MMAs (12, 16 and 32 cycles at N =
- * 16, 32 and 64) and in the end the power limit. A layer of 37 / 717 / 4096 tokens: 0.60 / 0.85 /
- * 2.40 ms with the weights in shared memory and 128 rows a tile, 0.21 / 0.46 / 1.95 ms with this.
+ * about a third of HBM's rate; from there to the largest batches the unpack and the MMAs (12, 16
+ * and 32 cycles at N = 16, 32 and 64) together, each about 70% of an SM's active time at 4096 tokens, and in the end
+ * the power limit. A layer of 37 / 717 / 4096 tokens: 0.60 / 0.85 / 2.40 ms with the weights in shared memory and 128 rows
+ * a tile, 0.19 / 0.43 / 1.85 ms with this.
  */
 #include <map>
 #include "prefill_tc.cuh"
@@ -633,7 +634,10 @@ void sp_tc_destroy(SpTcPlan *p) { if (!p) return; if (p->base) cudaFree(p->base)
 
 namespace {
 /* activation rows per tile: tiles of 32 have a second set of accumulators, tiles of 64 serve more rows per unpacked weight.
- * Measured per layer, 32 against 64: 205 / 213 us at 24 tokens, 282 / 294 at 128 (8 rows per expert), 324 / 311 at 256. */
+ * Us a layer with 32 / 64, E 2816, 128 experts, 8 each, FFE 704: 178 / 183 at 24 tokens, 240 / 246 at 128 (8 rows per expert),
+ * 247 / 252 at 160, 261 / 264 at 200, 297 / 289 at 256, 357 / 338 at 400. With 64 experts, 6 each, E 2048, FFE 1408: 169 / 166 at 64
+ * (6 rows), 182 / 192 at 96, 217 / 221 at 200 (19 rows); with 32, 4 each, E 1024, FFE 512: 46.7 / 58.1 at 64 (8 rows), 71 / 78 at
+ * 200 (25 rows). The line could lie higher: between 8 rows and the crossing 64 costs up to 2% in the first, 5 to 10% in the others. */
 int tile_rows(int groups, long long rows) { return rows > 8LL * groups ? 64 : 32; }
 
 template <bool PAIR, int NMAX>

@@ -20,8 +20,10 @@
  * of its next four tokens copied while it multiplies the current four. So the weight stream does not stop between units,
  * and experts nobody chose cost nothing. A unit's codes are one or two tensor copies (a box of all 128-byte slices of 16 to
  * 128 rows, swizzled, so that the eight rows an MMA operand takes lie on different banks): a copy costs its warp ~85 cycles
- * whatever its size, and a copy per row (for padded rows) took longer than the multiplication. What bounds it now is the
- * multiplying warps: ~30 instructions and 7 shared-memory wavefronts a chunk. One team of sixteen warps on a unit was slower
+ * whatever its size, and a copy per row (for padded rows) took longer than the multiplication. At 64
+ * tokens the multiplying warps bound it: ~30 instructions a chunk, row tile and four tokens, issued in 65% of the active
+ * cycles, with 12% (gate|up) and 18% (down) of the time lost to the start and the last units; at 16 tokens half the
+ * slots are used and the waits between stages count as much. One team of sixteen warps on a unit was slower
  * (199 us a layer at 64 tokens against 176): the latencies of a batch are then paid one after the other.
  */
 #include "rows_mma.cuh"
@@ -479,8 +481,12 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
     RowsArgs a{};
     cudaError_t e = cudaSuccess;
     a.nseg = nseg; a.status = status;
-    /* two chunks x two tokens per MMA while most chosen experts have one or two tokens (55 instead of 58 us a layer at five
-     * tokens of eight of 128 experts, even at 16, 204 instead of 176 at 64) and the rows are whole groups */
+    /* two chunks x two tokens per MMA while most chosen experts have one or two tokens and the rows are whole groups. Us a layer
+     * with one / two chunks, the line at one item per expert: E 2816, 128 experts, 8 each, FFE 704, line at 16 tokens: 57.5 / 54.0
+     * at 5, 91.3 / 91.2 at 16, 100.6 / 105.3 at 20, 175 / 202 at 64. E 2048, 64 experts, 6 each, FFE 1408, line at 10: 71 / 61 at
+     * 6, 95 / 81 at 10, 100 / 89 at 12, 113 / 106 at 16, 135 / 137 at 24. E 1024, 32 experts, 4 each, FFE 512, line at 8: 22.4 /
+     * 20.6 at 2, 23.3 / 23.9 at 4, 30.4 / 32.2 at 8, 34.4 / 35.8 at 10. The line is right for the first; the longer down rows of
+     * the second would move it to twice as many tokens, the short ones of the third to half. */
     bool whole = items <= seg[nseg - 1].groups;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
