@@ -33,6 +33,7 @@ static int fail(int code, const char *fmt, ...) {
 }
 static int fail_cuda(cudaError_t e, const char *where) {       /* CF:189-195 */
     const int code = (e == cudaErrorMemoryAllocation) ? SP_MOE_EBACKEND_OOM : SP_MOE_ECUDA;
+    cudaGetLastError();                                       /* reported here: not again by a later call's check */
     return fail(code, "CUDA: %s: %s (%d)", where, cudaGetErrorString(e), (int)e);
 }
 #define CK(call, where) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail_cuda(e_, where); } while (0)

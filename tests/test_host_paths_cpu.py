@@ -208,3 +208,25 @@ def test_one_block_per_sm_form_follows_the_device(fake, sms, M):
     few = [re.search(r"k_b_tokenILb[01]ELi\dELb[01]ELb([01])E", k.name).group(1) for k in fake.launches("k_b_token")]
     assert few == ["1" if M <= sms else "0"] * 2
     fake.L.sp_moe_close(h)
+
+
+@pytest.mark.parametrize("M,n_layers", [(1, 1), (1, 5), (8, 1), (70, 2)])
+@pytest.mark.parametrize("failing", [0, 2])
+def test_failed_launch_is_reported_once(fake, M, n_layers, failing):
+    """The call whose launch fails says so; the runtime's record of it does not reach a later call that is fine."""
+    cfg = orc.SMALL
+    h = fake.engine(cfg, n_layers=n_layers, max_tokens=M)
+    x = _floats(M * cfg["E"], 0)
+    forward = lambda: fake.L.sp_moe_forward_dev(h, 0, n_layers, 0, M, x.ctypes.data, x.ctypes.data, None, None, None)
+    count = [0]
+
+    def fail_one(_):
+        count[0] += 1
+        return 700 if count[0] == failing + 1 else 0
+    fake.on_launch = fail_one
+    assert forward() == -40
+    fake.on_launch = None
+    ints = np.zeros(4 * cfg["NE"] + M * cfg["NU"], np.int32).ctypes.data
+    assert fake.L.sp_moe_ep_recv_layout_dev(h, ints, 1, 0, M * cfg["NU"], ints, ints, None) == 0
+    assert forward() == 0
+    fake.L.sp_moe_close(h)
