@@ -380,7 +380,7 @@ extern "C" int sp_frob_matmul_q4_dev(const uint8_t *A_q4_dev, const uint8_t *B_q
         std::lock_guard<std::mutex> lk(g_mu);
         d->taken &= ~(1ull << w);
     }
-    g_word_free.notify_one();
+    g_word_free.notify_all();                             /* the waiters may be of several devices */
     if (moved) cudaFree(moved);
     return rc;
 }
