@@ -10,14 +10,13 @@ HOOK = C.CFUNCTYPE(C.c_int, C.c_char_p, C.c_char_p, C.c_void_p, C.c_void_p, C.c_
 
 
 def load(directory):
-    """Links the library's objects with the fake runtime and loads the result with the ABI's argument types."""
+    """Links the library's archive with the fake runtime and loads the result with the ABI's argument types."""
     from kairos_engine_b200 import _lib, build
     build.build()
     so = os.path.join(str(directory), "libsp_moe_fake.so")
-    objs = [build._obj(s) for s in build.sources()]
     rt = os.path.join(str(directory), "fake_cudart.o")
     subprocess.run(["gcc", "-O1", "-fPIC", "-std=gnu11", "-I/usr/local/cuda/include", "-c", os.path.join(HERE, "fake_cudart.c"), "-o", rt], check=True)
-    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", so, *objs, rt, "-ldl", "-lpthread"], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", so, "-Wl,--whole-archive", build.ARCHIVE, "-Wl,--no-whole-archive", rt, "-ldl", "-lpthread"], check=True)
     spec = importlib.util.spec_from_file_location("fake_abi", _lib.__file__)      # a second copy of the loader, with its own path
     abi = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(abi)

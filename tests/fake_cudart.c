@@ -1,5 +1,5 @@
 /* fake_cudart.c — the CUDA runtime calls the library makes, over host memory: device buffers are heap blocks, copies are
- * memcpy, a kernel launch runs nothing. Linked with the library's own objects (fake_cuda.py) it lets a test follow the host
+ * memcpy, a kernel launch runs nothing. Linked with the library's own archive (fake_cuda.py) it lets a test follow the host
  * side without a GPU: every launch, copy and synchronisation is told to a hook, which may answer with an error code. */
 #include <cuda.h>
 #include <cuda_runtime_api.h>
