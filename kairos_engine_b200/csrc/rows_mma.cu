@@ -7,24 +7,25 @@
  *   - One mma.sync m16n8k32 (s8 x s8) takes 16 weight rows x one chunk x four tokens: column 2t + h of B is token t
  *     restricted to half h, so lane (g, q) of the warp finds both block sums of rows g and g + 8 for token q in its C
  *     registers, for every chunk. It adds its slots by itself, in the order that completes subtrees (no shuffles, at most
- *     four partial sums waiting). Half of the MMA multiplies zeros; the MMA pipe has room for that (2.6 cycles per
- *     instruction and scheduler), and the epilogue's 10 fp32 instructions serve four tokens at a time. While most experts
+ *     four partial sums waiting). Half of the MMA multiplies zeros; the MMA pipe has room for that (8 cycles per
+ *     instruction and scheduler, 16% of the time), and the epilogue's 10 fp32 instructions serve four tokens at a time. While most experts
  *     have one or two tokens, two neighbouring chunks x two tokens share an epilogue instead (W = 2 below).
  *   - A operand: code nibbles moved to the top of a byte (16 * code as s8); C starts at 0x4B400000, so that one fma turns
  *     the s32 result into the float a conversion would give.
  *   - Gate|up: a 16-row MMA tile is 8 gate rows and the 8 up rows of the same outputs. A unit is 16 outputs = one
  *     quantisation block: it leaves the kernel as int8 codes and a scale, ready for the down rows.
  *
- * Work is cut into units of ~50 KB of weights x up to 16 tokens. One CTA per SM; one warp asks the copy engine for the
+ * Work is cut into units of ~50 KB of weights x up to 4 or 16 tokens. One CTA per SM; one warp asks the copy engine for the
  * units' rows (a ring of stages), two teams of eight warps consume them alternately, and a warp per team has the activations
- * of its next four tokens copied while it multiplies the current four. So the weight stream does not stop between units,
- * and experts nobody chose cost nothing. A unit's codes are one or two tensor copies (a box of all 128-byte slices of 16 to
- * 128 rows, swizzled, so that the eight rows an MMA operand takes lie on different banks): a copy costs its warp ~85 cycles
- * whatever its size, and a copy per row (for padded rows) took longer than the multiplication. At 64
- * tokens the multiplying warps bound it: ~30 instructions a chunk, row tile and four tokens, issued in 65% of the active
- * cycles, with 12% (gate|up) and 18% (down) of the time lost to the start and the last units; at 16 tokens half the
- * slots are used and the waits between stages count as much. One team of sixteen warps on a unit was slower
- * (199 us a layer at 64 tokens against 176): the latencies of a batch are then paid one after the other.
+ * of its next four tokens copied while it multiplies the current four. So the weight stream does not stop between units, and experts
+ * nobody chose cost nothing. A unit's codes are one or two tensor copies (a box of all 128-byte slices of 16 to 128 rows, swizzled, so that the eight
+ * rows an MMA operand takes lie on different banks): a copy costs its warp ~85 cycles whatever its size, and a copy per row (for
+ * padded rows) took longer than the multiplication. The multiplying warps bound it: at 16 tokens the launches take 50 + 36 us
+ * with units of 16, 46 + 33 without their copies and 31 + 21 without their dots. A team spends some 2200 cycles on a unit's dots
+ * (16 warps issue in 75% of them), 900 until the last of its sums is finished by two of them, and 300 to 1000 waiting. One team of
+ * sixteen warps on a unit was slower (199 us a layer at 64 tokens against 176), and so were sums finished by a warp of their
+ * own (one per team 165, for 160: ~300 instructions a unit are too long a chain for one warp) and four chunks x one token per
+ * MMA group (103 at 16 tokens: as many instructions a token).
  */
 #include "rows_mma.cuh"
 #include "launch.cuh"
@@ -34,7 +35,7 @@
 namespace {
 using namespace sp_tc;
 
-constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kUnitTok = 16, kMaxStages = 4, kMaxTeams = 2;
+constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kMaxStages = 4, kMaxTeams = 2;
 constexpr int kUnits = 128;                        /* unit descriptors of a CTA kept in shared memory */
 constexpr int kMagic = 0x4B400000;
 
@@ -45,7 +46,7 @@ struct SegGeo {                                    /* what the copies and the do
 };
 struct RowsArgs {
     SpRowsSeg seg[2]; SegGeo geo[2]; int nseg;
-    int stages, teams;
+    int stages, teams, unit_log;                   /* ...; log2 of the tokens of a unit at most */
     unsigned stage_bytes, act_bytes, zero_bytes;   /* one stage; one buffer of four tokens; the zeros B's other columns read */
     int *status;
     CUtensorMap codes[2][2];                       /* [segment][gate or only / up] */
@@ -107,6 +108,7 @@ __device__ __forceinline__ int group_count(const SpRowsSeg &s, int g) {
     const int c = __ldcg(s.count + g);
     return c > s.M ? s.M : c;
 }
+__device__ __forceinline__ int units_of(int cnt, int log) { return (cnt + (1 << log) - 1) >> log; }
 __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     Unit r{};
     r.seg = u >= p.total[0] ? 1 : 0;
@@ -116,10 +118,10 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     int lo = 0, hi = s.groups - 1;                          /* the last group that starts at or before u: never an empty one */
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (st[mid] <= u) lo = mid; else hi = mid - 1; }
     r.grp = lo;
-    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), nr = (cnt + kUnitTok - 1) / kUnitTok, k = u - st[lo];
+    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), nr = units_of(cnt, a.unit_log), k = u - st[lo];
     r.tile = k / nr;
-    r.t0 = (k - r.tile * nr) * kUnitTok;
-    r.nt = cnt - r.t0 < kUnitTok ? cnt - r.t0 : kUnitTok;
+    r.t0 = (k - r.tile * nr) << a.unit_log;
+    r.nt = cnt - r.t0 < 1 << a.unit_log ? cnt - r.t0 : 1 << a.unit_log;
     return r;
 }
 
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const SpRowsSeg &s = a.seg[k];
                 for (int g0 = 0; g0 < s.groups; g0 += 32) {
                     const int g = g0 + lane;
-                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * ((cnt + kUnitTok - 1) / kUnitTok);
+                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * units_of(cnt, a.unit_log);
                     if (k == 1 && g < s.groups) count_s[g] = cnt;
                     int v = n;
 #pragma unroll
@@ -482,12 +484,19 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
     cudaError_t e = cudaSuccess;
     a.nseg = nseg; a.status = status;
     /* two chunks x two tokens per MMA while most chosen experts have one or two tokens and the rows are whole groups. Us a layer
-     * with one / two chunks, the line at one item per expert: E 2816, 128 experts, 8 each, FFE 704, line at 16 tokens: 57.5 / 54.0
-     * at 5, 91.3 / 91.2 at 16, 100.6 / 105.3 at 20, 175 / 202 at 64. E 2048, 64 experts, 6 each, FFE 1408, line at 10: 71 / 61 at
-     * 6, 95 / 81 at 10, 100 / 89 at 12, 113 / 106 at 16, 135 / 137 at 24. E 1024, 32 experts, 4 each, FFE 512, line at 8: 22.4 /
-     * 20.6 at 2, 23.3 / 23.9 at 4, 30.4 / 32.2 at 8, 34.4 / 35.8 at 10. The line is right for the first; the longer down rows of
-     * the second would move it to twice as many tokens, the short ones of the third to half. */
+     * with one / two chunks, the line at one item per expert: E 2816, 128 experts, 8 each, FFE 704, line at 16 tokens: 42.7 / 39.6
+     * at 2, 56.3 / 54.0 at 5, 77.7 / 75.7 at 12, 88.7 / 88.4 at 16, 96.7 / 97.0 at 20, 112 / 123 at 32, 162 / 197 at 64. E 2048, 64
+     * experts, 6 each, FFE 1408, line at 10: 66.3 / 56.6 at 6, 85.1 / 71.9 at 10, 89.8 / 77.8 at 12, 101 / 92.4 at 16, 115 / 114 at 24.
+     * E 1024, 32 experts, 4 each, FFE 512, line at 8: 21.5 / 20.5 at 2, 23.4 / 24.2 at 4, 28.0 / 29.0 at 8, 29.1 / 30.7 at 10. The line
+     * is right for the first; the longer down rows of the second would move it to twice as many tokens, the short ones of the
+     * third to a quarter. */
     bool whole = items <= seg[nseg - 1].groups;
+    /* Small units all cost about the same: with up to 16 tokens to a unit, one of the shared expert held its stage for a third of
+     * the launch at 16 tokens and kept the other team waiting. What small ones fetch again comes from L2, until that is what
+     * bounds them. Us a layer of E 2816, 128 experts, 8 each, units of 16 / 8 / 4 tokens: 54.4 / 54.5 / 52.8 at 5 tokens, 92.2 / 88.5 /
+     * 86.6 at 16, 120 / 119 / 113 at 32, 176 / 174 / 160 at 64; of 16 / 4: 238 / 222 at 100, 412 / 395 at 200, 550 / 501 at 256, 772 / 760 at
+     * 400 (321: 693 / 623), 901 / 967 at 512, 1677 / 1870 at 1024: the line is at 384 tokens, 24 items to an expert. */
+    a.unit_log = items <= 24LL * seg[nseg - 1].groups ? 2 : 4;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
         const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
