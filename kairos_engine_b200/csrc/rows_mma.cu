@@ -84,7 +84,13 @@ __device__ __forceinline__ void mma_s8_add(int (&d)[4], unsigned a0, unsigned a1
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ float magic_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }     /* bits of magic + 16 S -> float(S) */
+/* bits of magic + 16 S -> float(S), for two neighbouring registers at once (a layer of 64 tokens 162.6 -> 159.0 us, of 16 86.7 -> 86.1) */
+__device__ __forceinline__ float2 magic_to_float2(int a, int b) {
+    float2 r;
+    asm("{ .reg .b64 v, m, c; mov.b64 v, {%2, %3}; mov.b64 m, {%4, %4}; mov.b64 c, {%5, %5}; fma.rn.f32x2 v, v, m, c; mov.b64 {%0, %1}, v; }"
+        : "=f"(r.x), "=f"(r.y) : "r"(a), "r"(b), "f"(0.0625f), "f"(-786432.0f));
+    return r;
+}
 
 /* ---------------------------------------------------------------- units of work */
 struct Unit { int seg, grp, tile, t0, nt; };                /* weight tile `tile` of group grp x its tokens [t0, t0 + nt) */
@@ -167,8 +173,9 @@ __device__ __forceinline__ float2 class_sum(const Frag &f, int r) {
                     mma_s8(d, (u0.x << 4) & 0xF0F0F0F0u, (u1.x << 4) & 0xF0F0F0F0u, u0.x & 0xF0F0F0F0u, u1.x & 0xF0F0F0F0u, b.x, b.y, kMagic);
                     mma_s8_add(d, (u0.y << 4) & 0xF0F0F0F0u, (u1.y << 4) & 0xF0F0F0F0u, u0.y & 0xF0F0F0F0u, u1.y & 0xF0F0F0F0u, b.z, b.w);
                 }
-                acc.x = __fmaf_rn(ws0, __fmaf_rn(magic_to_float(d[0]), s2.x, __fmul_rn(magic_to_float(d[1]), s2.y)), acc.x);
-                acc.y = __fmaf_rn(ws1, __fmaf_rn(magic_to_float(d[2]), s2.x, __fmul_rn(magic_to_float(d[3]), s2.y)), acc.y);
+                const float2 g = magic_to_float2(d[0], d[1]), h = magic_to_float2(d[2], d[3]);
+                acc.x = __fmaf_rn(ws0, __fmaf_rn(g.x, s2.x, __fmul_rn(g.y, s2.y)), acc.x);
+                acc.y = __fmaf_rn(ws1, __fmaf_rn(h.x, s2.x, __fmul_rn(h.y, s2.y)), acc.y);
             }
         }
         return acc;
