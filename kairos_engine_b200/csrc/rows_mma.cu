@@ -73,7 +73,9 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned
 __device__ __forceinline__ void box_g2s(uint32_t dst, const CUtensorMap *map, int row, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%4, %2, %4}], [%3];" ::"r"(dst), "l"(map), "r"(row), "r"(bar), "r"(0) : "memory");
 }
-__device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads) : "memory"); }
+/* the sums of a team's eight warps are there: for those that finish them; the others go on */
+__device__ __forceinline__ void sums_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTeamThreads) : "memory"); }
+__device__ __forceinline__ void sums_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kTeamThreads) : "memory"); }
 
 /* D = A x B + {magic, ...}, D += A x B (pure functions of their operands: the compiler may move them) */
 __device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
@@ -426,7 +428,10 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                     p[0] = v.x; p[8 * T] = v.y;
                 }
                 release();
-                team_sync(team);
+                /* Two warps (gate|up) or one per token finish the sums, other ones each time, and only they wait for the rest, which is
+                 * at its next tokens meanwhile: a warp loses the time of one finish in four (or two) times. The other buffer of sums
+                 * and the other barrier serve those next tokens; the buffer's next use but one waits for this one's end (aempty). */
+                const int id = 1 + 2 * team + buf;
                 auto total_of = [&](int m, int rw, int t) {                 /* the last levels of the tree */
                     const float *p = part + (m * 16 + rw) * T + t;
                     const int k = 32 * T;
@@ -434,25 +439,30 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                     return ((p[0] + p[4 * k]) + (p[2 * k] + p[6 * k])) + ((p[k] + p[5 * k]) + (p[3 * k] + p[7 * k]));
                 };
                 if (PAIR) {
-                    const int w0 = 2 * (n & 3);             /* two warps finish, other ones each time */
+                    const int w0 = 2 * (n & 3);
                     if (tw == w0 || (tw == w0 + 1 && T == 4)) {
+                        sums_wait(id);
                         const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
                         const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
                         const int it = bt.item[t] < 0 ? 0 : bt.item[t];
                         unsigned char *o = sg.out_act + (size_t)it * sp_act_pitch(sg.rows);
                         quant_elem16(h, bt.item[t] >= 0, reinterpret_cast<signed char *>(o) + tile * 16, reinterpret_cast<float *>(o + sg.rows) + tile);
-                    }
+                    } else sums_arrive(id);
                 } else {
                     const int t = tw - 4 * (n & 1);
                     if (t >= 0 && t < T) {
+                        sums_wait(id);
                         const int it = bt.item[t];
                         if (it >= 0 && r0 + lane < sg.rows) sg.out_f[(size_t)it * sg.out_stride + r0 + lane] = total_of(lane >> 4, lane & 15, t);
-                    }
+                    } else sums_arrive(id);
                 }
             }
             __syncwarp();
             mbar_arrive_lane0(aempty(team, buf), lane);
         }
+        /* a warp that gave up: the others may be waiting for its sums of these tokens or of the next, never of later ones (aempty) */
+        __syncwarp();
+        if (__any_sync(0xffffffffu, failed)) { sums_arrive(1 + 2 * team); sums_arrive(2 + 2 * team); }
     }
     if (failed) {
         if (lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
