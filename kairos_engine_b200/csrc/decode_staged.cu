@@ -113,6 +113,7 @@ struct Ctl {
     unsigned gs_off[2], us_off[2];          /* K2: where the two runs' gate / up scale rows start */
     unsigned sdelta[SP_MAX_NU];             /* K3: bytes before the first scale row of each slot's span */
     alignas(16) int zero[4];                /* K3: the activation operand of an MMA column that is not the lane's */
+    int2 cand[4 * SP_MAX_NU];               /* K2: the best of each router warp's candidates */
 };
 
 struct Lay1 { unsigned ctl, red, va, vb, ri, q_nx, q_in, s_nx, s_in, c_nx, c_in, st_r, st_gc, st_uc, st_gs, st_us, total; };
@@ -136,7 +137,7 @@ __host__ __device__ inline Lay2 lay2(const SpDims &d, int G) {
     auto take = [&](unsigned bytes) { const unsigned at = o; o = up16(o + bytes); return at; };
     const unsigned E = d.E, NE = d.NE, FFS = d.FFS, nj = cdiv(d.E, G), nP = cdiv(d.NU * d.FFE, G);
     L.ctl = take(sizeof(Ctl)); L.red = take(128 * 8); L.ex = take(8 * NE);
-    L.lg = take(4 * NE); L.p = take(4 * NE); L.dsc = take(4 * NE); L.wmax = take(4 * 32);
+    L.lg = take(4 * NE); L.p = take(4 * (NE < 128 ? 128 : NE)); L.dsc = take(4 * NE); L.wmax = take(4 * 32);
     L.q_in = take(E); L.s_in = take(4 * (E / 16)); L.c_in = take(4 * (E / 16));
     L.q_hd = take(FFS); L.s_hd = take(4 * (FFS / 16)); L.c_hd = take(4 * (FFS / 16));
     o = (o + 127u) & ~127u;
@@ -566,47 +567,8 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
 #pragma unroll
         for (int w = 0; w < kRW; w++) sum += red[w];
         const double rsum = 1.0 / sum;
-#pragma unroll 1
-        for (int i = t; i < NE; i += TR) p[i] = (float)(ex[i] * rsum);
-        bar_named(1, TR);
-        STAMP(1, 6);
-        if (NE <= 128) {
-            /* one warp, four candidates per lane in registers, NU rounds of (largest value, then lowest id among
-             * its holders): the order moe_topk_host's strict > insertion produces. key = bits(p) + 1 for a usable
-             * probability (p >= 0, so the bit pattern orders like the value), 0 for a NaN or an absent candidate */
-            if (warp == 0) {
-                unsigned key[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) { const int i = lane + 32 * k; const float v = i < NE ? p[i] : __int_as_float(0x7fc00000); key[k] = (v == v) ? __float_as_uint(v) + 1u : 0u; }
-#pragma unroll 1
-                for (int r = 0; r < NU; r++) {
-                    unsigned lm = key[0] > key[1] ? key[0] : key[1]; const unsigned l2 = key[2] > key[3] ? key[2] : key[3]; lm = lm > l2 ? lm : l2;
-                    const unsigned m = __reduce_max_sync(0xffffffffu, lm);
-                    if (m == 0u) break;
-                    unsigned cand = 0x7fffffffu;
-#pragma unroll
-                    for (int k = 3; k >= 0; k--) if (key[k] == m) cand = (unsigned)(lane + 32 * k);
-                    const unsigned w = __reduce_min_sync(0xffffffffu, cand);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) if ((unsigned)(lane + 32 * k) == w) key[k] = 0u;
-                    if (lane == 0) { ctl->sel_desc[r] = (int)w; ctl->p_desc[r] = __uint_as_float(m - 1u); }
-                }
-                __syncwarp();
-            }
-        } else {
-            /* rank of candidate i = how many candidates beat it (larger p, or equal p and lower id) */
-#pragma unroll 1
-            for (int i = t; i < NE; i += TR) {
-                const float pi = p[i]; int r = 0;
-#pragma unroll 4
-                for (int j = 0; j < NE; j++) { const float pj = p[j]; r += (pj > pi) || (pj == pi && j < i); }
-                if (r < NU && pi == pi) { ctl->sel_desc[r] = i; ctl->p_desc[r] = pi; }
-            }
-            bar_named(1, TR);
-        }
-        STAMP(1, 7);
-        if (warp == 0) {
-            /* the sum and the ascending place by shuffles, unrolled: the routed copies wait for this (22.50 -> 22.33 us a layer, 30 layers) */
+        /* sel_desc, p_desc -> normalised weights and ascending slots, by one warp */
+        auto finish = [&] {
             static_assert(SP_MAX_NU <= 32, "one lane per selected expert");
             const int e = lane < NU ? ctl->sel_desc[lane] : 0; const float pe = lane < NU ? ctl->p_desc[lane] : 0.0f;
             float ws = 0.0f; int slot = 0;
@@ -620,17 +582,11 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
             __syncwarp();
             if (lane < NU) { ctl->sel_asc[slot] = e; ctl->cw[slot] = __fmul_rn(wnorm, dsc[e]); ctl->p_desc[lane] = wnorm; }
             __syncwarp();
-            if (b == 0) asm volatile("bar.arrive 3, 64;" ::: "memory");      /* hands the selection to warp 1, which publishes it (below) */
-            if (nP > 0) {                                 /* the selection exists: start the first parts of the routed rows at once */
-                const int n1 = nP - n0;
-                const GuGeo gg{nP, n0, c0, ctl->sel_asc[slot0], n1 > 0 ? ctl->sel_asc[slot0 + 1] : ctl->sel_asc[slot0], 1 << LP, FFE, rbE, sbE};
-                gu_issue(sm, ly, ctl, L, gg, 0, nparts < kGuAhead ? nparts : kGuAhead, lane);
-            }
-        } else if (warp == 1 && b == 0) {
-            /* CTA 0 publishes the selection for the next kernel. A warp with nothing else to do takes it, so that the
-             * fence does not sit between the warp that feeds the copy engine and its copies; the CTA's signal to the
-             * dependent kernel follows every lane's fence. */
-            asm volatile("bar.sync 3, 64;" ::: "memory");
+        };
+        /* CTA 0 publishes the selection for the next kernel. A warp that starts no copies takes it, so that the fence does not sit
+         * between the warp that feeds the copy engine and its copies; the CTA's signal to the dependent kernel follows every
+         * lane's fence. */
+        auto publish = [&] {
             if (lane < NU) {
                 a.s.sel_asc[lane] = ctl->sel_asc[lane]; a.s.cw[lane] = ctl->cw[lane];
                 if (a.sel_out) a.sel_out[lane] = ctl->sel_desc[lane];
@@ -639,7 +595,89 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
             }
             __syncwarp();
             if (lane == 0) sp_pdl_next();
+        };
+        /* warp 0 finishes the selection and starts the routed rows' first parts, warp 1 publishes */
+        auto by_two = [&] {
+            if (warp == 0) {
+                finish();
+                if (b == 0) asm volatile("bar.arrive 3, 64;" ::: "memory");
+                if (nP > 0) {
+                    const int n1 = nP - n0;
+                    const GuGeo gg{nP, n0, c0, ctl->sel_asc[slot0], n1 > 0 ? ctl->sel_asc[slot0 + 1] : ctl->sel_asc[slot0], 1 << LP, FFE, rbE, sbE};
+                    gu_issue(sm, ly, ctl, L, gg, 0, nparts < kGuAhead ? nparts : kGuAhead, lane);
+                }
+            } else if (warp == 1 && b == 0) {
+                asm volatile("bar.sync 3, 64;" ::: "memory");
+                publish();
+            }
+        };
+        if (NE <= 128) {
+            STAMP(1, 6);
+            /* every warp ranks its 32 candidates among themselves, the first NU of each meet, and every warp ranks those: the order
+             * moe_topk_host's strict > insertion produces (largest probability, then lowest id; equal keys keep the order of their
+             * lanes, which is that of their ids). key = bits(p) + 1 for a usable probability (p >= 0, so the bit pattern orders like
+             * the value), 0 for a NaN or an absent candidate. Two rankings of 32 and a barrier take 0.9 us, NU rounds of a maximum
+             * and a minimum over all 128 took 1.1. */
+            auto rank = [&](int key, int *keys) {
+                keys[lane] = key;
+                __syncwarp();
+                int r = 0;
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const int4 o = *reinterpret_cast<const int4 *>(keys + j);
+                    r += (o.x > key - (j < lane)) + (o.y > key - (j + 1 < lane)) + (o.z > key - (j + 2 < lane)) + (o.w > key - (j + 3 < lane));
+                }
+                return r;
+            };
+            static_assert(TR == 128 && SP_MAX_NU * kRW == 32, "a candidate to a thread, a lane to each of the best");
+            int *const keys = reinterpret_cast<int *>(p);      /* a warp's 32 slots are its own */
+            const float v = t < NE ? (float)(ex[t] * rsum) : 0.0f;
+            const int key = t < NE && v == v ? __float_as_int(v) + 1 : 0, r = rank(key, keys + 32 * warp);
+            if (r < SP_MAX_NU) ctl->cand[SP_MAX_NU * warp + r] = make_int2(key, t);
+            bar_named(1, TR);
+            const int2 c = ctl->cand[lane];
+            const int rc = rank(c.x, keys + 32 * warp);
+            const bool chosen = rc < NU && c.x > 0;
+            if (__popc(__ballot_sync(0xffffffffu, chosen)) == NU) {
+                int slot = 0;                               /* ascending place: how many chosen ids are lower */
+#pragma unroll
+                for (int w = 0; w < kRW; w++) {
+                    const unsigned m = __reduce_or_sync(0xffffffffu, chosen && (c.y >> 5) == w ? 1u << (c.y & 31) : 0u);
+                    slot += __popc(w == c.y >> 5 ? m & ((1u << (c.y & 31)) - 1u) : w < c.y >> 5 ? m : 0u);
+                }
+                /* a warp starts one of the first parts of the routed rows, so that their copies (85 cycles of a warp each) do not queue
+                 * in one; the last has none and finishes the selection meanwhile */
+                const int e0 = __reduce_max_sync(0xffffffffu, chosen && slot == slot0 ? c.y : 0), e1 = __reduce_max_sync(0xffffffffu, chosen && slot == slot0 + 1 ? c.y : 0);
+                static_assert(kGuAhead == kRW - 1, "a part to each of the warps but the last");
+                if (warp < kGuAhead && warp < nparts) gu_issue(sm, ly, ctl, L, GuGeo{nP, n0, c0, e0, e1, 1 << LP, FFE, rbE, sbE}, warp, warp + 1, lane);
+                if (warp == kRW - 1) {
+                    if (chosen) { ctl->sel_desc[rc] = c.y; ctl->p_desc[rc] = __int_as_float(c.x - 1); }
+                    __syncwarp();
+                    finish();
+                    if (b == 0) publish();
+                }
+            } else {                                        /* fewer usable probabilities than experts to choose */
+                if (warp == 0 && chosen) { ctl->sel_desc[rc] = c.y; ctl->p_desc[rc] = __int_as_float(c.x - 1); }
+                bar_named(1, TR);
+                by_two();
+            }
+        } else {
+#pragma unroll 1
+            for (int i = t; i < NE; i += TR) p[i] = (float)(ex[i] * rsum);
+            bar_named(1, TR);
+            STAMP(1, 6);
+            /* rank of candidate i = how many candidates beat it (larger p, or equal p and lower id) */
+#pragma unroll 1
+            for (int i = t; i < NE; i += TR) {
+                const float pi = p[i]; int r = 0;
+#pragma unroll 4
+                for (int j = 0; j < NE; j++) { const float pj = p[j]; r += (pj > pi) || (pj == pi && j < i); }
+                if (r < NU && pi == pi) { ctl->sel_desc[r] = i; ctl->p_desc[r] = pi; }
+            }
+            bar_named(1, TR);
+            by_two();
         }
+        STAMP(1, 7);
     } else {
         /* ---- the routed experts' input (for the pairs below), the shared expert's hidden vector, its down rows */
         const int ts = t - TR, ws = warp - kRW;
