@@ -822,11 +822,11 @@ __device__ __forceinline__ void down_round(const unsigned char *sm, const Lay3 &
  * and one mul - and the slots are added in the shuffle tree's pairing. Rows past the slice repeat its last row and
  * are dropped. Valid while a row has at most 24 chunks (six groups of four). */
 __device__ __forceinline__ void mma_s8_acc(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void mma_s8_first(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
 __device__ __forceinline__ float magic16_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }   /* bits 0x4B400000 + 16 S -> float(S) */
@@ -838,24 +838,26 @@ __device__ __forceinline__ void down_tile_mma(const unsigned char *sm, const Lay
     const int gq = lane >> 2, q = lane & 3;
     const int r0 = ti * 16 + gq, r1 = r0 + 8;
     const int rc0 = r0 < nj ? r0 : nj - 1, rc1 = r1 < nj ? r1 : nj - 1;
-    const unsigned char *c0 = sm + ly.st_c + ((unsigned)s * (unsigned)njm + (unsigned)rc0) * rb;
-    const unsigned char *c1 = sm + ly.st_c + ((unsigned)s * (unsigned)njm + (unsigned)rc1) * rb;
-    const unsigned char *sbase = sm + ly.st_s + (unsigned)s * ly.span_max + ctl->sdelta[s];
+    /* each lane at its chunk of a group of four (4 jj + q). A last group may reach past the row: what those lanes load is some other
+     * row's, stays in shared memory, and only touches columns and sums that are not used */
+    const unsigned char *c0 = sm + ly.st_c + ((unsigned)s * (unsigned)njm + (unsigned)rc0) * rb + 16 * q;
+    const unsigned char *c1 = sm + ly.st_c + ((unsigned)s * (unsigned)njm + (unsigned)rc1) * rb + 16 * q;
+    const unsigned char *sbase = sm + ly.st_s + (unsigned)s * ly.span_max + ctl->sdelta[s] + 2 * q;
     const unsigned char *sc0 = sbase + (unsigned)rc0 * sb, *sc1 = sbase + (unsigned)rc1 * sb;
-    const unsigned char *qh = sm + ly.q_h + (unsigned)s * (unsigned)blk16 * 16u;
-    const float *sxp = reinterpret_cast<const float *>(sm + ly.s_h) + (unsigned)s * (unsigned)blk16;
+    const unsigned char *qh = sm + ly.q_h + (unsigned)s * (unsigned)blk16 * 16u + 32 * q;
+    const float *sxp = reinterpret_cast<const float *>(sm + ly.s_h) + (unsigned)s * (unsigned)blk16 + 2 * q;
     const unsigned char *zero = reinterpret_cast<const unsigned char *>(ctl->zero);
-    const bool bvalid = (gq >> 1) == q; const int bh = gq & 1;
+    const bool h0 = (gq >> 1) == q && !(gq & 1), h1 = (gq >> 1) == q && (gq & 1);
+    const unsigned char *b0 = h0 ? qh : zero, *b1 = h1 ? qh + 16 : zero;
+    const unsigned step0 = h0 ? 128u : 0u, step1 = h1 ? 128u : 0u;
     float acc[8][2];
 #pragma unroll
     for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = 0.0f;
 #pragma unroll
     for (int jj = 0; jj < kMmaGroups; jj++) {
         if (4 * jj < n32) {                               /* warp-uniform */
-            const int c = 4 * jj + q; const bool cv = c < n32; const int cc = cv ? c : n32 - 1;
-            uint4 w0 = *reinterpret_cast<const uint4 *>(c0 + 16 * cc), w1 = *reinterpret_cast<const uint4 *>(c1 + 16 * cc);
-            if (!cv) { w0 = make_uint4(0, 0, 0, 0); w1 = w0; }
-            const float s0 = h2f(*reinterpret_cast<const unsigned short *>(sc0 + 2 * cc)), s1 = h2f(*reinterpret_cast<const unsigned short *>(sc1 + 2 * cc));
+            const uint4 w0 = *reinterpret_cast<const uint4 *>(c0 + 64 * jj), w1 = *reinterpret_cast<const uint4 *>(c1 + 64 * jj);
+            const float s0 = h2f(*reinterpret_cast<const unsigned short *>(sc0 + 8 * jj)), s1 = h2f(*reinterpret_cast<const unsigned short *>(sc1 + 8 * jj));
             const unsigned x0[4] = {w0.x, w0.y, w0.z, w0.w}, x1[4] = {w1.x, w1.y, w1.z, w1.w};
             unsigned a[4][4];
 #pragma unroll
@@ -863,15 +865,15 @@ __device__ __forceinline__ void down_tile_mma(const unsigned char *sm, const Lay
                 a[i][0] = (x0[i] << 4) & 0xF0F0F0F0u; a[i][1] = (x1[i] << 4) & 0xF0F0F0F0u;
                 a[i][2] = x0[i] & 0xF0F0F0F0u;        a[i][3] = x1[i] & 0xF0F0F0F0u;
             }
-            const uint4 l0 = *reinterpret_cast<const uint4 *>(bvalid && cv && bh == 0 ? qh + c * 32 : zero);
-            const uint4 l1 = *reinterpret_cast<const uint4 *>(bvalid && cv && bh == 1 ? qh + c * 32 + 16 : zero);
+            const uint4 l0 = *reinterpret_cast<const uint4 *>(b0), l1 = *reinterpret_cast<const uint4 *>(b1);
+            b0 += step0; b1 += step1;
             int ca[4], cb[4];
             mma_s8_first(ca, a[0][0], a[0][1], a[0][2], a[0][3], l0.x, l0.y, kMagicBits);
             mma_s8_first(cb, a[2][0], a[2][1], a[2][2], a[2][3], l1.x, l1.y, kMagicBits);
             mma_s8_acc(ca, a[1][0], a[1][1], a[1][2], a[1][3], l0.z, l0.w);
             mma_s8_acc(cb, a[3][0], a[3][1], a[3][2], a[3][3], l1.z, l1.w);
-            if (cv) {
-                const float2 s2 = *reinterpret_cast<const float2 *>(sxp + 2 * c);
+            const float2 s2 = *reinterpret_cast<const float2 *>(sxp + 8 * jj);
+            if (4 * jj + q < n32) {
                 acc[jj][0] = __fmaf_rn(s0, __fmaf_rn(magic16_to_float(ca[0]), s2.x, __fmul_rn(magic16_to_float(cb[1]), s2.y)), acc[jj][0]);
                 acc[jj][1] = __fmaf_rn(s1, __fmaf_rn(magic16_to_float(ca[2]), s2.x, __fmul_rn(magic16_to_float(cb[3]), s2.y)), acc[jj][1]);
             }
@@ -912,6 +914,9 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
     const int n32 = FFE >> 5, blk16 = FFE >> 4, nblk = (NU * FFE) >> 4;
     const int SGs = (NU + kDnBars - 1) / kDnBars;         /* expert slots per landing part */
     STAMP(2, 0);
+    /* The selection was published and fenced before this kernel could be launched: this CTA's rows of every selected expert are
+     * requested now, before the wait for the predecessor's hidden vectors, an expert slot to a warp (sixteen copies of 85
+     * cycles each would queue in one) */
     if (t == 0) {
 #pragma unroll 1
         for (int i = 0; i < kDnBars; i++) mbar_init(smem_u32(&ctl->bar[i]), 1);
@@ -921,8 +926,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
     }
     __syncthreads();
     sp_pdl_next();
-    if (warp == 0) {                                      /* the selection was published and fenced before this kernel could be launched: start this
-                                                             CTA's rows of every selected expert now, before waiting for the predecessor's hidden vectors */
+    if (warp == 0) {
         const int e = lane < NU ? __ldcg(a.s.sel_asc + lane) : 0;
         const float w = lane < NU ? __ldcg(a.s.cw + lane) : 0.0f;
         if (lane < NU) { ctl->sel_asc[lane] = e; ctl->cw[lane] = w; }
@@ -930,7 +934,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
             const unsigned char *bs = reinterpret_cast<const unsigned char *>(L.dn_bs);
             const Span sp = make_span(bs + ((size_t)e * E + j0) * sb, (unsigned)nj * sb);
             if (lane < NU) ctl->sdelta[lane] = sp.delta;
-            const unsigned mine = lane < NU ? (unsigned)nj * rb + sp.bytes : 0u;       /* bytes per landing part: the lanes of its slots add up */
+            const unsigned mine = lane < NU ? (unsigned)nj * rb + sp.bytes : 0u;
             const int g = lane / SGs;
 #pragma unroll
             for (int gg = 0; gg < kDnBars; gg++) {
