@@ -113,7 +113,7 @@ struct Ctl {
     unsigned gs_off[2], us_off[2];          /* K2: where the two runs' gate / up scale rows start */
     unsigned sdelta[SP_MAX_NU];             /* K3: bytes before the first scale row of each slot's span */
     alignas(16) int zero[4];                /* K3: the activation operand of an MMA column that is not the lane's */
-    int2 cand[4 * SP_MAX_NU];               /* K2: the best of each router warp's candidates */
+    int2 cand[4 * SP_MAX_NU], rest[4];      /* K2: the best of each router warp's candidates (key, id); its next key and whether it met a NaN */
 };
 
 struct Lay1 { unsigned ctl, red, va, vb, ri, q_nx, q_in, s_nx, s_in, c_nx, c_in, st_r, st_gc, st_uc, st_gs, st_us, total; };
@@ -289,7 +289,7 @@ template <int KE, int NIT>
 __global__ void __launch_bounds__(kT, 1) k_ds_router_shared(SArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
     const SpDims d = a.d;
-    const int E = d.E, t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x, b = blockIdx.x;
+    const int E = d.E, t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x;
     const Lay1 &ly = *reinterpret_cast<const Lay1 *>(a.lay);
     Ctl *ctl = reinterpret_cast<Ctl *>(sm + ly.ctl);
     double *red = reinterpret_cast<double *>(sm + ly.red);
@@ -544,29 +544,6 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
     STAMP(1, 1);
     if (warp < kRW) {
         /* ---- moe_topk_host (CF:6220-6240): double softmax, order by (p descending, id ascending), clamp, renormalise */
-        float mx = -INFINITY; int bad = 0;
-#pragma unroll 1
-        for (int i = t; i < NE; i += TR) { const float l = __ldcg(a.s.logits + i); lg[i] = l; if (l != l) bad = 1; mx = fmaxf(mx, l); }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); bad |= __shfl_xor_sync(0xffffffffu, bad, o); }
-        if (lane == 0) wmax[warp] = mx;
-        if (bad && lane == 0) atomicExch(a.s.status, SP_KERR_NAN_ROUTER);
-        if (t < SP_MAX_NU) { ctl->sel_desc[t] = t < NE ? t : 0; ctl->p_desc[t] = 0.0f; }
-        bar_named(1, TR);
-        STAMP(1, 5);
-        mx = wmax[0];
-#pragma unroll
-        for (int w = 1; w < kRW; w++) mx = fmaxf(mx, wmax[w]);
-        double part = 0.0;
-#pragma unroll 1
-        for (int i = t; i < NE; i += TR) { const double e = exp((double)lg[i] - (double)mx); ex[i] = e; part += e; }
-        part = warp_sum_f64(part);
-        if (lane == 0) red[warp] = part;
-        bar_named(1, TR);
-        double sum = 0.0;
-#pragma unroll
-        for (int w = 0; w < kRW; w++) sum += red[w];
-        const double rsum = 1.0 / sum;
         /* sel_desc, p_desc -> normalised weights and ascending slots, by one warp */
         auto finish = [&] {
             static_assert(SP_MAX_NU <= 32, "one lane per selected expert");
@@ -611,34 +588,55 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
                 publish();
             }
         };
-        if (NE <= 128) {
-            STAMP(1, 6);
-            /* every warp ranks its 32 candidates among themselves, the first NU of each meet, and every warp ranks those: the order
-             * moe_topk_host's strict > insertion produces (largest probability, then lowest id; equal keys keep the order of their
-             * lanes, which is that of their ids). key = bits(p) + 1 for a usable probability (p >= 0, so the bit pattern orders like
-             * the value), 0 for a NaN or an absent candidate. Two rankings of 32 and a barrier take 0.9 us, NU rounds of a maximum
-             * and a minimum over all 128 took 1.1. */
-            auto rank = [&](int key, int *keys) {
-                keys[lane] = key;
-                __syncwarp();
-                int r = 0;
+        /* how many of the warp's 32 keys are larger, or equal in a lower lane */
+        auto rank = [&](int key, int *keys) {
+            keys[lane] = key;
+            __syncwarp();
+            int r = 0;
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                    const int4 o = *reinterpret_cast<const int4 *>(keys + j);
-                    r += (o.x > key - (j < lane)) + (o.y > key - (j + 1 < lane)) + (o.z > key - (j + 2 < lane)) + (o.w > key - (j + 3 < lane));
-                }
-                return r;
-            };
+            for (int j = 0; j < 32; j += 4) {
+                const int4 o = *reinterpret_cast<const int4 *>(keys + j);
+                r += (o.x > key - (j < lane)) + (o.y > key - (j + 1 < lane)) + (o.z > key - (j + 2 < lane)) + (o.w > key - (j + 3 < lane));
+            }
+            return r;
+        };
+        bool done = false;
+        if (NE <= 128) {
+            /* The selection straight from the logits: every warp ranks its 32 among themselves, the first NU of each meet, and every
+             * warp ranks those (equal keys keep the order of their lanes, which is that of their ids). Probabilities order as
+             * logits do, except that different logits can round to one probability; so it holds where no two neighbours among the
+             * first NU + 1 differ by less than 1e-6 without being equal (a probability is rounded to 6e-8 of itself) and none is
+             * 80 below the first (no underflow). Otherwise, and with a NaN, the probabilities decide, below. The routed copies wait
+             * for this: with the softmax first and NU rounds of a maximum and a minimum they went out 1.7 us later. */
             static_assert(TR == 128 && SP_MAX_NU * kRW == 32, "a candidate to a thread, a lane to each of the best");
-            int *const keys = reinterpret_cast<int *>(p);      /* a warp's 32 slots are its own */
-            const float v = t < NE ? (float)(ex[t] * rsum) : 0.0f;
-            const int key = t < NE && v == v ? __float_as_int(v) + 1 : 0, r = rank(key, keys + 32 * warp);
+            constexpr int kAbsent = (int)0x80000001;
+            int *const keys = reinterpret_cast<int *>(p) + 32 * warp;      /* a warp's 32 slots are its own */
+            const float l = t < NE ? __fadd_rn(__ldcg(a.s.logits + t), 0.0f) : -INFINITY;         /* -0 becomes 0 */
+            auto order = [](float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); };      /* its own inverse on int */
+            const int key = t < NE ? order(l) : kAbsent, r = rank(key, keys);
             if (r < SP_MAX_NU) ctl->cand[SP_MAX_NU * warp + r] = make_int2(key, t);
+            const bool bad = __any_sync(0xffffffffu, t < NE && l != l);
+            if (r == SP_MAX_NU) ctl->rest[warp] = make_int2(key, bad);
             bar_named(1, TR);
             const int2 c = ctl->cand[lane];
-            const int rc = rank(c.x, keys + 32 * warp);
-            const bool chosen = rc < NU && c.x > 0;
-            if (__popc(__ballot_sync(0xffffffffu, chosen)) == NU) {
+            const int rc = rank(c.x, keys);
+            __syncwarp();
+            keys[rc] = c.x;                                 /* sorted */
+            __syncwarp();
+            int after = keys[NU < 32 ? NU : 31], flag = 0;  /* the largest key not chosen */
+#pragma unroll
+            for (int w = 0; w < kRW; w++) { const int2 o = ctl->rest[w]; after = o.x > after ? o.x : after; flag |= o.y; }
+            auto value = [&](int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); };
+            const float first = value(keys[0]);
+            bool close = flag != 0;
+            if (lane < NU) {
+                const int k0 = keys[lane], k1 = lane + 1 < NU ? keys[lane + 1] : after;
+                const float gap = value(k0) - value(k1);
+                close |= k0 == kAbsent || !(value(k0) > first - 80.0f) || (k1 != kAbsent && k0 != k1 && !(gap >= 1e-6f));
+            }
+            done = !__any_sync(0xffffffffu, close);
+            if (done) {
+                const bool chosen = rc < NU;
                 int slot = 0;                               /* ascending place: how many chosen ids are lower */
 #pragma unroll
                 for (int w = 0; w < kRW; w++) {
@@ -646,26 +644,56 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
                     slot += __popc(w == c.y >> 5 ? m & ((1u << (c.y & 31)) - 1u) : w < c.y >> 5 ? m : 0u);
                 }
                 /* a warp starts one of the first parts of the routed rows, so that their copies (85 cycles of a warp each) do not queue
-                 * in one; the last has none and finishes the selection meanwhile */
+                 * in one; the last has none and finishes the selection */
                 const int e0 = __reduce_max_sync(0xffffffffu, chosen && slot == slot0 ? c.y : 0), e1 = __reduce_max_sync(0xffffffffu, chosen && slot == slot0 + 1 ? c.y : 0);
-                static_assert(kGuAhead == kRW - 1, "a part to each of the warps but the last");
-                if (warp < kGuAhead && warp < nparts) gu_issue(sm, ly, ctl, L, GuGeo{nP, n0, c0, e0, e1, 1 << LP, FFE, rbE, sbE}, warp, warp + 1, lane);
+                if (warp < kRW - 1)
+#pragma unroll 1
+                    for (int g = warp; g < kGuAhead && g < nparts; g += kRW - 1) gu_issue(sm, ly, ctl, L, GuGeo{nP, n0, c0, e0, e1, 1 << LP, FFE, rbE, sbE}, g, g + 1, lane);
+                STAMP(1, 5);
+                const double e = t < NE ? exp((double)l - (double)first) : 0.0;
+                if (t < NE) ex[t] = e;
+                const double part = warp_sum_f64(e);
+                if (lane == 0) red[warp] = part;
+                bar_named(1, TR);
+                STAMP(1, 6);
                 if (warp == kRW - 1) {
-                    if (chosen) { ctl->sel_desc[rc] = c.y; ctl->p_desc[rc] = __int_as_float(c.x - 1); }
+                    double sum = 0.0;
+#pragma unroll
+                    for (int w = 0; w < kRW; w++) sum += red[w];
+                    const double rsum = 1.0 / sum;
+                    if (chosen) { ctl->sel_desc[rc] = c.y; ctl->p_desc[rc] = (float)(ex[c.y] * rsum); }
                     __syncwarp();
                     finish();
                     if (b == 0) publish();
                 }
-            } else {                                        /* fewer usable probabilities than experts to choose */
-                if (warp == 0 && chosen) { ctl->sel_desc[rc] = c.y; ctl->p_desc[rc] = __int_as_float(c.x - 1); }
-                bar_named(1, TR);
-                by_two();
             }
-        } else {
+        }
+        if (!done) {
+            float mx = -INFINITY; int bad = 0;
+#pragma unroll 1
+            for (int i = t; i < NE; i += TR) { const float l = __ldcg(a.s.logits + i); lg[i] = l; if (l != l) bad = 1; mx = fmaxf(mx, l); }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); bad |= __shfl_xor_sync(0xffffffffu, bad, o); }
+            if (lane == 0) wmax[warp] = mx;
+            if (bad && lane == 0) atomicExch(a.s.status, SP_KERR_NAN_ROUTER);
+            if (t < SP_MAX_NU) { ctl->sel_desc[t] = t < NE ? t : 0; ctl->p_desc[t] = 0.0f; }
+            bar_named(1, TR);
+            mx = wmax[0];
+#pragma unroll
+            for (int w = 1; w < kRW; w++) mx = fmaxf(mx, wmax[w]);
+            double part = 0.0;
+#pragma unroll 1
+            for (int i = t; i < NE; i += TR) { const double e = exp((double)lg[i] - (double)mx); ex[i] = e; part += e; }
+            part = warp_sum_f64(part);
+            if (lane == 0) red[warp] = part;
+            bar_named(1, TR);
+            double sum = 0.0;
+#pragma unroll
+            for (int w = 0; w < kRW; w++) sum += red[w];
+            const double rsum = 1.0 / sum;
 #pragma unroll 1
             for (int i = t; i < NE; i += TR) p[i] = (float)(ex[i] * rsum);
             bar_named(1, TR);
-            STAMP(1, 6);
             /* rank of candidate i = how many candidates beat it (larger p, or equal p and lower id) */
 #pragma unroll 1
             for (int i = t; i < NE; i += TR) {
