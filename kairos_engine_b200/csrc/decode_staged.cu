@@ -59,7 +59,7 @@ struct SArgs {
     int has_next;
     unsigned flags;           /* SP_STAGED_* */
     long long *stamps;        /* [3][16] device time stamps of CTA 0, or NULL */
-    unsigned lay[20];         /* this kernel's shared-memory layout (Lay1 / Lay2 / Lay3), computed on the host */
+    unsigned lay[24];         /* this kernel's shared-memory layout (Lay1 / Lay2 / Lay3), computed on the host */
 };
 
 #define STAMP(k, i) do { if (a.stamps && blockIdx.x == 0 && threadIdx.x == 0) { long long t_; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_)); a.stamps[(k) * 16 + (i)] = t_; } } while (0)
@@ -131,7 +131,7 @@ __host__ __device__ inline Lay1 lay1(const SpDims &d, int G) {
     L.total = o;
     return L;
 }
-struct Lay2 { unsigned ctl, red, ex, lg, p, dsc, wmax, q_in, s_in, c_in, q_hd, s_hd, c_hd, st_sd, st_sds, st_gc, st_uc, st_gs, st_us, total; };
+struct Lay2 { unsigned ctl, red, ex, lg, p, dsc, wmax, q_in, s_in, c_in, q_hd, s_hd, c_hd, st_sd, st_sds, st_gc, st_uc, st_gs, st_us, part, total; };
 __host__ __device__ inline Lay2 lay2(const SpDims &d, int G) {
     Lay2 L; unsigned o = 0;
     auto take = [&](unsigned bytes) { const unsigned at = o; o = up16(o + bytes); return at; };
@@ -144,6 +144,7 @@ __host__ __device__ inline Lay2 lay2(const SpDims &d, int G) {
     L.st_sd = take(nj * (FFS / 2)); L.st_sds = take(nj * (FFS / 16) + 32);
     L.st_gc = take(nP * (E / 2)); L.st_uc = take(nP * (E / 2));
     L.st_gs = take(nP * (E / 16) + 64); L.st_us = take(nP * (E / 16) + 64);
+    L.part = take(1024 * ((nP + 7) / 8));
     L.total = o;
     return L;
 }
@@ -489,6 +490,70 @@ __device__ __forceinline__ void gu_issue(unsigned char *sm, const Lay2 &ly, Ctl 
     if (sz) bulk_g2s(sm + dst, src, sz, smem_u32(&ctl->bar[1 + g]));
 }
 
+__device__ __forceinline__ void mma_s8_acc(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_s8_first(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
+}
+__device__ __forceinline__ float magic16_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }   /* bits 0x4B400000 + 16 S -> float(S) */
+/* four chunks of a row and of its partner (a group), for the lane at chunk q of it: codes c0, c1, scales s0, s1, the lane's bytes of the
+ * activations' two halves (or zeros), their block scales */
+__device__ __forceinline__ void group_mma(const unsigned char *c0, const unsigned char *c1, const unsigned char *sc0, const unsigned char *sc1,
+                                          const unsigned char *b0, const unsigned char *b1, const float *sx, bool valid, float2 &acc) {
+    const uint4 w0 = *reinterpret_cast<const uint4 *>(c0), w1 = *reinterpret_cast<const uint4 *>(c1);
+    const float s0 = h2f(*reinterpret_cast<const unsigned short *>(sc0)), s1 = h2f(*reinterpret_cast<const unsigned short *>(sc1));
+    const unsigned x0[4] = {w0.x, w0.y, w0.z, w0.w}, x1[4] = {w1.x, w1.y, w1.z, w1.w};
+    unsigned a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        a[i][0] = (x0[i] << 4) & 0xF0F0F0F0u; a[i][1] = (x1[i] << 4) & 0xF0F0F0F0u;
+        a[i][2] = x0[i] & 0xF0F0F0F0u;        a[i][3] = x1[i] & 0xF0F0F0F0u;
+    }
+    const uint4 l0 = *reinterpret_cast<const uint4 *>(b0), l1 = *reinterpret_cast<const uint4 *>(b1);
+    int ca[4], cb[4];
+    mma_s8_first(ca, a[0][0], a[0][1], a[0][2], a[0][3], l0.x, l0.y, kMagicBits);
+    mma_s8_first(cb, a[2][0], a[2][1], a[2][2], a[2][3], l1.x, l1.y, kMagicBits);
+    mma_s8_acc(ca, a[1][0], a[1][1], a[1][2], a[1][3], l0.z, l0.w);
+    mma_s8_acc(cb, a[3][0], a[3][1], a[3][2], a[3][3], l1.z, l1.w);
+    const float2 s2 = *reinterpret_cast<const float2 *>(sx);
+    if (valid) {
+        acc.x = __fmaf_rn(s0, __fmaf_rn(magic16_to_float(ca[0]), s2.x, __fmul_rn(magic16_to_float(cb[1]), s2.y)), acc.x);
+        acc.y = __fmaf_rn(s1, __fmaf_rn(magic16_to_float(ca[2]), s2.x, __fmul_rn(magic16_to_float(cb[3]), s2.y)), acc.y);
+    }
+}
+/* Routed gate|up: the row dots of eight pairs on the tensor cores (as in k_ds_experts_down, below), a quarter of a row's slots to a warp:
+ * those with (slot / 4) % 4 = r, groups r, r + 4, r + 8, ... part: [tile][r][slot % 4][gate rows, up rows], each the first level of the
+ * tree. A warp then has a quarter of the instructions that dp4a takes for the same rows, and a part of the copies is worked
+ * off by four warps while the next one lands. */
+template <int NIT>
+__device__ __forceinline__ void pairs_mma(unsigned char *sm, const Lay2 &ly, Ctl *ctl, int tile, int r, int nP, int n0, unsigned rb, unsigned sb, int n32, int lane,
+                                          const signed char *q_in, const float *s_in, float *part) {
+    const int g = lane >> 2, q = lane & 3;
+    int i = 8 * tile + g;
+    if (i > nP - 1) i = nP - 1;                             /* rows past the slice repeat its last pair and are dropped */
+    const int run = i >= n0, idx = run ? i - n0 : i, o = 4 * r + q;
+    const unsigned char *c0 = sm + ly.st_gc + (unsigned)i * rb + 16 * o, *c1 = sm + ly.st_uc + (unsigned)i * rb + 16 * o;
+    const unsigned char *s0 = sm + ctl->gs_off[run] + (unsigned)idx * sb + 2 * o, *s1 = sm + ctl->us_off[run] + (unsigned)idx * sb + 2 * o;
+    const unsigned char *zero = reinterpret_cast<const unsigned char *>(ctl->zero), *qb = reinterpret_cast<const unsigned char *>(q_in) + 32 * o;
+    const bool h0 = (g >> 1) == q && !(g & 1), h1 = (g >> 1) == q && (g & 1);
+    const unsigned char *b0 = h0 ? qb : zero, *b1 = h1 ? qb + 16 : zero;
+    const unsigned st0 = h0 ? 512u : 0u, st1 = h1 ? 512u : 0u;
+    const float *sx = s_in + 2 * o;
+    float2 lo = make_float2(0.0f, 0.0f), hi = lo;           /* slots of groups r + 8 i, r + 4 + 8 i */
+    const int n = ((n32 + 3) >> 2) - r, left = n32 - o;
+#pragma unroll
+    for (int k = 0; k < 2 * NIT; k++)                       /* a last group may reach past the row: see down_tile_mma */
+        if (4 * k < n) {                                    /* warp-uniform */
+            group_mma(c0 + 256 * k, c1 + 256 * k, s0 + 32 * k, s1 + 32 * k, b0, b1, sx + 32 * k, 16 * k < left, k & 1 ? hi : lo);
+            b0 += st0; b1 += st1;
+        }
+    float *p = part + ((tile * 4 + r) * 4 + q) * 16 + g;
+    p[0] = lo.x + hi.x; p[8] = lo.y + hi.y;
+}
+
 template <int NIT_E, int NIT_S>
 __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -525,6 +590,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
 #pragma unroll 1
         for (int i = 0; i < 1 + kGuBars; i++) mbar_init(smem_u32(&ctl->bar[i]), 1);
         ctl->abort = 0;
+        ctl->zero[0] = ctl->zero[1] = ctl->zero[2] = ctl->zero[3] = 0;
         fence_barrier_init();
         if (nj > 0) {                                     /* shared-expert down rows: fixed addresses */
             mbar_expect_tx(bar_sd, (unsigned)nj * rbS + sds.bytes);
@@ -746,34 +812,15 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
         }
     }
     STAMP(1, 3);
-    /* routed gate|up pairs, as their part lands */
-    {
-        ActR<NIT_E> act;
-        act_load<NIT_E>(act, q_in, s_in, c_in, n32, lane);
-        /* four pairs (eight rows) per round: their lane partials wait in registers, one butterfly reduces all
-         * eight rows, and the lanes 0, 8, 16, 24 apply the GeGLU of the four pairs at the same time */
+    /* routed gate|up pairs, eight to a tile, as their part lands; units of work: (tile, quarter of the slots) */
+    float *const part = reinterpret_cast<float *>(sm + ly.part);
+    const int tiles = (nP + 7) >> 3;
 #pragma unroll 1
-        for (int i0 = warp; i0 < nP; i0 += 4 * kW) {
-            float f[8];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int i = i0 + k * kW;
-                f[2 * k] = 0.0f; f[2 * k + 1] = 0.0f;
-                if (i < nP) {                             /* warp-uniform */
-                    bar_wait(smem_u32(&ctl->bar[1]), &ctl->abort, a.s.status);              /* the scale rows travel with part 0 */
-                    bar_wait(smem_u32(&ctl->bar[1 + (i >> LP)]), &ctl->abort, a.s.status);
-                    const int run = i >= n0, idx = run ? i - n0 : i;
-                    RowW<NIT_E> wg, wu;
-                    row_fetch<NIT_E>(wg, sm + ly.st_gc + (unsigned)i * rbE, sm + ctl->gs_off[run] + (unsigned)idx * sbE, n32, lane);
-                    row_fetch<NIT_E>(wu, sm + ly.st_uc + (unsigned)i * rbE, sm + ctl->us_off[run] + (unsigned)idx * sbE, n32, lane);
-                    f[2 * k] = row_dot<NIT_E>(wg, act); f[2 * k + 1] = row_dot<NIT_E>(wu, act);
-                }
-            }
-            const float tot = tree8(f, lane);             /* lane 4r (and its three neighbours) holds row r: gate of pair k in lanes 8k.., up in lanes 8k+4.. */
-            const float upv = __shfl_down_sync(0xffffffffu, tot, 4);
-            const int k = lane >> 3, i = i0 + k * kW;
-            if ((lane & 7) == 0 && i < nP) a.s.h[P0 + i] = gelu_mul(tot, upv);
-        }
+    for (int u = warp; u < 4 * tiles; u += kW) {
+        bar_wait(smem_u32(&ctl->bar[1]), &ctl->abort, a.s.status);              /* the scale rows travel with part 0 */
+        bar_wait(smem_u32(&ctl->bar[1 + ((u >> 2) << 3 >> LP)]), &ctl->abort, a.s.status);
+        __syncwarp();
+        pairs_mma<NIT_E>(sm, ly, ctl, u >> 2, u & 3, nP, n0, rbE, sbE, n32, lane, q_in, s_in, part);
     }
     if ((a.flags & SP_STAGED_PREFETCH_DN) && nj > 0) {    /* the routed down rows the next kernel will stage: ask L2 for them */
 #pragma unroll 1
@@ -785,6 +832,17 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
     }
     STAMP(1, 12);
     __syncthreads();
+    /* the tree's other levels, eight lanes to a pair: (0 + 2) + (1 + 3) of the quarters, the same of the slots; then GeGLU */
+#pragma unroll 1
+    for (int i0 = t; (i0 & ~31) < 8 * nP; i0 += kT) {
+        const int i = i0 >> 3 < nP ? i0 >> 3 : nP - 1;
+        const float *f = part + (i >> 3) * 256 + (lane & 3) * 16 + 8 * ((lane >> 2) & 1) + (i & 7);
+        float v = (f[0] + f[128]) + (f[64] + f[192]);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        const float up = __shfl_down_sync(0xffffffffu, v, 4);
+        if ((lane & 7) == 0 && i0 >> 3 < nP) a.s.h[P0 + i] = gelu_mul(v, up);
+    }
     STAMP(1, 4);
 }
 
@@ -849,15 +907,6 @@ __device__ __forceinline__ void down_round(const unsigned char *sm, const Lay3 &
  * does what lane (4j+q) % 32 does in row_dot - one accumulator per slot, chunks in ascending order, the same two fmas
  * and one mul - and the slots are added in the shuffle tree's pairing. Rows past the slice repeat its last row and
  * are dropped. Valid while a row has at most 24 chunks (six groups of four). */
-__device__ __forceinline__ void mma_s8_acc(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_s8_first(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
-}
-__device__ __forceinline__ float magic16_to_float(int c) { return __fmaf_rn(__int_as_float(c), 0.0625f, -786432.0f); }   /* bits 0x4B400000 + 16 S -> float(S) */
 constexpr int kMmaGroups = 6;
 
 __device__ __forceinline__ void down_tile_mma(const unsigned char *sm, const Lay3 &ly, Ctl *ctl, int *status, int s, int ti, int nj, int njm, int SGs,
@@ -878,40 +927,21 @@ __device__ __forceinline__ void down_tile_mma(const unsigned char *sm, const Lay
     const bool h0 = (gq >> 1) == q && !(gq & 1), h1 = (gq >> 1) == q && (gq & 1);
     const unsigned char *b0 = h0 ? qh : zero, *b1 = h1 ? qh + 16 : zero;
     const unsigned step0 = h0 ? 128u : 0u, step1 = h1 ? 128u : 0u;
-    float acc[8][2];
+    float2 acc[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = 0.0f;
+    for (int i = 0; i < 8; i++) acc[i] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int jj = 0; jj < kMmaGroups; jj++) {
         if (4 * jj < n32) {                               /* warp-uniform */
-            const uint4 w0 = *reinterpret_cast<const uint4 *>(c0 + 64 * jj), w1 = *reinterpret_cast<const uint4 *>(c1 + 64 * jj);
-            const float s0 = h2f(*reinterpret_cast<const unsigned short *>(sc0 + 8 * jj)), s1 = h2f(*reinterpret_cast<const unsigned short *>(sc1 + 8 * jj));
-            const unsigned x0[4] = {w0.x, w0.y, w0.z, w0.w}, x1[4] = {w1.x, w1.y, w1.z, w1.w};
-            unsigned a[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                a[i][0] = (x0[i] << 4) & 0xF0F0F0F0u; a[i][1] = (x1[i] << 4) & 0xF0F0F0F0u;
-                a[i][2] = x0[i] & 0xF0F0F0F0u;        a[i][3] = x1[i] & 0xF0F0F0F0u;
-            }
-            const uint4 l0 = *reinterpret_cast<const uint4 *>(b0), l1 = *reinterpret_cast<const uint4 *>(b1);
+            group_mma(c0 + 64 * jj, c1 + 64 * jj, sc0 + 8 * jj, sc1 + 8 * jj, b0, b1, sxp + 8 * jj, 4 * jj + q < n32, acc[jj]);
             b0 += step0; b1 += step1;
-            int ca[4], cb[4];
-            mma_s8_first(ca, a[0][0], a[0][1], a[0][2], a[0][3], l0.x, l0.y, kMagicBits);
-            mma_s8_first(cb, a[2][0], a[2][1], a[2][2], a[2][3], l1.x, l1.y, kMagicBits);
-            mma_s8_acc(ca, a[1][0], a[1][1], a[1][2], a[1][3], l0.z, l0.w);
-            mma_s8_acc(cb, a[3][0], a[3][1], a[3][2], a[3][3], l1.z, l1.w);
-            const float2 s2 = *reinterpret_cast<const float2 *>(sxp + 8 * jj);
-            if (4 * jj + q < n32) {
-                acc[jj][0] = __fmaf_rn(s0, __fmaf_rn(magic16_to_float(ca[0]), s2.x, __fmul_rn(magic16_to_float(cb[1]), s2.y)), acc[jj][0]);
-                acc[jj][1] = __fmaf_rn(s1, __fmaf_rn(magic16_to_float(ca[2]), s2.x, __fmul_rn(magic16_to_float(cb[3]), s2.y)), acc[jj][1]);
-            }
         }
     }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = acc[i][r];
+        for (int i = 0; i < 8; i++) v[i] = r ? acc[i].y : acc[i].x;
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
