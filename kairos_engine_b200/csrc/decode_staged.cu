@@ -116,29 +116,28 @@ struct Ctl {
     int2 cand[4 * SP_MAX_NU], rest[4];      /* K2: the best of each router warp's candidates (key, id); its next key and whether it met a NaN */
 };
 
-struct Lay1 { unsigned ctl, red, va, vb, ri, q_nx, q_in, s_nx, s_in, c_nx, c_in, st_r, st_gc, st_uc, st_gs, st_us, total; };
+struct Lay1 { unsigned ctl, red, va, vb, ri, q_nx, s_nx, c_nx, st_r, st_gc, st_uc, st_gs, st_us, total; };
 __host__ __device__ inline Lay1 lay1(const SpDims &d, int G) {
     Lay1 L; unsigned o = 0;
     auto take = [&](unsigned bytes) { const unsigned at = o; o = up16(o + bytes); return at; };
     const unsigned E = d.E, nb = E / 16, nr = cdiv(d.NE, G), np = cdiv(d.FFS, G), rb = E / 2, sb = E / 16;
     L.ctl = take(sizeof(Ctl)); L.red = take(128 * 8);
     L.va = take(4 * E); L.vb = take(4 * E); L.ri = take(4 * E);
-    L.q_nx = take(E); L.q_in = take(E);
-    L.s_nx = take(4 * nb); L.s_in = take(4 * nb); L.c_nx = take(4 * nb); L.c_in = take(4 * nb);
+    L.q_nx = take(E); L.s_nx = take(4 * nb); L.c_nx = take(4 * nb);
     o = (o + 127u) & ~127u;
     L.st_r = take(nr * 4 * E); L.st_gc = take(np * rb); L.st_uc = take(np * rb);
     L.st_gs = take(np * sb + 32); L.st_us = take(np * sb + 32);
     L.total = o;
     return L;
 }
-struct Lay2 { unsigned ctl, red, ex, lg, p, dsc, wmax, q_in, s_in, c_in, q_hd, s_hd, c_hd, st_sd, st_sds, st_gc, st_uc, st_gs, st_us, part, total; };
+struct Lay2 { unsigned ctl, red, ex, lg, p, dsc, wmax, q_in, s_in, q_hd, s_hd, c_hd, st_sd, st_sds, st_gc, st_uc, st_gs, st_us, part, total; };
 __host__ __device__ inline Lay2 lay2(const SpDims &d, int G) {
     Lay2 L; unsigned o = 0;
     auto take = [&](unsigned bytes) { const unsigned at = o; o = up16(o + bytes); return at; };
     const unsigned E = d.E, NE = d.NE, FFS = d.FFS, nj = cdiv(d.E, G), nP = cdiv(d.NU * d.FFE, G);
     L.ctl = take(sizeof(Ctl)); L.red = take(128 * 8); L.ex = take(8 * NE);
     L.lg = take(4 * NE); L.p = take(4 * (NE < 128 ? 128 : NE)); L.dsc = take(4 * NE); L.wmax = take(4 * 32);
-    L.q_in = take(E); L.s_in = take(4 * (E / 16)); L.c_in = take(4 * (E / 16));
+    L.q_in = take(E); L.s_in = take(4 * (E / 16));
     L.q_hd = take(FFS); L.s_hd = take(4 * (FFS / 16)); L.c_hd = take(4 * (FFS / 16));
     o = (o + 127u) & ~127u;
     L.st_sd = take(nj * (FFS / 2)); L.st_sds = take(nj * (FFS / 16) + 32);
@@ -290,14 +289,14 @@ template <int KE, int NIT>
 __global__ void __launch_bounds__(kT, 1) k_ds_router_shared(SArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
     const SpDims d = a.d;
-    const int E = d.E, t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x;
+    const int E = d.E, t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x, b = blockIdx.x;
     const Lay1 &ly = *reinterpret_cast<const Lay1 *>(a.lay);
     Ctl *ctl = reinterpret_cast<Ctl *>(sm + ly.ctl);
     double *red = reinterpret_cast<double *>(sm + ly.red);
     float *va = reinterpret_cast<float *>(sm + ly.va), *vb = reinterpret_cast<float *>(sm + ly.vb), *ri = reinterpret_cast<float *>(sm + ly.ri);
-    signed char *q_nx = reinterpret_cast<signed char *>(sm + ly.q_nx), *q_in = reinterpret_cast<signed char *>(sm + ly.q_in);
-    float *s_nx = reinterpret_cast<float *>(sm + ly.s_nx), *s_in = reinterpret_cast<float *>(sm + ly.s_in);
-    int *c_nx = reinterpret_cast<int *>(sm + ly.c_nx), *c_in = reinterpret_cast<int *>(sm + ly.c_in);
+    signed char *q_nx = reinterpret_cast<signed char *>(sm + ly.q_nx);
+    float *s_nx = reinterpret_cast<float *>(sm + ly.s_nx);
+    int *c_nx = reinterpret_cast<int *>(sm + ly.c_nx);
     const SpLayerDev &L = a.L;
     /* this CTA's share of every phase, from the table the host built (no division in the kernel) */
     const int4 sl0 = __ldg(reinterpret_cast<const int4 *>(a.s.slices) + 3 * b), sl1 = __ldg(reinterpret_cast<const int4 *>(a.s.slices) + 3 * b + 1);
@@ -391,22 +390,24 @@ __global__ void __launch_bounds__(kT, 1) k_ds_router_shared(SArgs a) {
         }
     }
     __syncthreads();
+    /* the shared expert's input by every CTA for itself; the routed experts' input, which only the next kernel reads, block by block by
+     * one CTA each (all of it by every CTA, and by the first one to global memory: 30 layers 621.5 us, so 615.6) */
     const int nb = E >> 4;
 #pragma unroll 1
-    for (int bq = t; bq < 2 * nb; bq += kT) {
-        const bool first = bq < nb; const int bb = first ? bq : bq - nb;
-        const float *src = first ? va : vb;
+    for (int bq = t;; bq += kT) {
+        const bool nx = bq < nb; const int bb = nx ? bq : b + G * (bq - nb);
+        if (bb >= nb) break;
+        const float *src = nx ? va : vb;
         float v[16];
 #pragma unroll
         for (int i = 0; i < 4; i++) { const float4 f = reinterpret_cast<const float4 *>(src + 16 * bb)[i]; v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w; }
-        quant_block16_store(v, reinterpret_cast<int4 *>(first ? q_nx : q_in) + bb, (first ? s_nx : s_in) + bb, (first ? c_nx : c_in) + bb);
+        int4 w; float sx; int corr;
+        quant_block16_store(v, &w, &sx, &corr);
+        if (nx) { reinterpret_cast<int4 *>(q_nx)[bb] = w; s_nx[bb] = sx; c_nx[bb] = corr; }
+        else { reinterpret_cast<int4 *>(a.s.in_q)[bb] = w; a.s.in_s[bb] = sx; }
     }
     __syncthreads();
     STAMP(0, 6);
-    if (b == 0) {                                        /* the routed experts' input, for K2 */
-#pragma unroll 1
-        for (int i = t; i < nb; i += kT) { reinterpret_cast<int4 *>(a.s.in_q)[i] = reinterpret_cast<const int4 *>(q_in)[i]; a.s.in_s[i] = s_in[i]; a.s.in_c[i] = c_in[i]; }
-    }
     STAMP(0, 3);
     if (a.flags & SP_STAGED_PREFETCH_SD) {               /* the next kernel's routing-independent rows: ask L2 for them now */
         const int j0 = sl1.x, nj = sl1.y;
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
     float *wmax = reinterpret_cast<float *>(sm + ly.wmax);
     signed char *q_in = reinterpret_cast<signed char *>(sm + ly.q_in), *q_hd = reinterpret_cast<signed char *>(sm + ly.q_hd);
     float *s_in = reinterpret_cast<float *>(sm + ly.s_in), *s_hd = reinterpret_cast<float *>(sm + ly.s_hd);
-    int *c_in = reinterpret_cast<int *>(sm + ly.c_in), *c_hd = reinterpret_cast<int *>(sm + ly.c_hd);
+    int *c_hd = reinterpret_cast<int *>(sm + ly.c_hd);
     const SpLayerDev &L = a.L;
     const int4 sl1 = __ldg(reinterpret_cast<const int4 *>(a.s.slices) + 3 * b + 1), sl2 = __ldg(reinterpret_cast<const int4 *>(a.s.slices) + 3 * b + 2);
     const int j0 = sl1.x, nj = sl1.y, P0 = sl1.z, nP = sl1.w;
@@ -776,7 +777,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
         /* ---- the routed experts' input (for the pairs below), the shared expert's hidden vector, its down rows */
         const int ts = t - TR, ws = warp - kRW;
 #pragma unroll 1
-        for (int i = ts; i < E / 16; i += TS) { reinterpret_cast<int4 *>(q_in)[i] = __ldcg(reinterpret_cast<const int4 *>(a.s.in_q) + i); s_in[i] = __ldcg(a.s.in_s + i); c_in[i] = __ldcg(a.s.in_c + i); }
+        for (int i = ts; i < E / 16; i += TS) { reinterpret_cast<int4 *>(q_in)[i] = __ldcg(reinterpret_cast<const int4 *>(a.s.in_q) + i); s_in[i] = __ldcg(a.s.in_s + i); }
 #pragma unroll 1
         for (int bq = ts; bq < (FFS >> 4); bq += TS) quant_from_global(a.s.hd + 16 * bq, reinterpret_cast<int4 *>(q_hd) + bq, s_hd + bq, c_hd + bq);
         bar_named(2, TS);
