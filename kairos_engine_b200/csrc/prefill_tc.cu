@@ -221,25 +221,30 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
             const int j = t.mt * 2 * BLK + blk * BLK + (PAIR ? quad * 16 + (lane & 15) : quad * 32 + lane);
             const bool upper = lane >= 16, b2 = (lane & 4) != 0;
             /* pair: lane and lane ^ 4 hold k = j and j + 4, neighbours in the stored order: the lower one stores both hi, the upper both lo */
-            __half *pp = PAIR ? (b2 ? s.out_lo : s.out_hi) + kperm(j & ~4) : nullptr;
+            __half *pp = PAIR ? (b2 ? s.out_lo : s.out_hi) + kperm(j & ~4) + (size_t)(t.row0 + (upper ? 1 : 0)) * s.rows : nullptr;
 #pragma unroll 1
             for (int c0 = 0; c0 < t.nv; c0 += 32) {
                 int rm = t.row0 + c0 + lane;
                 if (!PAIR && s.rowmap) rm = c0 + lane < t.nv ? __ldcg(s.rowmap + rm) : 0;
 #pragma unroll
-                for (int n = 0; n < 32; n += 2) {
+                for (int n = 0; n < 32; n += PAIR ? 4 : 2) {
                     if (c0 + n >= t.nv) break;                          /* warp-uniform */
                     if (PAIR) {
-                        /* lanes 0-15 hold gate rows, 16-31 the up rows of the same outputs: the lower half finishes column n, the upper n + 1 */
-                        const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? v[n] : v[n + 1], 16);
-                        const float g = __uint_as_float(upper ? got : v[n]), u = __uint_as_float(upper ? v[n + 1] : got);
-                        const float h = gelu_mul(g, u);
-                        const __half x = __float2half_rn(h), y = __float2half_rn(__fsub_rn(h, __half2float(x)));
-                        const uint32_t hx = __half_as_ushort(x), hy = __half_as_ushort(y);
-                        const uint32_t other = __shfl_xor_sync(0xffffffffu, b2 ? hx : hy, 4);
-                        const uint32_t word = b2 ? (other | (hy << 16)) : (hx | (other << 16));
+                        /* lanes 0-15 hold gate rows, 16-31 the up rows of the same outputs: the lower half finishes columns n and n + 2, the upper n + 1, n + 3 */
+                        /* Issue-bound: four columns at a time, so that one exchange carries the hi and lo halves of two of them and the conversions
+                         * are packed. 30 layers: 37 tokens 5650 -> 5530 us, 4096 tokens 55.7 -> 54.8 ms, 717 tokens the same. */
+                        const uint32_t ga = __shfl_xor_sync(0xffffffffu, upper ? v[n] : v[n + 1], 16), gb = __shfl_xor_sync(0xffffffffu, upper ? v[n + 2] : v[n + 3], 16);
+                        const float2 h = make_float2(gelu_mul(__uint_as_float(upper ? ga : v[n]), __uint_as_float(upper ? v[n + 1] : ga)),
+                                                     gelu_mul(__uint_as_float(upper ? gb : v[n + 2]), __uint_as_float(upper ? v[n + 3] : gb)));
+                        const __half2 x = __floats2half2_rn(h.x, h.y);
+                        const float2 xf = __half22float2(x);
+                        const __half2 y = __floats2half2_rn(__fsub_rn(h.x, xf.x), __fsub_rn(h.y, xf.y));
+                        const uint32_t hx = *reinterpret_cast<const uint32_t *>(&x), hy = *reinterpret_cast<const uint32_t *>(&y);
+                        const uint32_t other = __shfl_xor_sync(0xffffffffu, b2 ? hx : hy, 4), a0 = b2 ? other : hx, a1 = b2 ? hy : other;
                         const int nn = c0 + n + (upper ? 1 : 0);
-                        if (nn < t.nv) *reinterpret_cast<uint32_t *>(pp + (size_t)(t.row0 + nn) * s.rows) = word;
+                        if (nn < t.nv) *reinterpret_cast<uint32_t *>(pp) = __byte_perm(a0, a1, 0x5410);
+                        if (nn + 2 < t.nv) *reinterpret_cast<uint32_t *>(pp + 2 * (size_t)s.rows) = __byte_perm(a0, a1, 0x7632);
+                        pp += 4 * (size_t)s.rows;
                     } else {
 #pragma unroll
                         for (int k = 0; k < 2; k++) {
