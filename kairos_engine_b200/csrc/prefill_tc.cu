@@ -50,7 +50,7 @@ namespace {
 using namespace sp_tc;
 
 constexpr int kBK = 64, kNGran = 16, kBoxBig = 64;
-constexpr int kEpiWarps = 8, kItems = 64;
+constexpr int kEpiWarps = 8, kItems = 8;                                /* items: the ring in which a CTA announces its next tiles */
 constexpr uint32_t kBoxRows = 64, kBoxBytes = 128 * kBoxRows;          /* codes: 128 B (256 weights) of 64 rows */
 constexpr uint32_t kChunkBytes = 4 * kBoxBytes;                        /* the four boxes of a tile: 32 KB per 256 k */
 /* 512 TMEM columns: 2 blocks x kAccBufs x NMAX of accumulators from column 0, then a ring of three stages of unpacked
@@ -62,9 +62,9 @@ template <int NMAX> struct Cfg {
     static constexpr int kAccBufs = NMAX == 32 ? 2 : 1, kACol = 2 * NMAX * kAccBufs, kAStages = 3, kACols = 2 * kBK;
     static constexpr int kBStages = 4, kCStages = 4;
     static constexpr uint32_t kBHalf = NMAX * 128u, kBStage = 2 * kBHalf;
-    static constexpr uint32_t kCOff = kBStages * kBStage, kBarOff = kCOff + kCStages * kChunkBytes, kItemOff = kBarOff + 320;
+    static constexpr uint32_t kCOff = kBStages * kBStage, kBarOff = kCOff + kCStages * kChunkBytes, kItemOff = kBarOff + 448;
     static constexpr uint32_t kScaleOff = kItemOff + 32 * kItems, kSmem = kScaleOff + 3 * 16 * 32 * kUnpWarps + 1024;     /* + alignment slack */
-    static constexpr int kLaunchRegs = 72, kEpiRegs = 104, kUnpRegs = 64, kMiscRegs = 32;
+    static constexpr int kLaunchRegs = 72, kEpiRegs = 96, kUnpRegs = 64, kMiscRegs = 48;
     static_assert(32 * (kEpiWarps * kEpiRegs + kUnpWarps * kUnpRegs + 4 * kMiscRegs) <= kThreads * kLaunchRegs, "register split exceeds what the block is launched with");
     static_assert(kACol + kACols * kAStages <= 512, "tensor memory");
 };
@@ -80,7 +80,7 @@ struct TcSeg {                     /* one GEMM of a launch: the shared expert's 
     __half *out_hi, *out_lo;       /* pair: geglu output rows of `rows` columns, split + permuted */
     float *out_f; int out_stride; const int *rowmap;  /* plain: out_f[(rowmap ? rowmap[r] : r) * stride + j] */
 };
-struct TcArgs { TcSeg seg[2]; int nseg; int K[2]; int *status; };
+struct TcArgs { TcSeg seg[2]; int nseg; int K[2]; int *ticket; int *status; };       /* ticket: tiles handed out beyond the first of each CTA; zero at launch */
 struct TcMaps { CUtensorMap codes[2][2], hi[2], lo[2], hi64[2], lo64[2]; };   /* [segment][gate / up]; activation boxes of 16 and of 64 rows */
 
 constexpr uint32_t kNegateA = 1u << 13;                                /* instruction descriptor: A enters with its sign flipped */
@@ -129,7 +129,7 @@ __device__ __forceinline__ void unpack_block(const int4 &w, unsigned short scale
 
 /* TERMS: 3 = all of w_hi*x_hi + w_lo*x_hi + w_hi*x_lo (exact to 2^-22); 2 = the weight rounded to fp16
  * (w_hi*x_hi + w_hi*x_lo); 1 = fp16 x fp16, the reference's SP_G4_GEMM_F16 mode (CF:13350-13365). */
-struct __align__(16) Item { int sg, mt, grp, row0, nv, n16, nblk, KB; };      /* rows [row0, row0 + nv) of group grp x weight tile mt */
+struct __align__(16) Item { int sg, mt, grp, row0, nv, n16, nblk, KB; };      /* rows [row0, row0 + nv) of group grp x weight tile mt; KB 0: no more */
 
 template <bool PAIR, int TERMS, int NMAX>
 __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid_constant__ TcArgs a, const __grid_constant__ TcMaps maps) {
@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
     auto tempty = [&](int b, int blk) { return bar0 + 256u + 8u * (2 * b + blk); };
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + C::kBarOff + 288);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::kBarOff + 292);
+    auto ifull = [&](int i) { return bar0 + 320u + 8u * (i % kItems); };                  /* items announced, and read by every other warp */
+    auto iempty = [&](int i) { return bar0 + 384u + 8u * (i % kItems); };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kBStages; s++) { mbar_init(bfull(s), 1); mbar_init(bempty(s), 2); }
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
             for (int s = 0; s < C::kAStages; s++) { mbar_init(afull(s, blk), 4); mbar_init(aempty(s, blk), 1); }
             for (int b = 0; b < 2; b++) { mbar_init(tfull(b, blk), 1); mbar_init(tempty(b, blk), kEpiWarps / 2); }
         }
+        for (int i = 0; i < kItems; i++) { mbar_init(ifull(i), 1); mbar_init(iempty(i), C::kWarps - 1); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -175,35 +178,22 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
     sp_pdl_wait();
     sp_pdl_next();
 
-    const int total0 = *a.seg[0].n_tiles * a.seg[0].m_tiles;
-    const int total = total0 + (a.nseg > 1 ? *a.seg[1].n_tiles * a.seg[1].m_tiles : 0);
-    /* work item -> segment, activation tile, weight tile (the weight tiles of one activation tile are neighbours). The
-     * first kItems of a CTA are worked out once, in parallel, and kept in shared memory: every role reads each of them */
-    auto item_at = [&](int w) {
-        Item t;
-        t.sg = w >= total0 ? 1 : 0;
-        const TcSeg &s = a.seg[t.sg];
-        const int r = w - (t.sg ? total0 : 0), nt = r / s.m_tiles;
-        t.mt = r - nt * s.m_tiles;
-        t.grp = __ldcg(s.tiles + 3 * nt); t.row0 = __ldcg(s.tiles + 3 * nt + 1); t.nv = __ldcg(s.tiles + 3 * nt + 2);
-        t.n16 = (t.nv + kNGran - 1) & ~(kNGran - 1);
-        t.nblk = s.rows - t.mt * 2 * BLK > BLK ? 2 : 1;
-        t.KB = a.K[t.sg] / kBK;
-        return t;
-    };
     Item *items = reinterpret_cast<Item *>(smem + C::kItemOff);
-    for (int i = threadIdx.x; i < kItems && (int)blockIdx.x + i * (int)gridDim.x < total; i += C::kThreads) items[i] = item_at(blockIdx.x + i * gridDim.x);
-    __syncthreads();
-    auto item = [&](int w, int i) { return i < kItems ? items[i] : item_at(w); };
     bool failed = false;
+    /* the CTA's i-th tile, for every warp but the one that announces it */
+    auto announced = [&](int i) { return mbar_wait(ifull(i), (uint32_t)(i / kItems) & 1u, abort_flag); };
+    auto read = [&](int i) { __syncwarp(); mbar_arrive_lane0(iempty(i), lane); };
 
     if (warp < kEpiWarps) {
         /* ---------------- epilogue: TMEM -> registers, the accumulators are free again, then -> global */
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
         const int quad = warp & 3, blk = warp >> 2;
         int lt = 0;
-        for (int w = blockIdx.x, i = 0; w < total; w += gridDim.x, i++) {
-            const Item t = item(w, i);
+        for (int i = 0;; i++) {
+            if (!announced(i)) { failed = true; break; }
+            const Item t = items[i % kItems];
+            read(i);
+            if (t.KB == 0) break;
             if (blk >= t.nblk) continue;
             const TcSeg &s = a.seg[t.sg];
             const int b = lt % C::kAccBufs; const uint32_t ph = (lt / C::kAccBufs) & 1;
@@ -273,19 +263,22 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
          * place of its own. */
         const uint32_t slot0 = smem_u32(smem) + C::kScaleOff + 16u * (threadIdx.x - 32 * kEpiWarps);
         constexpr uint32_t kSlot = 16u * 32u * C::kUnpWarps;
-        int pw = blockIdx.x, pi = 0, pk = 0, pKB = 0; uint32_t pslot = 0, uslot = 0;     /* next chunk to fetch: item, first 64-k step; slots of a ring of three */
+        int pi = 0, pk = 0, pKB = 0; uint32_t pslot = 0, uslot = 0;     /* next chunk to fetch: item, first 64-k step; slots of a ring of three */
         const uint32_t *sp = nullptr;
         auto fetch = [&]() {
-            if (pw < total) {
-                if (pk == 0) {
-                    const Item t = item(pw, pi);
+            if (pk == 0 && pKB >= 0) {
+                const Item &t = items[pi % kItems];
+                pKB = announced(pi) ? t.KB : 0;
+                if (pKB == 0) pKB = -1;                                 /* no more */
+                else {
                     const TcSeg &s = a.seg[t.sg];
                     int jj = t.mt * 2 * BLK + blk * BLK + rb;
                     if (jj > s.rows - 1) jj = s.rows - 1;
                     const size_t row = (size_t)((long long)t.grp * s.group_rows) + (size_t)(half ? s.up_off : 0) + (size_t)jj;
                     sp = reinterpret_cast<const uint32_t *>(s.bs[half] + row * (size_t)(2 * t.KB));
-                    pKB = t.KB;
                 }
+            }
+            if (pKB > 0) {
                 const uint32_t dst = slot0 + pslot * kSlot;
                 if ((pKB & 3) == 0) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(sp + pk) : "memory");      /* K a multiple of 256: rows of 16 bytes */
                 else {
@@ -294,16 +287,18 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                         if (pk + k < pKB) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * k), "l"(sp + pk + k) : "memory");
                 }
                 pk += 4;
-                if (pk >= pKB) { pk = 0; pw += gridDim.x; pi++; }
+                if (pk >= pKB) { pk = 0; pi++; }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
             pslot = pslot == 2 ? 0 : pslot + 1;
         };
         fetch(); fetch();
-        for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
-            const Item t = item(w, iw);
-            const int nst = blk < t.nblk ? t.KB : 0;
-            for (int c0 = 0; c0 < t.KB; c0 += 4) {
+        for (int iw = 0; !failed; iw++) {
+            if (!announced(iw)) { failed = true; break; }
+            const int KB = items[iw % kItems].KB, nst = blk < items[iw % kItems].nblk ? KB : 0;
+            read(iw);
+            if (KB == 0) break;
+            for (int c0 = 0; c0 < KB; c0 += 4) {
                 fetch();
                 asm volatile("cp.async.wait_group 2;" ::: "memory");
                 const uint32_t sc = slot0 + uslot * kSlot;
@@ -344,17 +339,20 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
             const bool leader = elect_one();
             const int blk = warp - kMma;
             uint32_t as = 0, aph = 0, bs = 0, bp = 0; int lt = 0;
-            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
-                const Item t = item(w, iw);
-                const bool mine = blk < t.nblk;
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(t.n16 >> 3) << 17) | ((128u >> 4) << 24);   /* f16 x f16 -> f32, K-major B, M = 128, N = n16 */
+            for (int iw = 0; !failed; iw++) {
+                if (!announced(iw)) { failed = true; break; }
+                const int KB = items[iw % kItems].KB, n16 = items[iw % kItems].n16;
+                const bool mine = blk < items[iw % kItems].nblk;
+                read(iw);
+                if (KB == 0) break;
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(n16 >> 3) << 17) | ((128u >> 4) << 24);   /* f16 x f16 -> f32, K-major B, M = 128, N = n16 */
                 const int b = lt % C::kAccBufs; const uint32_t bph = (lt / C::kAccBufs) & 1;
                 if (mine) {
                     lt++;
                     if (!mbar_wait(tempty(b, blk), bph ^ 1, abort_flag)) { failed = true; break; }
                 }
                 const uint32_t d = tmem + (uint32_t)((2 * b + blk) * NMAX);
-                for (int kb = 0; kb < t.KB; kb++) {
+                for (int kb = 0; kb < KB; kb++) {
                     if (!mbar_wait(bfull(bs), bp, abort_flag)) { failed = true; break; }
                     if (mine) {
                         const uint64_t x0 = make_desc(sbase + bs * C::kBStage);
@@ -371,7 +369,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                             }
                             umma_commit(aempty(as, blk));               /* both stages are free once these MMAs have read them */
                             umma_commit(bempty(bs));
-                            if (kb + 1 == t.KB) umma_commit(tfull(b, blk));
+                            if (kb + 1 == KB) umma_commit(tfull(b, blk));
                         }
                         __syncwarp();
                         if (++as == C::kAStages) { as = 0; aph ^= 1; }
@@ -383,19 +381,24 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
             /* ---------------- activation rows by TMA, 64 or 16 rows a copy. (Four gathered rows a copy, tile::gather4 from one
              * row per token, would save the sorted copy of the rows, but such copies are too slow: 1640 against 870 us for the
              * gate|up launch of 4096 tokens.) */
-            if (lane == 0) {
+            if (lane == 0) {                                            /* one lane walks the loop: with the warp in step this chain paces the CTA (30 layers of 24 tokens: +7%) */
                 uint32_t bs = 0, bp = 0;
-                for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
-                    const Item t = item(w, iw);
-                    for (int kb = 0; kb < t.KB; kb++) {
+                for (int iw = 0; !failed; iw++) {
+                    if (!announced(iw)) { failed = true; break; }
+                    const int KB = items[iw % kItems].KB, n16 = items[iw % kItems].n16, sg = items[iw % kItems].sg, row0 = items[iw % kItems].row0;
+                    mbar_arrive(iempty(iw));
+                    if (KB == 0) break;
+                    /* box and map are chosen once a tile: chosen at every copy, 30 layers of 400 / 4096 tokens took 9.73 / 54.1 ms instead of 9.34 / 53.7 */
+                    const bool big = NMAX >= kBoxBig && n16 == kBoxBig;
+                    const int step = big ? kBoxBig : kNGran;
+                    const CUtensorMap *mh = big ? &maps.hi64[sg] : &maps.hi[sg], *ml = big ? &maps.lo64[sg] : &maps.lo[sg];
+                    for (int kb = 0; kb < KB; kb++) {
                         if (!mbar_wait(bempty(bs), bp ^ 1, abort_flag)) { failed = true; break; }
                         const uint32_t dst = sbase + bs * C::kBStage, bar = bfull(bs);
-                        mbar_expect_tx(bar, (uint32_t)t.n16 * (TERMS >= 2 ? 256u : 128u));
-                        for (int i = 0; i < t.n16;) {
-                            const bool big = t.n16 - i >= kBoxBig;
-                            tma_load_2d(dst + 128u * i, big ? &maps.hi64[t.sg] : &maps.hi[t.sg], kb * kBK, t.row0 + i, bar);
-                            if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, big ? &maps.lo64[t.sg] : &maps.lo[t.sg], kb * kBK, t.row0 + i, bar);
-                            i += big ? kBoxBig : kNGran;
+                        mbar_expect_tx(bar, (uint32_t)n16 * (TERMS >= 2 ? 256u : 128u));
+                        for (int i = 0; i < n16; i += step) {
+                            tma_load_2d(dst + 128u * i, mh, kb * kBK, row0 + i, bar);
+                            if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, ml, kb * kBK, row0 + i, bar);
                         }
                         if (++bs == C::kBStages) { bs = 0; bp ^= 1; }
                     }
@@ -403,11 +406,34 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
             }
             if (failed || *abort_flag) __nanosleep(100000);             /* let copies in flight land before the CTA leaves */
         } else if (warp == kCodes && lane == 0) {
-            /* ---------------- packed codes by TMA, 256 k a copy */
+            /* ---------------- the tiles, and their packed codes by TMA, 256 k a copy. A CTA's first tile is its own number; each
+             * next one is drawn from a counter when the codes of the one before are on their way, some 16 stages before it is due.
+             * Tiles differ: the shared expert's K is three times the routed experts' in the down GEMM, the last tile of a group's
+             * rows may hold one block, and a CTA draws four to ten tiles in all when there are few rows. Dealt out in turn
+             * (CTA c: c, c + 148, ...), the CTAs with a long tile got as many others as the rest: 30 layers of 24 / 37 / 400 tokens
+             * 5480 / 5863 / 10149 us so, against 4866 / 5561 / 9913 drawn, all else the same. The order stays: shared expert first,
+             * so the long tiles are out early. */
+            const int total0 = *a.seg[0].n_tiles * a.seg[0].m_tiles;
+            const int total = total0 + (a.nseg > 1 ? *a.seg[1].n_tiles * a.seg[1].m_tiles : 0);
             uint32_t cc = 0;
-            for (int w = blockIdx.x, iw = 0; w < total && !failed; w += gridDim.x, iw++) {
-                const Item t = item(w, iw);
+            for (int w = blockIdx.x, i = 0; !failed; w = (int)gridDim.x + atomicAdd(a.ticket, 1), i++) {
+                if (!mbar_wait(iempty(i), ((uint32_t)(i / kItems) & 1u) ^ 1u, abort_flag)) { failed = true; break; }
+                /* work item -> segment, activation tile, weight tile (the weight tiles of one activation tile are neighbours) */
+                Item t;
+                t.sg = w >= total0 ? 1 : 0;
                 const TcSeg &s = a.seg[t.sg];
+                t.KB = 0;
+                if (w < total) {
+                    const int r = w - (t.sg ? total0 : 0), nt = r / s.m_tiles;
+                    t.mt = r - nt * s.m_tiles;
+                    t.grp = __ldcg(s.tiles + 3 * nt); t.row0 = __ldcg(s.tiles + 3 * nt + 1); t.nv = __ldcg(s.tiles + 3 * nt + 2);
+                    t.n16 = (t.nv + kNGran - 1) & ~(kNGran - 1);
+                    t.nblk = s.rows - t.mt * 2 * BLK > BLK ? 2 : 1;
+                    t.KB = a.K[t.sg] / kBK;
+                }
+                items[i % kItems] = t;
+                mbar_arrive(ifull(i));
+                if (t.KB == 0) break;
                 const int y0 = (int)((long long)t.grp * s.group_rows) + t.mt * 2 * BLK;
                 for (int kc = 0; kc < t.KB; kc += 4, cc++) {
                     const uint32_t cs = cc % C::kCStages, cp = (cc / C::kCStages) & 1;
@@ -491,7 +517,7 @@ __device__ __forceinline__ void write_tiles(int first, int cnt, int nmax, int *t
         const int left = cnt - i * per;
         tiles[3 * n] = (int)threadIdx.x; tiles[3 * n + 1] = first + i * per; tiles[3 * n + 2] = left < per ? left : per;
     }
-    if (threadIdx.x == 1023) *n_tiles = end < cap ? end : cap;
+    if (threadIdx.x == 1023) { *n_tiles = end < cap ? end : cap; n_tiles[1] = n_tiles[2] = 0; }
 }
 __global__ void __launch_bounds__(1024) k_tc_plan(const int *offsets, int groups, int fixed_rows, int max_rows, int nmax, int *tiles, int *n_tiles, int cap) {
     __shared__ int sh[32];
@@ -608,7 +634,7 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     size_t o = 0; auto take = [&](size_t b) { size_t at = o; o = up256(o + b); return at; };
     const size_t E = d.E, FFE = d.FFE, FFS = d.FFS, Mc = p->Mcap, Rc = p->Rcap;
     const size_t o_nx = take(4 * Mc * E), o_hd = take(4 * Mc * FFS), o_in = take(4 * Rc * E), o_h = take(4 * Rc * FFE), o_tk = take(4 * Mc * E);      /* hi rows, then lo rows */
-    const size_t o_tsh = take(12 * (size_t)p->cap_sh), o_nsh = take(4), o_tr = take(12 * (size_t)p->cap_r), o_nr = take(4);
+    const size_t o_tsh = take(12 * (size_t)p->cap_sh), o_nsh = take(12), o_tr = take(12 * (size_t)p->cap_r), o_nr = take(12);
     const size_t o_g = take(4 * Rc), o_rm = take(4 * Rc);
     p->bytes = o;
     e = cudaMalloc((void **)&p->base, o);
@@ -681,7 +707,8 @@ struct Launch {
         TcSeg &s = seg(d.FFE, p->h, L.dn_codes, L.dn_bs, L.dn_codes, L.dn_bs, (size_t)d.NE * d.E, d.E, (d.E + 255) / 256);
         s.group_rows = d.E; s.tiles = p->tiles_r; s.n_tiles = p->ntiles_r; s.out_f = out; s.out_stride = d.E; s.rowmap = rowmap;
     }
-    cudaError_t go(bool pair, int nmax, cudaStream_t st, int *nl) {
+    cudaError_t go(bool pair, int nmax, int *n_tiles, cudaStream_t st, int *nl) {      /* n_tiles: behind the count, the tickets of gate|up and of down */
+        a.ticket = n_tiles + (pair ? 1 : 2);
         if (err != cudaSuccess) return err;
         for (int i = a.nseg; i < 2; i++) { maps.hi[i] = maps.hi64[i] = maps.hi[0]; maps.lo[i] = maps.lo64[i] = maps.lo[0]; maps.codes[i][0] = maps.codes[i][1] = maps.codes[0][0]; a.K[i] = a.K[0]; }
         if (pair) return nmax == 64 ? launch_n<true, 64>(p, a, maps, st, nl) : launch_n<true, 32>(p, a, maps, st, nl);
@@ -702,11 +729,11 @@ cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M
     if (e != cudaSuccess) return e;
     Launch up(p, d, L, status);
     up.shared_up(); up.routed_up();
-    e = up.go(true, nmax, st, nl);
+    e = up.go(true, nmax, p->ntiles_r, st, nl);
     if (e != cudaSuccess) return e;
     Launch down(p, d, L, status);
     down.shared_down(dn); down.routed_down(eo, p->rowmap);
-    return down.go(false, nmax, st, nl);
+    return down.go(false, nmax, p->ntiles_r, st, nl);
 }
 
 cudaError_t sp_tc_shared_expert(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M, const float *nx, float *dn,
@@ -719,12 +746,12 @@ cudaError_t sp_tc_shared_expert(SpTcPlan *p, const SpDims &d, const SpLayerDev &
         k_tc_plan<<<1, 1024, 0, st>>>(nullptr, 1, M, M, nmax, p->tiles_sh, p->ntiles_sh, p->cap_sh); (*nl)++;
         Launch up(p, d, L, status);
         up.shared_up();
-        e = up.go(true, nmax, st, nl);
+        e = up.go(true, nmax, p->ntiles_sh, st, nl);
     }
     if (phase != 1 && e == cudaSuccess) {                 /* down: hd -> dn (the tile table of the first phase is still in place) */
         Launch down(p, d, L, status);
         down.shared_down(dn);
-        e = down.go(false, nmax, st, nl);
+        e = down.go(false, nmax, p->ntiles_sh, st, nl);
     }
     return e;
 }
@@ -738,9 +765,9 @@ cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int 
     k_tc_plan<<<1, 1024, 0, st>>>(offsets, d.NE, 0, R, nmax, p->tiles_r, p->ntiles_r, p->cap_r); (*nl)++;
     Launch up(p, d, L, status);
     up.routed_up();
-    cudaError_t e = up.go(true, nmax, st, nl);
+    cudaError_t e = up.go(true, nmax, p->ntiles_r, st, nl);
     if (e != cudaSuccess) return e;
     Launch down(p, d, L, status);
     down.routed_down(out, rowmap);
-    return down.go(false, nmax, st, nl);
+    return down.go(false, nmax, p->ntiles_r, st, nl);
 }
