@@ -49,7 +49,7 @@
 namespace {
 using namespace sp_tc;
 
-constexpr int kBK = 64, kNGran = 16, kBoxBig = 64;
+constexpr int kBK = 64, kNGran = 16, kNMax = 64;
 constexpr int kEpiWarps = 8, kItems = 8;                                /* items: the ring in which a CTA announces its next tiles */
 constexpr uint32_t kBoxRows = 64, kBoxBytes = 128 * kBoxRows;          /* codes: 128 B (256 weights) of 64 rows */
 constexpr uint32_t kChunkBytes = 4 * kBoxBytes;                        /* the four boxes of a tile: 32 KB per 256 k */
@@ -81,7 +81,7 @@ struct TcSeg {                     /* one GEMM of a launch: the shared expert's 
     float *out_f; int out_stride; const int *rowmap;  /* plain: out_f[(rowmap ? rowmap[r] : r) * stride + j] */
 };
 struct TcArgs { TcSeg seg[2]; int nseg; int K[2]; int *ticket; int *status; };       /* ticket: tiles handed out beyond the first of each CTA; zero at launch */
-struct TcMaps { CUtensorMap codes[2][2], hi[2], lo[2], hi64[2], lo64[2]; };   /* [segment][gate / up]; activation boxes of 16 and of 64 rows */
+struct TcMaps { CUtensorMap codes[2][2], act[2][kNMax / kNGran]; };    /* [segment][gate / up]; activation boxes of 16, 32, 48 and 64 rows, hi and lo */
 
 constexpr uint32_t kNegateA = 1u << 13;                                /* instruction descriptor: A enters with its sign flipped */
 
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                             const uint32_t wa = tmem + C::kACol + C::kACols * as + kBK * blk;
 #pragma unroll
                             for (int ks = 0; ks < kBK / 16; ks++) {
-                                const uint64_t xhi = x0 + 2u * ks, xlo = xhi + (C::kBHalf >> 4);       /* 32 bytes along k; the lo rows */
+                                const uint64_t xhi = x0 + 2u * ks, xlo = xhi + 8u * (uint32_t)n16;       /* 32 bytes along k; the lo rows behind the hi rows */
                                 if (ks == 0) umma_f16_ts(d, wa, xhi, idesc, kb ? 1u : 0u); else umma_f16_ts(d, wa + 8u * ks, xhi, idesc);
                                 if (TERMS >= 3) umma_f16_ts(d, wa + kBK / 2 + 8u * ks, xhi, idesc | kNegateA);
                                 if (TERMS >= 2) umma_f16_ts(d, wa + 8u * ks, xlo, idesc);
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                 }
             }
         } else if (warp == kActs) {
-            /* ---------------- activation rows by TMA, 64 or 16 rows a copy. (Four gathered rows a copy, tile::gather4 from one
+            /* ---------------- activation rows by TMA. (Four gathered rows a copy, tile::gather4 from one
              * row per token, would save the sorted copy of the rows, but such copies are too slow: 1640 against 870 us for the
              * gate|up launch of 4096 tokens.) */
             if (lane == 0) {                                            /* one lane walks the loop: with the warp in step this chain paces the CTA (30 layers of 24 tokens: +7%) */
@@ -388,18 +388,15 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
                     const int KB = items[iw % kItems].KB, n16 = items[iw % kItems].n16, sg = items[iw % kItems].sg, row0 = items[iw % kItems].row0;
                     mbar_arrive(iempty(iw));
                     if (KB == 0) break;
-                    /* box and map are chosen once a tile: chosen at every copy, 30 layers of 400 / 4096 tokens took 9.73 / 54.1 ms instead of 9.34 / 53.7 */
-                    const bool big = NMAX >= kBoxBig && n16 == kBoxBig;
-                    const int step = big ? kBoxBig : kNGran;
-                    const CUtensorMap *mh = big ? &maps.hi64[sg] : &maps.hi[sg], *ml = big ? &maps.lo64[sg] : &maps.lo[sg];
+                    /* hi and lo rows of a whole tile in one copy, a map per height: this lane's chain of wait, expect and copies is what
+                     * paces the CTA. In copies of 16 or 64 rows of hi or lo (6 for a tile of 48), 30 layers of 400 / 717 / 1500 tokens took
+                     * 9.38 / 12.6 / 23.2 ms instead of 9.15 / 12.1 / 22.6; of 37 tokens (2 copies) the same. */
+                    const CUtensorMap *map = &maps.act[sg][n16 / kNGran - 1];
                     for (int kb = 0; kb < KB; kb++) {
                         if (!mbar_wait(bempty(bs), bp ^ 1, abort_flag)) { failed = true; break; }
                         const uint32_t dst = sbase + bs * C::kBStage, bar = bfull(bs);
                         mbar_expect_tx(bar, (uint32_t)n16 * (TERMS >= 2 ? 256u : 128u));
-                        for (int i = 0; i < n16; i += step) {
-                            tma_load_2d(dst + 128u * i, mh, kb * kBK, row0 + i, bar);
-                            if (TERMS >= 2) tma_load_2d(dst + C::kBHalf + 128u * i, ml, kb * kBK, row0 + i, bar);
-                        }
+                        tma_load_3d(dst, map, kb * kBK, row0, 0, bar);
                         if (++bs == C::kBStages) { bs = 0; bp ^= 1; }
                     }
                 }
@@ -569,7 +566,7 @@ struct SpTcPlan {
     int *tiles_sh, *ntiles_sh, *tiles_r, *ntiles_r, *gather, *rowmap;
     int cap_sh, cap_r;
     int terms;                                         /* MMAs per k-step: 3, 2 or 1 */
-    CUtensorMap nx[4], hd[4], in[4], h[4];             /* boxes of 16 rows: hi, lo; of 64 rows: hi, lo */
+    CUtensorMap nx[4], hd[4], in[4], h[4];             /* boxes of 16, 32, 48 and 64 rows, hi and lo */
     sp_tc::EncodeTiledFn encode;
     std::map<const void *, CUtensorMap> codes;         /* one per weight tensor of the arena, made at first use */
 };
@@ -578,12 +575,13 @@ void sp_tc_inputs(SpTcPlan *p, __half **nx_hi, __half **nx_lo, __half **in_hi, _
 bool sp_tc_supported(const SpDims &d) { return (d.E % 64 == 0) && (d.FFE % 64 == 0) && (d.FFS % 64 == 0); }
 
 namespace {
-cudaError_t make_map(sp_tc::EncodeTiledFn fn, CUtensorMap *m, CUtensorMapDataType type, const void *ptr, size_t row_elems, size_t row_bytes, size_t rows, int box_elems, int box_rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)row_elems, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)box_elems, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(m, type, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+/* [plane][row][element], boxes of box_planes x box_rows rows of 128 bytes */
+cudaError_t make_map(sp_tc::EncodeTiledFn fn, CUtensorMap *m, CUtensorMapDataType type, const void *ptr, size_t row_elems, size_t row_bytes, size_t rows, int planes, int box_elems, int box_rows, int box_planes) {
+    const cuuint64_t dims[3] = {(cuuint64_t)row_elems, (cuuint64_t)rows, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)(row_bytes * rows)};
+    const cuuint32_t box[3] = {(cuuint32_t)box_elems, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(m, type, planes > 1 ? 3 : 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
@@ -592,7 +590,7 @@ cudaError_t codes_map(SpTcPlan *p, const uint8_t *codes, int K, size_t rows, CUt
     auto it = p->codes.find(codes);
     if (it == p->codes.end()) {
         CUtensorMap m;
-        const cudaError_t e = make_map(p->encode, &m, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, (size_t)K / 2, (size_t)K / 2, rows, 128, (int)kBoxRows);
+        const cudaError_t e = make_map(p->encode, &m, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, (size_t)K / 2, (size_t)K / 2, rows, 1, 128, (int)kBoxRows, 1);
         if (e != cudaSuccess) return e;
         it = p->codes.emplace(codes, m).first;
     }
@@ -646,18 +644,18 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
     p->tk_hi = (__half *)(b + o_tk); p->tk_lo = p->tk_hi + Mc * E;
     p->tiles_sh = (int *)(b + o_tsh); p->ntiles_sh = (int *)(b + o_nsh); p->tiles_r = (int *)(b + o_tr); p->ntiles_r = (int *)(b + o_nr);
     p->gather = (int *)(b + o_g); p->rowmap = (int *)(b + o_rm);
-    cudaError_t m = cudaSuccess;
-    auto mk = [&](CUtensorMap *t, const __half *hi, const __half *lo, size_t K, size_t rows) {
-        for (int i = 0; i < 4 && m == cudaSuccess; i++)
-            m = make_map(fn, t + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i & 1 ? lo : hi, K, 2 * K, rows, kBK, i < 2 ? kNGran : kBoxBig);
-    };
-    mk(p->nx, p->nx_hi, p->nx_lo, E, Mc); mk(p->hd, p->hd_hi, p->hd_lo, FFS, Mc);
-    mk(p->in, p->in_hi, p->in_lo, E, Rc); mk(p->h, p->h_hi, p->h_lo, FFE, Rc);
     /* house convention: behaviour switches are SP_* variables read once. 3 (default) keeps every product the fp32
      * reference arithmetic sees down to 2^-22; 2 rounds the dequantised weight to fp16; 1 also rounds the activation. */
     const char *tv = getenv("SP_MOE_PREFILL_TERMS");
     p->terms = tv ? atoi(tv) : 3;
     if (p->terms < 1 || p->terms > 3) p->terms = 3;
+    cudaError_t m = cudaSuccess;
+    auto mk = [&](CUtensorMap *t, const __half *hi, size_t K, size_t rows) {
+        for (int i = 0; i < kNMax / kNGran && m == cudaSuccess; i++)
+            m = make_map(fn, t + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, hi, K, 2 * K, rows, 2, kBK, (i + 1) * kNGran, p->terms >= 2 ? 2 : 1);
+    };
+    mk(p->nx, p->nx_hi, E, Mc); mk(p->hd, p->hd_hi, FFS, Mc);
+    mk(p->in, p->in_hi, E, Rc); mk(p->h, p->h_hi, FFE, Rc);
     if (m == cudaSuccess) m = p->terms == 3 ? prepare_terms<3>() : p->terms == 2 ? prepare_terms<2>() : prepare_terms<1>();
     if (m != cudaSuccess) { cudaFree(p->base); delete p; return m; }
     *out = p; *bytes = o;
@@ -684,7 +682,8 @@ struct Launch {
     Launch(SpTcPlan *p_, const SpDims &d_, const SpLayerDev &L_, int *status) : p(p_), d(d_), L(L_) { a.status = status; }
     TcSeg &seg(int K, const CUtensorMap *act, const uint8_t *c0, const uint16_t *b0, const uint8_t *c1, const uint16_t *b1, size_t tensor_rows, int rows, int m_tiles) {
         const int i = a.nseg++;
-        a.K[i] = K; maps.hi[i] = act[0]; maps.lo[i] = act[1]; maps.hi64[i] = act[2]; maps.lo64[i] = act[3];
+        a.K[i] = K;
+        for (int n = 0; n < kNMax / kNGran; n++) maps.act[i][n] = act[n];
         if (err == cudaSuccess) err = codes_map(p, c0, K, tensor_rows, &maps.codes[i][0]);
         if (err == cudaSuccess) err = codes_map(p, c1, K, tensor_rows, &maps.codes[i][1]);
         TcSeg &s = a.seg[i];
@@ -710,7 +709,10 @@ struct Launch {
     cudaError_t go(bool pair, int nmax, int *n_tiles, cudaStream_t st, int *nl) {      /* n_tiles: behind the count, the tickets of gate|up and of down */
         a.ticket = n_tiles + (pair ? 1 : 2);
         if (err != cudaSuccess) return err;
-        for (int i = a.nseg; i < 2; i++) { maps.hi[i] = maps.hi64[i] = maps.hi[0]; maps.lo[i] = maps.lo64[i] = maps.lo[0]; maps.codes[i][0] = maps.codes[i][1] = maps.codes[0][0]; a.K[i] = a.K[0]; }
+        for (int i = a.nseg; i < 2; i++) {
+            for (int n = 0; n < kNMax / kNGran; n++) maps.act[i][n] = maps.act[0][n];
+            maps.codes[i][0] = maps.codes[i][1] = maps.codes[0][0]; a.K[i] = a.K[0];
+        }
         if (pair) return nmax == 64 ? launch_n<true, 64>(p, a, maps, st, nl) : launch_n<true, 32>(p, a, maps, st, nl);
         return nmax == 64 ? launch_n<false, 64>(p, a, maps, st, nl) : launch_n<false, 32>(p, a, maps, st, nl);
     }
