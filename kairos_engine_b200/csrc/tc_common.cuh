@@ -39,6 +39,13 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
+/* two polls at once: have both phases completed? */
+__device__ __forceinline__ uint32_t mbar_try2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p, q; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4; and.pred p, p, q; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1) : "memory");
+    return ok;
+}
 /* one poll that may suspend the thread until the phase completes or kWaitNs pass: a waiting warp leaves the issue slots to
  * the warps that work */
 __device__ __forceinline__ uint32_t mbar_try_suspend(uint32_t bar, uint32_t parity) {
