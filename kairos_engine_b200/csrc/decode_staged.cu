@@ -14,10 +14,12 @@
  *     The copies run while all 16 warps do the per-layer prologue (norms, quantisation, top-k),
  *     so the prologue no longer delays the weight stream and no warp holds registers for loads in
  *     flight.
- *   - The warps then read rows from shared memory. A lane keeps its share of the quantised
- *     activation in registers across the rows it computes; rows are reduced two or eight at a
- *     time with a butterfly that performs exactly the additions of the reference's shuffle tree
- *     (same pairs, same tree shape), so results stay bit-identical.
+ *   - The warps then read rows from shared memory. The router and the shared gate|up rows take dp4a
+ *     chains, a lane keeping its share of the quantised activation in registers across the rows it
+ *     computes; the routed gate|up rows and the down rows take mma.sync tiles (exact integer sums of
+ *     16 weights). Rows are reduced two or eight at a time with a butterfly that performs exactly
+ *     the additions of the reference's shuffle tree (same pairs, same tree shape), so results stay
+ *     bit-identical.
  *
  * The single-pass layout needs a CTA's slice of every phase to fit shared memory at once
  * (sp_staged_fits); other geometries use decode_graph.cu.
@@ -36,7 +38,7 @@ using namespace sp_tc;
 #endif
 constexpr int kT = SP_DS_THREADS;       /* threads per CTA (a multiple of 128, at least 256) */
 constexpr int kW = kT / 32;
-constexpr int kRW = 4;                  /* K2: warps that run the softmax / top-NU while the others do the shared-expert rows */
+constexpr int kRW = 4;                  /* K2: warps that select the experts while the others do the shared-expert rows */
 #ifndef SP_DS_AHEAD
 #define SP_DS_AHEAD 3
 #endif

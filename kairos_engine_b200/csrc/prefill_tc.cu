@@ -668,11 +668,11 @@ void sp_tc_destroy(SpTcPlan *p) { if (!p) return; if (p->base) cudaFree(p->base)
 
 namespace {
 /* activation rows per tile: tiles of 32 have a second set of accumulators, tiles of 64 serve more rows per unpacked weight.
- * Us a layer with 32 / 64, E 2816, 128 experts, 8 each, FFE 704: 178 / 183 at 24 tokens, 240 / 246 at 128 (8 rows per expert),
- * 247 / 252 at 160, 261 / 264 at 200, 297 / 289 at 256, 357 / 338 at 400. With 64 experts, 6 each, E 2048, FFE 1408: 169 / 166 at 64
- * (6 rows), 182 / 192 at 96, 217 / 221 at 200 (19 rows); with 32, 4 each, E 1024, FFE 512: 46.7 / 58.1 at 64 (8 rows), 71 / 78 at
- * 200 (25 rows). The line could lie higher: between 8 rows and the crossing 64 costs up to 2% in the first, 5 to 10% in the others. */
-int tile_rows(int groups, long long rows) { return rows > 8LL * groups ? 64 : 32; }
+ * Us a layer with 32 / 64, E 2816, 128 experts, 8 each, FFE 704: 146 / 153 at 24 tokens, 189 / 193 at 64, 218 / 220 at 128 (8 rows
+ * per expert), 222 / 228 at 160, 233 / 237 at 200, 259 / 258 at 256, 312 / 298 at 400. With 64 experts, 6 each, E 2048, FFE 1408:
+ * 137 / 140 at 64 (6 rows), 158 / 155 at 128 (12 rows), 184 / 184 at 200 (19 rows); with 32, 4 each, E 1024, FFE 512: 42 / 50 at
+ * 64 (8 rows), 47 / 56 at 128, 62.8 / 61.7 at 200 (25 rows). */
+int tile_rows(int groups, long long rows) { return rows > 16LL * groups ? 64 : 32; }
 
 template <bool PAIR, int NMAX>
 cudaError_t launch_n(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st, int *nl) {

@@ -66,7 +66,7 @@ TC_MANY = _cfg(576, 160, 8, 64, 192)    # more experts than the warp-wide select
                                    (TC, 2), (TC, 15), (TC, 32), (TC, 33), (TC, 64), (TC, 65), (TC, 129), (TC, 257), (TC_MIN, 2), (TC_MIN, 17), (TC_MIN, 33), (TC_MIN, 130),
                                    (TC_MANY, 3), (TC_MANY, 50), (TC_MANY, 170), (TC_MANY, 400)])
 def test_prefill_tile_edges(cfg, M):
-    """Rows per expert on both sides of the eight at which the GEMMs go from 32 to 64 rows a tile, and of tiles of 16, 32 and
+    """Rows per expert on both sides of the sixteen at which the GEMMs go from 32 to 64 rows a tile, and of tiles of 16, 32 and
     64 rows."""
     eng, host = make_stack(cfg, 1, seed=73, rand_norms=True, max_tokens=M)
     x = np.random.default_rng(M).standard_normal((M, cfg["E"])).astype(np.float32)
