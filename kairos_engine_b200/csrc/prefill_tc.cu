@@ -34,12 +34,14 @@
  * Warps: 0-7 epilogue (TMEM lane quadrant = warp % 4, block = warp / 4), 8-23 unpack (the same, in
  * two sets that take alternate stages), 24 and 25 MMA issue (one per block), 26 activation TMA, 27
  * code TMA and TMEM allocation. Every wait is bounded.
- * What bounds it (Gemma geometry, one B200): up to some 40 rows per expert the unpack, ~136
- * instructions of the half-rate fp16 and integer pipes per 2048 weights, beside a weight stream at
- * about a third of HBM's rate; from there to the largest batches the unpack and the MMAs (12, 16
- * and 32 cycles at N = 16, 32 and 64) together, each about 70% of an SM's active time at 4096 tokens, and in the end
- * the power limit. A layer of 37 / 717 / 4096 tokens: 0.60 / 0.85 / 2.40 ms with the weights in shared memory and 128 rows
- * a tile, 0.19 / 0.43 / 1.85 ms with this.
+ * A CTA draws its tiles from a counter; the code warp announces them to the others through a ring.
+ * What bounds it (Gemma geometry, one B200): with a few rows per expert the chain of a stage in an MMA
+ * warp, ~740 cycles at 37 tokens (two polls at once, twelve MMAs and two commits 300, the loop), beside
+ * the unpack, ~136 instructions of the half-rate fp16 and integer pipes per 2048 weights, whose warps
+ * wait half their time for a stage to be free; with 48 and more rows the tensor time of the three terms
+ * (12, 16 and 32 cycles an MMA at N = 16, 32 and 64: 768 of ~870 cycles a stage at 64), and in the end
+ * the power limit. A layer of 37 / 717 / 4096 tokens: 0.60 / 0.85 / 2.40 ms with the weights in shared
+ * memory and 128 rows a tile, 0.18 / 0.40 / 1.78 ms with this.
  */
 #include <map>
 #include "prefill_tc.cuh"
