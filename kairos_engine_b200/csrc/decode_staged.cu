@@ -674,7 +674,8 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
             /* The selection straight from the logits: every warp ranks its 32 among themselves, the first NU of each meet, and every
              * warp ranks those (equal keys keep the order of their lanes, which is that of their ids). Probabilities order as
              * logits do, except that different logits can round to one probability; so it holds where no two neighbours among the
-             * first NU + 1 differ by less than 1e-6 without being equal (a probability is rounded to 6e-8 of itself) and none is
+             * first NU + 1 differ by less than 1e-6 without being equal (a probability is rounded to 6e-8 of itself), the last
+             * chosen is not equal to the first left out (a third, just below, could have their probability and a lower id) and none is
              * 80 below the first (no underflow). Otherwise, and with a NaN, the probabilities decide, below. The routed copies wait
              * for this: with the softmax first and NU rounds of a maximum and a minimum they went out 1.7 us later. */
             static_assert(TR == 128 && SP_MAX_NU * kRW == 32, "a candidate to a thread, a lane to each of the best");
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
             if (lane < NU) {
                 const int k0 = keys[lane], k1 = lane + 1 < NU ? keys[lane + 1] : after;
                 const float gap = value(k0) - value(k1);
-                close |= k0 == kAbsent || !(value(k0) > first - 80.0f) || (k1 != kAbsent && k0 != k1 && !(gap >= 1e-6f));
+                close |= k0 == kAbsent || !(value(k0) > first - 80.0f) || (k0 == k1 ? lane == NU - 1 : k1 != kAbsent && !(gap >= 1e-6f));
             }
             done = !__any_sync(0xffffffffu, close);
             if (done) {

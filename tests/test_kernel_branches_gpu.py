@@ -84,3 +84,43 @@ def test_prefill_drawn_tiles(cfg, M):
     for _ in range(8):
         assert np.array_equal(eng.forward(x, flavour=B)[0].view(np.uint32), y.view(np.uint32))
     eng.status(); eng.close()
+
+
+def _tie_then_one_ulp(NE, NU, same_warp):
+    """NU - 1 larger logits, two equal ones of which one is the last chosen, and one a float below with a lower id whose
+    probability rounds to theirs: the checker takes that one."""
+    near, tied = (3, (9, 11)) if same_warp else (3, (NE - 5, NE - 2))
+    rest = [i for i in range(NE) if i not in (near, *tied)]
+    for k in range(1, 200):
+        v = -1.0 - np.arange(NE, dtype=np.float32) / NE
+        v[rest[-(NU - 1):] if NU > 1 else []] = np.float32(2.0) + np.arange(NU - 1, dtype=np.float32)
+        v[list(tied)] = np.float32(0.001 * k)
+        v[near] = np.nextafter(np.float32(0.001 * k), np.float32(0.0))
+        _, idx, _ = orc.topk(v, NU)
+        if idx[NU - 1] == near:
+            return v
+    raise AssertionError("no such logits")
+
+
+@pytest.mark.parametrize("same_warp", [True, False])
+@pytest.mark.parametrize("cfg", [orc.GEMMA, _cfg(256, 128, 1, 64, 128), _cfg(96, 37, 5, 96, 32)])
+def test_single_token_tie_at_the_last_place(cfg, same_warp):
+    """The last chosen logit equals the first one left out and a third is one float below: probabilities decide, in the
+    single-token kernels as in a batch of two."""
+    import torch
+    from kairos_engine_b200 import MoeEngine, synth
+    bias = _tie_then_one_ulp(cfg["NE"], cfg["NU"], same_warp)
+    layer = synth.make_layer(cfg, 78, rand_norms=True, bias=torch.from_numpy(bias).cuda())
+    layer["router_w"] = torch.zeros_like(layer["router_w"])
+    eng = MoeEngine(n_layers=1, max_tokens=2, **cfg)
+    eng.upload_layer(0, layer, on_device=True)
+    x = np.random.default_rng(6).standard_normal((2, cfg["E"])).astype(np.float32)
+    ry, rsel, rwts, _ = oracle_stack(cfg, [orc.LayerWeights(**synth.layer_to_host(layer))], x, A)
+    y, sel, wts = eng.forward(x, flavour=A)
+    assert np.array_equal(sel, rsel) and np.array_equal(wts.view(np.uint32), rwts.view(np.uint32))
+    for t in range(2):
+        y1, sel1, wts1 = eng.forward(x[t:t + 1], flavour=A)
+        assert np.array_equal(sel1[:, 0], rsel[:, t])
+        assert np.array_equal(wts1[:, 0].view(np.uint32), rwts[:, t].view(np.uint32)) and np.array_equal(y1[0].view(np.uint32), ry[t].view(np.uint32))
+        assert np.array_equal(y1[0].view(np.uint32), y[t].view(np.uint32))
+    eng.close()
