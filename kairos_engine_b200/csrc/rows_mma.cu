@@ -73,9 +73,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned
 __device__ __forceinline__ void box_g2s(uint32_t dst, const CUtensorMap *map, int row, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%4, %2, %4}], [%3];" ::"r"(dst), "l"(map), "r"(row), "r"(bar), "r"(0) : "memory");
 }
-/* the sums of a team's eight warps are there: for those that finish them; the others go on */
-__device__ __forceinline__ void sums_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTeamThreads) : "memory"); }
-__device__ __forceinline__ void sums_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kTeamThreads) : "memory"); }
 
 /* D = A x B + {magic, ...}, D += A x B (pure functions of their operands: the compiler may move them) */
 __device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, int c) {
@@ -217,7 +214,7 @@ struct Batch { int seg, tile, flags, item[kTok], pad; };     /* up to four token
 template <bool PAIR, int W>
 __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const __grid_constant__ RowsArgs a) {
     unsigned char *const sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
-    __shared__ unsigned long long bars[(1 + kMaxTeams) * kMaxStages + 4 * kMaxTeams];
+    __shared__ unsigned long long bars[(1 + kMaxTeams) * kMaxStages + 6 * kMaxTeams];
     __shared__ int abort_s;
     __shared__ Batch batch_s[kMaxTeams][2];
     __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
@@ -231,8 +228,9 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     auto full = [&](int team, int s) { return bar0 + 8u * (kMaxStages * (1 + team) + s); };
     auto empty = [&](int s) { return bar0 + 8u * s; };
     constexpr int kActBars = (1 + kMaxTeams) * kMaxStages;
-    auto afull = [&](int team, int b) { return bar0 + 8u * (kActBars + 4 * team + b); };      /* a team's two buffers of activations */
-    auto aempty = [&](int team, int b) { return bar0 + 8u * (kActBars + 4 * team + 2 + b); };
+    auto afull = [&](int team, int b) { return bar0 + 8u * (kActBars + 6 * team + b); };      /* a team's two buffers of activations */
+    auto aempty = [&](int team, int b) { return bar0 + 8u * (kActBars + 6 * team + 2 + b); };
+    auto sums = [&](int team, int b) { return bar0 + 8u * (kActBars + 6 * team + 4 + b); };      /* and of sums: all eight warps' are there */
     if (tid == 0) {
         for (int s = 0; s < a.stages; s++) {
             for (int t = 0; t < a.teams; t++) mbar_init(full(t, s), 1);
@@ -240,7 +238,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         }
         for (int t = 0; t < a.teams; t++)
             for (int b = 0; b < 2; b++) {
-                mbar_init(afull(t, b), 1); mbar_init(aempty(t, b), kTeamWarps);
+                mbar_init(afull(t, b), 1); mbar_init(aempty(t, b), kTeamWarps); mbar_init(sums(t, b), kTeamWarps);
             }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -350,7 +348,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         const int team = warp / kTeamWarps, tw = warp % kTeamWarps, gq = lane >> 2, q = lane & 3;
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
         int s = team % a.stages;
-        unsigned phs = 0;                                   /* bit s: parity of this team's next use of stage s */
+        unsigned phs = 0, psum = 0;                         /* bit s: parity of this team's next use of stage s; bit b: of buffer b of sums */
         Frag f;
         /* lanes whose 8-byte loads share a wavefront (W = 2) take rows whose pieces differ by more than the group's two */
         f.row = W == 1 ? gq : (gq & 1) << 2 | (gq & 2) | gq >> 2;
@@ -430,8 +428,13 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 release();
                 /* Two warps (gate|up) or one per token finish the sums, other ones each time, and only they wait for the rest, which is
                  * at its next tokens meanwhile: a warp loses the time of one finish in four (or two) times. The other buffer of sums
-                 * and the other barrier serve those next tokens; the buffer's next use but one waits for this one's end (aempty). */
-                const int id = 1 + 2 * team + buf;
+                 * and the other barrier serve those next tokens; the buffer's next use but one waits for this one's end (aempty). The
+                 * wait gives up when a warp of the team did, whose sums never come (on named barriers, which cannot, the give-up path
+                 * would have to arrive for others; 64 tokens take 160.1 us a layer so, 159.2 on those). */
+                const uint32_t par = psum >> buf & 1u;
+                psum ^= 1u << buf;
+                __syncwarp();
+                mbar_arrive_lane0(sums(team, buf), lane);
                 auto total_of = [&](int m, int rw, int t) {                 /* the last levels of the tree */
                     const float *p = part + (m * 16 + rw) * T + t;
                     const int k = 32 * T;
@@ -441,28 +444,26 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 if (PAIR) {
                     const int w0 = 2 * (n & 3);
                     if (tw == w0 || (tw == w0 + 1 && T == 4)) {
-                        sums_wait(id);
+                        if (!mbar_wait_out(sums(team, buf), par, abort_flag)) { failed = true; break; }
+                        __syncwarp();                       /* the quantisation takes the whole warp */
                         const int idx = (tw - w0) * 32 + lane, t = idx >> 4, col = idx & 15;
                         const float h = gelu_mul(total_of(col >> 3, col & 7, t), total_of(col >> 3, (col & 7) + 8, t));
                         const int it = bt.item[t] < 0 ? 0 : bt.item[t];
                         unsigned char *o = sg.out_act + (size_t)it * sp_act_pitch(sg.rows);
                         quant_elem16(h, bt.item[t] >= 0, reinterpret_cast<signed char *>(o) + tile * 16, reinterpret_cast<float *>(o + sg.rows) + tile);
-                    } else sums_arrive(id);
+                    }
                 } else {
                     const int t = tw - 4 * (n & 1);
                     if (t >= 0 && t < T) {
-                        sums_wait(id);
+                        if (!mbar_wait_out(sums(team, buf), par, abort_flag)) { failed = true; break; }
                         const int it = bt.item[t];
                         if (it >= 0 && r0 + lane < sg.rows) sg.out_f[(size_t)it * sg.out_stride + r0 + lane] = total_of(lane >> 4, lane & 15, t);
-                    } else sums_arrive(id);
+                    }
                 }
             }
             __syncwarp();
             mbar_arrive_lane0(aempty(team, buf), lane);
         }
-        /* a warp that gave up: the others may be waiting for its sums of these tokens or of the next, never of later ones (aempty) */
-        __syncwarp();
-        if (__any_sync(0xffffffffu, failed)) { sums_arrive(1 + 2 * team); sums_arrive(2 + 2 * team); }
     }
     if (failed) {
         if (lane == 0) atomicExch(a.status, SP_KERR_BARRIER_TIMEOUT);
