@@ -45,6 +45,7 @@ constexpr int kRW = 4;                  /* K2: warps that select the experts whi
 #ifndef SP_DS_LP
 #define SP_DS_LP 3
 #endif
+static_assert(SP_DS_LP >= 3, "a part holds whole tiles of eight pairs: a tile waits for the part of its first pair only");
 constexpr int kGuBars = 10;             /* the routed gate|up slice lands in up to 10 parts ... */
 constexpr int kGuAhead = SP_DS_AHEAD;             /* ... of which this many are in flight at a time, so they land in the order they are consumed */
 constexpr int kDnBars = 4;              /* the routed down slice too */
