@@ -116,9 +116,9 @@ struct Ctl {
     unsigned gs_off[2], us_off[2];          /* K2: where the two runs' gate / up scale rows start */
     unsigned sdelta[SP_MAX_NU];             /* K3: bytes before the first scale row of each slot's span */
     alignas(16) int zero[4];                /* K3: the activation operand of an MMA column that is not the lane's */
-    int2 cand[4 * SP_MAX_NU], rest[4];      /* K2: the best of each router warp's candidates (key, id); its next key and whether it met a NaN */
 };
 
+constexpr unsigned kSmemMax = 227 * 1024;   /* shared memory of a CTA, sm_100 */
 struct Lay1 { unsigned ctl, red, va, vb, ri, q_nx, s_nx, c_nx, st_r, st_gc, st_uc, st_gs, st_us, total; };
 __host__ __device__ inline Lay1 lay1(const SpDims &d, int G) {
     Lay1 L; unsigned o = 0;
@@ -133,20 +133,32 @@ __host__ __device__ inline Lay1 lay1(const SpDims &d, int G) {
     L.total = o;
     return L;
 }
+/* K2's selection from the logits, in the part of the reduction scratch that K2 does not use */
+struct Sel {
+    int keys[4][32];                        /* a router warp's keys, then the best of all in order */
+    int2 cand[4 * SP_MAX_NU], rest[4];      /* the best of each router warp's candidates (key, id); its next key and whether it met a NaN */
+};
+constexpr unsigned kRedBytes = 128 * 8, kSelAt = 64;
+static_assert(kRW * sizeof(double) <= kSelAt && kSelAt + sizeof(Sel) <= kRedBytes && kRW == 4, "the selection's scratch");
 struct Lay2 { unsigned ctl, red, ex, lg, p, dsc, wmax, q_in, s_in, q_hd, s_hd, c_hd, st_sd, st_sds, st_gc, st_uc, st_gs, st_us, part, total; };
 __host__ __device__ inline Lay2 lay2(const SpDims &d, int G) {
     Lay2 L; unsigned o = 0;
     auto take = [&](unsigned bytes) { const unsigned at = o; o = up16(o + bytes); return at; };
     const unsigned E = d.E, NE = d.NE, FFS = d.FFS, nj = cdiv(d.E, G), nP = cdiv(d.NU * d.FFE, G);
-    L.ctl = take(sizeof(Ctl)); L.red = take(128 * 8); L.ex = take(8 * NE);
-    L.lg = take(4 * NE); L.p = take(4 * (NE < 128 ? 128 : NE)); L.dsc = take(4 * NE); L.wmax = take(4 * 32);
+    L.ctl = take(sizeof(Ctl)); L.red = take(kRedBytes); L.ex = take(8 * NE);
+    L.lg = take(4 * NE); L.p = take(4 * NE); L.dsc = take(4 * NE); L.wmax = take(4 * 32);
     L.q_in = take(E); L.s_in = take(4 * (E / 16));
     L.q_hd = take(FFS); L.s_hd = take(4 * (FFS / 16)); L.c_hd = take(4 * (FFS / 16));
     o = (o + 127u) & ~127u;
     L.st_sd = take(nj * (FFS / 2)); L.st_sds = take(nj * (FFS / 16) + 32);
     L.st_gc = take(nP * (E / 2)); L.st_uc = take(nP * (E / 2));
     L.st_gs = take(nP * (E / 16) + 64); L.st_us = take(nP * (E / 16) + 64);
-    L.part = take(1024 * ((nP + 7) / 8));
+    /* The pairs' sums have a place of their own where there is room. Elsewhere they take that of the code rows, a round of tiles after
+     * all warps have read it (1024 bytes a tile of eight rows: never past the rows of the tiles that are done, and after the last
+     * round nothing of the slice is read). Without that, geometries whose rows fill the shared memory would not fit. */
+    const unsigned tiles = (nP + 7) / 8, before = o;
+    L.part = take(1024 * tiles);
+    if (o > kSmemMax && E >= 256 && 1024 * tiles <= nP * E) { L.part = L.st_gc; o = before; }
     L.total = o;
     return L;
 }
@@ -529,12 +541,12 @@ __device__ __forceinline__ void group_mma(const unsigned char *c0, const unsigne
     }
 }
 /* Routed gate|up: the row dots of eight pairs on the tensor cores (as in k_ds_experts_down, below), a quarter of a row's slots to a warp:
- * those with (slot / 4) % 4 = r, groups r, r + 4, r + 8, ... part: [tile][r][slot % 4][gate rows, up rows], each the first level of the
- * tree. A warp then has a quarter of the instructions that dp4a takes for the same rows, and a part of the copies is worked
+ * those with (slot / 4) % 4 = r, groups r, r + 4, r + 8, ... Lane (g, q) returns the sums of slot % 4 = q of gate row g and up row g, the
+ * first level of the tree. A warp then has a quarter of the instructions that dp4a takes for the same rows, and a part of the copies is worked
  * off by four warps while the next one lands. */
 template <int NIT>
-__device__ __forceinline__ void pairs_mma(unsigned char *sm, const Lay2 &ly, Ctl *ctl, int tile, int r, int nP, int n0, unsigned rb, unsigned sb, int n32, int lane,
-                                          const signed char *q_in, const float *s_in, float *part) {
+__device__ __forceinline__ float2 pairs_mma(unsigned char *sm, const Lay2 &ly, Ctl *ctl, int tile, int r, int nP, int n0, unsigned rb, unsigned sb, int n32, int lane,
+                                            const signed char *q_in, const float *s_in) {
     const int g = lane >> 2, q = lane & 3;
     int i = 8 * tile + g;
     if (i > nP - 1) i = nP - 1;                             /* rows past the slice repeat its last pair and are dropped */
@@ -554,8 +566,7 @@ __device__ __forceinline__ void pairs_mma(unsigned char *sm, const Lay2 &ly, Ctl
             group_mma(c0 + 256 * k, c1 + 256 * k, s0 + 32 * k, s1 + 32 * k, b0, b1, sx + 32 * k, 16 * k < left, k & 1 ? hi : lo);
             b0 += st0; b1 += st1;
         }
-    float *p = part + ((tile * 4 + r) * 4 + q) * 16 + g;
-    p[0] = lo.x + hi.x; p[8] = lo.y + hi.y;
+    return make_float2(lo.x + hi.x, lo.y + hi.y);
 }
 
 template <int NIT_E, int NIT_S>
@@ -681,22 +692,23 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
              * for this: with the softmax first and NU rounds of a maximum and a minimum they went out 1.7 us later. */
             static_assert(TR == 128 && SP_MAX_NU * kRW == 32, "a candidate to a thread, a lane to each of the best");
             constexpr int kAbsent = (int)0x80000001;
-            int *const keys = reinterpret_cast<int *>(p) + 32 * warp;      /* a warp's 32 slots are its own */
+            Sel *const sel = reinterpret_cast<Sel *>(sm + ly.red + kSelAt);
+            int *const keys = sel->keys[warp];
             const float l = t < NE ? __fadd_rn(__ldcg(a.s.logits + t), 0.0f) : -INFINITY;         /* -0 becomes 0 */
             auto order = [](float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); };      /* its own inverse on int */
             const int key = t < NE ? order(l) : kAbsent, r = rank(key, keys);
-            if (r < SP_MAX_NU) ctl->cand[SP_MAX_NU * warp + r] = make_int2(key, t);
+            if (r < SP_MAX_NU) sel->cand[SP_MAX_NU * warp + r] = make_int2(key, t);
             const bool bad = __any_sync(0xffffffffu, t < NE && l != l);
-            if (r == SP_MAX_NU) ctl->rest[warp] = make_int2(key, bad);
+            if (r == SP_MAX_NU) sel->rest[warp] = make_int2(key, bad);
             bar_named(1, TR);
-            const int2 c = ctl->cand[lane];
+            const int2 c = sel->cand[lane];
             const int rc = rank(c.x, keys);
             __syncwarp();
             keys[rc] = c.x;                                 /* sorted */
             __syncwarp();
             int after = keys[NU < 32 ? NU : 31], flag = 0;  /* the largest key not chosen */
 #pragma unroll
-            for (int w = 0; w < kRW; w++) { const int2 o = ctl->rest[w]; after = o.x > after ? o.x : after; flag |= o.y; }
+            for (int w = 0; w < kRW; w++) { const int2 o = sel->rest[w]; after = o.x > after ? o.x : after; flag |= o.y; }
             auto value = [&](int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); };
             const float first = value(keys[0]);
             bool close = flag != 0;
@@ -820,12 +832,23 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
     /* routed gate|up pairs, eight to a tile, as their part lands; units of work: (tile, quarter of the slots) */
     float *const part = reinterpret_cast<float *>(sm + ly.part);
     const int tiles = (nP + 7) >> 3;
+    static_assert(kW % 4 == 0, "a round is whole tiles");
+    const bool over = ly.part == ly.st_gc;                /* the sums take the place of rows that are done: see lay2 */
 #pragma unroll 1
-    for (int u = warp; u < 4 * tiles; u += kW) {
-        bar_wait(smem_u32(&ctl->bar[1]), &ctl->abort, a.s.status);              /* the scale rows travel with part 0 */
-        bar_wait(smem_u32(&ctl->bar[1 + ((u >> 2) << 3 >> LP)]), &ctl->abort, a.s.status);
-        __syncwarp();
-        pairs_mma<NIT_E>(sm, ly, ctl, u >> 2, u & 3, nP, n0, rbE, sbE, n32, lane, q_in, s_in, part);
+    for (int u0 = 0; u0 < 4 * tiles; u0 += kW) {
+        const int u = u0 + warp;
+        float2 v = make_float2(0.0f, 0.0f);
+        if (u < 4 * tiles) {
+            bar_wait(smem_u32(&ctl->bar[1]), &ctl->abort, a.s.status);              /* the scale rows travel with part 0 */
+            bar_wait(smem_u32(&ctl->bar[1 + ((u >> 2) << 3 >> LP)]), &ctl->abort, a.s.status);
+            __syncwarp();
+            v = pairs_mma<NIT_E>(sm, ly, ctl, u >> 2, u & 3, nP, n0, rbE, sbE, n32, lane, q_in, s_in);
+        }
+        if (over) __syncthreads();
+        if (u < 4 * tiles) {                              /* part: [tile][r][slot % 4][gate rows, up rows] */
+            float *p = part + (u * 4 + (lane & 3)) * 16 + (lane >> 2);
+            p[0] = v.x; p[8] = v.y;
+        }
     }
     if ((a.flags & SP_STAGED_PREFETCH_DN) && nj > 0) {    /* the routed down rows the next kernel will stage: ask L2 for them */
 #pragma unroll 1
