@@ -761,6 +761,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
             if (bad && lane == 0) atomicExch(a.s.status, SP_KERR_NAN_ROUTER);
             if (t < SP_MAX_NU) { ctl->sel_desc[t] = t < NE ? t : 0; ctl->p_desc[t] = 0.0f; }
             bar_named(1, TR);
+            STAMP(1, 5);
             mx = wmax[0];
 #pragma unroll
             for (int w = 1; w < kRW; w++) mx = fmaxf(mx, wmax[w]);
@@ -777,6 +778,7 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_up(SArgs a) {
 #pragma unroll 1
             for (int i = t; i < NE; i += TR) p[i] = (float)(ex[i] * rsum);
             bar_named(1, TR);
+            STAMP(1, 6);
             if (NE <= 128) {
                 /* one warp, four candidates per lane in registers, NU rounds of (largest value, then lowest id among
                  * its holders): the order moe_topk_host's strict > insertion produces. key = bits(p) + 1 for a usable
