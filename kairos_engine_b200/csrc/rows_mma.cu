@@ -36,6 +36,7 @@ namespace {
 using namespace sp_tc;
 
 constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kMaxStages = 4, kMaxTeams = 2;
+constexpr int kFewItems = 24, kManyItems = 48;     /* items to a group up to which units are of 4 tokens: on average, and in any one group */
 constexpr int kUnits = 128;                        /* unit descriptors of a CTA kept in shared memory */
 constexpr int kMagic = 0x4B400000;
 
@@ -46,7 +47,8 @@ struct SegGeo {                                    /* what the copies and the do
 };
 struct RowsArgs {
     SpRowsSeg seg[2]; SegGeo geo[2]; int nseg;
-    int stages, teams, unit_log;                   /* ...; log2 of the tokens of a unit at most */
+    int stages, teams;
+    int many[2];                                   /* a group of more items than this has units of up to 16 tokens, others of up to 4 */
     unsigned stage_bytes, act_bytes, zero_bytes;   /* one stage; one buffer of four tokens; the zeros B's other columns read */
     int *status;
     CUtensorMap codes[2][2];                       /* [segment][gate or only / up] */
@@ -113,6 +115,7 @@ __device__ __forceinline__ int group_count(const SpRowsSeg &s, int g) {
     const int c = __ldcg(s.count + g);
     return c > s.M ? s.M : c;
 }
+__device__ __forceinline__ int unit_log(int cnt, int many) { return cnt > many ? 4 : 2; }      /* log2 of the tokens of a group's units at most */
 __device__ __forceinline__ int units_of(int cnt, int log) { return (cnt + (1 << log) - 1) >> log; }
 __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     Unit r{};
@@ -123,10 +126,10 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     int lo = 0, hi = s.groups - 1;                          /* the last group that starts at or before u: never an empty one */
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (st[mid] <= u) lo = mid; else hi = mid - 1; }
     r.grp = lo;
-    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), nr = units_of(cnt, a.unit_log), k = u - st[lo];
+    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), log = unit_log(cnt, a.many[r.seg]), nr = units_of(cnt, log), k = u - st[lo];
     r.tile = k / nr;
-    r.t0 = (k - r.tile * nr) << a.unit_log;
-    r.nt = cnt - r.t0 < 1 << a.unit_log ? cnt - r.t0 : 1 << a.unit_log;
+    r.t0 = (k - r.tile * nr) << log;
+    r.nt = cnt - r.t0 < 1 << log ? cnt - r.t0 : 1 << log;
     return r;
 }
 
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const SpRowsSeg &s = a.seg[k];
                 for (int g0 = 0; g0 < s.groups; g0 += 32) {
                     const int g = g0 + lane;
-                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * units_of(cnt, a.unit_log);
+                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * units_of(cnt, unit_log(cnt, a.many[k]));
                     if (k == 1 && g < s.groups) count_s[g] = cnt;
                     int v = n;
 #pragma unroll
@@ -513,10 +516,18 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
      * the launch at 16 tokens and kept the other team waiting. What small ones fetch again comes from L2, until that is what
      * bounds them. Us a layer of E 2816, 128 experts, 8 each, units of 16 / 8 / 4 tokens: 54.4 / 54.5 / 52.8 at 5 tokens, 92.2 / 88.5 /
      * 86.6 at 16, 120 / 119 / 113 at 32, 176 / 174 / 160 at 64; of 16 / 4: 238 / 222 at 100, 412 / 395 at 200, 550 / 501 at 256, 772 / 760 at
-     * 400 (321: 693 / 623), 901 / 967 at 512, 1677 / 1870 at 1024: the line is at 384 tokens, 24 items to an expert. */
-    a.unit_log = items <= 24LL * seg[nseg - 1].groups ? 2 : 4;
+     * 400 (321: 693 / 623), 901 / 967 at 512, 1677 / 1870 at 1024: the line is at 384 tokens, 24 items to an expert on average
+     * (E 2048, 64 experts, 6 each: 869 / 746 at 24 items, 1029 / 1083 at 36; E 1024, 32 experts, 4 each: 121 / 103 at 24, 136 /
+     * 128 at 32, where it could lie higher). Where the router sends most tokens to a few experts, those alone are above the
+     * line: a group of more than 48 items has units of 16 whatever the average (a Zipf 1.2 router over 128 experts, units of 4 everywhere /
+     * so: 242 / 237 at 128 tokens, 463 / 428 at 256, 687 / 613 at 384). 48, because units of both sizes side by side cost
+     * more than they save while the counts only scatter about their average (384 tokens, 24 on average: a line of 24 per group 757,
+     * of 48 721). Rows sorted for one rank's experts belong to fewer groups than there are, how many is not known here: their line
+     * is 24 for each group by itself. */
+    const bool few = items <= (long long)kFewItems * seg[nseg - 1].groups;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
+        a.many[i] = seg[i].offset ? kFewItems : !few ? 0 : seg[i].groups > 1 ? kManyItems : 0x7fffffff;
         const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
         const unsigned sb = up1024(g.scale_off + 16 * g.mt_n * g.sb), ab = kTok * g.ast;
         const unsigned zb = (unsigned)seg[i].in + 128;
