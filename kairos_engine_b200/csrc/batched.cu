@@ -941,15 +941,16 @@ cudaError_t ep_route(const SpDims &d, const SpLayerDev &L, int M, const float *x
  * (token dispatch); the outputs still go to the pair's own row (row_index). */
 template <bool FA>
 cudaError_t ep_experts(const SpDims &d, const SpLayerDev &L, int R, const float *rows_in, const int32_t *row_index, const int32_t *offsets, float *rows_out,
-                       const int32_t *in_index, int n_in, BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
+                       const int32_t *in_index, int n_in, int owners, BView &v, SpTcPlan *tc, int *status, cudaStream_t st, int *nl) {
     const int E = d.E, NE = d.NE, FFE = d.FFE;
     if (R == 0) return cudaSuccess;
-    if (!FA && tc) return sp_tc_routed(tc, d, L, R, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
+    if (!FA && tc) return sp_tc_routed(tc, d, L, R, owners, rows_in, in_index ? in_index : row_index, offsets, row_index, rows_out, status, st, nl);
     if (FA) {
         cudaError_t e = sp_launch((uintptr_t)rows_in & 15 ? k_b_quant_rows<false> : k_b_quant_rows<true>, dim3((unsigned)(in_index ? n_in : R)), (unsigned)((E / 4 + 31) & ~31), 0, st, nl, rows_in, E, v.ep_q);
         if (e != cudaSuccess) return e;
         SpRowsSeg up = seg_routed_up(d, L, R, v.ep_q, v), down = seg_routed_down(d, L, R, v, rows_out);
         up.offset = down.offset = offsets; up.index = down.index = row_index; up.act_index = in_index;      /* h has one row per pair */
+        up.owners = down.owners = owners;
         e = sp_rows_launch(&up, 1, true, R, status, st, nl);
         return e != cudaSuccess ? e : sp_rows_launch(&down, 1, false, R, status, st, nl);
     }
@@ -989,12 +990,12 @@ cudaError_t sp_batched_ep_shared(const SpDims &d, const SpLayerDev &L, int flavo
     return flavour == SP_MOE_FLAVOUR_DECODE ? ep_shared<true>(d, L, M, v, s->tc, status, st, nlaunch, phase) : ep_shared<false>(d, L, M, v, s->tc, status, st, nlaunch, phase);
 }
 cudaError_t sp_batched_ep_experts(const SpDims &d, const SpLayerDev &L, int flavour, int R, const float *rows_in, const int32_t *row_index, const int32_t *offsets,
-                                  float *rows_out, SpBatchedScratch *s, int *status, cudaStream_t st, int *nlaunch, const int32_t *in_index, int n_in) {
+                                  float *rows_out, SpBatchedScratch *s, int *status, cudaStream_t st, int *nlaunch, const int32_t *in_index, int n_in, int owners) {
     *nlaunch = 0;
     if (!s->base || R > s->max_rows || (in_index && (n_in <= 0 || n_in > s->max_rows))) return cudaErrorInvalidValue;
     BView v = bview(d, s);
-    return flavour == SP_MOE_FLAVOUR_DECODE ? ep_experts<true>(d, L, R, rows_in, row_index, offsets, rows_out, in_index, n_in, v, s->tc, status, st, nlaunch)
-                                            : ep_experts<false>(d, L, R, rows_in, row_index, offsets, rows_out, in_index, n_in, v, s->tc, status, st, nlaunch);
+    return flavour == SP_MOE_FLAVOUR_DECODE ? ep_experts<true>(d, L, R, rows_in, row_index, offsets, rows_out, in_index, n_in, owners, v, s->tc, status, st, nlaunch)
+                                            : ep_experts<false>(d, L, R, rows_in, row_index, offsets, rows_out, in_index, n_in, owners, v, s->tc, status, st, nlaunch);
 }
 /* token dispatch, sender side (after sp_batched_ep_route of the same tokens with rows == NULL): tokrows
  * [n_ranks][cap_tokens][E], tokidx [n_ranks][capacity] (the pair order of the padded exchange), slot = scratch of

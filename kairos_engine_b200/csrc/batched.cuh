@@ -43,7 +43,7 @@ cudaError_t sp_batched_ep_recv_layout(const SpDims &d, const int32_t *counts_all
 cudaError_t sp_batched_ep_shared(const SpDims &d, const SpLayerDev &L, int flavour, int M, SpBatchedScratch *s, int *status, cudaStream_t st, int *nlaunch, int t0 = 0, int slice = 0, int phase = 0);
 cudaError_t sp_batched_ep_experts(const SpDims &d, const SpLayerDev &L, int flavour, int R, const float *rows_in, const int32_t *row_index, const int32_t *offsets,
                                   float *rows_out, SpBatchedScratch *s, int *status, cudaStream_t st, int *nlaunch,
-                                  const int32_t *in_index = nullptr, int n_in = 0);   /* in_index: sorted position -> input row when pairs share input rows */
+                                  const int32_t *in_index = nullptr, int n_in = 0, int owners = 0);   /* in_index: sorted position -> input row when pairs share input rows; owners: experts that can have rows, 0 = not known */
 /* token dispatch (each token's input row travels once per destination rank): sender side after a route call made with
  * rows == NULL, and the receiver's input index after the receive layout */
 cudaError_t sp_batched_ep_tokens(const SpDims &d, int M, int n_ranks, int capacity, int cap_tokens, const int32_t *sel_asc, const int32_t *pair_index,

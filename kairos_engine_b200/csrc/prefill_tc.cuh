@@ -15,8 +15,9 @@ cudaError_t sp_tc_shared_expert(SpTcPlan *p, const SpDims &d, const SpLayerDev &
                                 int *status, cudaStream_t st, int *nl, int phase = 0);
 /* routed experts on R rows sorted by expert (expert e owns rows [offsets[e], offsets[e+1]), device
  * array of NE+1 ints): out[rowmap ? rowmap[r] : r][E] = Wdn[e] . geglu(Wgu[e] . rows[r]).
- * gather != NULL: row r is src[gather[r]] instead of src[r]. R <= max_rows. */
-cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int R, const float *src, const int *gather,
+ * gather != NULL: row r is src[gather[r]] instead of src[r]. R <= max_rows. owners: how many experts the rows can belong to, 0 =
+ * not known. */
+cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int R, int owners, const float *src, const int *gather,
                          const int *offsets, const int *rowmap, float *out, int *status, cudaStream_t st, int *nl);
 /* one whole layer's GEMMs on one GPU, the shared expert and the routed experts in one launch each for gate|up and down:
  * sel_asc / pairpos [M*NU] and count [NE] from the selection -> dn [M][E], eo [M*NU][E] (row = pair). The experts' normalised

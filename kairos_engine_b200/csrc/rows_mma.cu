@@ -511,7 +511,7 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
      * E 1024, 32 experts, 4 each, FFE 512, line at 8: 21.5 / 20.5 at 2, 23.4 / 24.2 at 4, 28.0 / 29.0 at 8, 29.1 / 30.7 at 10. The line
      * is right for the first; the longer down rows of the second would move it to twice as many tokens, the short ones of the
      * third to a quarter. */
-    bool whole = items <= seg[nseg - 1].groups;
+    bool whole = items <= (seg[nseg - 1].owners ? seg[nseg - 1].owners : seg[nseg - 1].groups);
     /* Small units all cost about the same: with up to 16 tokens to a unit, one of the shared expert held its stage for a third of
      * the launch at 16 tokens and kept the other team waiting. What small ones fetch again comes from L2, until that is what
      * bounds them. Us a layer of E 2816, 128 experts, 8 each, units of 16 / 8 / 4 tokens: 54.4 / 54.5 / 52.8 at 5 tokens, 92.2 / 88.5 /

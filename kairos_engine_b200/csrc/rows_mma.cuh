@@ -10,6 +10,7 @@ struct SpRowsSeg {
     long long rows_per_group; int up_off;
     int in, rows;                                  /* columns; output rows (pairs) per group, a multiple of 16 */
     int groups;                                    /* 1, or one per expert */
+    int owners;                                    /* how many of them can have items, where the caller knows; 0: all, or not known */
     /* which activations: group g owns list[g * list_stride ..] of count[g] items (list NULL: items 0..M-1), or positions
      * [offset[g], offset[g + 1]) of an order sorted by group, with item = index[position] (NULL: the position) */
     const int *count, *list; int list_stride;
