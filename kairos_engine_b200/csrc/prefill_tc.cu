@@ -669,12 +669,18 @@ cudaError_t sp_tc_create(const SpDims &d, int max_tokens, int max_rows, SpTcPlan
 void sp_tc_destroy(SpTcPlan *p) { if (!p) return; if (p->base) cudaFree(p->base); delete p; }
 
 namespace {
-/* activation rows per tile: tiles of 32 have a second set of accumulators, tiles of 64 serve more rows per unpacked weight.
- * Us a layer with 32 / 64, E 2816, 128 experts, 8 each, FFE 704: 146 / 153 at 24 tokens, 189 / 193 at 64, 218 / 220 at 128 (8 rows
- * per expert), 222 / 228 at 160, 233 / 237 at 200, 259 / 258 at 256, 312 / 298 at 400. With 64 experts, 6 each, E 2048, FFE 1408:
- * 137 / 140 at 64 (6 rows), 158 / 155 at 128 (12 rows), 184 / 184 at 200 (19 rows); with 32, 4 each, E 1024, FFE 512: 42 / 50 at
- * 64 (8 rows), 47 / 56 at 128, 62.8 / 61.7 at 200 (25 rows). */
-int tile_rows(int groups, long long rows) { return rows > 16LL * groups ? 64 : 32; }
+/* activation rows per tile: tiles of 32 have a second set of accumulators, tiles of 64 serve more rows per unpacked weight. The
+ * line is at 12 rows per expert, and at 16 where tiles of 64 would be fewer than the SMs. Us a layer with 32 / 64, E 2816, 128 experts,
+ * 8 each, FFE 704: 146 / 153 at 24 tokens, 189 / 193 at 64, 208 / 214 at 130 (8 rows per expert), 210 / 215 at 160, 219 / 223 at 200,
+ * 255 / 256 at 256, 312 / 298 at 400. With a router that sends most tokens to a few experts (Zipf 1.2) 129 / 117 at 130,
+ * 148 / 127 at 200, 171 / 139 at 256: what a line above 12 gives the even one it takes several times from that one. With 64 experts, 6
+ * each, E 2048, FFE 1408: 153 / 159 at 100 (9 rows), 156 / 162 at 130, 173 / 172 at 170 (16 rows), Zipf 130 / 112. With 32, 4 each, E
+ * 1024, FFE 512, 136 tiles of gate|up with 64: 42 / 50 at 64 (8 rows), 47 / 56 at 128, 62.8 / 61.7 at 200 (25 rows). groups: the experts that the
+ * rows can belong to; M: rows of the shared expert in the same launch. */
+int tile_rows(const SpTcPlan *p, const SpDims &d, int groups, long long rows, int M) {
+    const long long tiles = (long long)groups * ((d.FFE + 127) / 128) + (long long)((M + 63) / 64) * ((d.FFS + 127) / 128);
+    return rows > (tiles < p->sms ? 16LL : 12LL) * groups ? 64 : 32;
+}
 
 template <bool PAIR, int NMAX>
 cudaError_t launch_n(const SpTcPlan *p, const TcArgs &a, const TcMaps &maps, cudaStream_t st, int *nl) {
@@ -728,7 +734,7 @@ cudaError_t sp_tc_layer(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int M
                         int *status, cudaStream_t st, int *nl) {
     const int R = M * d.NU;
     if (!p || M > p->Mcap || (long long)M * d.NU > p->Rcap) return cudaErrorInvalidValue;
-    const int nmax = tile_rows(d.NE, R);
+    const int nmax = tile_rows(p, d, d.NE, R, M);
     SortArgs s{count, sel_asc, pairpos, d.NE, M, d.NU, nmax, p->gather, p->rowmap, p->tiles_r, p->ntiles_r, p->tiles_sh, p->ntiles_sh, p->cap_r, p->cap_sh};
     cudaError_t e = sp_launch(k_tc_sort, dim3((unsigned)((R + 1023) / 1024)), 1024, 0, st, nl, s);
     if (e != cudaSuccess) return e;
@@ -767,9 +773,9 @@ cudaError_t sp_tc_routed(SpTcPlan *p, const SpDims &d, const SpLayerDev &L, int 
                          const int *offsets, const int *rowmap, float *out, int *status, cudaStream_t st, int *nl) {
     if (!p || R > p->Rcap) return cudaErrorInvalidValue;
     if (R == 0) return cudaSuccess;
-    /* the rows belong to one rank's experts. Where their number is not known the line is at half the rows per expert: right for two
-     * ranks, and a single rank loses 1 to 3% between 8 and 16 rows per expert (above), where four ranks have 32 to 64 */
-    const int nmax = owners ? tile_rows(owners, R) : tile_rows(d.NE, 2LL * R);
+    /* where the caller does not know how many of the experts are its rank's, the line is at 8 rows per expert of the model: two thirds
+     * of it, as they are fewer */
+    const int nmax = owners ? tile_rows(p, d, owners, R, 0) : tile_rows(p, d, d.NE, 3LL * R / 2, 0);
     k_tc_split<<<R, 256, 0, st>>>(src, gather, d.E, p->in_hi, p->in_lo); (*nl)++;
     k_tc_plan<<<1, 1024, 0, st>>>(offsets, d.NE, 0, R, nmax, p->tiles_r, p->ntiles_r, p->cap_r); (*nl)++;
     Launch up(p, d, L, status);
