@@ -126,7 +126,7 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     int lo = 0, hi = s.groups - 1;                          /* the last group that starts at or before u: never an empty one */
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (st[mid] <= u) lo = mid; else hi = mid - 1; }
     r.grp = lo;
-    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), log = unit_log(cnt, a.many[r.seg]), nr = units_of(cnt, log), k = u - st[lo];
+    const int cnt = r.seg && p.count ? p.count[lo] : group_count(s, lo), log = unit_log(cnt, r.seg ? a.many[1] : a.many[0]), nr = units_of(cnt, log), k = u - st[lo];
     r.tile = k / nr;
     r.t0 = (k - r.tile * nr) << log;
     r.nt = cnt - r.t0 < 1 << log ? cnt - r.t0 : 1 << log;
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 const SpRowsSeg &s = a.seg[k];
                 for (int g0 = 0; g0 < s.groups; g0 += 32) {
                     const int g = g0 + lane;
-                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * units_of(cnt, unit_log(cnt, a.many[k]));
+                    const int cnt = g < s.groups ? group_count(s, g) : 0, n = a.geo[k].tiles * units_of(cnt, unit_log(cnt, k ? a.many[1] : a.many[0]));
                     if (k == 1 && g < s.groups) count_s[g] = cnt;
                     int v = n;
 #pragma unroll
