@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
         const int team = warp / kTeamWarps, tw = warp % kTeamWarps, gq = lane >> 2, q = lane & 3;
         const unsigned char *const aptr = sm + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
         int s = team % a.stages;
-        unsigned phs = 0, psum = 0;                         /* bit s: parity of this team's next use of stage s; bit b: of buffer b of sums */
+        unsigned phs = 0, psum = 0;                         /* bit s: parity of this team's next use of stage s; bit b: of buffer b of sums (pairs: of every batch) */
         Frag f;
         /* lanes whose 8-byte loads share a wavefront (W = 2) take rows whose pieces differ by more than the group's two */
         f.row = W == 1 ? gq : (gq & 1) << 2 | (gq & 2) | gq >> 2;
@@ -382,9 +382,9 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                 f.b = bvalid ? act + (first + btok) * ge.ast + bo : z;
                 f.sx = act + (first + ctok) * ge.ast + sg.in + 8 * cs;
             };
-            auto release = [&] {                            /* the stage, once the warp has read it for the last time */
+            auto release = [&] {                            /* the stage, once the warp has read it for the last time; its lanes meet */
+                __syncwarp();
                 if (flags & 2) {
-                    __syncwarp();
                     mbar_arrive_lane0(empty(s), lane);
                     phs ^= 1u << s;
                     s += a.teams;
@@ -434,9 +434,8 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                  * and the other barrier serve those next tokens; the buffer's next use but one waits for this one's end (aempty). The
                  * wait gives up when a warp of the team did, whose sums never come (on named barriers, which cannot, the give-up path
                  * would have to arrive for others; 64 tokens take 160.1 us a layer so, 159.2 on those). */
-                const uint32_t par = psum >> buf & 1u;
-                psum ^= 1u << buf;
-                __syncwarp();
+                const uint32_t par = PAIR ? (uint32_t)(n >> 1) & 1u : psum >> buf & 1u;
+                if (!PAIR) psum ^= 1u << buf;
                 mbar_arrive_lane0(sums(team, buf), lane);
                 auto total_of = [&](int m, int rw, int t) {                 /* the last levels of the tree */
                     const float *p = part + (m * 16 + rw) * T + t;
