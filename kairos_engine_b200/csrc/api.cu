@@ -263,10 +263,10 @@ static cudaError_t align_x(sp_moe *h, const float **x, int M, cudaStream_t st) {
     return e;
 }
 /* Short runs of one token are launched one kernel after the other, longer ones replayed from a graph. On the device the launches
- * are ahead up to about twelve layers (us a layer, launched / replayed: 24.0 / 33.7 at one layer a call, 23.3 / 28.0 at two,
- * 23.0 / 24.8 at four, 22.8 / 23.4 at eight, 22.75 / 22.90 at twelve, 22.65 / 22.32 at thirty), but they cost the calling thread 7 us
- * a layer where a replay costs it 17 us a call. At four layers the device still gains 7 us for 14 of the thread's; beyond, the
- * gain of a call shrinks while the thread's share grows. */
+ * are ahead up to about fifteen layers (us a layer, launched / replayed: 22.0 / 30.4 at one layer a call, 21.5 / 26.1 at two,
+ * 21.2 / 23.6 at four, 21.0 / 22.3 at six, 20.95 / 21.9 at eight, 20.9 / 21.4 at twelve, 20.85 / 21.0 at fifteen, 20.8 / 20.5 at
+ * thirty), but they cost the calling thread 7 to 8 us a layer where a replay costs it 13 to 17 us a call. At four layers the device
+ * still gains 10 us for 22 of the thread's; beyond, the gain of a call shrinks while the thread's share grows. */
 constexpr int kDirectLayers = 4;
 extern "C" int sp_moe_forward_dev(sp_moe *h, int lf, int nl, int flavour, int M,
                                   const float *x_dev, float *y_dev, int32_t *sel_dev, float *wts_dev, void *stream) {

@@ -11,7 +11,7 @@
  *     engine for them (cp.async.bulk, completion counted on mbarriers in shared memory), whole
  *     slices at a time: rows whose address does not depend on the routing are requested before
  *     the kernel waits for its predecessor, routed rows the moment the top-NU selection exists.
- *     The copies run while all 16 warps do the per-layer prologue (norms, quantisation, top-k),
+ *     The copies run while all twenty warps do the per-layer prologue (norms, quantisation, top-k),
  *     so the prologue no longer delays the weight stream and no warp holds registers for loads in
  *     flight.
  *   - The warps then read rows from shared memory. The router and the shared gate|up rows take dp4a
@@ -1029,8 +1029,8 @@ __global__ void __launch_bounds__(kT, 1) k_ds_experts_down(SArgs a) {
     const int SGs = (NU + kDnBars - 1) / kDnBars;         /* expert slots per landing part */
     STAMP(2, 0);
     /* The selection was published and fenced before this kernel could be launched: this CTA's rows of every selected expert are
-     * requested now, before the wait for the predecessor's hidden vectors, an expert slot to a warp (sixteen copies of 85
-     * cycles each would queue in one) */
+     * requested now, before the wait for the predecessor's hidden vectors, by warp 0, a lane per expert slot (spread over eight
+     * warps they were not there any sooner) */
     if (t == 0) {
 #pragma unroll 1
         for (int i = 0; i < kDnBars; i++) mbar_init(smem_u32(&ctl->bar[i]), 1);

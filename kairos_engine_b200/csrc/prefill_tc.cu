@@ -412,8 +412,8 @@ __global__ void __launch_bounds__(Cfg<NMAX>::kThreads, 1) k_tc_gemm(const __grid
              * next one is drawn from a counter when the codes of the one before are on their way, some 16 stages before it is due.
              * Tiles differ: the shared expert's K is three times the routed experts' in the down GEMM, the last tile of a group's
              * rows may hold one block, and a CTA draws four to ten tiles in all when there are few rows. Dealt out in turn
-             * (CTA c: c, c + 148, ...), the CTAs with a long tile got as many others as the rest: 30 layers of 24 / 37 / 400 tokens
-             * 5480 / 5863 / 10149 us so, against 4866 / 5561 / 9913 drawn, all else the same. The order stays: shared expert first,
+             * (CTA c: c, c + 148, ...), the CTAs with a long tile got as many others as the rest: a layer of 24 / 37 / 400 / 717 tokens takes
+             * 165 / 180 / 299 / 392 us so, 148 / 168 / 293 / 386 drawn, all else the same. The order stays: shared expert first,
              * so the long tiles are out early. */
             const int total0 = *a.seg[0].n_tiles * a.seg[0].m_tiles;
             const int total = total0 + (a.nseg > 1 ? *a.seg[1].n_tiles * a.seg[1].m_tiles : 0);

@@ -509,7 +509,7 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
      * experts, 6 each, FFE 1408, line at 10: 66.3 / 56.6 at 6, 85.1 / 71.9 at 10, 89.8 / 77.8 at 12, 101 / 92.4 at 16, 115 / 114 at 24.
      * E 1024, 32 experts, 4 each, FFE 512, line at 8: 21.5 / 20.5 at 2, 23.4 / 24.2 at 4, 28.0 / 29.0 at 8, 29.1 / 30.7 at 10. The line
      * is right for the first; the longer down rows of the second would move it to twice as many tokens, the short ones of the
-     * third to a quarter. */
+     * third to a quarter of them. */
     bool whole = items <= (seg[nseg - 1].owners ? seg[nseg - 1].owners : seg[nseg - 1].groups);
     /* Small units all cost about the same: with up to 16 tokens to a unit, one of the shared expert held its stage for a third of
      * the launch at 16 tokens and kept the other team waiting. What small ones fetch again comes from L2, until that is what
