@@ -133,6 +133,9 @@ __device__ Unit locate(const RowsArgs &a, const Plan &p, int u) {
     return r;
 }
 
+/* out of line, for the units after the first: rare, and no code of it in the loops of the copy warps */
+__device__ __noinline__ UnitWord locate_out(const RowsArgs &a, const Plan &p, int u) { return pack(locate(a, p, u)); }
+
 /* ---------------------------------------------------------------- the dots of one warp: 16 rows x four tokens */
 /* W = 1: one chunk x four tokens fill the eight columns of B. W = 2: two neighbouring chunks (a group) x two tokens; lane q of
  * a row reads two words, one per MMA, and column 2 u + h takes half h of the (token, chunk) u. Either way lane q's C registers
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     __shared__ int abort_s;
     __shared__ Batch batch_s[kMaxTeams][2];
     __shared__ float part_s[kMaxTeams][2][4 * 2 * 16 * kTok];
-    __shared__ UnitWord units_s[kUnits];
+    __shared__ UnitWord units_s[kUnits], later_s[32];
     __shared__ int start_s[1 + 1024], total_s[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     volatile int *abort_flag = &abort_s;
@@ -281,40 +284,64 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
     plan.count = nullptr;
     __syncthreads();
     const int mine = total > (int)blockIdx.x ? (total - blockIdx.x + G - 1) / G : 0;
-    auto unit = [&](int i) { return i < kUnits ? unpack(units_s[i]) : locate(a, plan, blockIdx.x + i * G); };
+    /* units beyond the table: a warp finds its next 32 at once, a lane each. One after the other, 274 tokens of E 1344, 160 experts, 7
+     * each, FFE 1472 (300 units a CTA) took 640 us a layer, 509 so; 256 tokens of E 2816, 128 experts, 8 each, FFE 704 493, 467 so. The
+     * copy warps' loops over the table stay free of it (one loop for both: 1% at 32 and 64 tokens). */
+    auto later = [&](int i) { return i < mine ? locate_out(a, plan, blockIdx.x + i * G) : UnitWord{0u, 0}; };
     const uint32_t sbase = smem_u32(sm);
     bool failed = false;
 
     if (warp == a.teams * kTeamWarps) {
         /* ---------------- weights */
-        if (lane == 0)
-            for (int i = 0, s = 0, ph = 0; i < mine; i++) {
-                const Unit u = unit(i);
-                const SpRowsSeg &sg = a.seg[u.seg];
-                const SegGeo &ge = a.geo[u.seg];
-                const int per = PAIR ? 16 : 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
-                const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(i % a.teams, s);
-                const int row = (int)((long long)u.grp * sg.rows_per_group) + r0;
-                const unsigned sbytes = (unsigned)nr * ge.sb;
-                const unsigned char *const ssrc = reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb;
-                if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) { failed = true; break; }
-                mbar_expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
-                box_g2s(dst, &a.codes[u.seg][0], row, bar);
-                if (PAIR) {
-                    box_g2s(dst + ge.box_bytes, &a.codes[u.seg][1], row + sg.up_off, bar);
-                    bulk_g2s(sdst + 16 * ge.sb, reinterpret_cast<const unsigned char *>(sg.ubs) + (size_t)(row + sg.up_off) * ge.sb, sbytes, bar);
-                }
-                bulk_g2s(sdst, ssrc, sbytes, bar);
-                if (++s == a.stages) { s = 0; ph ^= 1; }
+        int s = 0, ph = 0;
+        auto issue = [&](const Unit &u, int i) {
+            const SpRowsSeg &sg = a.seg[u.seg];
+            const SegGeo &ge = a.geo[u.seg];
+            const int per = PAIR ? 16 : 16 * ge.mt_n, r0 = u.tile * per, nr = sg.rows - r0 < per ? sg.rows - r0 : per;
+            const uint32_t dst = sbase + (unsigned)s * a.stage_bytes, sdst = dst + ge.scale_off, bar = full(i % a.teams, s);
+            const int row = (int)((long long)u.grp * sg.rows_per_group) + r0;
+            const unsigned sbytes = (unsigned)nr * ge.sb;
+            const unsigned char *const ssrc = reinterpret_cast<const unsigned char *>(sg.bs) + (size_t)row * ge.sb;
+            if (!mbar_wait(empty(s), ph ^ 1, abort_flag)) return false;
+            mbar_expect_tx(bar, (PAIR ? 2 : 1) * (ge.box_bytes + sbytes));       /* rows past the tensor arrive as zeros */
+            box_g2s(dst, &a.codes[u.seg][0], row, bar);
+            if (PAIR) {
+                box_g2s(dst + ge.box_bytes, &a.codes[u.seg][1], row + sg.up_off, bar);
+                bulk_g2s(sdst + 16 * ge.sb, reinterpret_cast<const unsigned char *>(sg.ubs) + (size_t)(row + sg.up_off) * ge.sb, sbytes, bar);
             }
+            bulk_g2s(sdst, ssrc, sbytes, bar);
+            if (++s == a.stages) { s = 0; ph ^= 1; }
+            return true;
+        };
+        const int table = mine < kUnits ? mine : kUnits;
+        if (lane == 0)
+            for (int i = 0; i < table; i++)
+                if (!issue(unpack(units_s[i]), i)) { failed = true; break; }
+        for (int i0 = kUnits; i0 < mine; i0 += 32) {
+            __syncwarp();                                   /* lane 0 has read the words */
+            if (__shfl_sync(0xffffffffu, failed, 0)) break;
+            later_s[lane] = later(i0 + lane);
+            __syncwarp();
+            if (lane == 0)
+                for (int i = i0; i < mine && i < i0 + 32; i++)
+                    if (!issue(unpack(later_s[i - i0]), i)) { failed = true; break; }
+        }
         __syncwarp();
     } else if (warp > a.teams * kTeamWarps) {
         /* ---------------- activations of one team: four tokens ahead of it, one lane per token */
         const int team = warp - a.teams * kTeamWarps - 1;
         const uint32_t abase = sbase + (unsigned)a.stages * a.stage_bytes + (unsigned)team * 2u * a.act_bytes;
-        int n = 0;
+        int n = 0, nl = 0;
+        UnitWord ahead{0u, 0};
         for (int i = team; i < mine && !failed; i += a.teams) {
-            const Unit u = unit(i);
+            UnitWord w;
+            if (i < kUnits) w = units_s[i];
+            else {
+                if ((nl & 31) == 0) ahead = later(i + lane * a.teams);
+                w.w = __shfl_sync(0xffffffffu, ahead.w, nl & 31); w.t0 = __shfl_sync(0xffffffffu, ahead.t0, nl & 31);
+                nl++;
+            }
+            const Unit u = unpack(w);
             const SpRowsSeg &s = a.seg[u.seg];
             const SegGeo &ge = a.geo[u.seg];
             const int first = group_first(s, u.grp) + u.t0;
@@ -503,6 +530,10 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
     RowsArgs a{};
     cudaError_t e = cudaSuccess;
     a.nseg = nseg; a.status = status;
+    int dev = 0, sms = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     /* two chunks x two tokens per MMA while most chosen experts have one or two tokens and the rows are whole groups. Us a layer
      * with one / two chunks, the line at one item per expert: E 2816, 128 experts, 8 each, FFE 704, line at 16 tokens: 42.7 / 39.6
      * at 2, 56.3 / 54.0 at 5, 77.7 / 75.7 at 12, 88.7 / 88.4 at 16, 96.7 / 97.0 at 20, 112 / 123 at 32, 162 / 197 at 64. E 2048, 64
@@ -545,10 +576,6 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
     a.stages = (int)((kSmemLimit - 1024 - acts) / a.stage_bytes);
     if (a.stages > kMaxStages) a.stages = kMaxStages;
     if (a.stages < 1) return cudaErrorInvalidValue;
-    int dev = 0, sms = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
     const unsigned threads = (unsigned)(a.teams * kTeamThreads + 32 + 32 * a.teams);
     const size_t smem = acts + (size_t)a.stages * a.stage_bytes + 1024;
     return sp_launch(pair ? whole ? k_rows<true, 2> : k_rows<true, 1> : whole ? k_rows<false, 2> : k_rows<false, 1>, dim3((unsigned)sms), threads, smem, st, nl, a);

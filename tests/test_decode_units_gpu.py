@@ -69,3 +69,23 @@ def test_expert_parallel_units(M, owned):
     eng.status()
     assert torch.equal(y.view(torch.int32), y2.view(torch.int32))
     eng.close()
+
+
+@pytest.mark.parametrize("cfg,M", [(_cfg(64, 160, 8, 2048, 64), 120), (_cfg(2080, 160, 8, 1056, 64), 200)])
+def test_more_units_than_the_table_holds(cfg, M):
+    """Some 200 units a CTA of gate|up, and of down: those beyond the first 128 are found later, 32 at a time."""
+    import torch
+    from kairos_engine_b200 import MoeEngine, synth
+    eng = MoeEngine(n_layers=1, max_tokens=M, **cfg)
+    eng.upload_layer(0, synth.make_layer(cfg, 83, rand_norms=True), on_device=True)
+    x = synth.make_inputs(cfg, M, 84)
+    y, y1 = torch.empty_like(x), torch.empty_like(x[:1])
+    eng.forward_dev(x, y, flavour=A)
+    for t in range(0, M, 7):
+        eng.forward_dev(x[t:t + 1].contiguous(), y1, flavour=A)
+        assert torch.equal(y1[0].view(torch.int32), y[t].view(torch.int32)), t
+    again = torch.empty_like(x)
+    for _ in range(10):
+        eng.forward_dev(x, again, flavour=A)
+        assert torch.equal(again.view(torch.int32), y.view(torch.int32))
+    eng.status(); eng.close()
