@@ -37,6 +37,7 @@ using namespace sp_tc;
 
 constexpr int kTeamWarps = 8, kTeamThreads = 32 * kTeamWarps, kTok = 4, kMaxStages = 4, kMaxTeams = 2;
 constexpr int kFewItems = 24, kManyItems = 48;     /* items to a group up to which units are of 4 tokens: on average, and in any one group */
+constexpr int kSmUnits = 16;                       /* ... in one group: where units of 16 are at least this many to an SM */
 constexpr int kUnits = 128;                        /* unit descriptors of a CTA kept in shared memory */
 constexpr int kMagic = 0x4B400000;
 
@@ -552,12 +553,15 @@ cudaError_t sp_rows_launch(const SpRowsSeg *seg, int nseg, bool pair, long long 
      * line: a group of more than 48 items has units of 16 whatever the average (a Zipf 1.2 router over 128 experts, units of 4 everywhere /
      * so: 242 / 237 at 128 tokens, 463 / 428 at 256, 687 / 613 at 384). 48, because units of both sizes side by side cost
      * more than they save while the counts only scatter about their average (384 tokens, 24 on average: a line of 24 per group 757,
-     * of 48 721). Rows sorted for one rank's experts belong to fewer groups than there are, how many is not known here: their line
-     * is 24 for each group by itself. */
+     * of 48 721). And only where there would still be 16 units of that size to an SM: the few of a small launch end unevenly (60 experts, 7
+     * each, E 2688, FFE 1088, Zipf, 49 tokens: 138 with units of 16, 124; 16 experts, 2 each, E 576, FFE 832, 113 tokens: 54, 49). Rows sorted for one rank's experts belong to fewer groups than there are, how many is not known here: their line
+     * is 24 for each group by itself, with the same condition. */
     const bool few = items <= (long long)kFewItems * seg[nseg - 1].groups;
     for (int i = 0; i < nseg; i++) {
         a.seg[i] = seg[i];
-        a.many[i] = seg[i].offset ? kFewItems : !few ? 0 : seg[i].groups > 1 ? kManyItems : 0x7fffffff;
+        const long long units = (long long)seg_geo(seg[i], pair).tiles * (i + 1 < nseg ? seg[i].M : items) / 16;
+        const int line = units >= kSmUnits * (long long)sms ? (seg[i].offset ? kFewItems : kManyItems) : 0x7fffffff;
+        a.many[i] = !few && !seg[i].offset ? 0 : seg[i].groups > 1 ? line : 0x7fffffff;
         const SegGeo &g = a.geo[i] = seg_geo(seg[i], pair);
         const unsigned sb = up1024(g.scale_off + 16 * g.mt_n * g.sb), ab = kTok * g.ast;
         const unsigned zb = (unsigned)seg[i].in + 128;
