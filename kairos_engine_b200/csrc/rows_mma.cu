@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kMaxTeams *kTeamThreads + 96, 1) k_rows(const 
                  * at its next tokens meanwhile: a warp loses the time of one finish in four (or two) times. The other buffer of sums
                  * and the other barrier serve those next tokens; the buffer's next use but one waits for this one's end (aempty). The
                  * wait gives up when a warp of the team did, whose sums never come (on named barriers, which cannot, the give-up path
-                 * would have to arrive for others; 64 tokens take 160.1 us a layer so, 159.2 on those). */
+                 * would have to arrive for others; 64 tokens take 158.5 us a layer either way, 512 tokens 866 so, 859 on those). */
                 const uint32_t par = PAIR ? (uint32_t)(n >> 1) & 1u : psum >> buf & 1u;
                 if (!PAIR) psum ^= 1u << buf;
                 mbar_arrive_lane0(sums(team, buf), lane);
