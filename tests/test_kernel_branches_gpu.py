@@ -88,7 +88,7 @@ def test_prefill_drawn_tiles(cfg, M):
 
 def _tie_then_one_ulp(NE, NU, same_warp):
     """NU - 1 larger logits, two equal ones of which one is the last chosen, and one a float below with a lower id whose
-    probability rounds to theirs: the checker takes that one."""
+    probability rounds to theirs: the oracle takes that one."""
     near, tied = (3, (9, 11)) if same_warp else (3, (NE - 5, NE - 2))
     rest = [i for i in range(NE) if i not in (near, *tied)]
     for k in range(1, 200):

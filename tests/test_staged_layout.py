@@ -27,7 +27,7 @@ def test_full_geometries_keep_the_staged_path(tmp_path_factory, geo):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("geo", FULL)
-def test_full_geometries_give_the_checkers_bits(geo):
+def test_full_geometries_give_the_oracles_bits(geo):
     from gpu_common import make_stack, oracle_stack
     cfg = _cfg(*geo)
     eng, host = make_stack(cfg, 2, seed=91, rand_norms=True, max_tokens=2)
